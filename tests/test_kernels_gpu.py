@@ -131,6 +131,26 @@ def test_gemm_f32_is_true_fp32(M, N, K, bias):
     assert torch.equal(gemm_f32(x[:1].contiguous(), w, b), got[:1])
 
 
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 128, 129, 300])
+@pytest.mark.parametrize("N,K,lda", [(33, 68, 68), (129, 64, 80), (1536, 1540, 1540), (4097, 260, 260),
+                                     (32800, 132, 136), (40, 515, 519), (31, 4, 4)])
+def test_gemm_f32_at_the_edges_of_its_kernels(M, N, K, lda):
+    """Every row kernel and tile, with remainders of rows, columns, chunks and cluster shares, rows of
+    A apart, 16-byte and 4-byte copies: close to 64 bits, and each row as if it were alone."""
+    from ginfer_b200.ops.linear import gemm_f32
+    g = torch.Generator(device=DEV).manual_seed(M * 31 + N)
+    x = torch.randn(M, lda, device=DEV, generator=g)[:, :K]
+    w = torch.randn(N, K, device=DEV, generator=g)
+    b = torch.randn(N, device=DEV, generator=g)
+    got = gemm_f32(x, w, b)
+    # chains of at most K / 4 + 16 FMAs (even or odd k of a segment), their sum, at most 8 segments and the
+    # bias: as many roundings of 2^-24, of partial sums that stay below sum |x w|
+    bound = (K / 4 + 16 + 10) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t() + b.double().abs())
+    assert ((got.double() - (x.double() @ w.double().t() + b.double())).abs() <= bound).all()
+    for m in {0, M // 2, M - 1}:
+        assert torch.equal(gemm_f32(x[m:m + 1], w, b), got[m:m + 1])
+
+
 def _paged_case(B_lens, q_lens, nh, nkv, hd, P, window, dtype, seed=0, spike=True):
     """Random paged cache and queries for requests with kv lengths ``B_lens`` whose last
     ``q_lens`` tokens are this step's queries.  Returns the kernel inputs and the plain result."""
