@@ -12,7 +12,8 @@
 //   moe_plan_kernel     a block an expert: (token, choice) pairs counted per expert, the experts' ranges in
 //                       the sorted order, each pair's place, and the list of row tiles (expert,
 //                       first row) that the grouped products walk over.
-//   moe_gemm_mma_kernel the grouped products of the bf16 path, on the tensor cores (see there).
+//   moe_stream_kernel   the grouped products of decode steps: an expert's weights streamed once (see there).
+//   moe_gemm_mma_kernel those of more pairs, in tiles of 64 rows (see there).
 //   moe_gemm_kernel     (32-bit path, and sizes the other refuses) grouped product over the sorted pairs, a block a (row tile, column tile):
 //                       FIRST: rows gathered from the tokens, W = the expert's row-interleaved
 //                       gate/up matrix, epilogue = clamped sigmoid-gated GLU (MODE 1), or W = the
@@ -504,113 +505,145 @@ moe_gemm_mma_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfl
     }
 }
 
-// ---- the same grouped products for a handful of pairs (decode steps of few requests) ------------
-// There the work is the experts' weight bytes, and a tile of 64 rows that walks its whole reduction
-// alone keeps too few of them under way (4 pairs: 45 us for 35 MB).  Here a tile is up to 8 rows of
-// one expert, kept in shared memory; a block takes 16, 32 or 64 weight rows of that expert (the
-// fewer pairs, the fewer rows, so that enough blocks keep loads under way), a warp two
-// neighbouring rows at a time (a gate and its up value in the gated form), streamed once with
-// 16-byte loads, each lane a strided share of the reduction, a warp sum at the end.  The order of
-// the sums depends on K alone, so a pair's result does not depend on the batch.
-constexpr int kFewRows = 8, kFewWarps = 8, kFewChunkMax = 64;
+// ---- the same grouped products where the experts' weight bytes are the work (decode steps) --------
+// Up to some hundred pairs every expert that is reached has a few rows, and its matrix is read once for
+// them: the time is the stream of weights.  The weights are the 16-row operand of mma.sync and go from
+// memory straight into its registers (k is a summed index, so a lane may hold any k as long as both
+// operands agree: a lane takes 16 bytes of a row, 4 lanes a 64-byte run, two runs a step of 64 k);
+// the pairs' rows, at most 16 of one expert, are staged in shared memory and are the 8-column operand.
+// No weight is staged, so a warp keeps 8 loads of 16 bytes a lane under way whatever the other warps do.
+// A warp owns 16 weight rows; `parts` warps (1, 2, 4 or 8 of the block's eight) split its reduction
+// where the rows alone give too few warps.  Lane group g has weight rows 2 g and 2 g + 1: a gate and
+// its up value meet in one lane.
+// Measured on a B200 (both products of a layer, 32 experts of 2048 x 2112, 4 choices; floor = the
+// reached experts' bytes at 6.54 TB/s), against a kernel that kept eight rows in shared memory and
+// multiplied on the FMA pipes (up to 20 pairs) and the 64-row tiles below (from 21 on): 4 pairs 26.5
+// us (29.5; floor 10.6), 20 pairs 53.5 (97.5; 39.6), 64 pairs 91.6 (120; 60.8), 256 pairs 113.5 (172; 82),
+// 512 pairs 144.5 (182; 84.6), 1,020 pairs 214 (209: the line lies at 768).
+constexpr int kStRows = 16, kStWarps = 8, kStUnroll = 2;
+constexpr int kStMaxShared = 160 * 1024;                     // K up to 5,088
 
-__device__ __forceinline__ void bf16x8_to_f32(const uint4& raw, float (&v)[8]) {
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 f = __bfloat1622float2(h[i]);
-    v[2 * i] = f.x, v[2 * i + 1] = f.y;
-  }
+__host__ __device__ inline size_t stream_pitch(int K) {      // of a staged row, bytes: 64 mod 128
+  return ((size_t)K * 2 + 127) / 128 * 128 + 64;
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(kFewWarps * 32)
-moe_gemv_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfloat16* __restrict__ w,
-                int N, int K, const int* __restrict__ offsets, const int* __restrict__ pair_of_pos,
-                int top, const int* __restrict__ tile_expert, const int* __restrict__ tile_row0,
-                const int* __restrict__ num_tiles, void* __restrict__ out_, float limit,
-                float alpha, float up_shift, const float* __restrict__ row_w, int chunk) {
-  extern __shared__ __align__(16) __nv_bfloat16 xrows[];           // [kFewRows][K]
+__global__ void __launch_bounds__(kStWarps * 32, 2)
+moe_stream_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfloat16* __restrict__ w,
+                  int N, int K, const int* __restrict__ offsets, const int* __restrict__ pair_of_pos,
+                  int top, const int* __restrict__ tile_expert, const int* __restrict__ tile_row0,
+                  const int* __restrict__ num_tiles, void* __restrict__ out_, float limit,
+                  float alpha, float up_shift, const float* __restrict__ row_w, int parts) {
+  extern __shared__ __align__(16) uint8_t staged[];          // [kStRows] rows of stream_pitch(K)
+  __shared__ float sums[kStWarps][32][8];
   pdl_trigger();
   pdl_wait();
   if ((int)blockIdx.x >= fresh_index(num_tiles)) return;
   const int e = fresh_index(tile_expert + blockIdx.x), row0 = fresh_index(tile_row0 + blockIdx.x);
-  const int rows = min(kFewRows, fresh_index(offsets + e + 1) - row0);
-  const int k8 = K >> 3;
-  for (int i = threadIdx.x; i < rows * k8; i += blockDim.x) {
-    const int r = i / k8, c = (i - r * k8) * 8;
-    const int src = MODE != 0 ? fresh_index(pair_of_pos + row0 + r) / top : row0 + r;
-    *reinterpret_cast<uint4*>(xrows + (size_t)r * K + c) =
-        *reinterpret_cast<const uint4*>(a + (size_t)src * lda + c);
-  }
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const __nv_bfloat16* we = w + (size_t)e * N * K;
-  for (int i = warp; i < chunk / 2; i += kFewWarps) {
-    const int n = blockIdx.y * chunk + 2 * i;
-    if (n >= N) break;                                             // N is even
-    const __nv_bfloat16 *w0 = we + (size_t)n * K, *w1 = w0 + K;
-    float acc0[kFewRows], acc1[kFewRows];
+  const int rows = min(kStRows, fresh_index(offsets + e + 1) - row0);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int part = warp % parts, n0 = (blockIdx.y * (kStWarps / parts) + warp / parts) * 16;
+  const size_t pitch = stream_pitch(K);
+  const int units = (K + 63) / 64;
+  const int u0 = units * part / parts, u1 = units * (part + 1) / parts;
+  const int n = n0 + 2 * g;                                  // N is even: both rows are there, or none
+  const __nv_bfloat16* w0 = w + ((size_t)e * N + (n < N ? n : 0)) * K + 8 * t;
+  const __nv_bfloat16* w1 = w0 + K;
+  uint4 ra[kStUnroll][2], rb[kStUnroll][2];                  // rows 2 g and 2 g + 1
+  auto load = [&](int u) {
 #pragma unroll
-    for (int r = 0; r < kFewRows; ++r) acc0[r] = acc1[r] = 0.f;
-    // four steps of the reduction at a time: their eight loads go out together, before any
-    // arithmetic (left to the compiler, the loads of a step waited behind the branches of the
-    // step before: 1.2 TB/s)
-    for (int c0 = lane * 8; c0 < K; c0 += 4 * 256) {
-      uint4 wa[4], wb[4];
+    for (int i = 0; i < kStUnroll; ++i)
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int c = c0 + u * 256;
-        if (c < K) {
-          wa[u] = __ldg(reinterpret_cast<const uint4*>(w0 + c));
-          wb[u] = __ldg(reinterpret_cast<const uint4*>(w1 + c));
+      for (int h = 0; h < 2; ++h) {
+        const int k = (u + i) * 64 + h * 32;
+        ra[i][h] = rb[i][h] = make_uint4(0u, 0u, 0u, 0u);
+        if (u + i < u1 && k + 8 * t < K) {
+          ra[i][h] = __ldg(reinterpret_cast<const uint4*>(w0 + k));
+          rb[i][h] = __ldg(reinterpret_cast<const uint4*>(w1 + k));
         }
       }
+  };
+  load(u0);
+  {                                                          // the rows, zeros up to whole steps
+    const int k8 = units * 8, staged_rows = rows <= 8 ? 8 : 16;
+    for (int i = threadIdx.x; i < staged_rows * k8; i += kStWarps * 32) {
+      const int r = i / k8, c = (i - r * k8) * 8;
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (r < rows && c < K) {
+        const int src = MODE != 0 ? fresh_index(pair_of_pos + row0 + r) / top : row0 + r;
+        v = *reinterpret_cast<const uint4*>(a + (size_t)src * lda + c);
+      }
+      *reinterpret_cast<uint4*>(staged + r * pitch + (size_t)c * 2) = v;
+    }
+  }
+  __syncthreads();
+  float acc[2][4] = {};                                      // pairs 8 j + 2 t, + 1 of rows 2 g | 2 g + 1
+  const uint8_t* x0 = staged + g * pitch + 16 * t;
+  const bool second = rows > 8;
+  for (int u = u0; u < u1; u += kStUnroll) {
+    uint4 ca[kStUnroll][2], cb[kStUnroll][2];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int c = c0 + u * 256;
-        if (c >= K) break;
-        float f0[8], f1[8];
-        bf16x8_to_f32(wa[u], f0);
-        bf16x8_to_f32(wb[u], f1);
+    for (int i = 0; i < kStUnroll; ++i)
 #pragma unroll
-        for (int r = 0; r < kFewRows; ++r) {
-          if (r < rows) {
-            float x[8];
-            bf16x8_to_f32(*reinterpret_cast<const uint4*>(xrows + (size_t)r * K + c), x);
+      for (int h = 0; h < 2; ++h) ca[i][h] = ra[i][h], cb[i][h] = rb[i][h];
+    load(u + kStUnroll);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              acc0[r] = fmaf(f0[j], x[j], acc0[r]);
-              acc1[r] = fmaf(f1[j], x[j], acc1[r]);
-            }
-          }
+    for (int i = 0; i < kStUnroll; ++i) {
+      if (u + i >= u1) break;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint8_t* x = x0 + (size_t)(u + i) * 128 + h * 64;
+        const uint32_t lo[4] = {ca[i][h].x, cb[i][h].x, ca[i][h].y, cb[i][h].y};
+        const uint32_t hi[4] = {ca[i][h].z, cb[i][h].z, ca[i][h].w, cb[i][h].w};
+        const uint4 v = *reinterpret_cast<const uint4*>(x);
+        const uint32_t b0[2] = {v.x, v.y}, b1[2] = {v.z, v.w};
+        mma_bf16(acc[0], lo, b0);
+        mma_bf16(acc[0], hi, b1);
+        if (second) {
+          const uint4 y = *reinterpret_cast<const uint4*>(x + 8 * pitch);
+          const uint32_t d0[2] = {y.x, y.y}, d1[2] = {y.z, y.w};
+          mma_bf16(acc[1], lo, d0);
+          mma_bf16(acc[1], hi, d1);
         }
       }
     }
+  }
+  if (parts > 1) {                                           // the first of a group's warps adds up
 #pragma unroll
-    for (int r = 0; r < kFewRows; ++r) {
-      if (r >= rows) break;                                        // uniform over the warp
-      const float c0 = warp_sum(acc0[r]), c1 = warp_sum(acc1[r]);
-      if (lane != 0) continue;
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sums[warp][lane][j * 4 + i] = acc[j][i];
+    __syncthreads();
+    if (part) return;
+    for (int p = 1; p < parts; ++p)
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[j][i] += sums[warp + p][lane][j * 4 + i];
+  }
+  if (n >= N) return;
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int r = 8 * j + 2 * t + i;
+      if (r >= rows) continue;
       const size_t s = (size_t)(row0 + r);
+      const float c0 = acc[j][i], c1 = acc[j][2 + i];        // weight rows n, n + 1
       if (MODE == 2) {
-        const float rw = row_w ? row_w[pair_of_pos[s]] : 1.f;
-        const float u0 = fmaxf(to_f32(from_f32<__nv_bfloat16>(c0 * rw)), 0.f);
-        const float u1 = fmaxf(to_f32(from_f32<__nv_bfloat16>(c1 * rw)), 0.f);
-        __nv_bfloat16* out = (__nv_bfloat16*)out_ + s * N + n;
-        out[0] = from_f32<__nv_bfloat16>(u0 * u0);
-        out[1] = from_f32<__nv_bfloat16>(u1 * u1);
+        const float rw = row_w ? row_w[fresh_index(pair_of_pos + s)] : 1.f;
+        const float v0 = fmaxf(to_f32(from_f32<__nv_bfloat16>(c0 * rw)), 0.f);
+        const float v1 = fmaxf(to_f32(from_f32<__nv_bfloat16>(c1 * rw)), 0.f);
+        *reinterpret_cast<__nv_bfloat162*>((__nv_bfloat16*)out_ + s * N + n) =
+            __floats2bfloat162_rn(v0 * v0, v1 * v1);
       } else if (MODE == 1) {
         const float gt = to_f32(from_f32<__nv_bfloat16>(c0)), up = to_f32(from_f32<__nv_bfloat16>(c1));
         ((__nv_bfloat16*)out_)[s * (N / 2) + n / 2] =
             from_f32<__nv_bfloat16>(clamped_glu(gt, up, limit, alpha, up_shift));
       } else {
-        float* out = (float*)out_ + s * N + n;
-        out[0] = c0;
-        out[1] = c1;
+        *reinterpret_cast<float2*>((float*)out_ + s * N + n) = make_float2(c0, c1);
       }
     }
-  }
 }
 
 // xs[s, :] = x[pair_of_pos[s] / top, :]: the tokens' rows in sorted order, 16 bytes an access, for
@@ -656,9 +689,10 @@ using bf = __nv_bfloat16;
 
 GF_DEFINE_PDL_SWITCH
 
-// Rows of a tile: of the plain kernel (tensor_cores == 0) or of the tensor-core kernel.
+// Rows of a tile: of the plain kernel (tensor_cores == 0), of the tensor-core kernel (1) or of the
+// weight-streaming kernel (2).
 GF_EXPORT int gf_moe_tile_rows(int tensor_cores) {
-  return tensor_cores == 2 ? kFewRows : tensor_cores ? kTM : kBM;
+  return tensor_cores == 2 ? kStRows : tensor_cores ? kTM : kBM;
 }
 
 // sigmoid != 0: a score is the sigmoid of its logit instead of the softmax over all experts.
@@ -712,32 +746,33 @@ GF_EXPORT int gf_moe_gemm(const void* a, int lda, const void* w, int N, int K, c
                           int pairs) {
   if (max_tiles <= 0) return 0;
   auto st = (cudaStream_t)stream;
-  if (tensor_cores == 2) {                     // a handful of pairs: the weight-streaming kernel
-    const size_t smem = (size_t)kFewRows * K * sizeof(bf);
+  if (tensor_cores == 2) {                     // the weight-streaming kernel
+    const size_t smem = kStRows * stream_pitch(K);
     if (dtype != GF_BF16 || K % 8 || lda % 8 || N % 2 || (uintptr_t)a % 16 || (uintptr_t)w % 16 ||
-        smem > 64 * 1024)
+        (uintptr_t)out % 8 || smem > kStMaxShared)
       return -3;
-    // at most min(pairs, max_tiles) tiles hold rows; about four blocks an SM should be busy
-    int chunk = kFewChunkMax;
+    // at most min(pairs, max_tiles) tiles hold rows; about 16 warps an SM should be busy
     const int busy = pairs > 0 && pairs < max_tiles ? pairs : max_tiles;
-    while (chunk > 2 * kFewWarps && (long long)busy * ((N + chunk - 1) / chunk) < 4 * 148) chunk /= 2;
-    const dim3 fgrid(max_tiles, (N + chunk - 1) / chunk), fblock(kFewWarps * 32);
-#define GF_FEW(MODE)                                                                              \
+    int parts = 1;
+    while (parts < kStWarps && (long long)busy * (N / 16 + 1) * parts < 16 * 148 && K >= parts * 256) parts *= 2;
+    const int span = 16 * (kStWarps / parts);
+    const dim3 sgrid(max_tiles, (N + span - 1) / span), sblock(kStWarps * 32);
+#define GF_ST(MODE)                                                                               \
   {                                                                                               \
     static OncePerDevice attrs;                                                                   \
     if (int rc = attrs.run([&] {                                                                  \
-          return cudaFuncSetAttribute(moe_gemv_kernel<MODE>,                                      \
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);    \
+          return cudaFuncSetAttribute(moe_stream_kernel<MODE>,                                    \
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, kStMaxShared); \
         }))                                                                                       \
       return rc;                                                                                  \
-    return launch_kernel(moe_gemv_kernel<MODE>, fgrid, fblock, smem, st, (const bf*)a, lda,        \
-                         (const bf*)w, N, K, offsets, pair_of_pos, top, tile_expert, tile_row0,    \
-                         num_tiles, out, limit, alpha, up_shift, row_w, chunk);                    \
+    return launch_kernel(moe_stream_kernel<MODE>, sgrid, sblock, smem, st, (const bf*)a, lda,     \
+                         (const bf*)w, N, K, offsets, pair_of_pos, top, tile_expert, tile_row0,   \
+                         num_tiles, out, limit, alpha, up_shift, row_w, parts);                   \
   }
-    if (first == 2) GF_FEW(2)
-    if (first) GF_FEW(1)
-    GF_FEW(0)
-#undef GF_FEW
+    if (first == 2) GF_ST(2)
+    if (first) GF_ST(1)
+    GF_ST(0)
+#undef GF_ST
   }
   if (tensor_cores) {
     if (dtype != GF_BF16 || K % 8 || lda % 8 || (uintptr_t)a % 16 || (uintptr_t)w % 16) return -3;

@@ -13,7 +13,7 @@ _tile_rows: dict = {}
 
 def tile_rows(tensor_cores) -> int:
     """Rows of a tile of the plain kernel (``False``), of the ``mma.sync`` kernel (``True``), of
-    the tcgen05 kernel (``"tcgen05"``) or of the kernel for a handful of pairs (``"few"``)."""
+    the tcgen05 kernel (``"tcgen05"``) or of the weight-streaming kernel (``"few"``)."""
     if tensor_cores not in _tile_rows:
         if tensor_cores == "tcgen05":
             _tile_rows[tensor_cores] = int(load_library("gemm_prefill").gf_gemm_grouped_tile_rows())
@@ -26,19 +26,21 @@ def tile_rows(tensor_cores) -> int:
 
 # From this many (token, expert) pairs on, the grouped products of the bf16 path run on the
 # persistent tcgen05 kernel (csrc/gemm_prefill.cu, tiles of 128 rows x 256 columns, the rows brought
-# into sorted order first); below it on the mma.sync kernel with its tiles of 64 rows, which is
-# bound by the experts' weight bytes there.
+# into sorted order first); below it on one of the two mma.sync kernels, which are bound by the
+# experts' weight bytes there.
 TCGEN05_MIN_PAIRS = 1024
-# Up to this many pairs (decode steps of few requests) the products run on the kernel that streams
-# an expert's rows once for up to eight pairs; it keeps the rows in shared memory, which bounds the
-# reduction size.
-FEW_MAX_PAIRS = 20
+# Up to this many pairs (decode steps) the products run on the kernel that streams an expert's weights
+# once for up to 16 pairs; it keeps the pairs' rows in shared memory, which bounds the reduction size.
+# On a B200, both products of 32 experts of 2048 x 2112 with 4 choices a token: 512 pairs 144 us
+# against 182 on the mma.sync kernel, 1,020 pairs 214 against 209; 16 experts of 1024 x 1056 with 2
+# choices: 510 pairs 47 against 62.
+FEW_MAX_PAIRS = 768
 FEW_MAX_K = 4096
 
 
 def kernel_for(x: torch.Tensor, pairs: int, reductions, widths) -> object:
     """Which grouped-product kernel serves activations ``x`` with these reduction sizes and output
-    widths: ``"tcgen05"``, ``"few"`` (a handful of pairs), ``True`` (``mma.sync``) or ``False``
+    widths: ``"tcgen05"``, ``"few"`` (weights streamed), ``True`` (``mma.sync``) or ``False``
     (plain)."""
     if not (on_tensor_cores(x.dtype, *reductions) and x.stride(0) % 8 == 0):
         return False

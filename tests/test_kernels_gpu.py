@@ -503,3 +503,47 @@ def test_temperature_sampling_is_the_inverse_cdf(V):
     freq = torch.bincount(picks.long(), minlength=5).double() / 4000
     want = torch.softmax(row[0].double() / 0.7, -1).cpu()
     assert (freq.cpu() - want).abs().max() < 0.03
+
+
+@pytest.mark.parametrize("K,F,T,E,top", [(8, 2, 1, 1, 1), (72, 34, 40, 3, 2), (1024, 704, 2, 16, 2),
+                                         (1416, 136, 33, 5, 3), (4096, 64, 20, 4, 1), (2048, 2112, 9, 32, 4),
+                                         (128, 50, 384, 7, 2)])
+def test_grouped_products_that_stream_the_weights(K, F, T, E, top):
+    """One pair to several tiles of an expert, reductions that are no multiple of a step, fewer weight
+    rows than a warp takes, one to eight warps a reduction: against 64 bits."""
+    from ginfer_b200.ops import moe
+    g = torch.Generator(device=DEV).manual_seed(K + F)
+    x = torch.randn(T, K, generator=g, device=DEV).bfloat16()
+    up = (torch.randn(E, F, K, generator=g, device=DEV) * K ** -0.5).bfloat16()
+    gate_up = (torch.randn(E, 2 * F, K, generator=g, device=DEV) * K ** -0.5).bfloat16()
+    idx = torch.rand(T, E, generator=g, device=DEV).argsort(1)[:, :top].int()
+    idx[: T // 2, 0] = 0                                   # a crowded expert (twice in a row is no matter)
+    wgt = torch.rand(T, top, generator=g, device=DEV) + 0.2
+    plan = moe.Plan(idx, E, "few")
+    tok, exp = torch.arange(T, device=DEV).repeat_interleave(top), idx.reshape(-1).long()
+    place = plan.pos_of_pair.long()
+    eps = 2.0 ** -8                                        # of a rounding to bf16: half of 2^-7, eight digits
+    acc = K * 2.0 ** -24                                   # of K sums in fp32, relative to sum |x w|
+    z = torch.einsum("pk,pfk->pf", x[tok].double(), up[exp].double()) * wgt.reshape(-1, 1).double()
+    size = torch.einsum("pk,pfk->pf", x[tok].double().abs(), up[exp].double().abs()) * wgt.reshape(-1, 1)
+    # u = relu(z) is rounded once (and z summed in fp32), u^2 again
+    want, off = z.relu() ** 2, (z.abs() * eps + acc * size)
+    got = moe.grouped_relu2(x, up, plan, wgt)[place].double()
+    assert ((got - want).abs() <= (2 * z.abs() + off) * off + eps * (z.abs() + off) ** 2 + 1e-37).all()
+    # the gated form with its clamp far away: s(g) u, s with a slope of at most 1.1
+    h = torch.einsum("pk,pfk->pf", x[tok].double(), gate_up[exp].double())
+    hs = torch.einsum("pk,pfk->pf", x[tok].double().abs(), gate_up[exp].double().abs())
+    gt, u = h[:, 0::2], h[:, 1::2]
+    og, ou = gt.abs() * eps + acc * hs[:, 0::2], u.abs() * eps + acc * hs[:, 1::2]
+    s = gt * torch.sigmoid(gt)
+    got = moe.grouped_glu(x, gate_up, plan, 1e9, 1.0, 0.0)[place].double()
+    off = 1.1 * og * (u.abs() + ou) + s.abs() * ou
+    assert ((got - s * u).abs() <= off + eps * ((s * u).abs() + off) + 1e-6).all()
+    y = moe.grouped_relu2(x, up, plan, wgt)
+    down = (torch.randn(E, K, F, generator=g, device=DEV) * F ** -0.5).bfloat16()
+    if F % 8 == 0:
+        got = moe.grouped_down(y, down, plan)[place].double()
+        yp = y[place].double()
+        want = torch.einsum("pf,pkf->pk", yp, down[exp].double())
+        size = torch.einsum("pf,pkf->pk", yp.abs(), down[exp].double().abs())
+        assert ((got - want).abs() <= (F + 8) * 2.0 ** -24 * size).all()
