@@ -16,8 +16,8 @@
 //                            independent: four lanes or a warp share a column (a share of the rows
 //                            each, in registers).  The tokens' operands come through two stages of
 //                            shared memory, a chunk ahead (cp.async).
-//   delta_chunk_coef_kernel, delta_chunk_recurrence_kernel   the recurrence of long portions with one
-//                            decay a head, eight tokens at a time (see there).
+//   delta_chunk_coef(_channels)_kernel, delta_chunk_recurrence_kernel   the recurrence of long
+//                            portions, eight tokens at a time (see there).
 //   delta_output_kernel      a warp a (token, head): o / rms(o) * w * sigmoid(gate).
 #include "common.cuh"
 
@@ -550,43 +550,144 @@ delta_chunk_coef_kernel(const float* __restrict__ qn, const float* __restrict__ 
   }
 }
 
-// A block = (request, head, 16 columns of S); LANES (8 or 16) lanes a column.  Lane p of a column owns
+// The same with a decay a key channel, where G_i, R and G_7 are vectors: R stands inside the dot products
+// L and M are made of, and the recurrence reads G_i k_i, G_i q_i and R(j, 7) k_j (elementwise) in the
+// places of k_i, q_i and k_j.  A warp a (chunk, head): those three for every token, [T, H, D] each, L, M
+// and beta, and the chunk's G_7.  On a B200, 2,251 tokens of four requests, the longest 1,201, 16 heads
+// of 128 x 128: 26 us and 391 us for the recurrence behind it; token by token 736 us.
+__global__ void __launch_bounds__(128)
+delta_chunk_coef_channels_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
+                                 const float* __restrict__ g, const float* __restrict__ beta,
+                                 const int* __restrict__ cu_seqlens, DeltaDims dm,
+                                 float* __restrict__ coef, float* __restrict__ total,
+                                 float* __restrict__ kg, float* __restrict__ qg, float* __restrict__ ke) {
+  const int lane = threadIdx.x & 31;
+  const int c = blockIdx.x * 4 + (threadIdx.x >> 5), b = blockIdx.y, h = blockIdx.z;
+  pdl_wait();
+  const int t0 = cu_seqlens[b], ta = t0 + c * CT, n = min(CT, cu_seqlens[b + 1] - ta);
+  if (n <= 0) return;
+  const int D = dm.D, H = dm.H, kvh = h / (H / dm.G);
+  const size_t GD = (size_t)dm.G * D, HD = (size_t)H * D;
+  const size_t chunk = (size_t)chunk_number(t0, b, c) * H + h;
+  float val[64];                                             // pairs as above
+#pragma unroll
+  for (int m = 0; m < 64; ++m) val[m] = 0.f;
+  for (int d = 4 * lane; d < D; d += 128) {
+    float k[CT][4], q[CT][4], gd[CT][4];
+#pragma unroll
+    for (int i = 0; i < CT; ++i) {
+#pragma unroll
+      for (int x = 0; x < 4; ++x) k[i][x] = q[i][x] = 0.f, gd[i][x] = 1.f;
+      if (i < n) {
+        const size_t at = (size_t)(ta + i) * GD + (size_t)kvh * D + d;
+        Quad<float>::load(kn + at, k[i]);
+        Quad<float>::load(qn + at, q[i]);
+        Quad<float>::load(g + (size_t)(ta + i) * HD + (size_t)h * D + d, gd[i]);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < CT; ++j) {
+      float kr[4];                                           // R(j, i) k_j
+#pragma unroll
+      for (int x = 0; x < 4; ++x) kr[x] = k[j][x], val[9 * j] = fmaf(kr[x], q[j][x], val[9 * j]);
+#pragma unroll
+      for (int i = j + 1; i < CT; ++i)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          kr[x] *= gd[i][x];
+          val[8 * i + j] = fmaf(kr[x], k[i][x], val[8 * i + j]);
+          val[8 * j + i] = fmaf(kr[x], q[i][x], val[8 * j + i]);
+        }
+      if (j < n) Quad<float>::store(ke + (size_t)(ta + j) * HD + (size_t)h * D + d, kr);
+    }
+    float G[4] = {1.f, 1.f, 1.f, 1.f};
+#pragma unroll
+    for (int i = 0; i < CT; ++i) {
+      float a[4], e[4];
+#pragma unroll
+      for (int x = 0; x < 4; ++x) G[x] *= gd[i][x], a[x] = G[x] * k[i][x], e[x] = G[x] * q[i][x];
+      if (i < n) {
+        const size_t at = (size_t)(ta + i) * HD + (size_t)h * D + d;
+        Quad<float>::store(kg + at, a);
+        Quad<float>::store(qg + at, e);
+      }
+    }
+    Quad<float>::store(total + chunk * D + d, G);
+  }
+#pragma unroll
+  for (int half = 16; half >= 1; half >>= 1) {               // lane l ends with m = l, l + 32, as above
+    const bool up = lane & half;
+#pragma unroll
+    for (int hi = 0; hi < 2; ++hi)
+#pragma unroll
+      for (int m = 0; m < half; ++m) {
+        const float lo_v = val[32 * hi + m], hi_v = val[32 * hi + m + half];
+        const float got = __shfl_xor_sync(0xffffffffu, up ? lo_v : hi_v, half);
+        val[32 * hi + m] = (up ? hi_v : lo_v) + got;
+      }
+  }
+  const float mine[2] = {val[0], val[32]};
+  const float bl = lane < n ? beta[(size_t)(ta + lane) * H + h] : 0.f;
+  float* dst = coef + chunk * kCoefs;
+#pragma unroll
+  for (int x = 0; x < 2; ++x) {
+    const int m = lane + 32 * x, a = m >> 3, e = m & 7;
+    const float bi = __shfl_sync(0xffffffffu, bl, a);
+    if (a > e) {
+      dst[kCoefL + a * CT + e] = bi * mine[x];
+      dst[kCoefM + e * CT + a] = 0.f;                        // (M is read as whole rows)
+    } else {
+      dst[kCoefM + e * CT + a] = mine[x];
+      if (a == e) dst[kCoefL + a * CT + a] = 0.f;
+    }
+  }
+  if (lane < CT) dst[kCoefBeta + lane] = bl;
+}
+
+// A block = (request, head, 16 CP columns of S); LANES (8 or 16) lanes a column, CP columns a lane (a read
+// of k or q serves them all: shared-memory reads bound a block, and two columns a lane halve them where
+// there are blocks enough without).  Lane p of a column owns
 // the rows 4 (p + LANES i) .. + 3, i < DPER / 4, so that the lanes' reads of a token's k and q are one run of
 // shared memory.  Stages as in the kernel above, one barrier a chunk.
-template <int DPER, int LANES>
+// CHANNELS: a decay a key channel; kn, qn and ke are [T, H, D] as delta_chunk_coef_channels_kernel leaves
+// them, total the chunks' G_7.  With a decay a head ke and total are not read.
+template <int DPER, int LANES, int CP, bool CHANNELS>
 __global__ void __launch_bounds__(16 * LANES)
 delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
+                              const float* __restrict__ ke, const float* __restrict__ total,
                               const float* __restrict__ v, const float* __restrict__ coef,
                               float* __restrict__ state, const int* __restrict__ cu_seqlens,
                               const int* __restrict__ slot_ids, DeltaDims dm, float* __restrict__ o) {
-  constexpr int Dp = LANES * DPER, COLS = 16, NQ = DPER / 4;
-  constexpr int kQ = CT * Dp, kVc = 2 * CT * Dp, kC = kVc + CT * COLS, kStage = kC + kCoefs;
+  constexpr int Dp = LANES * DPER, COLS = 16 * CP, NQ = DPER / 4;
+  constexpr int kQ = CT * Dp, kE = CHANNELS ? 2 * CT * Dp : 0, kG = (CHANNELS ? 3 : 2) * CT * Dp;
+  constexpr int kVc = kG + (CHANNELS ? Dp : 0), kC = kVc + CT * COLS, kStage = kC + kCoefs;
   extern __shared__ __align__(16) float stage[];               // [kStages][kStage]
   const int b = blockIdx.x / dm.H, h = blockIdx.x - b * dm.H;
   const int p = threadIdx.x % LANES, lc = threadIdx.x / LANES;
-  const int col0 = blockIdx.y * COLS, col = col0 + lc;
+  const int col0 = blockIdx.y * COLS;                          // a lane's columns: col0 + lc + 16 c
   pdl_trigger();
   const int D = dm.D, Vd = dm.Vd;
   for (int i = threadIdx.x; i < kStages * kStage; i += blockDim.x) stage[i] = 0.f;
   __syncthreads();
   pdl_wait();
-  const bool col_ok = col < Vd;
-  const int cj = col_ok ? col : 0;
-  const int kvh = h / (dm.H / dm.G);
-  float* Sg = state + (size_t)slot_ids[b] * dm.state_stride + ((size_t)h * D) * Vd + cj;
-  float S[NQ][4];
+  const int kvh = CHANNELS ? h : h / (dm.H / dm.G);
+  float* Sg = state + (size_t)slot_ids[b] * dm.state_stride + ((size_t)h * D) * Vd;
+  float S[CP][NQ][4];
 #pragma unroll
-  for (int i = 0; i < NQ; ++i)
+  for (int y = 0; y < CP; ++y)
 #pragma unroll
-    for (int x = 0; x < 4; ++x) {
-      const int row = 4 * (p + LANES * i) + x;
-      S[i][x] = row < D ? Sg[(size_t)row * Vd] : 0.f;
-    }
+    for (int i = 0; i < NQ; ++i)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const int row = 4 * (p + LANES * i) + x, col = col0 + lc + 16 * y;
+        S[y][i][x] = row < D ? Sg[(size_t)row * Vd + (col < Vd ? col : 0)] : 0.f;
+      }
   const int t0 = cu_seqlens[b], t1 = cu_seqlens[b + 1];
-  const size_t GD = (size_t)dm.G * D, HV = (size_t)dm.H * Vd;
+  const size_t KD = (size_t)(CHANNELS ? dm.H : dm.G) * D, HV = (size_t)dm.H * Vd;
   const int vq = min(COLS, Vd - col0) >> 2, dq = D >> 2;
   const int nchunks = (t1 - t0 + CT - 1) / CT;
-  const float* coef0 = coef + ((size_t)chunk_number(t0, b, 0) * dm.H + h) * kCoefs;
+  const int chunk0 = chunk_number(t0, b, 0);
+  const float* coef0 = coef + ((size_t)chunk0 * dm.H + h) * kCoefs;
   auto copy16 = [](float* dst, const float* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
   };
@@ -595,10 +696,14 @@ delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restr
     const int ta = t0 + c * CT, n = min(CT, t1 - ta);
     for (int e = threadIdx.x; e < n * dq; e += blockDim.x) {
       const int t = e / dq, d = 4 * (e - t * dq);
-      const size_t at = (size_t)(ta + t) * GD + (size_t)kvh * D + d;
+      const size_t at = (size_t)(ta + t) * KD + (size_t)kvh * D + d;
       copy16(st + t * Dp + d, kn + at);
       copy16(st + kQ + t * Dp + d, qn + at);
+      if (CHANNELS) copy16(st + kE + t * Dp + d, ke + at);
     }
+    if (CHANNELS)
+      for (int e = threadIdx.x; e < dq; e += blockDim.x)
+        copy16(st + kG + 4 * e, total + ((size_t)(chunk0 + c) * dm.H + h) * D + 4 * e);
     for (int e = threadIdx.x; e < n * vq; e += blockDim.x) {
       const int t = e / vq, d = 4 * (e - t * vq);
       copy16(st + kVc + t * COLS + d, v + (size_t)(ta + t) * HV + (size_t)h * Vd + col0 + d);
@@ -618,16 +723,22 @@ delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restr
     const float* st = stage + (size_t)(c % kStages) * kStage;
     const float* cf = st + kC;
     // this lane's share of S^T k_i (x[i]) and S^T q_i (x[8 + i])
-    float x[2 * CT];
+    float x[CP][2 * CT];
 #pragma unroll
-    for (int i = 0; i < 2 * CT; ++i) x[i] = 0.f;
+    for (int y = 0; y < CP; ++y)
+#pragma unroll
+      for (int i = 0; i < 2 * CT; ++i) x[y][i] = 0.f;
 #pragma unroll
     for (int i = 0; i < NQ; ++i) {
       const float* at = st + 4 * (p + LANES * i);
 #pragma unroll
       for (int t = 0; t < 2 * CT; ++t) {
         const float4 a = *reinterpret_cast<const float4*>(at + t * Dp);
-        x[t] = fmaf(S[i][0], a.x, fmaf(S[i][1], a.y, fmaf(S[i][2], a.z, fmaf(S[i][3], a.w, x[t]))));
+#pragma unroll
+        for (int y = 0; y < CP; ++y) {
+          const float(&s)[4] = S[y][i];
+          x[y][t] = fmaf(s[0], a.x, fmaf(s[1], a.y, fmaf(s[2], a.z, fmaf(s[3], a.w, x[y][t]))));
+        }
       }
     }
     // add up across the column's lanes: of eight, lane p ends with both sums of token p; of sixteen,
@@ -636,75 +747,112 @@ delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restr
     for (int half = LANES / 2; half >= 1; half >>= 1) {
       const bool up = p & half;
 #pragma unroll
-      for (int hi = 0; hi < 2 * CT / LANES; ++hi)
+      for (int y = 0; y < CP; ++y)
 #pragma unroll
-        for (int m = 0; m < half; ++m) {
-          const float lo_v = x[LANES * hi + m], hi_v = x[LANES * hi + m + half];
-          const float got = __shfl_xor_sync(0xffffffffu, up ? lo_v : hi_v, half);
-          x[LANES * hi + m] = (up ? hi_v : lo_v) + got;
-        }
+        for (int hi = 0; hi < 2 * CT / LANES; ++hi)
+#pragma unroll
+          for (int m = 0; m < half; ++m) {
+            const float lo_v = x[y][LANES * hi + m], hi_v = x[y][LANES * hi + m + half];
+            const float got = __shfl_xor_sync(0xffffffffu, up ? lo_v : hi_v, half);
+            x[y][LANES * hi + m] = (up ? hi_v : lo_v) + got;
+          }
     }
     const int tok = p % CT;                                     // the token this lane looks after
-    const float Gp = cf[kCoefG + tok];
-    const float rp = cf[kCoefBeta + tok] * (st[kVc + tok * COLS + lc] - Gp * x[0]);
-    float u[CT];
+    const float Gp = CHANNELS ? 1.f : cf[kCoefG + tok];
+    float u[CP][CT];
 #pragma unroll
-    for (int i = 0; i < CT; ++i) u[i] = __shfl_sync(0xffffffffu, rp, i, LANES);
+    for (int y = 0; y < CP; ++y) {
+      const float rp = cf[kCoefBeta + tok] * (st[kVc + tok * COLS + lc + 16 * y] - Gp * x[y][0]);
+#pragma unroll
+      for (int i = 0; i < CT; ++i) u[y][i] = __shfl_sync(0xffffffffu, rp, i, LANES);
+    }
 #pragma unroll
     for (int j = 0; j < CT - 1; ++j)
 #pragma unroll
-      for (int i = j + 1; i < CT; ++i) u[i] = fmaf(-cf[kCoefL + i * CT + j], u[j], u[i]);
+      for (int i = j + 1; i < CT; ++i) {
+        const float l = -cf[kCoefL + i * CT + j];
+#pragma unroll
+        for (int y = 0; y < CP; ++y) u[y][i] = fmaf(l, u[y][j], u[y][i]);
+      }
     {
       const float4* Mp = reinterpret_cast<const float4*>(cf + kCoefM + tok * CT);
       const float4 m0 = Mp[0], m1 = Mp[1];
-      float out = Gp * (LANES == CT ? x[CT] : x[0]);
-      out = fmaf(m0.x, u[0], fmaf(m0.y, u[1], fmaf(m0.z, u[2], fmaf(m0.w, u[3], out))));
-      out = fmaf(m1.x, u[4], fmaf(m1.y, u[5], fmaf(m1.z, u[6], fmaf(m1.w, u[7], out))));
       const int row = t0 + c * CT + tok;
-      if (col_ok && row < t1 && p >= LANES - CT) o[(size_t)row * HV + (size_t)h * Vd + col] = out;
-    }
-    const float Gc = cf[kCoefG + CT - 1];
 #pragma unroll
-    for (int j = 0; j < CT; ++j) u[j] *= cf[kCoefE + j];
+      for (int y = 0; y < CP; ++y) {
+        const float(&w)[CT] = u[y];
+        float out = Gp * (LANES == CT ? x[y][CT] : x[y][0]);
+        out = fmaf(m0.x, w[0], fmaf(m0.y, w[1], fmaf(m0.z, w[2], fmaf(m0.w, w[3], out))));
+        out = fmaf(m1.x, w[4], fmaf(m1.y, w[5], fmaf(m1.z, w[6], fmaf(m1.w, w[7], out))));
+        const int col = col0 + lc + 16 * y;
+        if (col < Vd && row < t1 && p >= LANES - CT) o[(size_t)row * HV + (size_t)h * Vd + col] = out;
+      }
+    }
+    const float Gc = CHANNELS ? 1.f : cf[kCoefG + CT - 1];
+    if (!CHANNELS)
+#pragma unroll
+      for (int j = 0; j < CT; ++j) {
+        const float e = cf[kCoefE + j];
+#pragma unroll
+        for (int y = 0; y < CP; ++y) u[y][j] *= e;
+      }
 #pragma unroll
     for (int i = 0; i < NQ; ++i) {
-      const float* at = st + 4 * (p + LANES * i);
+      const float* at = st + kE + 4 * (p + LANES * i);
+      float4 g4 = make_float4(Gc, Gc, Gc, Gc);
+      if (CHANNELS) g4 = *reinterpret_cast<const float4*>(st + kG + 4 * (p + LANES * i));
 #pragma unroll
-      for (int y = 0; y < 4; ++y) S[i][y] *= Gc;
+      for (int y = 0; y < CP; ++y)
+        S[y][i][0] *= g4.x, S[y][i][1] *= g4.y, S[y][i][2] *= g4.z, S[y][i][3] *= g4.w;
 #pragma unroll
       for (int t = 0; t < CT; ++t) {
         const float4 a = *reinterpret_cast<const float4*>(at + t * Dp);
-        S[i][0] = fmaf(a.x, u[t], S[i][0]);
-        S[i][1] = fmaf(a.y, u[t], S[i][1]);
-        S[i][2] = fmaf(a.z, u[t], S[i][2]);
-        S[i][3] = fmaf(a.w, u[t], S[i][3]);
+#pragma unroll
+        for (int y = 0; y < CP; ++y) {
+          S[y][i][0] = fmaf(a.x, u[y][t], S[y][i][0]);
+          S[y][i][1] = fmaf(a.y, u[y][t], S[y][i][1]);
+          S[y][i][2] = fmaf(a.z, u[y][t], S[y][i][2]);
+          S[y][i][3] = fmaf(a.w, u[y][t], S[y][i][3]);
+        }
       }
     }
   }
-  if (col_ok) {
+#pragma unroll
+  for (int y = 0; y < CP; ++y)
 #pragma unroll
     for (int i = 0; i < NQ; ++i)
 #pragma unroll
       for (int x = 0; x < 4; ++x) {
-        const int row = 4 * (p + LANES * i) + x;
-        if (row < D) Sg[(size_t)row * Vd] = S[i][x];
+        const int row = 4 * (p + LANES * i) + x, col = col0 + lc + 16 * y;
+        if (row < D && col < Vd) Sg[(size_t)row * Vd + col] = S[y][i][x];
       }
-  }
 }
 
-template <int DPER, int LANES>
-static int launch_chunks(const float* qn, const float* kn, const float* v, const float* coef,
-                         float* state, const int* cu_seqlens, const int* slot_ids, int B,
-                         const DeltaDims& dm, float* o, cudaStream_t st) {
-  const size_t smem = (size_t)kStages * (2 * CT * LANES * DPER + CT * 16 + kCoefs) * sizeof(float);
+template <int DPER, int LANES, int CP, bool CHANNELS>
+static int launch_chunk_columns(const float* qn, const float* kn, const float* ke, const float* total,
+                                const float* v, const float* coef, float* state, const int* cu_seqlens,
+                                const int* slot_ids, int B, const DeltaDims& dm, float* o,
+                                cudaStream_t st) {
+  const size_t smem = (size_t)kStages * sizeof(float) *
+                      ((CHANNELS ? 3 * CT + 1 : 2 * CT) * LANES * DPER + CT * 16 * CP + kCoefs);
   static OncePerDevice attrs;
   if (int rc = attrs.run([&] {
-        return cudaFuncSetAttribute(delta_chunk_recurrence_kernel<DPER, LANES>,
+        return cudaFuncSetAttribute(delta_chunk_recurrence_kernel<DPER, LANES, CP, CHANNELS>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       }))
     return rc;
-  return launch_kernel(delta_chunk_recurrence_kernel<DPER, LANES>, dim3(B * dm.H, (dm.Vd + 15) / 16),
-                       dim3(16 * LANES), smem, st, qn, kn, v, coef, state, cu_seqlens, slot_ids, dm, o);
+  return launch_kernel(delta_chunk_recurrence_kernel<DPER, LANES, CP, CHANNELS>,
+                       dim3(B * dm.H, (dm.Vd + 16 * CP - 1) / (16 * CP)), dim3(16 * LANES), smem, st, qn,
+                       kn, ke, total, v, coef, state, cu_seqlens, slot_ids, dm, o);
+}
+
+template <int DPER, int LANES, bool CHANNELS, typename... Args>
+static int launch_chunks(int B, const DeltaDims& dm, float* o, cudaStream_t st, Args... args) {
+  // two blocks an SM of 16 columns: then one of 32 each does the same work with half the reads (512
+  // blocks of 16 columns 434 us, 256 of 32 391)
+  if (LANES * DPER <= 128 && (long long)B * dm.H * ((dm.Vd + 15) / 16) >= 2 * 148 && dm.Vd > 16)
+    return launch_chunk_columns<DPER, LANES, LANES * DPER <= 128 ? 2 : 1, CHANNELS>(args..., B, dm, o, st);
+  return launch_chunk_columns<DPER, LANES, 1, CHANNELS>(args..., B, dm, o, st);
 }
 
 template <typename T>
@@ -818,31 +966,44 @@ GF_EXPORT int gf_delta_prepare_heads(const float* proj, int ld, int a_off, int b
                        0, st, proj, ld, state, cu_seqlens, slot_ids, dm);
 }
 
-// fp32 words of scratch with which gf_delta_recurrence takes eight tokens at a time (one decay a head).
-GF_EXPORT long long gf_delta_chunk_words(int T, int B, int H) {
-  return (long long)(T / CT + B + 1) * H * kCoefs;
+// fp32 words of scratch with which gf_delta_recurrence takes eight tokens at a time.
+GF_EXPORT long long gf_delta_chunk_words(int T, int B, int H, int D, int one_decay) {
+  const long long chunks = (long long)(T / CT + B + 1) * H;
+  return one_decay ? chunks * kCoefs : chunks * (kCoefs + D) + 3ll * T * H * D;
 }
 
-// one_decay: g is [T, H] (a decay a head), else [T, H, D].  scratch (gf_delta_chunk_words; null: token
-// by token) and max_q_len, the longest portion, are for steps with one decay a head.
+// one_decay: g is [T, H] (a decay a head), else [T, H, D].  scratch: gf_delta_chunk_words, or null: token
+// by token; max_q_len: the longest portion.
 GF_EXPORT int gf_delta_recurrence(const float* qn, const float* kn, const float* v, const float* g,
                                   const float* beta, float* state, const int* cu_seqlens,
-                                  const int* slot_ids, int B, int H, int G, int D, int Vd,
+                                  const int* slot_ids, int T, int B, int H, int G, int D, int Vd,
                                   int state_stride, float* o, int one_decay, float* scratch,
                                   int max_q_len, void* stream) {
   if (B <= 0) return 0;
   if (H % G) return -3;
   const DeltaDims dm = dims_of(H, G, D, Vd, 1, state_stride, 0);
   auto st = (cudaStream_t)stream;
-  if (one_decay && scratch && D % 4 == 0 && Vd % 4 == 0 && D <= 256 && B <= 65535 && G <= 65535 &&
-      (((uintptr_t)qn | (uintptr_t)kn | (uintptr_t)v | (uintptr_t)scratch) & 15) == 0) {
-    const int chunks = (max_q_len + CT - 1) / CT;
-    if (int rc = launch_kernel(delta_chunk_coef_kernel, dim3((chunks + 3) / 4, B, G), dim3(128), 0, st,
-                               qn, kn, g, beta, cu_seqlens, dm, scratch))
-      return rc;
+  if (scratch && D % 4 == 0 && Vd % 4 == 0 && D <= 256 && B <= 65535 && H <= 65535 &&
+      (((uintptr_t)qn | (uintptr_t)kn | (uintptr_t)v | (uintptr_t)scratch) & 15) == 0 &&
+      (one_decay || ((uintptr_t)g & 15) == 0)) {
+    const dim3 cgrid(((max_q_len + CT - 1) / CT + 3) / 4, B, one_decay ? G : H);
+    const size_t chunks = (size_t)(T / CT + B + 1) * H, HTD = (size_t)T * H * D;
+    float* total = scratch + chunks * kCoefs;
+    float *kg = total + chunks * D, *qg = kg + HTD, *ke = qg + HTD;      // (a decay a channel only)
+    const int rc = one_decay ? launch_kernel(delta_chunk_coef_kernel, cgrid, dim3(128), 0, st, qn, kn, g,
+                                             beta, cu_seqlens, dm, scratch)
+                             : launch_kernel(delta_chunk_coef_channels_kernel, cgrid, dim3(128), 0, st, qn,
+                                             kn, g, beta, cu_seqlens, dm, scratch, total, kg, qg, ke);
+    if (rc) return rc;
 #define GF_GO(DPER, LANES)                                                                         \
-  if (D <= DPER * LANES)                                                                           \
-    return launch_chunks<DPER, LANES>(qn, kn, v, scratch, state, cu_seqlens, slot_ids, B, dm, o, st);
+  if (D <= DPER * LANES) {                                                                         \
+    if (one_decay)                                                                                 \
+      return launch_chunks<DPER, LANES, false>(B, dm, o, st, qn, kn, (const float*)nullptr,        \
+                                               (const float*)nullptr, v, scratch, state,           \
+                                               cu_seqlens, slot_ids);                              \
+    return launch_chunks<DPER, LANES, true>(B, dm, o, st, qg, kg, ke, total, v, scratch, state,    \
+                                            cu_seqlens, slot_ids);                                 \
+  }
     GF_GO(4, 8)
     GF_GO(8, 8)
     GF_GO(16, 8)             // (sixteen lanes of 8 rows: 348 us for a prompt that takes 317 so)

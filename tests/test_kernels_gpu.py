@@ -547,3 +547,52 @@ def test_grouped_products_that_stream_the_weights(K, F, T, E, top):
         want = torch.einsum("pf,pkf->pk", yp, down[exp].double())
         size = torch.einsum("pf,pkf->pk", yp.abs(), down[exp].double().abs())
         assert ((got - want).abs() <= (F + 8) * 2.0 ** -24 * size).all()
+
+
+@pytest.mark.parametrize("H,G,D,Vd,lens", [(2, 1, 12, 20, [16, 1, 7]), (4, 2, 64, 64, [40, 8, 9, 3]),
+                                           (2, 2, 128, 128, [33, 17]), (3, 3, 100, 36, [24, 25, 31, 1]),
+                                           (2, 1, 256, 48, [65]), (1, 1, 128, 4, [1, 1, 23]),
+                                           (8, 8, 128, 100, [17] * 6)])
+def test_delta_rule_with_channel_decays_eight_tokens_at_a_time(H, G, D, Vd, lens):
+    """Chunks whole and cut, portions shorter than a chunk, one and two columns a lane, decays from none
+    to all gone: outputs and states against the recurrence token by token in 64 bits, beside the
+    token-by-token kernel."""
+    from types import SimpleNamespace
+    from ginfer_b200.ops import delta
+    g0 = torch.Generator().manual_seed(D + Vd)
+    B, T = len(lens), sum(lens)
+    q = torch.randn(T, G, D, generator=g0) / D ** 0.5
+    k = torch.nn.functional.normalize(torch.randn(T, G, D, generator=g0), dim=-1)
+    v, beta = torch.randn(T, H, Vd, generator=g0), torch.rand(T, H, generator=g0)
+    g = torch.rand(T, H, D, generator=g0)
+    g[:, :, ::3] = 1.0 - g[:, :, ::3] * 0.01
+    g[T // 2, :, 1::4] = 1e-30                              # a channel forgets all it held
+    state0 = torch.randn(B + 2, H * D * Vd + 8, generator=g0)
+    cu = torch.tensor([0] + lens).cumsum(0)
+    slots = torch.randperm(B + 2, generator=g0)[:B]
+    got = []
+    for longest in (max(lens), 0):
+        state = state0.clone().cuda()
+        ctx = SimpleNamespace(num_seqs=B, slot_ids=slots.int().cuda(), cu_seqlens_q=cu.int().cuda(),
+                              max_q_len=longest)
+        o = delta.recurrence(q.cuda(), k.cuda(), v.cuda(), g.cuda(), beta.cuda(), state, ctx)
+        got.append((o.cpu().double(), state.cpu()))
+    err = [0.0, 0.0]
+    for b in range(B):
+        S = state0[slots[b], :H * D * Vd].double().reshape(H, D, Vd).clone()
+        kv = torch.arange(H) // (H // G)
+        for t in range(int(cu[b]), int(cu[b + 1])):
+            S = g[t].double()[:, :, None] * S
+            u = beta[t].double()[:, None] * (v[t].double() - torch.einsum("hdv,hd->hv", S, k[t, kv].double()))
+            S = S + k[t, kv].double()[:, :, None] * u[:, None]
+            want = torch.einsum("hdv,hd->hv", S, q[t, kv].double())
+            for i in range(2):
+                err[i] = max(err[i], float((got[i][0][t] - want).abs().max()))
+        for i in range(2):
+            kept = got[i][1][slots[b]]
+            err[i] = max(err[i], float((kept[:H * D * Vd].double() - S.reshape(-1)).abs().max()))
+            assert torch.equal(kept[H * D * Vd:], state0[slots[b], H * D * Vd:])
+    # values of a few units, sums of at most 256 products of unit vectors' channels in fp32
+    assert err[0] <= 2e-5 and err[1] <= 2e-5, err
+    rest = [s for s in range(B + 2) if s not in slots.tolist()]
+    assert torch.equal(got[0][1][rest], state0[rest])
