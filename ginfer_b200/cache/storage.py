@@ -78,6 +78,7 @@ class CacheStorage:
         self.num_slots = num_slots
         self.state = {cid: torch.zeros((num_slots + 1, *s.shape), dtype=s.dtype, device=device)
                       for cid, s in cache_specs.items() if isinstance(s, StateSpec)}
+        self._spans = None           # the states' addresses and slot sizes on the device
 
     def group_of(self, cache_id: int) -> int:
         return self._where[cache_id][0]
@@ -95,6 +96,19 @@ class CacheStorage:
     def is_paged(self, cache_id: int) -> bool:
         return cache_id in self._where
 
+    def reset_slots(self, slots: list[int]) -> None:
+        """The slots' state becomes zero, all of it by one kernel."""
+        if not self.state or not slots:
+            return
+        if any(not 0 <= s <= self.num_slots for s in slots):
+            raise IndexError(f"slots {slots} of {self.num_slots}")
+        if self._spans is None:
+            self._spans = torch.tensor([[t.data_ptr(), t.stride(0) * t.element_size()]
+                                        for t in self.state.values()], dtype=torch.int64,
+                                       device=next(iter(self.state.values())).device)
+        from ..ops import zero_slots
+        with torch.cuda.device(self._spans.device):      # (a step is prepared outside any guard)
+            zero_slots(self._spans, slots)
+
     def reset_slot(self, slot: int) -> None:
-        for t in self.state.values():
-            t[slot].zero_()
+        self.reset_slots([slot])

@@ -6,6 +6,25 @@
 
 namespace gf {
 
+// The states of requests that start: a step of 32 of them had 64 fills, 5 us of host time each, where
+// one kernel does.
+struct SlotList {
+  static constexpr int kMax = 64;
+  int count;
+  int slot[kMax];
+};
+__global__ void zero_slots_kernel(const longlong2* __restrict__ spans, const SlotList list) {
+  pdl_trigger();
+  pdl_wait();
+  const longlong2 s = spans[blockIdx.y];
+  uint8_t* base = reinterpret_cast<uint8_t*>(s.x) + (size_t)list.slot[blockIdx.z] * s.y;
+  const long long at = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  if (((uintptr_t)base | s.y) % 16 == 0)
+    for (long long i = at; i < s.y / 16; i += step) reinterpret_cast<uint4*>(base)[i] = make_uint4(0, 0, 0, 0);
+  else
+    for (long long i = at; i < s.y / 4; i += step) reinterpret_cast<uint32_t*>(base)[i] = 0;
+}
+
 // ----------------------------------------------------------------------------- embedding
 // out[t, :] = W[ids[t], :], copied in `unit`-byte words (16 when rows allow it).
 template <typename V>
@@ -416,6 +435,21 @@ GF_EXPORT int gf_rope_kv_write(void* qkv, int row_stride, const float* table, in
   return launch_kernel(rope_kv_write_kernel<__nv_bfloat16>, dim3(T), dim3(threads), 0, st,
                        (__nv_bfloat16*)qkv, row_stride, table, rot, positions, slot_mapping,
                        (__nv_bfloat16*)kpages, (__nv_bfloat16*)vpages, nh, nkv, hd);
+}
+
+// spans[i] = {address of a state's first slot, bytes a slot}, i < n; the slots named by `slots` (host) of
+// each become zero.  Slot sizes are multiples of four bytes.
+GF_EXPORT int gf_zero_slots(const long long* spans, int n, const int* slots, int count, void* stream) {
+  for (int at = 0; at < count; at += SlotList::kMax) {
+    SlotList list;
+    list.count = count - at < SlotList::kMax ? count - at : SlotList::kMax;
+    for (int i = 0; i < list.count; ++i) list.slot[i] = slots[at + i];
+    if (n <= 0) return 0;
+    const int rc = launch_kernel(zero_slots_kernel, dim3(16, n, list.count), dim3(256), 0,
+                                 (cudaStream_t)stream, (const longlong2*)spans, list);
+    if (rc) return rc;
+  }
+  return 0;
 }
 
 GF_EXPORT int gf_silu_mul(const void* gu, void* out, int T, int I, int dtype, void* stream) {

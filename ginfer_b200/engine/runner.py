@@ -173,9 +173,8 @@ class ModelRunner:
             slots = np.fromiter((cache.requests[i].slot for i in ids), dtype=np.int32, count=B)
         q_starts = cache.lengths(slots).astype(np.int64)
         if self.storage.state:
-            for sl, n0 in zip(slots, q_starts):
-                if n0 == 0:                  # a sequence starts (again): its state starts at zero
-                    self.storage.reset_slot(int(sl))
+            # a sequence starts (again): its state starts at zero
+            self.storage.reset_slots([int(sl) for sl, n0 in zip(slots, q_starts) if n0 == 0])
         cache.reserve_step(slots, q_lens)
 
         tokens = np.concatenate([np.asarray(e.tokens, dtype=np.int64).reshape(-1)

@@ -31,11 +31,13 @@ def _p(t):
     if not t.is_cuda:
         raise RuntimeError("ginfer_b200 kernels run on a CUDA device only; got a tensor on "
                            f"{t.device}")
-    return c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 def _stream():
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current stream's handle.  (``torch.cuda.current_stream()`` makes a stream object, 8 us a call, of
+    which a step that is launched kernel by kernel makes one a kernel.)"""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _cuda(*ts):
@@ -311,7 +313,6 @@ def paged_attention_simt(qkv, pages, block_table, seq_of_token, positions, nh, n
     ``cap * tanh(s / cap)``; ``slopes`` (fp32, a head): ``slope * (p - c)`` is taken off the score
     of the key at ``c`` for the query at ``p``, after the cap; ``sink``: ``exp(sink)`` is added to the
     softmax's denominator (a score without a key and a value; a tensor: one a head)."""
-    from . import attention_bf16
     _cuda(qkv, pages[0], pages[1], block_table, seq_of_token, positions, slopes)
     assert slopes is None or (slopes.dtype == torch.float32 and slopes.numel() == nh
                               and slopes.is_contiguous())
@@ -337,7 +338,6 @@ def paged_attention_simt(qkv, pages, block_table, seq_of_token, positions, nh, n
 def attention_fuses_rope(qkv: torch.Tensor, ctx, nh: int, nkv: int, hd: int) -> bool:
     """True if :func:`paged_attention` can rotate q and k and write the new k and v itself for
     this step (pass ``rope=`` then, and skip :func:`rope_kv_write`)."""
-    from . import attention_bf16
     return attention_bf16.fuses_rope(qkv, ctx, hd, nh, nkv)
 
 
@@ -353,7 +353,6 @@ def paged_attention(qkv: torch.Tensor, pages, block_table: torch.Tensor, ctx,
     (``pages`` is then the pair of the cache's two planes; the result is ``[T, nh * vd]``).
     ``softcap``, ``slopes``, ``sink``: a soft cap on the scores, a distance bias a head and a sink, see
     :func:`paged_attention_simt`."""
-    from . import attention_bf16
     shaped = dict(softcap=float(softcap or 0.0), slopes=slopes, sink=sink)
     if vd is not None and vd != hd:        # keys and values of different widths: the plain kernel
         assert rope is None
@@ -421,6 +420,16 @@ def scatter_tokens(dst: torch.Tensor, dst_idx: torch.Tensor, src: torch.Tensor,
     _ok(f(_p(dst), _p(dst_idx), _p(src), _p(src_idx), n, _stream()), "scatter_tokens")
 
 
+def zero_slots(spans: torch.Tensor, slots) -> None:
+    """``spans [n, 2]`` int64 on the device: address and bytes a slot of ``n`` states; the slots named
+    become zero in all of them."""
+    _cuda(spans)
+    assert spans.dtype == torch.int64 and spans.dim() == 2 and spans.shape[1] == 2 and spans.is_contiguous()
+    f = _fn("elementwise", "gf_zero_slots", [c_void_p, c_int, c_void_p, c_int, c_void_p])
+    names = (c_int * len(slots))(*slots)
+    _ok(f(_p(spans), spans.shape[0], names, len(slots), _stream()), "zero_slots")
+
+
 def qkv_rope_write(x, linear, table, rot, positions, slot_mapping, pages, nh, nkv, hd):
     """``linear(x)`` with q and k rotated and k and v written to the cache by the product's own
     epilogue, where that is served (bf16, many tokens; see ``gemm_prefill.qkv_rope_write``), else
@@ -428,7 +437,6 @@ def qkv_rope_write(x, linear, table, rot, positions, slot_mapping, pages, nh, nk
     if (getattr(linear, "dtype", None) != torch.bfloat16 or x.dtype != torch.bfloat16
             or linear.out_dtype != torch.bfloat16):
         return None
-    from . import gemm_prefill
     return gemm_prefill.qkv_rope_write(x, linear.weight, linear._bias_f32, table, rot, positions,
                                        slot_mapping, pages, nh, nkv, hd)
 
@@ -443,6 +451,7 @@ def bmm_f32_out(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     return torch.bmm(a, b, out_dtype=torch.float32)
 
 
+from . import attention_bf16, gemm_bf16, gemm_prefill  # noqa: E402,F401
 from .linear import GatedLinear, Linear, add_to  # noqa: E402,F401
 from . import prenorm  # noqa: E402,F401
 from . import depth, hyper, rotary, shift  # noqa: E402,F401

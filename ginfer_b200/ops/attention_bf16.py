@@ -7,6 +7,9 @@ from ctypes import c_float, c_int, c_void_p
 
 import torch
 
+from . import _Counter, _fn, _ok, _p, _stream
+from .gemm_bf16 import _dev_state, error_word, num_sms
+
 KEY_TILE = 64
 CTAS_PER_SM = 2                # resident CTAs of the decode kernel on one SM
 MAX_SPLITS = 64
@@ -19,7 +22,6 @@ def sink_args(sink):
     """What the kernels are told of a sink: one score for all heads (``None``: none), or an fp32 tensor
     with one a head -> ``(score, pointer)``."""
     if torch.is_tensor(sink):
-        from . import _p
         assert sink.dtype == torch.float32 and sink.dim() == 1 and sink.is_contiguous()
         return NO_SINK, _p(sink)
     return (NO_SINK if sink is None else float(sink)), None
@@ -33,7 +35,6 @@ def decode_splits(batch: int, nh: int, nkv: int, max_keys: int, sms: int | None 
     """How many ways to split each request's keys so that the grid fills the GPU without a second
     wave: a power of two up to 8, so that the splits of a request can form a thread-block cluster.  ``sms``: the
     device's SM count (asked of the current device if ``None``)."""
-    from .gemm_bf16 import num_sms
     chunks = (nh // nkv + 15) // 16
     base = max(1, batch * nkv * chunks)
     target = (sms or num_sms()) * CTAS_PER_SM
@@ -59,7 +60,6 @@ def decode_partition(batch: int, nh: int, nkv: int, max_keys: int,
     memory, and how many such clusters share a request's keys (their results are added up by a
     second kernel).  More than one cluster only where 8 CTAs a request and kv head leave most of
     the GPU idle: few requests with many keys."""
-    from .gemm_bf16 import num_sms
     splits = decode_splits(batch, nh, nkv, max_keys, sms)
     if splits < 8:
         return splits, 1
@@ -104,7 +104,6 @@ def decode(qkv, pages, block_table, cu_seqlens_q, positions, B, nh, nkv, hd, sca
     they take the kernel that loads its tiles with ``cp.async`` (no rotation inside it).
     ``sink``: the score of a sink in the softmax's denominator, a number or an fp32 tensor with one a
     head (every kernel takes it; no rotation inside it either)."""
-    from . import _fn, _ok, _p, _stream
     defines = (f"GF_HEAD_DIM={hd}",)
     is_shaped = bool(softcap) or slopes is not None
     if is_shaped:
@@ -124,7 +123,6 @@ def decode(qkv, pages, block_table, cu_seqlens_q, positions, B, nh, nkv, hd, sca
         else:
             scratch = _scratch_for(nbytes, qkv.device)
     if use_tma and hd % 64 == 0 and scratch is None and not through_scratch:
-        from .gemm_bf16 import error_word
         table, rot, write = rope if rope is not None else (None, 0, False)
         parts = max(1, int(parts))
         part_scratch = None
@@ -147,7 +145,6 @@ def decode(qkv, pages, block_table, cu_seqlens_q, positions, B, nh, nkv, hd, sca
                int(bool(write)), _p(error_word(qkv.device)), _stream(), parts, _p(part_scratch),
                sink_score, sinks)
         if rc == 0 and parts > 1:
-            from . import _Counter
             _Counter.launches += 1                     # the kernel that adds the parts up
         if rc != -6:
             _ok(rc, "attn_decode_tma")
@@ -187,7 +184,6 @@ def decode(qkv, pages, block_table, cu_seqlens_q, positions, B, nh, nkv, hd, sca
 def prefill(qkv, pages, block_table, cu_seqlens_q, kv_lens, B, max_q_len, nh, nkv, hd, scale,
             window, page_size, out=None, softcap: float = 0.0, slopes=None,
             sink=None):
-    from . import _fn, _ok, _p, _stream
     if out is None:
         out = torch.empty((qkv.shape[0], nh * hd), dtype=torch.bfloat16, device=qkv.device)
     if softcap or slopes is not None or sink is not None:
@@ -232,10 +228,6 @@ def prefill_tc(qkv, pages, block_table, cu_seqlens_q, kv_lens, B, max_q_len, nh,
     ``softcap`` > 0, ``slopes`` (fp32, a head): shaped scores as in ``ops.paged_attention_simt``
     (an instance of the kernel of its own).  ``sink``: the score of a sink in the softmax's
     denominator."""
-    from ctypes import c_float, c_int, c_void_p
-
-    from . import _fn, _ok, _p, _stream
-    from .gemm_bf16 import _dev_state
     if not tc_supports(hd, page_size) or qkv.stride(0) % 8:
         return None
     T = qkv.shape[0]

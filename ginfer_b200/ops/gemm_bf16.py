@@ -7,6 +7,8 @@ from dataclasses import dataclass
 
 import torch
 
+from . import _fn, _ok, _p, _stream
+
 B200_SMS = 148                 # what the split choices assume where no device can be asked
 _state: dict = {}
 _sms: dict = {}
@@ -15,13 +17,15 @@ _sms: dict = {}
 def num_sms(device=None) -> int:
     """Streaming multiprocessors of ``device`` (the current one if ``None``), read from the
     device; without a CUDA device (host-side tests of the split choices) a B200's count."""
-    if not torch.cuda.is_available():
-        return B200_SMS
     key = torch.device(device).index if device is not None else None
     if key is None:
+        if not torch.cuda.is_initialized() and not torch.cuda.is_available():
+            return B200_SMS
         key = torch.cuda.current_device()
     n = _sms.get(key)
     if n is None:
+        if not torch.cuda.is_available():
+            return B200_SMS
         n = _sms[key] = torch.cuda.get_device_properties(key).multi_processor_count
     return n
 
@@ -122,7 +126,6 @@ def gemm(x, weight, bias_f32=None, out_dtype=torch.bfloat16, epi: int = 0, split
     is ``(s, scaled, sumsq)`` with ``s = resid + x W^T (+ bias)`` in fp32, ``scaled = bf16(s *
     gamma)`` (``None`` without ``gamma``) and the partial sums of squares of ``s``'s rows.
     Returns ``None`` if the kernel cannot serve the shape."""
-    from . import _fn, _ok, _p, _stream
     if not supports(x, weight):
         return None
     M, K = x.shape

@@ -9,6 +9,9 @@ from ctypes import c_int, c_void_p
 
 import torch
 
+from . import _cuda, _fn, _ok, _p, _stream
+from .gemm_bf16 import error_word
+
 
 def supports(x: torch.Tensor, weight: torch.Tensor) -> bool:
     K = weight.shape[1]
@@ -27,8 +30,6 @@ def gemm(x, weight, bias_f32=None, out_dtype=torch.bfloat16, epi: int = 0, ctas:
     ``ctas``: CTAs to launch (0: one an SM).  ``pair``: on CTA pairs (tiles of 256 tokens x 256
     weight rows, tcgen05 ``cta_group::2``; ``None``: the default).  ``None`` if the kernel cannot
     serve the shape."""
-    from . import _cuda, _fn, _ok, _p, _stream
-    from .gemm_bf16 import error_word
     if not supports(x, weight):
         return None
     _cuda(x, weight, bias_f32)
@@ -90,8 +91,6 @@ def qkv_rope_write(x, weight, bias_f32, table, rot, positions, slot_mapping, pag
     does behind a plain product).  ``pages [2, num_pages, page, nkv, hd]`` bf16.  Returns
     ``[T, (nh + 2 nkv) hd]`` with q and k rotated, or ``None`` if the kernel does not serve the
     case (:func:`qkv_epilogue_serves`; ``min_tokens`` is ``QKV_MIN_TOKENS`` unless given)."""
-    from . import _cuda, _fn, _ok, _p, _stream
-    from .gemm_bf16 import error_word
     M, K = x.shape
     if min_tokens is None:
         if not QKV_EPILOGUE:

@@ -13,7 +13,8 @@ from ctypes import c_int, c_void_p
 
 import torch
 
-from . import _cuda, _fn, _ok, _p, _stream, silu_mul
+from . import (_cuda, _fn, _ok, _p, _stream, activation_, clamped_glu, gemm_bf16, gemm_prefill,
+               silu_mul)
 
 
 def gemm_f32(x: torch.Tensor, w: torch.Tensor, bias=None) -> torch.Tensor:
@@ -68,12 +69,10 @@ class Linear:
             return self._product(x)
         if (self.dtype == torch.bfloat16 and not hasattr(x, "materialize")
                 and x.dtype == self.dtype):
-            from . import gemm_bf16
             y = gemm_bf16.try_linear(x, self.weight, self._bias_f32, self.out_dtype,
                                      activation=self.activation, act_consts=self.act_consts)
             if y is not None:
                 return y
-        from . import activation_
         return activation_(self._product(x), self.activation, *(self.act_consts or ()))
 
     def deferring_bias(self, x):
@@ -84,7 +83,6 @@ class Linear:
         if (self.activation is None and self.dtype == torch.bfloat16 and self.bias is not None
                 and self.out_dtype == torch.float32 and not hasattr(x, "materialize")
                 and x.dtype == self.dtype):
-            from . import gemm_bf16
             y = gemm_bf16.try_linear(x, self.weight, self._bias_f32, self.out_dtype)
             if y is not None:
                 return y, None
@@ -94,7 +92,6 @@ class Linear:
     def _product(self, x) -> torch.Tensor:
         if hasattr(x, "materialize"):                 # a normalisation not computed yet
             if self.dtype == torch.bfloat16 and x.scaled is not None:
-                from . import gemm_bf16
                 y = gemm_bf16.gemm(x.scaled, self.weight, self._bias_f32, self.out_dtype,
                                    scale=gemm_bf16.RowScale(x.summed.sumsq, x.eps))
                 if y is not None:
@@ -104,7 +101,6 @@ class Linear:
             raise TypeError(f"Linear holds {self.dtype} weights but got {x.dtype} input")
         if self.dtype == torch.float32:
             return gemm_f32(x, self.weight, self.bias)
-        from . import gemm_bf16
         y = gemm_bf16.try_linear(x, self.weight, self._bias_f32, self.out_dtype)
         if y is not None:
             return y
@@ -125,7 +121,6 @@ def add_to(linear: "Linear", x: torch.Tensor, residual: torch.Tensor, gamma=None
     weight of the RMS norm that follows, if it can be folded."""
     if linear.dtype != torch.bfloat16 or residual.dtype != torch.float32:
         return None
-    from . import gemm_bf16
     if x.shape[0] > gemm_bf16.plain_limit(linear.weight):
         return None
     got = gemm_bf16.gemm(x, linear.weight, linear._bias_f32, resid=residual, gamma=gamma)
@@ -142,11 +137,6 @@ def add_to(linear: "Linear", x: torch.Tensor, residual: torch.Tensor, gamma=None
 # 8,192 tokens 304 against 386; at the 7B shape (37888 x 3584) 768 tokens 151 against 153, 1,024
 # tokens 193 against 210, 2,048 tokens 367 against 392.
 PREFILL_GATED_MIN_TOKENS = 768
-
-
-def _gemm_bf16():
-    from . import gemm_bf16
-    return gemm_bf16
 
 
 class GatedLinear:
@@ -171,15 +161,13 @@ class GatedLinear:
     def __call__(self, x) -> torch.Tensor:
         if hasattr(x, "materialize"):                 # a normalisation not computed yet
             if self.proj.dtype == torch.bfloat16 and x.scaled is not None \
-                    and x.scaled.shape[0] <= _gemm_bf16().MAX_TOKENS:
-                gb = _gemm_bf16()
-                z = gb.gemm(x.scaled, self.proj.weight, self.act, torch.bfloat16, epi=2,
-                            scale=gb.RowScale(x.summed.sumsq, x.eps))
+                    and x.scaled.shape[0] <= gemm_bf16.MAX_TOKENS:
+                z = gemm_bf16.gemm(x.scaled, self.proj.weight, self.act, torch.bfloat16, epi=2,
+                            scale=gemm_bf16.RowScale(x.summed.sumsq, x.eps))
                 if z is not None:
                     return z
             x = x.materialize()
         if x.dtype == torch.bfloat16:
-            from . import gemm_bf16, gemm_prefill
             if x.shape[0] <= gemm_bf16.MAX_TOKENS:
                 z = gemm_bf16.gemm(x, self.proj.weight, self.act, torch.bfloat16, epi=2)
                 if z is not None:
@@ -189,6 +177,5 @@ class GatedLinear:
                 if z is not None:
                     return z
         if self.clamped is not None:
-            from . import clamped_glu
             return clamped_glu(self.proj(x), *self.clamped)
         return silu_mul(self.proj(x))

@@ -7,6 +7,7 @@ from ctypes import c_float, c_int, c_void_p
 import torch
 
 from . import _code, _cuda, _fn, _ok, _p, _stream, load_library
+from .gemm_bf16 import _dev_state
 
 _tile_rows: dict = {}
 
@@ -184,7 +185,6 @@ def gather_rows(x: torch.Tensor, plan: Plan) -> torch.Tensor:
 
 def _grouped_tc(a, w, plan: Plan, out, epi: int, act=None, row_w=None) -> bool:
     """The grouped product on the persistent tcgen05 kernel; ``False`` if it refuses the shape."""
-    from .gemm_bf16 import _dev_state
     E, N, K = w.shape
     f = _fn("gemm_prefill", "gf_gemm_grouped",
             [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,

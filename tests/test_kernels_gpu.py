@@ -596,3 +596,18 @@ def test_delta_rule_with_channel_decays_eight_tokens_at_a_time(H, G, D, Vd, lens
     assert err[0] <= 2e-5 and err[1] <= 2e-5, err
     rest = [s for s in range(B + 2) if s not in slots.tolist()]
     assert torch.equal(got[0][1][rest], state0[rest])
+
+
+@pytest.mark.parametrize("slots", [[2], [0, 4, 1], list(range(69, -1, -1))])
+def test_zero_slots_clears_the_named_slots_of_every_state(slots):
+    """States of several types and slot sizes (whole 16 bytes and not), more slots than a launch names."""
+    n = max(max(slots) + 2, 6)
+    states = [torch.ones((n, 7), dtype=torch.int32, device=DEV), torch.ones((n, 1), dtype=torch.int32, device=DEV),
+              torch.ones((n, 12345), device=DEV), torch.ones((n, 64), device=DEV)]
+    from ginfer_b200 import ops
+    spans = torch.tensor([[t.data_ptr(), t.stride(0) * t.element_size()] for t in states], device=DEV)
+    ops.zero_slots(spans, slots)
+    for t in states:
+        want = torch.ones(n, dtype=torch.bool, device=DEV)
+        want[slots] = False
+        assert torch.equal((t == 1).all(dim=1), want) and torch.equal((t == 0).all(dim=1), ~want)
