@@ -31,6 +31,24 @@ __device__ __forceinline__ float xielu(float z, float a, float b) {
   return fmaf(0.5f, z, z > 0.f ? a * z2 : b * below);
 }
 
+// The gated activation in a product's epilogue; gate and up are rounded to bf16 first, as a plain product
+// would store them.  `act` null: silu(gate) * up.  Else act = {limit, alpha, shift} (passed in a gated
+// product's place for a bias):
+// min(gate, limit) * sigmoid(alpha * min(gate, limit)) * (clamp(up, -limit, limit) + shift).
+__device__ __forceinline__ float gated_activation(float g, float u, const float* __restrict__ act) {
+  float gg = __bfloat162float(__float2bfloat16_rn(g));
+  float uu = __bfloat162float(__float2bfloat16_rn(u));
+  if (act) {
+    const float limit = __ldg(act), alpha = __ldg(act + 1), shift = __ldg(act + 2);
+    gg = fminf(gg, limit);
+    uu = fminf(fmaxf(uu, -limit), limit);
+    // alpha < 0: the gate's sigmoid sharpened to a step (relu)
+    const float sg = alpha < 0.f ? (gg > 0.f ? 1.0f : 0.0f) : 1.0f / (1.0f + expf(-alpha * gg));
+    return gg * sg * (uu + shift);
+  }
+  return gg * (1.0f / (1.0f + expf(-gg))) * uu;
+}
+
 template <typename T> __device__ __forceinline__ float to_f32(T v);
 template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; }
 template <> __device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 v) {

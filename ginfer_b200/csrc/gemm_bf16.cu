@@ -12,7 +12,7 @@
 // 2..5 read the accumulator back with tcgen05.ld and run the epilogue:
 //   EPI_STORE  out = acc (+ bias[n]) as bf16 or fp32
 //   EPI_SILU   W rows are interleaved (gate_i, up_i): out[m, i] = silu(bf16(gate)) * bf16(up), or the
-//              clamped sigmoid-gated form when `bias` holds its three constants (see silu_mul)
+//              clamped sigmoid-gated form when `bias` holds its three constants (see gated_activation)
 //   EPI_RESID  s = resid + acc (+ bias[n]) in fp32, the new residual stream; beside it
 //              bf16(s * gamma[n]) (the operand of the product behind the next RMS norm) and, per
 //              token, this CTA's share of sum_n s^2
@@ -114,23 +114,6 @@ __device__ __forceinline__ float gamma_at(const GemmExtra& ex, int n) {
   return ex.gamma_f32 ? reinterpret_cast<const float*>(ex.gamma)[n]
                       : __bfloat162float(reinterpret_cast<const bf16*>(ex.gamma)[n]);
 }
-// The gated activation of EPI_SILU.  `act` null: silu(gate) * up.  Else act = {limit, alpha, shift}
-// (the kernel's `bias` argument, which EPI_SILU has no other use for):
-// min(gate, limit) * sigmoid(alpha * min(gate, limit)) * (clamp(up, -limit, limit) + shift).
-__device__ __forceinline__ float silu_mul(float g, float u, const float* __restrict__ act) {
-  float gg = __bfloat162float(__float2bfloat16_rn(g));
-  float uu = __bfloat162float(__float2bfloat16_rn(u));
-  if (act) {
-    const float limit = __ldg(act), alpha = __ldg(act + 1), shift = __ldg(act + 2);
-    gg = fminf(gg, limit);
-    uu = fminf(fmaxf(uu, -limit), limit);
-    // alpha < 0: the gate's sigmoid sharpened to a step (relu)
-    const float sg = alpha < 0.f ? (gg > 0.f ? 1.0f : 0.0f) : 1.0f / (1.0f + expf(-alpha * gg));
-    return gg * sg * (uu + shift);
-  }
-  return gg * (1.0f / (1.0f + expf(-gg))) * uu;
-}
-
 // Epilogue of 16 accumulator columns (tokens m_base .. m_base + 15) of W row n for one thread.
 // `scale`: per-token factors of a deferred normalisation (shared memory, indexed from the tile's
 // first token) or null.  EPI_RESID: sq[j] receives the square of what was stored (0 where nothing).
@@ -180,7 +163,7 @@ __device__ __forceinline__ void epilogue16(float (&v)[16], OUT* __restrict__ out
         const float g = (lane & 1) ? other : v[j], u = (lane & 1) ? v[j] : other;
         const int pair = n >> 1;
         if ((n | 1) < N && m_base + j < M)
-          store_out<OUT>(out + (size_t)(m_base + j) * ldo + pair, silu_mul(g, u, bias));
+          store_out<OUT>(out + (size_t)(m_base + j) * ldo + pair, gated_activation(g, u, bias));
       }
     }
   }
@@ -291,7 +274,7 @@ __device__ __forceinline__ void cluster_reduce(uint32_t red, const float* recv, 
         if (EPI == EPI_SILU) {
           // rows are (gate, up) pairs: two results
           const int pair = n >> 1;
-          const float r0 = silu_mul(v[0], v[1], bias), r1 = silu_mul(v[2], v[3], bias);
+          const float r0 = gated_activation(v[0], v[1], bias), r1 = gated_activation(v[2], v[3], bias);
           OUT* dst = out + (size_t)m * ldo + pair;
           if (n + 1 < N) store_out<OUT>(dst, r0);
           if (n + 3 < N) store_out<OUT>(dst + 1, r1);

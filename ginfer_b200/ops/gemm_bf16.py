@@ -139,6 +139,10 @@ def gemm(x, weight, bias_f32=None, out_dtype=torch.bfloat16, epi: int = 0, split
     out = torch.empty((M, cols), dtype=out_dtype, device=x.device)
     if M == 0:
         return out if resid is None else None
+    if (M <= STREAM_MAX_TOKENS and N * K <= STREAM_MAX_WEIGHTS and split_k is None
+            and not through_workspace and scale is None and resid is None
+            and stream(x, weight, bias_f32, out, epi, act_consts)):
+        return out
     sk = split_k_for(M, N, K) if split_k is None else int(split_k)
     ws = None
     if sk > 1 and through_workspace:
@@ -172,6 +176,32 @@ def gemm(x, weight, bias_f32=None, out_dtype=torch.bfloat16, epi: int = 0, split
         return None
     _ok(rc, "gemm_bf16_tc")
     return out if resid is None else (out, scaled, sumsq)
+
+
+# Up to this many rows of x and weights (14.5 MB: eight warps on each of 148 SMs hold 8 KB each, and half as
+# much again is streamed) the products run on the kernel that has its weights in registers before the
+# kernel ahead is done (csrc/gemm_stream.cu).  Decode steps on a B200 with products of up to 9.7 MB / of
+# up to 14.5 MB / of up to 27 MB on it, none: pimidra m, 2 requests 0.589 / 0.569 / 0.581, 0.610 ms;
+# lasizen m, 4 requests 0.513 / 0.499 / 0.501, 0.509; vilepel m, 4 requests 0.872 / 0.874 / 0.892, 0.960.
+STREAM_MAX_TOKENS = 8
+STREAM_MAX_WEIGHTS = 148 * 8 * 6144
+
+
+def stream(x, weight, bias_f32, out, epi: int = 0, act_consts=None, parts: int = 0) -> bool:
+    """``x [M <= 8, K] @ weight[N, K]^T`` into ``out`` with the epilogues 0, 1, 2 and 4 of
+    :func:`gemm`; ``False`` where the kernel does not take the case.  ``parts``: warps that share a
+    row's reduction (0 picks)."""
+    f = _fn("gemm_stream", "gf_gemm_stream",
+            [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
+             c_float, c_float, c_int, c_void_p])
+    a, b = act_consts or (0.0, 0.0)
+    rc = f(_p(x), x.stride(0), _p(weight), _p(bias_f32), _p(out), out.stride(0), x.shape[0],
+           weight.shape[0], weight.shape[1], int(epi), int(out.dtype == torch.float32), float(a),
+           float(b), int(parts), _stream())
+    if rc == -6:
+        return False
+    _ok(rc, "gemm_stream")
+    return True
 
 
 # The residual epilogue takes the token tiles of decode steps.

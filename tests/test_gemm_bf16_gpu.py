@@ -196,3 +196,41 @@ def test_a_wait_that_runs_out_is_reported_and_the_kernel_returns(M, N, K, split_
     got = gemm_bf16.gemm(x, w, None, torch.bfloat16, split_k=split_k)
     torch.testing.assert_close(got.double(), _ref(x, w), atol=2e-2, rtol=1e-2)
     gemm_bf16.check_errors()
+
+
+@pytest.mark.parametrize("N,K", [(2, 8), (33, 72), (250, 1032), (1001, 264), (2048, 2048), (48, 4096)])
+@pytest.mark.parametrize("M", [1, 3, 8])
+@pytest.mark.parametrize("parts", [0, 1, 2, 4, 8])
+def test_products_with_their_weights_in_registers(M, N, K, parts):
+    """Every split of the reduction, rows and columns that fill no tile, reductions shorter than a step and
+    no multiple of one, rows of x apart, all epilogues: against 64 bits."""
+    from ginfer_b200.ops import gemm_bf16
+    g = torch.Generator(device=DEV).manual_seed(N + K + M)
+    x = torch.randn(M, K + 16, generator=g, device=DEV).bfloat16()[:, 8:8 + K]
+    w = (torch.randn(N, K, generator=g, device=DEV) * K ** -0.5).bfloat16()
+    b = torch.randn(N, generator=g, device=DEV)
+    z = x.double() @ w.double().t()
+    acc = K * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())     # K sums in fp32
+    def run(dtype, epi, bias, cols, consts=None):
+        out = torch.full((M, cols), float("nan"), dtype=dtype, device=DEV)
+        assert gemm_bf16.stream(x, w, bias, out, epi, consts, parts)
+        return out.double()
+    zb = z + b.double()
+    assert ((run(torch.float32, 0, b, N) - zb).abs() <= acc + 2.0 ** -22 * zb.abs()).all()
+    assert ((run(torch.bfloat16, 0, None, N) - z).abs() <= acc + 2.0 ** -8 * (z.abs() + acc)).all()
+    want = zb.relu() ** 2
+    off = (2 * zb.abs() + acc) * (acc + 2.0 ** -22 * zb.abs())
+    assert ((run(torch.float32, 1, b, N) - want).abs() <= off + 2.0 ** -22 * want).all()
+    want = torch.where(z > 0, 0.7 * z * z, 0.3 * (z.expm1() - z)) + z / 2
+    off = (1.4 * z.abs() + 1) * acc + 2.0 ** -20 * (want.abs() + z.abs() + z * z)   # its slope, its own roundings
+    assert ((run(torch.float32, 4, None, N, (0.7, 0.3)) - want).abs() <= off).all()
+    if N % 2 == 0:
+        gt, u = z[:, 0::2], z[:, 1::2]
+        eg, eu = (a.abs() * 2.0 ** -8 + e for a, e in ((gt, acc[:, 0::2]), (u, acc[:, 1::2])))
+        for act in (None, torch.tensor([1e9, 1.0, 0.5], device=DEV)):
+            shift = 0.0 if act is None else 0.5
+            s = gt * torch.sigmoid(gt)
+            off = 1.1 * eg * ((u + shift).abs() + eu) + s.abs() * eu    # silu's slope is at most 1.1
+            want = s * (u + shift)
+            got = run(torch.bfloat16, 2, act, N // 2)
+            assert ((got - want).abs() <= off + 2.0 ** -8 * (want.abs() + off) + 1e-6).all()
