@@ -555,9 +555,13 @@ delta_chunk_coef_kernel(const float* __restrict__ qn, const float* __restrict__ 
 // places of k_i, q_i and k_j.  A warp a (chunk, head): those three for every token, [T, H, D] each, L, M
 // and beta, and the chunk's G_7.  On a B200, 2,251 tokens of four requests, the longest 1,201, 16 heads
 // of 128 x 128: 26 us and 391 us for the recurrence behind it; token by token 736 us.
+// DELTA false: a plain linear attention, S <- diag(g) S + k v^T; its u is v, so there is no L, no beta
+// and no G_i k_i.  ld_q, ld_k, ld_g: floats between two tokens.
+template <bool DELTA>
 __global__ void __launch_bounds__(128)
-delta_chunk_coef_channels_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
-                                 const float* __restrict__ g, const float* __restrict__ beta,
+delta_chunk_coef_channels_kernel(const float* __restrict__ qn, int ld_q, const float* __restrict__ kn,
+                                 int ld_k, const float* __restrict__ g, int ld_g,
+                                 const float* __restrict__ beta,
                                  const int* __restrict__ cu_seqlens, DeltaDims dm,
                                  float* __restrict__ coef, float* __restrict__ total,
                                  float* __restrict__ kg, float* __restrict__ qg, float* __restrict__ ke) {
@@ -567,7 +571,7 @@ delta_chunk_coef_channels_kernel(const float* __restrict__ qn, const float* __re
   const int t0 = cu_seqlens[b], ta = t0 + c * CT, n = min(CT, cu_seqlens[b + 1] - ta);
   if (n <= 0) return;
   const int D = dm.D, H = dm.H, kvh = h / (H / dm.G);
-  const size_t GD = (size_t)dm.G * D, HD = (size_t)H * D;
+  const size_t HD = (size_t)H * D;
   const size_t chunk = (size_t)chunk_number(t0, b, c) * H + h;
   float val[64];                                             // pairs as above
 #pragma unroll
@@ -579,10 +583,10 @@ delta_chunk_coef_channels_kernel(const float* __restrict__ qn, const float* __re
 #pragma unroll
       for (int x = 0; x < 4; ++x) k[i][x] = q[i][x] = 0.f, gd[i][x] = 1.f;
       if (i < n) {
-        const size_t at = (size_t)(ta + i) * GD + (size_t)kvh * D + d;
-        Quad<float>::load(kn + at, k[i]);
-        Quad<float>::load(qn + at, q[i]);
-        Quad<float>::load(g + (size_t)(ta + i) * HD + (size_t)h * D + d, gd[i]);
+        const size_t r = ta + i;
+        Quad<float>::load(kn + r * ld_k + (size_t)kvh * D + d, k[i]);
+        Quad<float>::load(qn + r * ld_q + (size_t)kvh * D + d, q[i]);
+        Quad<float>::load(g + r * ld_g + (size_t)h * D + d, gd[i]);
       }
     }
 #pragma unroll
@@ -595,7 +599,7 @@ delta_chunk_coef_channels_kernel(const float* __restrict__ qn, const float* __re
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
           kr[x] *= gd[i][x];
-          val[8 * i + j] = fmaf(kr[x], k[i][x], val[8 * i + j]);
+          if (DELTA) val[8 * i + j] = fmaf(kr[x], k[i][x], val[8 * i + j]);
           val[8 * j + i] = fmaf(kr[x], q[i][x], val[8 * j + i]);
         }
       if (j < n) Quad<float>::store(ke + (size_t)(ta + j) * HD + (size_t)h * D + d, kr);
@@ -608,7 +612,7 @@ delta_chunk_coef_channels_kernel(const float* __restrict__ qn, const float* __re
       for (int x = 0; x < 4; ++x) G[x] *= gd[i][x], a[x] = G[x] * k[i][x], e[x] = G[x] * q[i][x];
       if (i < n) {
         const size_t at = (size_t)(ta + i) * HD + (size_t)h * D + d;
-        Quad<float>::store(kg + at, a);
+        if (DELTA) Quad<float>::store(kg + at, a);
         Quad<float>::store(qg + at, e);
       }
     }
@@ -627,7 +631,7 @@ delta_chunk_coef_channels_kernel(const float* __restrict__ qn, const float* __re
       }
   }
   const float mine[2] = {val[0], val[32]};
-  const float bl = lane < n ? beta[(size_t)(ta + lane) * H + h] : 0.f;
+  const float bl = DELTA && lane < n ? beta[(size_t)(ta + lane) * H + h] : 0.f;
   float* dst = coef + chunk * kCoefs;
 #pragma unroll
   for (int x = 0; x < 2; ++x) {
@@ -649,18 +653,23 @@ delta_chunk_coef_channels_kernel(const float* __restrict__ qn, const float* __re
 // there are blocks enough without).  Lane p of a column owns
 // the rows 4 (p + LANES i) .. + 3, i < DPER / 4, so that the lanes' reads of a token's k and q are one run of
 // shared memory.  Stages as in the kernel above, one barrier a chunk.
-// CHANNELS: a decay a key channel; kn, qn and ke are [T, H, D] as delta_chunk_coef_channels_kernel leaves
-// them, total the chunks' G_7.  With a decay a head ke and total are not read.
-template <int DPER, int LANES, int CP, bool CHANNELS>
+// HEADS: the delta rule with a decay a head; ke and total are not read.  CHANNELS: a decay a key channel;
+// kn, qn and ke are [T, H, D] as delta_chunk_coef_channels_kernel leaves them, total the chunks' G_7.
+// PLAIN: the same without the delta rule (u = v; kn is not read; eight lanes a column).
+enum { HEADS = 0, CHANNELS = 1, PLAIN = 2 };
+template <int DPER, int LANES, int CP, int MODE>
 __global__ void __launch_bounds__(16 * LANES)
 delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
                               const float* __restrict__ ke, const float* __restrict__ total,
-                              const float* __restrict__ v, const float* __restrict__ coef,
+                              const float* __restrict__ v, int ld_v, const float* __restrict__ coef,
                               float* __restrict__ state, const int* __restrict__ cu_seqlens,
                               const int* __restrict__ slot_ids, DeltaDims dm, float* __restrict__ o) {
   constexpr int Dp = LANES * DPER, COLS = 16 * CP, NQ = DPER / 4;
-  constexpr int kQ = CT * Dp, kE = CHANNELS ? 2 * CT * Dp : 0, kG = (CHANNELS ? 3 : 2) * CT * Dp;
-  constexpr int kVc = kG + (CHANNELS ? Dp : 0), kC = kVc + CT * COLS, kStage = kC + kCoefs;
+  static_assert(MODE != PLAIN || LANES == CT, "a lane a token of a chunk");
+  constexpr int SETS = MODE == CHANNELS ? 3 : 2;               // [CT][Dp] each: k | q, k | q | ke, or q | ke
+  constexpr int kQ = MODE == PLAIN ? 0 : CT * Dp, kE = MODE == HEADS ? 0 : kQ + CT * Dp, kG = SETS * CT * Dp;
+  constexpr int kVc = kG + (MODE == HEADS ? 0 : Dp), kC = kVc + CT * COLS, kStage = kC + kCoefs;
+  constexpr int DOTS = MODE == PLAIN ? CT : 2 * CT;            // with S: the chunk's q, and k in front of them
   extern __shared__ __align__(16) float stage[];               // [kStages][kStage]
   const int b = blockIdx.x / dm.H, h = blockIdx.x - b * dm.H;
   const int p = threadIdx.x % LANES, lc = threadIdx.x / LANES;
@@ -670,7 +679,7 @@ delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restr
   for (int i = threadIdx.x; i < kStages * kStage; i += blockDim.x) stage[i] = 0.f;
   __syncthreads();
   pdl_wait();
-  const int kvh = CHANNELS ? h : h / (dm.H / dm.G);
+  const int kvh = MODE == HEADS ? h / (dm.H / dm.G) : h;
   float* Sg = state + (size_t)slot_ids[b] * dm.state_stride + ((size_t)h * D) * Vd;
   float S[CP][NQ][4];
 #pragma unroll
@@ -683,7 +692,7 @@ delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restr
         S[y][i][x] = row < D ? Sg[(size_t)row * Vd + (col < Vd ? col : 0)] : 0.f;
       }
   const int t0 = cu_seqlens[b], t1 = cu_seqlens[b + 1];
-  const size_t KD = (size_t)(CHANNELS ? dm.H : dm.G) * D, HV = (size_t)dm.H * Vd;
+  const size_t KD = (size_t)(MODE == HEADS ? dm.G : dm.H) * D, HV = (size_t)dm.H * Vd;
   const int vq = min(COLS, Vd - col0) >> 2, dq = D >> 2;
   const int nchunks = (t1 - t0 + CT - 1) / CT;
   const int chunk0 = chunk_number(t0, b, 0);
@@ -697,16 +706,16 @@ delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restr
     for (int e = threadIdx.x; e < n * dq; e += blockDim.x) {
       const int t = e / dq, d = 4 * (e - t * dq);
       const size_t at = (size_t)(ta + t) * KD + (size_t)kvh * D + d;
-      copy16(st + t * Dp + d, kn + at);
+      if (MODE != PLAIN) copy16(st + t * Dp + d, kn + at);
       copy16(st + kQ + t * Dp + d, qn + at);
-      if (CHANNELS) copy16(st + kE + t * Dp + d, ke + at);
+      if (MODE != HEADS) copy16(st + kE + t * Dp + d, ke + at);
     }
-    if (CHANNELS)
+    if (MODE != HEADS)
       for (int e = threadIdx.x; e < dq; e += blockDim.x)
         copy16(st + kG + 4 * e, total + ((size_t)(chunk0 + c) * dm.H + h) * D + 4 * e);
     for (int e = threadIdx.x; e < n * vq; e += blockDim.x) {
       const int t = e / vq, d = 4 * (e - t * vq);
-      copy16(st + kVc + t * COLS + d, v + (size_t)(ta + t) * HV + (size_t)h * Vd + col0 + d);
+      copy16(st + kVc + t * COLS + d, v + (size_t)(ta + t) * ld_v + (size_t)h * Vd + col0 + d);
     }
     for (int e = threadIdx.x; e < kCoefs / 4; e += blockDim.x)
       copy16(st + kC + 4 * e, coef0 + (size_t)c * dm.H * kCoefs + 4 * e);
@@ -722,17 +731,17 @@ delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restr
     copy_async_commit();
     const float* st = stage + (size_t)(c % kStages) * kStage;
     const float* cf = st + kC;
-    // this lane's share of S^T k_i (x[i]) and S^T q_i (x[8 + i])
-    float x[CP][2 * CT];
+    // this lane's share of S^T k_i (x[i]) and S^T q_i (x[8 + i]; PLAIN: x[i])
+    float x[CP][DOTS];
 #pragma unroll
     for (int y = 0; y < CP; ++y)
 #pragma unroll
-      for (int i = 0; i < 2 * CT; ++i) x[y][i] = 0.f;
+      for (int i = 0; i < DOTS; ++i) x[y][i] = 0.f;
 #pragma unroll
     for (int i = 0; i < NQ; ++i) {
       const float* at = st + 4 * (p + LANES * i);
 #pragma unroll
-      for (int t = 0; t < 2 * CT; ++t) {
+      for (int t = 0; t < DOTS; ++t) {
         const float4 a = *reinterpret_cast<const float4*>(at + t * Dp);
 #pragma unroll
         for (int y = 0; y < CP; ++y) {
@@ -749,7 +758,7 @@ delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restr
 #pragma unroll
       for (int y = 0; y < CP; ++y)
 #pragma unroll
-        for (int hi = 0; hi < 2 * CT / LANES; ++hi)
+        for (int hi = 0; hi < DOTS / LANES; ++hi)
 #pragma unroll
           for (int m = 0; m < half; ++m) {
             const float lo_v = x[y][LANES * hi + m], hi_v = x[y][LANES * hi + m + half];
@@ -758,8 +767,15 @@ delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restr
           }
     }
     const int tok = p % CT;                                     // the token this lane looks after
-    const float Gp = CHANNELS ? 1.f : cf[kCoefG + tok];
+    const float Gp = MODE == HEADS ? cf[kCoefG + tok] : 1.f;
     float u[CP][CT];
+    if constexpr (MODE == PLAIN) {
+      const int n = t1 - t0 - c * CT;                           // (what lies behind the end is an older chunk's)
+#pragma unroll
+      for (int y = 0; y < CP; ++y)
+#pragma unroll
+        for (int i = 0; i < CT; ++i) u[y][i] = i < n ? st[kVc + i * COLS + lc + 16 * y] : 0.f;
+    } else {
 #pragma unroll
     for (int y = 0; y < CP; ++y) {
       const float rp = cf[kCoefBeta + tok] * (st[kVc + tok * COLS + lc + 16 * y] - Gp * x[y][0]);
@@ -774,6 +790,7 @@ delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restr
 #pragma unroll
         for (int y = 0; y < CP; ++y) u[y][i] = fmaf(l, u[y][j], u[y][i]);
       }
+    }
     {
       const float4* Mp = reinterpret_cast<const float4*>(cf + kCoefM + tok * CT);
       const float4 m0 = Mp[0], m1 = Mp[1];
@@ -781,15 +798,15 @@ delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restr
 #pragma unroll
       for (int y = 0; y < CP; ++y) {
         const float(&w)[CT] = u[y];
-        float out = Gp * (LANES == CT ? x[y][CT] : x[y][0]);
+        float out = Gp * x[y][LANES == CT && MODE != PLAIN ? CT : 0];
         out = fmaf(m0.x, w[0], fmaf(m0.y, w[1], fmaf(m0.z, w[2], fmaf(m0.w, w[3], out))));
         out = fmaf(m1.x, w[4], fmaf(m1.y, w[5], fmaf(m1.z, w[6], fmaf(m1.w, w[7], out))));
         const int col = col0 + lc + 16 * y;
         if (col < Vd && row < t1 && p >= LANES - CT) o[(size_t)row * HV + (size_t)h * Vd + col] = out;
       }
     }
-    const float Gc = CHANNELS ? 1.f : cf[kCoefG + CT - 1];
-    if (!CHANNELS)
+    const float Gc = MODE == HEADS ? cf[kCoefG + CT - 1] : 1.f;
+    if (MODE == HEADS)
 #pragma unroll
       for (int j = 0; j < CT; ++j) {
         const float e = cf[kCoefE + j];
@@ -800,7 +817,7 @@ delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restr
     for (int i = 0; i < NQ; ++i) {
       const float* at = st + kE + 4 * (p + LANES * i);
       float4 g4 = make_float4(Gc, Gc, Gc, Gc);
-      if (CHANNELS) g4 = *reinterpret_cast<const float4*>(st + kG + 4 * (p + LANES * i));
+      if (MODE != HEADS) g4 = *reinterpret_cast<const float4*>(st + kG + 4 * (p + LANES * i));
 #pragma unroll
       for (int y = 0; y < CP; ++y)
         S[y][i][0] *= g4.x, S[y][i][1] *= g4.y, S[y][i][2] *= g4.z, S[y][i][3] *= g4.w;
@@ -828,31 +845,38 @@ delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restr
       }
 }
 
-template <int DPER, int LANES, int CP, bool CHANNELS>
-static int launch_chunk_columns(const float* qn, const float* kn, const float* ke, const float* total,
-                                const float* v, const float* coef, float* state, const int* cu_seqlens,
-                                const int* slot_ids, int B, const DeltaDims& dm, float* o,
-                                cudaStream_t st) {
+struct ChunkArgs {
+  const float *q, *k, *ke, *total, *v;
+  int ld_v;
+  const float* coef;
+  float* state;
+  const int *cu_seqlens, *slot_ids;
+  float* o;
+};
+
+template <int DPER, int LANES, int CP, int MODE>
+static int launch_chunk_columns(int B, const DeltaDims& dm, const ChunkArgs& a, cudaStream_t st) {
   const size_t smem = (size_t)kStages * sizeof(float) *
-                      ((CHANNELS ? 3 * CT + 1 : 2 * CT) * LANES * DPER + CT * 16 * CP + kCoefs);
+                      (((MODE == CHANNELS ? 3 : 2) * CT + (MODE == HEADS ? 0 : 1)) * LANES * DPER +
+                       CT * 16 * CP + kCoefs);
   static OncePerDevice attrs;
   if (int rc = attrs.run([&] {
-        return cudaFuncSetAttribute(delta_chunk_recurrence_kernel<DPER, LANES, CP, CHANNELS>,
+        return cudaFuncSetAttribute(delta_chunk_recurrence_kernel<DPER, LANES, CP, MODE>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       }))
     return rc;
-  return launch_kernel(delta_chunk_recurrence_kernel<DPER, LANES, CP, CHANNELS>,
-                       dim3(B * dm.H, (dm.Vd + 16 * CP - 1) / (16 * CP)), dim3(16 * LANES), smem, st, qn,
-                       kn, ke, total, v, coef, state, cu_seqlens, slot_ids, dm, o);
+  return launch_kernel(delta_chunk_recurrence_kernel<DPER, LANES, CP, MODE>,
+                       dim3(B * dm.H, (dm.Vd + 16 * CP - 1) / (16 * CP)), dim3(16 * LANES), smem, st, a.q,
+                       a.k, a.ke, a.total, a.v, a.ld_v, a.coef, a.state, a.cu_seqlens, a.slot_ids, dm, a.o);
 }
 
-template <int DPER, int LANES, bool CHANNELS, typename... Args>
-static int launch_chunks(int B, const DeltaDims& dm, float* o, cudaStream_t st, Args... args) {
+template <int DPER, int LANES, int MODE>
+static int launch_chunks(int B, const DeltaDims& dm, const ChunkArgs& a, cudaStream_t st) {
   // two blocks an SM of 16 columns: then one of 32 each does the same work with half the reads (512
   // blocks of 16 columns 434 us, 256 of 32 391)
   if (LANES * DPER <= 128 && (long long)B * dm.H * ((dm.Vd + 15) / 16) >= 2 * 148 && dm.Vd > 16)
-    return launch_chunk_columns<DPER, LANES, LANES * DPER <= 128 ? 2 : 1, CHANNELS>(args..., B, dm, o, st);
-  return launch_chunk_columns<DPER, LANES, 1, CHANNELS>(args..., B, dm, o, st);
+    return launch_chunk_columns<DPER, LANES, LANES * DPER <= 128 ? 2 : 1, MODE>(B, dm, a, st);
+  return launch_chunk_columns<DPER, LANES, 1, MODE>(B, dm, a, st);
 }
 
 template <typename T>
@@ -990,20 +1014,18 @@ GF_EXPORT int gf_delta_recurrence(const float* qn, const float* kn, const float*
     const size_t chunks = (size_t)(T / CT + B + 1) * H, HTD = (size_t)T * H * D;
     float* total = scratch + chunks * kCoefs;
     float *kg = total + chunks * D, *qg = kg + HTD, *ke = qg + HTD;      // (a decay a channel only)
-    const int rc = one_decay ? launch_kernel(delta_chunk_coef_kernel, cgrid, dim3(128), 0, st, qn, kn, g,
-                                             beta, cu_seqlens, dm, scratch)
-                             : launch_kernel(delta_chunk_coef_channels_kernel, cgrid, dim3(128), 0, st, qn,
-                                             kn, g, beta, cu_seqlens, dm, scratch, total, kg, qg, ke);
+    const int rc =
+        one_decay ? launch_kernel(delta_chunk_coef_kernel, cgrid, dim3(128), 0, st, qn, kn, g, beta,
+                                  cu_seqlens, dm, scratch)
+                  : launch_kernel(delta_chunk_coef_channels_kernel<true>, cgrid, dim3(128), 0, st, qn, G * D,
+                                  kn, G * D, g, H * D, beta, cu_seqlens, dm, scratch, total, kg, qg, ke);
     if (rc) return rc;
+    const ChunkArgs a{one_decay ? qn : qg, one_decay ? kn : kg, ke, total, v, H * Vd, scratch, state,
+                      cu_seqlens, slot_ids, o};
 #define GF_GO(DPER, LANES)                                                                         \
-  if (D <= DPER * LANES) {                                                                         \
-    if (one_decay)                                                                                 \
-      return launch_chunks<DPER, LANES, false>(B, dm, o, st, qn, kn, (const float*)nullptr,        \
-                                               (const float*)nullptr, v, scratch, state,           \
-                                               cu_seqlens, slot_ids);                              \
-    return launch_chunks<DPER, LANES, true>(B, dm, o, st, qg, kg, ke, total, v, scratch, state,    \
-                                            cu_seqlens, slot_ids);                                 \
-  }
+  if (D <= DPER * LANES)                                                                           \
+    return one_decay ? launch_chunks<DPER, LANES, HEADS>(B, dm, a, st)                             \
+                     : launch_chunks<DPER, LANES, CHANNELS>(B, dm, a, st);
     GF_GO(4, 8)
     GF_GO(8, 8)
     GF_GO(16, 8)             // (sixteen lanes of 8 rows: 348 us for a prompt that takes 317 so)
@@ -1042,6 +1064,35 @@ GF_EXPORT int gf_delta_recurrence(const float* qn, const float* kn, const float*
 #undef GF_GO
 #undef GF_AS
   return -3;
+}
+
+// A plain linear attention with a decay a key channel, S <- diag(g) S + k v^T, o = S^T q, eight tokens at a
+// time.  Rows of q, k (G heads of D), v (H of Vd) and g (H of D) are ld_* floats apart; scratch:
+// gf_delta_chunk_words with one_decay 0; o [T, H, Vd].  Returns -6 for what it does not take (key sizes over
+// 128, sizes or rows that are no multiples of four).
+GF_EXPORT int gf_decay_channels_chunked(const float* q, int ld_q, const float* k, int ld_k, const float* v,
+                                        int ld_v, const float* g, int ld_g, float* state, int state_stride,
+                                        const int* cu_seqlens, const int* slot_ids, int T, int B, int H,
+                                        int G, int D, int Vd, float* o, float* scratch, int max_q_len,
+                                        void* stream) {
+  if (B <= 0) return 0;
+  if (H % G || D > 128 || D % 4 || Vd % 4 || ld_q % 4 || ld_k % 4 || ld_v % 4 || ld_g % 4 || B > 65535 ||
+      H > 65535 ||
+      (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)g | (uintptr_t)scratch) & 15))
+    return -6;
+  const DeltaDims dm = dims_of(H, G, D, Vd, 1, state_stride, 0);
+  auto st = (cudaStream_t)stream;
+  const size_t chunks = (size_t)(T / CT + B + 1) * H, HTD = (size_t)T * H * D;
+  float *total = scratch + chunks * kCoefs, *qg = total + chunks * D, *ke = qg + HTD;
+  if (int rc = launch_kernel(delta_chunk_coef_channels_kernel<false>,
+                             dim3(((max_q_len + CT - 1) / CT + 3) / 4, B, H), dim3(128), 0, st, q, ld_q, k,
+                             ld_k, g, ld_g, (const float*)nullptr, cu_seqlens, dm, scratch, total,
+                             (float*)nullptr, qg, ke))
+    return rc;
+  const ChunkArgs a{qg, nullptr, ke, total, v, ld_v, scratch, state, cu_seqlens, slot_ids, o};
+  if (D <= 32) return launch_chunks<4, 8, PLAIN>(B, dm, a, st);
+  if (D <= 64) return launch_chunks<8, 8, PLAIN>(B, dm, a, st);
+  return launch_chunks<16, 8, PLAIN>(B, dm, a, st);
 }
 
 GF_EXPORT int gf_delta_output(const float* o, const void* gate, int gate_ld, const float* w,

@@ -83,13 +83,14 @@ def prepare_heads(proj: torch.Tensor, a_off: int, b_off: int, conv_w: torch.Tens
     return qn, kn, v, g, beta
 
 
-def _fn_words():
+def chunk_words(T: int, B: int, H: int, D: int, one_decay: int) -> int:
+    """fp32 words of scratch with which a step goes eight tokens at a time."""
     from ctypes import c_longlong
 
     from .build import load_library
     f = load_library("delta_rule").gf_delta_chunk_words
     f.argtypes, f.restype = [c_int] * 5, c_longlong
-    return f
+    return int(f(T, B, H, D, one_decay))
 
 
 def recurrence(qn, kn, v, g, beta, state: torch.Tensor, ctx) -> torch.Tensor:
@@ -105,8 +106,8 @@ def recurrence(qn, kn, v, g, beta, state: torch.Tensor, ctx) -> torch.Tensor:
     # (a context that does not say how long its portions are: token by token)
     scratch, longest = None, int(getattr(ctx, "max_q_len", 0))
     if longest >= CHUNKED_MIN_TOKENS:
-        words = _fn_words()(T, ctx.num_seqs, H, D, one)
-        scratch = torch.empty(words, dtype=torch.float32, device=qn.device)
+        scratch = torch.empty(chunk_words(T, ctx.num_seqs, H, D, one), dtype=torch.float32,
+                              device=qn.device)
     rc = f(_p(qn), _p(kn), _p(v), _p(g), _p(beta), _p(state), _p(ctx.cu_seqlens_q),
            _p(ctx.slot_ids), T, ctx.num_seqs, H, G, D, Vd, state.stride(0), _p(o), one,
            _p(scratch), longest, _stream())

@@ -611,3 +611,41 @@ def test_zero_slots_clears_the_named_slots_of_every_state(slots):
         want = torch.ones(n, dtype=torch.bool, device=DEV)
         want[slots] = False
         assert torch.equal((t == 1).all(dim=1), want) and torch.equal((t == 0).all(dim=1), ~want)
+
+
+@pytest.mark.parametrize("H,G,D,Vd,lens", [(2, 1, 12, 20, [64, 1, 7]), (4, 2, 64, 64, [80, 8, 9]),
+                                           (2, 2, 128, 128, [66, 17]), (3, 3, 100, 36, [24, 65, 1]),
+                                           (16, 16, 128, 48, [64, 3, 9, 70, 8, 1, 65, 64]), (1, 1, 32, 4, [71])])
+def test_linear_attention_with_channel_decays_eight_tokens_at_a_time(H, G, D, Vd, lens):
+    """Rows of a wider projection, chunks whole and cut, one and two columns a lane, decays from none to all
+    gone: outputs and states against the recurrence token by token in 64 bits."""
+    from types import SimpleNamespace
+    from ginfer_b200.ops import decay
+    g0 = torch.Generator().manual_seed(D + Vd)
+    B, T = len(lens), sum(lens)
+    q, k = torch.randn(T, G, D, generator=g0) / D ** 0.5, torch.randn(T, G, D, generator=g0) / D ** 0.5
+    v, g = torch.randn(T, H, Vd, generator=g0), torch.rand(T, H, D, generator=g0)
+    g[:, :, ::3] = 1.0 - g[:, :, ::3] * 0.01
+    g[T // 2, :, 1::4] = 1e-30
+    state0 = torch.randn(B + 2, H * D * Vd + 8, generator=g0)
+    cu = torch.tensor([0] + lens).cumsum(0)
+    slots = torch.randperm(B + 2, generator=g0)[:B]
+    wide = torch.cat([q.reshape(T, -1), k.reshape(T, -1), v.reshape(T, -1), torch.ones(T, 4)], 1).cuda()
+    qd, kd, vd = wide[:, :G * D], wide[:, G * D:2 * G * D], wide[:, 2 * G * D:2 * G * D + H * Vd]
+    state = state0.clone().cuda()
+    ctx = SimpleNamespace(num_seqs=B, slot_ids=slots.int().cuda(), cu_seqlens_q=cu.int().cuda(),
+                          max_q_len=max(lens), q_lens_host=lens)
+    o = decay.recurrence(qd, kd, vd, g.reshape(T, -1).cuda(), state, ctx, H, G, D, Vd)
+    o, state = o.cpu().double().reshape(T, H, Vd), state.cpu()
+    err, kv = 0.0, torch.arange(H) // (H // G)
+    for b in range(B):
+        S = state0[slots[b], :H * D * Vd].double().reshape(H, D, Vd).clone()
+        for t in range(int(cu[b]), int(cu[b + 1])):
+            S = g[t].double()[:, :, None] * S + k[t, kv].double()[:, :, None] * v[t].double()[:, None]
+            err = max(err, float((o[t] - torch.einsum("hdv,hd->hv", S, q[t, kv].double())).abs().max()))
+        err = max(err, float((state[slots[b], :H * D * Vd].double() - S.reshape(-1)).abs().max()))
+        assert torch.equal(state[slots[b], H * D * Vd:], state0[slots[b], H * D * Vd:])
+    # values of a few units (a state holds some 200 terms of at most one), fp32 sums of at most 128 of them
+    assert err <= 2e-5, err
+    rest = [s for s in range(B + 2) if s not in slots.tolist()]
+    assert torch.equal(state[rest], state0[rest])
