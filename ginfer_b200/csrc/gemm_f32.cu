@@ -6,7 +6,7 @@
 // The order of every sum is fixed by N and K alone, so a row's result does not depend on what else is
 // in the batch, nor on which of the two kernels below computes it: K is cut into 2, 4 or 8 segments, a
 // segment is two chains of FMAs in ascending k (even and odd k) and their sum, and the segments are
-// added in ascending order.  The two chains are the halves of fma.rn.f32x2: one FMA an instruction
+// added in pairs, pairs of pairs, and so on.  The two chains are the halves of fma.rn.f32x2: one FMA an instruction
 // leaves the pipes of an sm_100 SM at half their rate (37 TFLOP/s at 148 SMs), and pairs of
 // neighbouring k are what a 16-byte load of either operand holds.
 //
@@ -154,13 +154,14 @@ gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W,
   cg::cluster_group cluster = cg::this_cluster();
   cluster.sync();
   for (int m = rank; m < M; m += ranks) {
-    float v = 0.f;
-    for (int r = 0; r < ranks; ++r) {
-      const float* part = cluster.map_shared_rank(&sm.sum[0][m][lane], r);
-      v += part[0];
-      v += part[MT * 32];
-    }
-    if (n < N) C[(size_t)m * ldc + n] = v + add;
+    float p[4] = {0.f, 0.f, 0.f, 0.f};                    // (adding the zeros of ranks that are not there is exact)
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      if (r < ranks) {
+        const float* part = cluster.map_shared_rank(&sm.sum[0][m][lane], r);
+        p[r] = part[0] + part[MT * 32];
+      }
+    if (n < N) C[(size_t)m * ldc + n] = ((p[0] + p[1]) + (p[2] + p[3])) + add;
   }
   cluster.sync();                                         // nobody leaves while its sums are read
 }
@@ -250,8 +251,11 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W,
   for (int e = tid; e < rows * BN; e += THREADS) {
     const int r = rank * rows + e / BN, m = m0 + r, n = n0 + e % BN;
     if (m >= M || n >= N) continue;
-    float v = 0.f;
-    for (int s = 0; s < ranks; ++s) v += *cluster.map_shared_rank(ring + r * OP + e % BN, s);
+    float p[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int s = 0; s < 8; ++s)
+      if (s < ranks) p[s] = *cluster.map_shared_rank(ring + r * OP + e % BN, s);
+    const float v = ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7]));
     C[(size_t)m * ldc + n] = v + (bias ? bias[n] : 0.f);
   }
   cluster.sync();
