@@ -649,3 +649,27 @@ def test_linear_attention_with_channel_decays_eight_tokens_at_a_time(H, G, D, Vd
     assert err <= 2e-5, err
     rest = [s for s in range(B + 2) if s not in slots.tolist()]
     assert torch.equal(state[rest], state0[rest])
+
+
+@pytest.mark.parametrize("C", [16, 48, 80, 512])
+@pytest.mark.parametrize("lens", [[600], [700, 3, 64], [1000, 520, 1, 65]])
+def test_shares_of_a_tokens_keys_are_put_together(C, lens):
+    """Latent attention of few tokens over many keys in several shares, some of them empty, latent sizes that
+    fill no warp: against 64 bits."""
+    from types import SimpleNamespace
+    from ginfer_b200.ops import latent
+    B, H, page = len(lens), 5, 16
+    assert latent.key_splits(B, H, max(lens)) > 1
+    g = torch.Generator(device=DEV).manual_seed(C + B)
+    W = -(-max(lens) // page)
+    pages = torch.randn(B * W, page, 1, C, generator=g, device=DEV).bfloat16()
+    table = torch.randperm(B * W, generator=g, device=DEV).int().view(B, W)
+    q = torch.randn(H, B, C, generator=g, device=DEV).bfloat16().float()      # (the kernel rounds q to bf16)
+    ctx = SimpleNamespace(seq_of_token=torch.arange(B, dtype=torch.int32, device=DEV), max_kv_len=max(lens),
+                          positions=torch.tensor([n - 1 for n in lens], dtype=torch.int32, device=DEV))
+    out = latent.attention(q, None, pages, None, table, ctx, 0, C ** -0.5, page).double()
+    for b, n in enumerate(lens):
+        c = pages[table[b].long()].reshape(-1, C)[:n].double()
+        p = torch.softmax(q[:, b].double() @ c.t() * C ** -0.5, dim=-1)
+        # probabilities and result are rounded to bf16: 2^-8 each, of at most sum p |c|
+        assert ((out[:, b] - p @ c).abs() <= 2 * 2.0 ** -8 * (p @ c.abs()) + 1e-6).all()
