@@ -149,6 +149,9 @@ def recurrence(q, k, v, g, state: torch.Tensor, ctx, H: int, G: int, D: int, Vd:
     assert state.dtype == torch.float32 and state.dim() == 2 and state.is_contiguous()
     o = torch.empty((T, H * Vd), dtype=torch.float32, device=v.device)
     o_n = None if normaliser is None else torch.empty((T, H), dtype=torch.float32, device=v.device)
+    if (ctx.max_q_len == 1 and o_n is None
+            and delta.state_step(q, k, v, g, state, ctx, H, G, D, Vd, o, c=k_scale, skip=skip)):
+        return o
     # long portions with one decay a head go a chunk at a time; single tokens in front of them (as the
     # scheduler orders a mixed step) token by token
     seqs, q_lens = ctx.num_seqs, getattr(ctx, "q_lens_host", ())

@@ -83,6 +83,24 @@ def prepare_heads(proj: torch.Tensor, a_off: int, b_off: int, conv_w: torch.Tens
     return qn, kn, v, g, beta
 
 
+def state_step(q, k, v, g, state, ctx, H: int, G: int, D: int, Vd: int, o, c=None, skip=None,
+               beta=None) -> bool:
+    """One token of every request (``csrc/state_step.cu``): rows of ``q``, ``k`` (``G D``), ``v``, ``o``
+    (``H Vd``), ``g`` (``H`` or ``H D``) and ``c`` (``H``), all fp32 with a row stride; with ``beta [T, H]``
+    the delta rule, else ``S <- g S + c k v^T``.  ``False`` where the kernel does not take the case."""
+    f = _fn("state_step", "gf_state_step",
+            [c_void_p, c_int] * 4 + [c_int, c_void_p, c_int] + [c_void_p] * 3 + [c_int, c_void_p, c_void_p] +
+            [c_int] * 5 + [c_void_p, c_int, c_void_p])
+    rc = f(_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(g), g.stride(0),
+           g.shape[1] // H, _p(c), c.stride(0) if c is not None else 0, _p(skip), _p(beta), _p(state),
+           state.stride(0), _p(ctx.cu_seqlens_q), _p(ctx.slot_ids), ctx.num_seqs, H, G, D, Vd, _p(o),
+           o.stride(0), _stream())
+    if rc == -6:
+        return False
+    _ok(rc, "state_step")
+    return True
+
+
 def chunk_words(T: int, B: int, H: int, D: int, one_decay: int) -> int:
     """fp32 words of scratch with which a step goes eight tokens at a time."""
     from ctypes import c_longlong
@@ -105,6 +123,9 @@ def recurrence(qn, kn, v, g, beta, state: torch.Tensor, ctx) -> torch.Tensor:
     one = int(g.dim() == 2)
     # (a context that does not say how long its portions are: token by token)
     scratch, longest = None, int(getattr(ctx, "max_q_len", 0))
+    if longest == 1 and state_step(qn.view(T, G * D), kn.view(T, G * D), v.view(T, H * Vd), g.view(T, -1),
+                                   state, ctx, H, G, D, Vd, o.view(T, H * Vd), beta=beta):
+        return o
     if longest >= CHUNKED_MIN_TOKENS:
         scratch = torch.empty(chunk_words(T, ctx.num_seqs, H, D, one), dtype=torch.float32,
                               device=qn.device)

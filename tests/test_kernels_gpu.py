@@ -673,3 +673,49 @@ def test_shares_of_a_tokens_keys_are_put_together(C, lens):
         p = torch.softmax(q[:, b].double() @ c.t() * C ** -0.5, dim=-1)
         # probabilities and result are rounded to bf16: 2^-8 each, of at most sum p |c|
         assert ((out[:, b] - p @ c).abs() <= 2 * 2.0 ** -8 * (p @ c.abs()) + 1e-6).all()
+
+
+@pytest.mark.parametrize("H,G,D,Vd,B", [(2, 1, 12, 20, 3), (4, 2, 64, 64, 1), (16, 16, 128, 128, 5), (3, 3, 100, 36, 2),
+                                        (2, 1, 256, 48, 2), (1, 1, 200, 132, 1), (2, 2, 130, 8, 2), (64, 1, 128, 64, 2)])
+@pytest.mark.parametrize("channels", [False, True])
+@pytest.mark.parametrize("rule", ["delta", "linear", "scaled"])
+def test_one_token_of_every_request_through_its_state(H, G, D, Vd, B, channels, rule):
+    """Rows and columns that fill no block, keys of every size class, operands as columns of a wider row, a
+    decay a head and a channel: against 64 bits; slots that are not named stay."""
+    from types import SimpleNamespace
+    from ginfer_b200.ops import delta
+    g0 = torch.Generator(device=DEV).manual_seed(D + Vd + B)
+    def rnd(*shape):
+        return torch.randn(*shape, generator=g0, device=DEV)
+    wide = rnd(B, 2 * G * D + H * Vd + 8)
+    q, k = wide[:, :G * D], wide[:, G * D:2 * G * D]
+    wide[:, :2 * G * D] *= D ** -0.5
+    v = wide[:, 2 * G * D:2 * G * D + H * Vd] if G * D % 2 == 0 and wide.shape[1] % 4 == 0 else rnd(B, H * Vd)
+    g = torch.rand(B, H * D if channels else H, generator=g0, device=DEV)
+    beta, c, skip = torch.rand(B, H, generator=g0, device=DEV), rnd(B, H), rnd(H)
+    state0 = rnd(B + 2, H * D * Vd + 8)
+    slots = torch.randperm(B + 2, generator=g0, device=DEV)[:B]
+    state, o = state0.clone(), torch.empty(B, H * Vd, device=DEV)
+    ctx = SimpleNamespace(num_seqs=B, slot_ids=slots.int(),
+                          cu_seqlens_q=torch.arange(B + 1, dtype=torch.int32, device=DEV))
+    kw = dict(beta=beta) if rule == "delta" else dict(c=c, skip=skip) if rule == "scaled" else {}
+    assert delta.state_step(q, k, v, g, state, ctx, H, G, D, Vd, o, **kw)
+    kv = torch.arange(H, device=DEV) // (H // G)
+    qd, kd = (t.double().reshape(B, G, D)[:, kv] for t in (q, k))
+    vd, S = v.double().reshape(B, H, Vd), state0[slots, :H * D * Vd].double().reshape(B, H, D, Vd)
+    S = S * (g.double().reshape(B, H, -1)[..., None])
+    size = S.abs().sum(2).amax() + 8
+    if rule == "delta":
+        u = beta.double()[..., None] * (vd - torch.einsum("bhdv,bhd->bhv", S, kd))
+    else:
+        u = vd * (c.double()[..., None] if rule == "scaled" else 1.0)
+    S = S + kd[..., None] * u[:, :, None]
+    want = torch.einsum("bhdv,bhd->bhv", S, qd) + (skip.double()[:, None] * vd if rule == "scaled" else 0.0)
+    # at most 256 products of a state of a few units and unit vectors' channels, summed in fp32
+    tol = 2e-6 * float(size)
+    assert float((o.double().reshape(B, H, Vd) - want).abs().max()) <= tol
+    got = state[slots]
+    assert float((got[:, :H * D * Vd].double() - S.reshape(B, -1)).abs().max()) <= tol
+    assert torch.equal(got[:, H * D * Vd:], state0[slots, H * D * Vd:])
+    rest = [i for i in range(B + 2) if i not in slots.tolist()]
+    assert torch.equal(state[rest], state0[rest])
