@@ -76,6 +76,8 @@ gemm_stream_kernel(const StreamArgs args) {
   pdl_trigger();
   pdl_wait();
 
+  // x from L2: this block may have shared its SM with readers of what the buffer held before, and no two
+  // warps read the same of it.
   uint4 xs[2][2];
   const bf16* xr = args.x + (size_t)(g < M ? g : 0) * args.ldx + 8 * t;
   auto load_x = [&](int slot, int u) {
@@ -83,7 +85,7 @@ gemm_stream_kernel(const StreamArgs args) {
     for (int h = 0; h < 2; ++h) {
       const int k = u * 64 + h * 32;
       xs[slot][h] = make_uint4(0u, 0u, 0u, 0u);
-      if (g < M && k < k_end) xs[slot][h] = *reinterpret_cast<const uint4*>(xr + k);
+      if (g < M && k < k_end) xs[slot][h] = __ldcg(reinterpret_cast<const uint4*>(xr + k));
     }
   };
   load_x(0, u0);

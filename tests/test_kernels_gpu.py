@@ -719,3 +719,24 @@ def test_one_token_of_every_request_through_its_state(H, G, D, Vd, B, channels, 
     assert torch.equal(got[:, H * D * Vd:], state0[slots, H * D * Vd:])
     rest = [i for i in range(B + 2) if i not in slots.tolist()]
     assert torch.equal(state[rest], state0[rest])
+
+
+@pytest.mark.parametrize("T,top,N", [(1, 1, 4), (3, 4, 2048), (5, 6, 516), (2, 9, 37), (40, 2, 130)])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_pairs_rows_are_added_up_in_the_order_chosen(T, top, N, weighted):
+    """Widths of quads and others, more choices than are asked for at a time, choices without a row: equal to
+    the sum in that order in 32-bit."""
+    from types import SimpleNamespace
+    from ginfer_b200.ops import moe
+    g = torch.Generator(device=DEV).manual_seed(N)
+    y = torch.randn(T * top, N, generator=g, device=DEV)
+    pos = torch.randperm(T * top, generator=g, device=DEV).int()
+    pos[::5] = -1
+    wgt = torch.rand(T, top, generator=g, device=DEV) if weighted else None
+    got = moe.combine(y, SimpleNamespace(pos_of_pair=pos, top=top), wgt, T)
+    want, size = torch.zeros(T, N, dtype=torch.float64, device=DEV), torch.zeros(T, N, device=DEV)
+    for k in range(top):
+        p = pos.view(T, top)[:, k].long()
+        row = torch.where(p[:, None] >= 0, y[p.clamp(min=0)], 0.0) * (wgt[:, k:k + 1] if weighted else 1.0)
+        want, size = want + row.double(), size + row.abs()
+    assert ((got.double() - want).abs() <= top * 2.0 ** -23 * size).all()
