@@ -73,8 +73,10 @@ gemm_stream_kernel(const StreamArgs args) {
   for (int i = 0; i < RING; ++i) load_w(i, u0 + i);
   float b0 = 0.f, b1 = 0.f;
   if (EPI != ST_GATED && args.bias) b0 = n < N ? args.bias[n] : 0.f, b1 = n + 1 < N ? args.bias[n + 1] : 0.f;
-  pdl_trigger();
+  // The kernel behind may only start now: earlier, its own loads (a large product's ring) compete with
+  // those that this chain waits for (8 requests, 32 experts: 30.7 -> 28.6 ms for the whole batch).
   pdl_wait();
+  pdl_trigger();
 
   // x from L2: this block may have shared its SM with readers of what the buffer held before, and no two
   // warps read the same of it.
