@@ -32,13 +32,15 @@ namespace gf {
 
 namespace cg = cooperative_groups;
 
-constexpr int KU = 32;                                    // segments are multiples of this
+constexpr int KS = 8;                                     // segments are multiples of this
+constexpr int KU = 32;                                    // k of a stage of the rows kernel
 
 // Segments of K, a function of the matrix alone (it fixes the order of the sums): enough for a few
-// blocks an SM.
+// blocks an SM; eight where each has 32 k at least, four where each has 8 (short reductions are cut too,
+// for shorter chains of roundings).
 inline int k_segments(int N, int K) {
   int s = N <= 4096 ? 8 : N <= 32768 ? 4 : 2;
-  while (s > 2 && s * KU > K) s >>= 1;
+  while (s > 2 && s * (s > 4 ? 4 * KS : KS) > K) s >>= 1;
   return s;
 }
 
@@ -84,7 +86,7 @@ gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W,
   auto& sm = *reinterpret_cast<RowsShared<MT, STAGES>*>(raw);
   const int lane = threadIdx.x, half = lane >> 4, row = lane & 15;
   const int rank = blockIdx.x, ranks = gridDim.x, n0 = blockIdx.y * 32;
-  const int kbase = 2 * rank * seg;                       // seg: a multiple of KU
+  const int kbase = 2 * rank * seg;                       // seg: a multiple of KS
   const int steps = max(0, min(seg, K - kbase) + KU - 1) / KU;
   pdl_trigger();
   pdl_wait();
@@ -96,15 +98,15 @@ gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W,
 #pragma unroll 16
       for (int e = lane; e < 64 * PER; e += 32) {
         const int h = e / (32 * PER), r = e / PER % 32, kk = (e % PER) * VEC;
-        const int k = kbase + h * seg + step * KU + kk;
-        const bool in = n0 + r < N && k < K;
+        const int at = step * KU + kk, k = kbase + h * seg + at;
+        const bool in = n0 + r < N && at < seg && k < K;
         copy_async<VEC>(&sm.w[st][h][r][kk], in ? W + (size_t)(n0 + r) * K + k : W, in);
       }
 #pragma unroll
       for (int e = lane; e < 2 * MT * PER; e += 32) {
         const int h = e / (MT * PER), r = e / PER % MT, kk = (e % PER) * VEC;
-        const int k = kbase + h * seg + step * KU + kk;
-        const bool in = r < M && k < K;
+        const int at = step * KU + kk, k = kbase + h * seg + at;
+        const bool in = r < M && at < seg && k < K;
         copy_async<VEC>(&sm.x[st][h][r][kk], in ? A + (size_t)r * lda + k : A, in);
       }
     }
@@ -168,7 +170,6 @@ gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W,
 
 // ---------------------------------------------------------------------------------- more rows
 constexpr int BN = 128, BK = 16, BP = BK + 4, TILE_STAGES = 4, OP = BN + 16;
-static_assert(KU % BK == 0);
 
 template <int BM> constexpr size_t tile_shared() {
   const size_t ring = (size_t)TILE_STAGES * (BM + BN) * BP, out = (size_t)BM * OP;
@@ -192,18 +193,18 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W,
   auto fetch = [&](int step) {
     if (step < steps) {
       float* st = ring + (size_t)(step % TILE_STAGES) * (BM + BN) * BP;
-      const int k0 = kbase + step * BK;
+      const int k0 = kbase + step * BK, k_end = min(kbase + seg, K);
       constexpr int PER = BK / VEC;
 #pragma unroll 8
       for (int e = tid; e < BM * PER; e += THREADS) {
         const int r = e / PER, kk = (e % PER) * VEC, k = k0 + kk;
-        const bool in = m0 + r < M && k < K;
+        const bool in = m0 + r < M && k < k_end;
         copy_async<VEC>(st + r * BP + kk, in ? A + (size_t)(m0 + r) * lda + k : A, in);
       }
 #pragma unroll 8
       for (int e = tid; e < BN * PER; e += THREADS) {
         const int r = e / PER, kk = (e % PER) * VEC, k = k0 + kk;
-        const bool in = n0 + r < N && k < K;
+        const bool in = n0 + r < N && k < k_end;
         copy_async<VEC>(st + (BM + r) * BP + kk, in ? W + (size_t)(n0 + r) * K + k : W, in);
       }
     }
@@ -317,8 +318,8 @@ GF_DEFINE_PDL_SWITCH
 GF_EXPORT int gf_gemm_f32(const float* A, int lda, const float* W, const float* bias, float* C,
                           int ldc, int M, int N, int K, void* stream) {
   if (M <= 0 || N <= 0) return 0;
-  const int segments = k_segments(N, K), units = (K + KU - 1) / KU;
-  const F32Args a{A, W, bias, C, M, N, K, lda, ldc, segments, (units + segments - 1) / segments * KU,
+  const int segments = k_segments(N, K), units = (K + KS - 1) / KS;
+  const F32Args a{A, W, bias, C, M, N, K, lda, ldc, segments, (units + segments - 1) / segments * KS,
                   (cudaStream_t)stream};
   const bool whole = K % 4 == 0 && lda % 4 == 0 && ((uintptr_t)A | (uintptr_t)W) % 16 == 0;
   return whole ? start_by_rows<4>(a) : start_by_rows<1>(a);
