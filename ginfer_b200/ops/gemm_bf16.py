@@ -140,7 +140,7 @@ def gemm(x, weight, bias_f32=None, out_dtype=torch.bfloat16, epi: int = 0, split
     if M == 0:
         return out if resid is None else None
     if (M <= STREAM_MAX_TOKENS and N * K <= STREAM_MAX_WEIGHTS and split_k is None
-            and (out_dtype == torch.float32 or epi != 0)
+            and (M <= STREAM_MAX_TOKENS_BF16 or out_dtype == torch.float32 or epi != 0)
             and not through_workspace and scale is None and resid is None
             and stream(x, weight, bias_f32, out, epi, act_consts)):
         return out
@@ -184,10 +184,12 @@ def gemm(x, weight, bias_f32=None, out_dtype=torch.bfloat16, epi: int = 0, split
 # kernel ahead is done (csrc/gemm_stream.cu).  Decode steps on a B200 with products of up to 9.7 MB / of
 # up to 14.5 MB / of up to 27 MB on it, none: pimidra m, 2 requests 0.589 / 0.569 / 0.581, 0.610 ms;
 # lasizen m, 4 requests 0.513 / 0.499 / 0.501, 0.509; vilepel m, 4 requests 0.872 / 0.874 / 0.892, 0.960.
-# Plain products with bf16 results stay: behind and in front of Qwen2's large products they cost its decode
-# step of 8 requests 2 % at the 1.5B shape (47.4 -> 48.5 ms for the whole batch of 512-token prompts), and
-# give one or four requests less than 1 %.
+# Plain products with bf16 results come up to four rows only: beside Qwen2's large products they cost its
+# decode step of 8 requests 2 % at the 1.5B shape (47.5 -> 48.4 ms for the whole batch of 512-token prompts)
+# and give 4 requests 1 %; lasizen s, one request: 9.7 ms without them, 9.1 with; bapivik s, 4 requests:
+# 12.1 and 11.3.
 STREAM_MAX_TOKENS = 8
+STREAM_MAX_TOKENS_BF16 = 4
 STREAM_MAX_WEIGHTS = 148 * 8 * 6144
 
 
