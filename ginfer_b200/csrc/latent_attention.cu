@@ -557,216 +557,6 @@ latent_attention_mma_kernel(const float* __restrict__ q_lat, const float* __rest
   }
 }
 
-// ---- several tokens a block (prompt portions) -----------------------------------------------------
-// The kernel above reads a token's keys for that token alone: 2,251 tokens of four prompts with a window of
-// 1,024 keys of 576 channels asked L2 for 1.6 GB a layer.  Neighbouring tokens of a request see nearly the
-// same keys, so a block takes four tokens: 64 rows (16 heads each) share every tile of 32 keys.  A warp
-// belongs to a token and a quarter: a quarter of the key channels for the scores (the quarters' parts
-// meet in shared memory), eight of the tile's keys for the softmax, a quarter of the latent channels for
-// the output.  What a token does not see of the tile is masked; tokens of several requests in one block
-// are taken request by request.  Rounding is that of the kernel above (queries and probabilities to bf16).
-// Those 2,251 tokens (16 heads) on a B200: 258 us a layer, 556 with a block a token.
-constexpr int kRowTokens = 4, kRowTile = 32, kRowSld = kRowTile + 4, kRowPld = kRowTile + 8;
-
-__device__ __forceinline__ void ldsm_x4_trans(uint32_t (&r)[4], const void* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(smem_u32(p)));
-}
-// The four warps of a token.
-__device__ __forceinline__ void token_sync(int tok) {
-  asm volatile("bar.sync %0, 128;" ::"r"(tok + 1) : "memory");
-}
-
-__host__ __device__ inline size_t rows_shared(int Dk) {
-  return (size_t)(64 + 2 * kRowTile) * (Dk + 8) * 2 + (size_t)(4 * 64 * kRowSld + 4 * 64) * 4 + 64 * kRowPld * 2;
-}
-
-// NT: tiles of 8 latent channels a warp.
-template <int NT>
-__global__ void __launch_bounds__(512, 1)
-latent_attention_rows_kernel(const float* __restrict__ q_lat, const float* __restrict__ q_rot,
-                             const bf16* __restrict__ c_pages, const bf16* __restrict__ r_pages,
-                             const int* __restrict__ block_table, int table_stride,
-                             const int* __restrict__ seq_of_token, const int* __restrict__ positions,
-                             bf16* __restrict__ out, int num_tokens, int H, int C, int R, int page_size,
-                             int window, float scale) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int Dk = C + R, ld = Dk + 8;
-  bf16* Qs = reinterpret_cast<bf16*>(smem_raw);              // [64][ld], row 16 token + head
-  bf16* Ks = Qs + 64 * ld;                                   // [2][32][ld]
-  float* sred = reinterpret_cast<float*>(Ks + 2 * kRowTile * ld);   // [4 quarters][64][kRowSld]
-  float* red = sred + 4 * 64 * kRowSld;                      // [4 quarters][64]
-  bf16* Ps = reinterpret_cast<bf16*>(red + 4 * 64);          // [64][kRowPld]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
-  const int tok = warp & 3, qr = warp >> 2, h0 = blockIdx.y * 16;
-  // the last tokens of a prompt see the most keys: they go first
-  const int base = ((int)gridDim.x - 1 - (int)blockIdx.x) * kRowTokens;
-  const int here = min(kRowTokens, num_tokens - base);
-  pdl_trigger();
-  pdl_wait();
-  const int dq = Dk >> 2;
-  for (int i = threadIdx.x; i < 64 * dq; i += 512) {
-    const int row = i / dq, d = (i - row * dq) * 4, t = base + (row >> 4), h = h0 + (row & 15);
-    float v[4] = {0.f, 0.f, 0.f, 0.f};
-    if ((row >> 4) < here && h < H)
-      Quad<float>::load(d < C ? q_lat + ((size_t)h * num_tokens + t) * C + d
-                              : q_rot + ((size_t)t * H + h) * R + (d - C), v);
-    Quad<bf16>::store(Qs + row * ld + d, v);
-  }
-  const int mine = base + min(tok, here - 1);
-  const int my_p = positions[mine];
-  const int my_lo = window > 0 ? max(0, my_p - window + 1) : 0;
-  float o[NT][4];
-#pragma unroll
-  for (int j = 0; j < NT; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
-  float m[2] = {-INFINITY, -INFINITY}, lsum[2] = {0.f, 0.f};
-  const int kj = threadIdx.x >> 4, nchunk = Dk >> 3;         // sixteen threads a key
-  const int steps = Dk >> 4, k_lo = (steps * qr / 4) << 4, k_hi = (steps * (qr + 1) / 4) << 4;
-  const int ctiles = C >> 3, ntw = (((ctiles + 3) >> 2) + 1) & ~1, ct0 = qr * ntw;   // (ctiles is even)
-  const bf16* qa = Qs + (tok * 16 + (lane & 15)) * ld + ((lane >> 4) << 3);
-  const int b_row = ((lane >> 4) << 3) + (lane & 7), b_col = ((lane >> 3) & 1) << 3;
-
-  for (int g0 = 0; g0 < here;) {                             // the requests of the block's tokens
-    const int b = seq_of_token[base + g0];
-    int g1 = g0 + 1;
-    while (g1 < here && seq_of_token[base + g1] == b) ++g1;
-    const int p_first = positions[base + g0], p = positions[base + g1 - 1];
-    const int lo = window > 0 ? max(0, p_first - window + 1) : 0;
-    const bool active = tok >= g0 && tok < g1;
-    const int* tbl = block_table + (size_t)b * table_stride;
-    const int tiles = (p - lo) / kRowTile + 1;
-    auto ask = [&](int tile) {
-      bf16* dst = Ks + (size_t)(tile & 1) * kRowTile * ld + (size_t)kj * ld;
-      const int c = lo + tile * kRowTile + kj;
-      const bool ok = c <= p;
-      const size_t slot = ok ? (size_t)tbl[c / page_size] * page_size + c % page_size : 0;
-      for (int i = threadIdx.x & 15; i < nchunk; i += 16) {
-        const int d = i << 3;
-        cp_async_16(dst + d, d < C ? c_pages + slot * C + d : r_pages + slot * R + (d - C), ok);
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    ask(0);
-    for (int it = 0; it < tiles; ++it) {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-      __syncthreads();                                       // the tile is there, the other stage is free
-      if (it + 1 < tiles) ask(it + 1);
-      if (!active) continue;
-      const bf16* K = Ks + (size_t)(it & 1) * kRowTile * ld;
-      float s[4][4] = {};                                    // this quarter's part of 16 heads x 32 keys
-      const bf16* kb = K + (size_t)b_row * ld + b_col;
-#pragma unroll 3
-      for (int k = k_lo; k < k_hi; k += 16) {
-        uint32_t a[4], b0[4], b1[4];
-        ldsm_x4(a, qa + k);
-        ldsm_x4(b0, kb + k);
-        ldsm_x4(b1, kb + 16 * ld + k);
-        const uint32_t c0[2] = {b0[0], b0[1]}, c1[2] = {b0[2], b0[3]};
-        const uint32_t c2[2] = {b1[0], b1[1]}, c3[2] = {b1[2], b1[3]};
-        mma_bf16(s[0], a, c0);
-        mma_bf16(s[1], a, c1);
-        mma_bf16(s[2], a, c2);
-        mma_bf16(s[3], a, c3);
-      }
-      float* part = sred + (size_t)(qr * 64 + tok * 16) * kRowSld + 2 * t4;
-#pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        *reinterpret_cast<float2*>(part + g * kRowSld + 8 * n) = make_float2(s[n][0], s[n][1]);
-        *reinterpret_cast<float2*>(part + (g + 8) * kRowSld + 8 * n) = make_float2(s[n][2], s[n][3]);
-      }
-      token_sync(tok);
-      float x[4] = {0.f, 0.f, 0.f, 0.f};                     // rows g | g + 8, keys 8 qr + 2 t4, + 1
-#pragma unroll
-      for (int z = 0; z < 4; ++z) {
-        const float* at = sred + (size_t)(z * 64 + tok * 16) * kRowSld + 8 * qr + 2 * t4;
-        const float2 u = *reinterpret_cast<const float2*>(at + g * kRowSld);
-        const float2 w = *reinterpret_cast<const float2*>(at + (g + 8) * kRowSld);
-        x[0] += u.x, x[1] += u.y, x[2] += w.x, x[3] += w.y;
-      }
-      const int key = lo + it * kRowTile + 8 * qr + 2 * t4;
-      float mx[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int c = key + (e & 1);
-        x[e] = c >= my_lo && c <= my_p ? x[e] * scale : -INFINITY;
-        mx[e >> 1] = fmaxf(mx[e >> 1], x[e]);
-      }
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
-        mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
-        if (t4 == 0) red[qr * 64 + tok * 16 + g + 8 * r] = mx[r];
-      }
-      token_sync(tok);
-      float corr[2], ref[2];
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        const float* at = red + tok * 16 + g + 8 * r;
-        const float mn = fmaxf(m[r], fmaxf(fmaxf(at[0], at[64]), fmaxf(at[128], at[192])));
-        ref[r] = mn == -INFINITY ? 0.f : mn;                 // (a token that sees none of the tile yet)
-        corr[r] = expf(m[r] - ref[r]);
-        m[r] = mn;
-      }
-      const float p0 = expf(x[0] - ref[0]), p1 = expf(x[1] - ref[0]);
-      const float p2 = expf(x[2] - ref[1]), p3 = expf(x[3] - ref[1]);
-      lsum[0] = lsum[0] * corr[0] + (p0 + p1);
-      lsum[1] = lsum[1] * corr[1] + (p2 + p3);
-      bf16* pw = Ps + (size_t)(tok * 16) * kRowPld + 8 * qr + 2 * t4;
-      *reinterpret_cast<uint32_t*>(pw + g * kRowPld) = pack_bf16(p0, p1);
-      *reinterpret_cast<uint32_t*>(pw + (g + 8) * kRowPld) = pack_bf16(p2, p3);
-#pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        o[j][0] *= corr[0], o[j][1] *= corr[0];
-        o[j][2] *= corr[1], o[j][3] *= corr[1];
-      }
-      token_sync(tok);
-#pragma unroll
-      for (int ks = 0; ks < kRowTile; ks += 16) {
-        uint32_t a[4];
-        ldsm_x4(a, Ps + (size_t)(tok * 16 + (lane & 15)) * kRowPld + ks + ((lane >> 4) << 3));
-        const bf16* vrow = K + (size_t)(ks + (lane & 15)) * ld + ((lane >> 4) << 3);
-#pragma unroll
-        for (int j = 0; j < NT; j += 2) {
-          const int ct = ct0 + j;
-          if (j < ntw && ct < ctiles) {
-            uint32_t v[4];
-            ldsm_x4_trans(v, vrow + ct * 8);
-            const uint32_t v0[2] = {v[0], v[1]}, v1[2] = {v[2], v[3]};
-            mma_bf16(o[j], a, v0);
-            mma_bf16(o[j + 1], a, v1);
-          }
-        }
-      }
-    }
-    __syncthreads();                                         // the stages are free for the next request
-    g0 = g1;
-  }
-#pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    lsum[r] += __shfl_xor_sync(0xffffffffu, lsum[r], 1);
-    lsum[r] += __shfl_xor_sync(0xffffffffu, lsum[r], 2);
-    if (t4 == 0) red[qr * 64 + tok * 16 + g + 8 * r] = lsum[r];
-  }
-  __syncthreads();
-  if (tok >= here) return;
-#pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    const int h = h0 + g + 8 * r;
-    if (h >= H) continue;
-    const float* at = red + tok * 16 + g + 8 * r;
-    const float inv = 1.f / ((at[0] + at[64]) + (at[128] + at[192]));
-    bf16* dst = out + ((size_t)h * num_tokens + mine) * C;
-#pragma unroll
-    for (int j = 0; j < NT; ++j) {
-      const int ct = ct0 + j;
-      if (j < ntw && ct < ctiles)
-        *reinterpret_cast<uint32_t*>(dst + ct * 8 + 2 * t4) =
-            pack_bf16(o[j][2 * r] * inv, o[j][2 * r + 1] * inv);
-    }
-  }
-}
-
 // out[h, t, :] = sum_z o_z exp(m_z - M) / sum_z l_z exp(m_z - M): a block a (token, head), a thread four
 // channels.  Bound by latency: the shares' sums are asked for before their weights are known (what an
 // empty share left there is not used), all at once.  32 tokens, 16 heads of 512 channels in 4 shares on a
@@ -873,34 +663,13 @@ GF_EXPORT int gf_latent_attention(const float* q_lat, const float* q_rot, const 
                                   const void* r_pages, const int* block_table, int table_stride,
                                   const int* seq_of_token, const int* positions, void* out, int T,
                                   int H, int C, int R, int page_size, int window, float scale,
-                                  int dtype, int nsplit, float* part_o, float* part_ml, int portions,
+                                  int dtype, int nsplit, float* part_o, float* part_ml,
                                   void* stream) {
   if (T <= 0) return 0;
   if (C > kLatMaxC || C <= 0 || R < 0) return -3;
   const int Dk = C + R;
   if (dtype == GF_BF16 && C % 16 == 0 && R % 16 == 0 && (uintptr_t)c_pages % 16 == 0 &&
       (uintptr_t)r_pages % 16 == 0) {
-    if (portions && C <= 512 && rows_shared(Dk) <= 220 * 1024 && (uintptr_t)q_lat % 16 == 0 &&
-        (uintptr_t)q_rot % 16 == 0 && (uintptr_t)out % 4 == 0) {
-      static OncePerDevice once_rows;
-      if (int rc = once_rows.run([] {
-            for (auto k : {latent_attention_rows_kernel<4>, latent_attention_rows_kernel<8>,
-                           latent_attention_rows_kernel<16>}) {
-              const cudaError_t e =
-                  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-              if (e != cudaSuccess) return e;
-            }
-            return cudaSuccess;
-          }))
-        return rc;
-      const auto kernel = C <= 128   ? latent_attention_rows_kernel<4>
-                          : C <= 256 ? latent_attention_rows_kernel<8>
-                                     : latent_attention_rows_kernel<16>;
-      return launch_kernel(kernel, dim3((T + kRowTokens - 1) / kRowTokens, (H + 15) / 16), dim3(512),
-                           rows_shared(Dk), (cudaStream_t)stream, q_lat, q_rot, (const bf*)c_pages,
-                           (const bf*)r_pages, block_table, table_stride, seq_of_token, positions, (bf*)out,
-                           T, H, C, R, page_size, window, scale);
-    }
     const int ld = Dk + 8;
     const size_t bytes = ((size_t)16 * ld + (size_t)2 * kMmaTile * ld + 16 * (kMmaTile + 8)) * 2 +
                          (8 * 16 + 2 * 16 * kMmaTile) * sizeof(float);

@@ -85,14 +85,6 @@ MAX_SPLITS = 8
 MIN_TILES_A_SPLIT = 4   # a share shorter than this costs more in the merge than it saves
 
 
-# Steps of at least this many tokens, in portions of at least so many on average, take the kernel whose
-# blocks share every key among four neighbouring tokens (bf16).  With fewer blocks than SMs the kernel
-# with a block a token has four times as many; single tokens have no neighbours (a block takes the
-# requests of its tokens one after another).
-ROWS_MIN_TOKENS = 320
-ROWS_MIN_PORTION = 8
-
-
 def key_splits(num_tokens: int, num_heads: int, max_keys: int, sms: int = 148) -> int:
     """How many blocks share the keys of a token: one unless the step's blocks would leave most
     SMs idle and a token has several tiles of keys."""
@@ -124,15 +116,14 @@ def attention(q_lat: torch.Tensor, q_rot: torch.Tensor, c_pages: torch.Tensor,
         if nsplit > 1:
             part_o = torch.empty((nsplit, T, H, C), dtype=torch.float32, device=q_lat.device)
             part_ml = torch.empty((nsplit, T, H, 2), dtype=torch.float32, device=q_lat.device)
-    portions = nsplit == 1 and T >= ROWS_MIN_TOKENS and T >= ROWS_MIN_PORTION * int(getattr(ctx, "num_seqs", T))
     f = _fn("latent_attention", "gf_latent_attention",
             [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
              c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p,
-             c_void_p, c_int, c_void_p], kernels=2 if nsplit > 1 else 1)
+             c_void_p, c_void_p], kernels=2 if nsplit > 1 else 1)
     rc = f(_p(q_lat), _p(q_rot), _p(c_pages), _p(r_pages), _p(block_table),
            block_table.stride(0), _p(ctx.seq_of_token), _p(ctx.positions), _p(out), T, H, C, R,
            int(page_size), int(window), float(scale), _code(c_pages.dtype), nsplit, _p(part_o),
-           _p(part_ml), int(portions), _stream())
+           _p(part_ml), _stream())
     if rc == -3:
         raise ValueError(f"latent attention takes latent vectors of up to 1024 channels whose key "
                          f"tile fits shared memory; got kv_rank={C}, rot_dim={R}")

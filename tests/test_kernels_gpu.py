@@ -740,49 +740,3 @@ def test_pairs_rows_are_added_up_in_the_order_chosen(T, top, N, weighted):
         row = torch.where(p[:, None] >= 0, y[p.clamp(min=0)], 0.0) * (wgt[:, k:k + 1] if weighted else 1.0)
         want, size = want + row.double(), size + row.abs()
     assert ((got.double() - want).abs() <= top * 2.0 ** -23 * size).all()
-
-
-@pytest.mark.parametrize("H,C,R,window", [(5, 16, 0, 0), (16, 512, 64, 40), (20, 80, 16, 0), (3, 144, 32, 33),
-                                          (16, 256, 0, 1)])
-@pytest.mark.parametrize("spans", [[(0, 37)], [(0, 1), (9, 2), (100, 6), (31, 33)], [(70, 3), (0, 130), (200, 1)]])
-def test_latent_attention_of_portions_shares_its_keys(monkeypatch, H, C, R, window, spans):
-    """Portions ``(first position, tokens)`` of several requests, whose ends fall inside a block; windows that
-    start anywhere in a tile; heads and channels that fill no tile: against 64 bits, and beside the kernel
-    with a block a token."""
-    from types import SimpleNamespace
-    from ginfer_b200.ops import latent
-    g = torch.Generator(device=DEV).manual_seed(C + H + len(spans))
-    page, B = 16, len(spans)
-    W = max(-(-(a + n) // page) for a, n in spans)
-    cp = torch.randn(B * W + 1, page, 1, C, generator=g, device=DEV).bfloat16()
-    rp = torch.randn(B * W + 1, page, 1, R, generator=g, device=DEV).bfloat16() if R else None
-    table = torch.randperm(B * W, generator=g, device=DEV).int().view(B, W)
-    seq = [b for b, (a, n) in enumerate(spans) for _ in range(n)]
-    pos = [a + i for a, n in spans for i in range(n)]
-    T = len(seq)
-    ql = torch.randn(H, T, C, generator=g, device=DEV).bfloat16().float()     # (rounded to bf16 inside)
-    qr = torch.randn(T, H, R, generator=g, device=DEV).bfloat16().float() if R else None
-    scale = (C + R) ** -0.5
-    seen = table.clone()
-    if window:                          # pages that no query of the step sees are given back
-        for b, (a, n) in enumerate(spans):
-            seen[b, :max(0, a - window + 1) // page] = -1
-    ctx = SimpleNamespace(seq_of_token=torch.tensor(seq, dtype=torch.int32, device=DEV), num_seqs=B,
-                          positions=torch.tensor(pos, dtype=torch.int32, device=DEV))
-    got = []
-    for least in (1, 1 << 30):
-        monkeypatch.setattr(latent, "ROWS_MIN_TOKENS", least)
-        monkeypatch.setattr(latent, "ROWS_MIN_PORTION", 0)
-        got.append(latent.attention(ql, qr, cp, rp, seen, ctx, window, scale, page).double())
-    for t in range(T):
-        b, p = seq[t], pos[t]
-        lo = max(0, p - window + 1) if window else 0
-        c = cp[table[b].long()].reshape(-1, C)[lo:p + 1].double()
-        s = ql[:, t].double() @ c.t()
-        if R:
-            s = s + qr[t].double() @ rp[table[b].long()].reshape(-1, R)[lo:p + 1].double().t()
-        w = torch.softmax(s * scale, dim=-1)
-        # probabilities and result are rounded to bf16: 2^-8 each, of at most sum w |c|
-        bound = 2 * 2.0 ** -8 * (w @ c.abs()) + 1e-6
-        for i in range(2):
-            assert ((got[i][:, t] - w @ c).abs() <= bound).all(), (t, i)

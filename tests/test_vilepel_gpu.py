@@ -477,3 +477,28 @@ def test_latent_attention_shares_a_tokens_keys_among_blocks_in_small_steps(windo
     slow = latent.attention(q_lat, q_rot, c_pages.float(), r_pages.float(), table, ctx, window,
                             0.2, page)
     assert float((fast.float() - slow).abs().max()) <= 0.02 * float(slow.abs().max())
+
+
+@pytest.mark.parametrize("H, C, R, window", [(5, 48, 16, 0), (16, 256, 32, 100)])
+def test_latent_attention_of_a_token_does_not_depend_on_its_step(H, C, R, window):
+    """A long portion in one step and cut into steps of some hundred tokens: equal bit for bit.  (A router
+    behind the layer makes close calls: a token's bits decide which experts it gets.)"""
+    from ginfer_b200.ops import latent
+    T, page = 430, 16
+    g = torch.Generator(device="cuda").manual_seed(C)
+    W = -(-T // page)
+    c_pages = torch.randn(W, page, 1, C, generator=g, device="cuda").bfloat16()
+    r_pages = torch.randn(W, page, 1, R, generator=g, device="cuda").bfloat16()
+    table = torch.randperm(W, generator=g, device="cuda").int().view(1, W)
+    q_lat = torch.randn(H, T, C, generator=g, device="cuda")
+    q_rot = torch.randn(T, H, R, generator=g, device="cuda")
+
+    def run(a, b):
+        ctx = _Ctx()
+        ctx.num_seqs = 1
+        ctx.seq_of_token = torch.zeros(b - a, dtype=torch.int32, device="cuda")
+        ctx.positions = torch.arange(a, b, dtype=torch.int32, device="cuda")
+        return latent.attention(q_lat[:, a:b].contiguous(), q_rot[a:b].contiguous(), c_pages, r_pages,
+                                table, ctx, window, 0.05, page)
+    whole = run(0, T)
+    assert torch.equal(whole, torch.cat([run(a, min(a + 110, T)) for a in range(0, T, 110)], dim=1))
