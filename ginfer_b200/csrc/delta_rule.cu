@@ -16,8 +16,9 @@
 //                            independent: four lanes or a warp share a column (a share of the rows
 //                            each, in registers).  The tokens' operands come through two stages of
 //                            shared memory, a chunk ahead (cp.async).
-//   delta_chunk_coef(_channels)_kernel, delta_chunk_recurrence_kernel   the recurrence of long
-//                            portions, eight tokens at a time (see there).
+//   delta_chunk_coef_kernel, linear_chunk_coef_kernel, delta_chunk_recurrence_kernel   the recurrence of
+//                            long portions, eight tokens at a time: the delta rule with one decay a head,
+//                            plain linear attention with a decay a key channel (see there).
 //   delta_output_kernel      a warp a (token, head): o / rms(o) * w * sigmoid(gate).
 #include "common.cuh"
 
@@ -550,21 +551,19 @@ delta_chunk_coef_kernel(const float* __restrict__ qn, const float* __restrict__ 
   }
 }
 
-// The same with a decay a key channel, where G_i, R and G_7 are vectors: R stands inside the dot products
-// L and M are made of, and the recurrence reads G_i k_i, G_i q_i and R(j, 7) k_j (elementwise) in the
-// places of k_i, q_i and k_j.  A warp a (chunk, head): those three for every token, [T, H, D] each, L, M
-// and beta, and the chunk's G_7.  On a B200, 2,251 tokens of four requests, the longest 1,201, 16 heads
-// of 128 x 128: 26 us and 391 us for the recurrence behind it; token by token 736 us.
-// DELTA false: a plain linear attention, S <- diag(g) S + k v^T; its u is v, so there is no L, no beta
-// and no G_i k_i.  ld_q, ld_k, ld_g: floats between two tokens.
-template <bool DELTA>
+// The same for a plain linear attention with a decay a key channel, S <- diag(g) S + k v^T: its u is v, so
+// there is no L and no beta.  G_i, R and G_7 are vectors: R stands inside the dot products M is made of,
+// and the recurrence reads G_i q_i and R(j, 7) k_j (elementwise) in the places of q_i and k_j.  A warp a
+// (chunk, head): those two for every token, [T, H, D] each, M, and the chunk's G_7.  On a B200, two
+// prompts of 1,500 and 1,700 tokens, 16 heads of 128 x 128: 20 us, and 360 for the recurrence behind it.
+// (The delta rule itself with a decay a channel goes token by token in steps of every length: a router
+// behind it makes close calls, so its sums keep one order.)  ld_q, ld_k, ld_g: floats between two tokens.
 __global__ void __launch_bounds__(128)
-delta_chunk_coef_channels_kernel(const float* __restrict__ qn, int ld_q, const float* __restrict__ kn,
-                                 int ld_k, const float* __restrict__ g, int ld_g,
-                                 const float* __restrict__ beta,
-                                 const int* __restrict__ cu_seqlens, DeltaDims dm,
-                                 float* __restrict__ coef, float* __restrict__ total,
-                                 float* __restrict__ kg, float* __restrict__ qg, float* __restrict__ ke) {
+linear_chunk_coef_kernel(const float* __restrict__ qn, int ld_q, const float* __restrict__ kn,
+                         int ld_k, const float* __restrict__ g, int ld_g,
+                         const int* __restrict__ cu_seqlens, DeltaDims dm,
+                         float* __restrict__ coef, float* __restrict__ total,
+                         float* __restrict__ qg, float* __restrict__ ke) {
   const int lane = threadIdx.x & 31;
   const int c = blockIdx.x * 4 + (threadIdx.x >> 5), b = blockIdx.y, h = blockIdx.z;
   pdl_wait();
@@ -599,7 +598,6 @@ delta_chunk_coef_channels_kernel(const float* __restrict__ qn, int ld_q, const f
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
           kr[x] *= gd[i][x];
-          if (DELTA) val[8 * i + j] = fmaf(kr[x], k[i][x], val[8 * i + j]);
           val[8 * j + i] = fmaf(kr[x], q[i][x], val[8 * j + i]);
         }
       if (j < n) Quad<float>::store(ke + (size_t)(ta + j) * HD + (size_t)h * D + d, kr);
@@ -607,14 +605,10 @@ delta_chunk_coef_channels_kernel(const float* __restrict__ qn, int ld_q, const f
     float G[4] = {1.f, 1.f, 1.f, 1.f};
 #pragma unroll
     for (int i = 0; i < CT; ++i) {
-      float a[4], e[4];
+      float e[4];
 #pragma unroll
-      for (int x = 0; x < 4; ++x) G[x] *= gd[i][x], a[x] = G[x] * k[i][x], e[x] = G[x] * q[i][x];
-      if (i < n) {
-        const size_t at = (size_t)(ta + i) * HD + (size_t)h * D + d;
-        if (DELTA) Quad<float>::store(kg + at, a);
-        Quad<float>::store(qg + at, e);
-      }
+      for (int x = 0; x < 4; ++x) G[x] *= gd[i][x], e[x] = G[x] * q[i][x];
+      if (i < n) Quad<float>::store(qg + (size_t)(ta + i) * HD + (size_t)h * D + d, e);
     }
     Quad<float>::store(total + chunk * D + d, G);
   }
@@ -631,21 +625,12 @@ delta_chunk_coef_channels_kernel(const float* __restrict__ qn, int ld_q, const f
       }
   }
   const float mine[2] = {val[0], val[32]};
-  const float bl = DELTA && lane < n ? beta[(size_t)(ta + lane) * H + h] : 0.f;
   float* dst = coef + chunk * kCoefs;
 #pragma unroll
   for (int x = 0; x < 2; ++x) {
     const int m = lane + 32 * x, a = m >> 3, e = m & 7;
-    const float bi = __shfl_sync(0xffffffffu, bl, a);
-    if (a > e) {
-      dst[kCoefL + a * CT + e] = bi * mine[x];
-      dst[kCoefM + e * CT + a] = 0.f;                        // (M is read as whole rows)
-    } else {
-      dst[kCoefM + e * CT + a] = mine[x];
-      if (a == e) dst[kCoefL + a * CT + a] = 0.f;
-    }
+    dst[kCoefM + e * CT + a] = a > e ? 0.f : mine[x];        // (M is read as whole rows)
   }
-  if (lane < CT) dst[kCoefBeta + lane] = bl;
 }
 
 // A block = (request, head, 16 CP columns of S); LANES (8 or 16) lanes a column, CP columns a lane (a read
@@ -653,10 +638,10 @@ delta_chunk_coef_channels_kernel(const float* __restrict__ qn, int ld_q, const f
 // there are blocks enough without).  Lane p of a column owns
 // the rows 4 (p + LANES i) .. + 3, i < DPER / 4, so that the lanes' reads of a token's k and q are one run of
 // shared memory.  Stages as in the kernel above, one barrier a chunk.
-// HEADS: the delta rule with a decay a head; ke and total are not read.  CHANNELS: a decay a key channel;
-// kn, qn and ke are [T, H, D] as delta_chunk_coef_channels_kernel leaves them, total the chunks' G_7.
-// PLAIN: the same without the delta rule (u = v; kn is not read; eight lanes a column).
-enum { HEADS = 0, CHANNELS = 1, PLAIN = 2 };
+// HEADS: the delta rule with a decay a head; ke and total are not read.  PLAIN: linear attention with a
+// decay a key channel (u = v; kn is not read; eight lanes a column); qn and ke are [T, H, D] as
+// linear_chunk_coef_kernel leaves them, total the chunks' G_7.
+enum { HEADS = 0, PLAIN = 1 };
 template <int DPER, int LANES, int CP, int MODE>
 __global__ void __launch_bounds__(16 * LANES)
 delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
@@ -666,8 +651,8 @@ delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restr
                               const int* __restrict__ slot_ids, DeltaDims dm, float* __restrict__ o) {
   constexpr int Dp = LANES * DPER, COLS = 16 * CP, NQ = DPER / 4;
   static_assert(MODE != PLAIN || LANES == CT, "a lane a token of a chunk");
-  constexpr int SETS = MODE == CHANNELS ? 3 : 2;               // [CT][Dp] each: k | q, k | q | ke, or q | ke
-  constexpr int kQ = MODE == PLAIN ? 0 : CT * Dp, kE = MODE == HEADS ? 0 : kQ + CT * Dp, kG = SETS * CT * Dp;
+  // two sets of [CT][Dp]: k | q, or q | ke
+  constexpr int kQ = MODE == PLAIN ? 0 : CT * Dp, kE = MODE == HEADS ? 0 : CT * Dp, kG = 2 * CT * Dp;
   constexpr int kVc = kG + (MODE == HEADS ? 0 : Dp), kC = kVc + CT * COLS, kStage = kC + kCoefs;
   constexpr int DOTS = MODE == PLAIN ? CT : 2 * CT;            // with S: the chunk's q, and k in front of them
   extern __shared__ __align__(16) float stage[];               // [kStages][kStage]
@@ -857,8 +842,7 @@ struct ChunkArgs {
 template <int DPER, int LANES, int CP, int MODE>
 static int launch_chunk_columns(int B, const DeltaDims& dm, const ChunkArgs& a, cudaStream_t st) {
   const size_t smem = (size_t)kStages * sizeof(float) *
-                      (((MODE == CHANNELS ? 3 : 2) * CT + (MODE == HEADS ? 0 : 1)) * LANES * DPER +
-                       CT * 16 * CP + kCoefs);
+                      ((2 * CT + (MODE == HEADS ? 0 : 1)) * LANES * DPER + CT * 16 * CP + kCoefs);
   static OncePerDevice attrs;
   if (int rc = attrs.run([&] {
         return cudaFuncSetAttribute(delta_chunk_recurrence_kernel<DPER, LANES, CP, MODE>,
@@ -990,42 +974,33 @@ GF_EXPORT int gf_delta_prepare_heads(const float* proj, int ld, int a_off, int b
                        0, st, proj, ld, state, cu_seqlens, slot_ids, dm);
 }
 
-// fp32 words of scratch with which gf_delta_recurrence takes eight tokens at a time.
+// fp32 words of scratch with which a step goes eight tokens at a time: gf_delta_recurrence (one_decay 1),
+// gf_decay_channels_chunked (0).
 GF_EXPORT long long gf_delta_chunk_words(int T, int B, int H, int D, int one_decay) {
   const long long chunks = (long long)(T / CT + B + 1) * H;
-  return one_decay ? chunks * kCoefs : chunks * (kCoefs + D) + 3ll * T * H * D;
+  return one_decay ? chunks * kCoefs : chunks * (kCoefs + D) + 2ll * T * H * D;
 }
 
-// one_decay: g is [T, H] (a decay a head), else [T, H, D].  scratch: gf_delta_chunk_words, or null: token
-// by token; max_q_len: the longest portion.
+// one_decay: g is [T, H] (a decay a head), else [T, H, D].  scratch (gf_delta_chunk_words; null: token by
+// token) and max_q_len, the longest portion, are for steps with one decay a head.
 GF_EXPORT int gf_delta_recurrence(const float* qn, const float* kn, const float* v, const float* g,
                                   const float* beta, float* state, const int* cu_seqlens,
-                                  const int* slot_ids, int T, int B, int H, int G, int D, int Vd,
+                                  const int* slot_ids, int B, int H, int G, int D, int Vd,
                                   int state_stride, float* o, int one_decay, float* scratch,
                                   int max_q_len, void* stream) {
   if (B <= 0) return 0;
   if (H % G) return -3;
   const DeltaDims dm = dims_of(H, G, D, Vd, 1, state_stride, 0);
   auto st = (cudaStream_t)stream;
-  if (scratch && D % 4 == 0 && Vd % 4 == 0 && D <= 256 && B <= 65535 && H <= 65535 &&
-      (((uintptr_t)qn | (uintptr_t)kn | (uintptr_t)v | (uintptr_t)scratch) & 15) == 0 &&
-      (one_decay || ((uintptr_t)g & 15) == 0)) {
-    const dim3 cgrid(((max_q_len + CT - 1) / CT + 3) / 4, B, one_decay ? G : H);
-    const size_t chunks = (size_t)(T / CT + B + 1) * H, HTD = (size_t)T * H * D;
-    float* total = scratch + chunks * kCoefs;
-    float *kg = total + chunks * D, *qg = kg + HTD, *ke = qg + HTD;      // (a decay a channel only)
-    const int rc =
-        one_decay ? launch_kernel(delta_chunk_coef_kernel, cgrid, dim3(128), 0, st, qn, kn, g, beta,
-                                  cu_seqlens, dm, scratch)
-                  : launch_kernel(delta_chunk_coef_channels_kernel<true>, cgrid, dim3(128), 0, st, qn, G * D,
-                                  kn, G * D, g, H * D, beta, cu_seqlens, dm, scratch, total, kg, qg, ke);
-    if (rc) return rc;
-    const ChunkArgs a{one_decay ? qn : qg, one_decay ? kn : kg, ke, total, v, H * Vd, scratch, state,
-                      cu_seqlens, slot_ids, o};
+  if (one_decay && scratch && D % 4 == 0 && Vd % 4 == 0 && D <= 256 && B <= 65535 && G <= 65535 &&
+      (((uintptr_t)qn | (uintptr_t)kn | (uintptr_t)v | (uintptr_t)scratch) & 15) == 0) {
+    const int chunks = (max_q_len + CT - 1) / CT;
+    if (int rc = launch_kernel(delta_chunk_coef_kernel, dim3((chunks + 3) / 4, B, G), dim3(128), 0, st,
+                               qn, kn, g, beta, cu_seqlens, dm, scratch))
+      return rc;
+    const ChunkArgs a{qn, kn, nullptr, nullptr, v, H * Vd, scratch, state, cu_seqlens, slot_ids, o};
 #define GF_GO(DPER, LANES)                                                                         \
-  if (D <= DPER * LANES)                                                                           \
-    return one_decay ? launch_chunks<DPER, LANES, HEADS>(B, dm, a, st)                             \
-                     : launch_chunks<DPER, LANES, CHANNELS>(B, dm, a, st);
+  if (D <= DPER * LANES) return launch_chunks<DPER, LANES, HEADS>(B, dm, a, st);
     GF_GO(4, 8)
     GF_GO(8, 8)
     GF_GO(16, 8)             // (sixteen lanes of 8 rows: 348 us for a prompt that takes 317 so)
@@ -1084,10 +1059,9 @@ GF_EXPORT int gf_decay_channels_chunked(const float* q, int ld_q, const float* k
   auto st = (cudaStream_t)stream;
   const size_t chunks = (size_t)(T / CT + B + 1) * H, HTD = (size_t)T * H * D;
   float *total = scratch + chunks * kCoefs, *qg = total + chunks * D, *ke = qg + HTD;
-  if (int rc = launch_kernel(delta_chunk_coef_channels_kernel<false>,
-                             dim3(((max_q_len + CT - 1) / CT + 3) / 4, B, H), dim3(128), 0, st, q, ld_q, k,
-                             ld_k, g, ld_g, (const float*)nullptr, cu_seqlens, dm, scratch, total,
-                             (float*)nullptr, qg, ke))
+  if (int rc = launch_kernel(linear_chunk_coef_kernel, dim3(((max_q_len + CT - 1) / CT + 3) / 4, B, H),
+                             dim3(128), 0, st, q, ld_q, k, ld_k, g, ld_g, cu_seqlens, dm, scratch, total, qg,
+                             ke))
     return rc;
   const ChunkArgs a{qg, nullptr, ke, total, v, ld_v, scratch, state, cu_seqlens, slot_ids, o};
   if (D <= 32) return launch_chunks<4, 8, PLAIN>(B, dm, a, st);

@@ -10,7 +10,8 @@ from . import _code, _cuda, _fn, _ok, _p, _stream
 
 
 MAX_KEY_SIZE = 256        # the recurrence kernel's largest
-# Steps with a portion of at least this many tokens take the recurrence eight tokens at a time.
+# Steps with a portion of at least this many tokens take the recurrence with one decay a head eight
+# tokens at a time.
 CHUNKED_MIN_TOKENS = 16
 
 
@@ -113,16 +114,16 @@ def chunk_words(T: int, B: int, H: int, D: int, one_decay: int) -> int:
 
 def recurrence(qn, kn, v, g, beta, state: torch.Tensor, ctx) -> torch.Tensor:
     """Advance every request's state over its tokens of this step; returns ``o [T, H, Vd]`` fp32.
-    ``g``: ``[T, H, D]``, or ``[T, H]`` for one decay a head.  Long portions go eight tokens at a
-    time."""
+    ``g``: ``[T, H, D]``, or ``[T, H]`` for one decay a head (long portions then go eight tokens at a
+    time, and steps of single tokens on a kernel of their own; with a decay a channel every step goes token
+    by token, so that a token's bits do not depend on how the portions are cut)."""
     T, G, D = qn.shape
     H, Vd = v.shape[1], v.shape[2]
     o = torch.empty((T, H, Vd), dtype=torch.float32, device=qn.device)
     f = _fn("delta_rule", "gf_delta_recurrence",
-            [c_void_p] * 8 + [c_int] * 7 + [c_void_p, c_int, c_void_p, c_int, c_void_p])
+            [c_void_p] * 8 + [c_int] * 6 + [c_void_p, c_int, c_void_p, c_int, c_void_p])
     one = int(g.dim() == 2)
-    # (a context that does not say how long its portions are: token by token)
-    scratch, longest = None, int(getattr(ctx, "max_q_len", 0))
+    scratch, longest = None, int(ctx.max_q_len) if one else 0
     if longest == 1 and state_step(qn.view(T, G * D), kn.view(T, G * D), v.view(T, H * Vd), g.view(T, -1),
                                    state, ctx, H, G, D, Vd, o.view(T, H * Vd), beta=beta):
         return o
@@ -130,7 +131,7 @@ def recurrence(qn, kn, v, g, beta, state: torch.Tensor, ctx) -> torch.Tensor:
         scratch = torch.empty(chunk_words(T, ctx.num_seqs, H, D, one), dtype=torch.float32,
                               device=qn.device)
     rc = f(_p(qn), _p(kn), _p(v), _p(g), _p(beta), _p(state), _p(ctx.cu_seqlens_q),
-           _p(ctx.slot_ids), T, ctx.num_seqs, H, G, D, Vd, state.stride(0), _p(o), one,
+           _p(ctx.slot_ids), ctx.num_seqs, H, G, D, Vd, state.stride(0), _p(o), one,
            _p(scratch), longest, _stream())
     if rc == -3:
         raise ValueError(f"the delta-rule recurrence takes key sizes up to {MAX_KEY_SIZE}, got {D}")

@@ -553,10 +553,10 @@ def test_grouped_products_that_stream_the_weights(K, F, T, E, top):
                                            (2, 2, 128, 128, [33, 17]), (3, 3, 100, 36, [24, 25, 31, 1]),
                                            (2, 1, 256, 48, [65]), (1, 1, 128, 4, [1, 1, 23]),
                                            (8, 8, 128, 100, [17] * 6)])
-def test_delta_rule_with_channel_decays_eight_tokens_at_a_time(H, G, D, Vd, lens):
-    """Chunks whole and cut, portions shorter than a chunk, one and two columns a lane, decays from none
-    to all gone: outputs and states against the recurrence token by token in 64 bits, beside the
-    token-by-token kernel."""
+def test_delta_rule_with_channel_decays(H, G, D, Vd, lens):
+    """Portions of one token and of many, decays from none to all gone: outputs and states against the
+    recurrence in 64 bits, and equal bit for bit however the portions are cut into steps (a router behind
+    the layer makes close calls)."""
     from types import SimpleNamespace
     from ginfer_b200.ops import delta
     g0 = torch.Generator().manual_seed(D + Vd)
@@ -577,6 +577,23 @@ def test_delta_rule_with_channel_decays_eight_tokens_at_a_time(H, G, D, Vd, lens
                               max_q_len=longest)
         o = delta.recurrence(q.cuda(), k.cuda(), v.cuda(), g.cuda(), beta.cuda(), state, ctx)
         got.append((o.cpu().double(), state.cpu()))
+    # the same portions in two steps, and a token a step
+    for at in ([max(n // 2, n - 16) for n in lens], None):
+        state, o = state0.clone().cuda(), torch.empty_like(got[0][0])
+        for step in range(2 if at else max(lens)):
+            lo = [0 if not step else a for a in at] if at else [min(step, n) for n in lens]
+            hi = [(at if not step else lens)[b] if at else min(step + 1, n) for b, n in enumerate(lens)]
+            live = [b for b in range(B) if hi[b] > lo[b]]
+            if len(live) < B and not at:              # (the kernel's lanes are chosen by the requests' number)
+                break
+            rows = torch.cat([torch.arange(int(cu[b]) + lo[b], int(cu[b]) + hi[b]) for b in live])
+            ctx = SimpleNamespace(num_seqs=B, slot_ids=slots.int().cuda(), max_q_len=max(h - a for a, h in zip(lo, hi)),
+                                  cu_seqlens_q=torch.tensor([0] + [h - a for a, h in zip(lo, hi)]).cumsum(0).int().cuda())
+            part = delta.recurrence(*(t[rows].cuda() for t in (q, k, v, g, beta)), state, ctx).cpu().double()
+            o[rows] = part
+            assert torch.equal(part, got[0][0][rows])
+        if at:
+            assert torch.equal(o, got[0][0]) and torch.equal(state.cpu(), got[0][1])
     err = [0.0, 0.0]
     for b in range(B):
         S = state0[slots[b], :H * D * Vd].double().reshape(H, D, Vd).clone()
