@@ -115,7 +115,7 @@ def sumsq_ld(M: int) -> int:
 
 def gemm(x, weight, bias_f32=None, out_dtype=torch.bfloat16, epi: int = 0, split_k=None,
          through_workspace: bool = False, scale: RowScale | None = None, resid=None, gamma=None,
-         act_consts=None):
+         act_consts=None, streamed: bool = True):
     """``x [M, K] @ weight[N, K]^T``; ``epi`` 0: (+ bias) -> ``[M, N]``; ``epi`` 1: the same
     through ``relu(.)^2``; ``epi`` 4: the same through xIELU with ``act_consts = (a, b)`` (``a z^2 +
     z/2`` above zero, ``b (e^z - 1 - z) + z/2`` below); ``epi`` 2: weight rows
@@ -125,6 +125,7 @@ def gemm(x, weight, bias_f32=None, out_dtype=torch.bfloat16, epi: int = 0, split
     is multiplied by its factor first (a deferred RMS normalisation).  ``resid`` (fp32 ``[M, N]``): the result
     is ``(s, scaled, sumsq)`` with ``s = resid + x W^T (+ bias)`` in fp32, ``scaled = bf16(s *
     gamma)`` (``None`` without ``gamma``) and the partial sums of squares of ``s``'s rows.
+    ``streamed``: up to 8 rows may run on the register-streaming kernel (see :func:`stream`).
     Returns ``None`` if the kernel cannot serve the shape."""
     if not supports(x, weight):
         return None
@@ -139,7 +140,7 @@ def gemm(x, weight, bias_f32=None, out_dtype=torch.bfloat16, epi: int = 0, split
     out = torch.empty((M, cols), dtype=out_dtype, device=x.device)
     if M == 0:
         return out if resid is None else None
-    if (M <= STREAM_MAX_TOKENS and N * K <= STREAM_MAX_WEIGHTS and split_k is None
+    if (streamed and M <= STREAM_MAX_TOKENS and N * K <= STREAM_MAX_WEIGHTS and split_k is None
             and (M <= STREAM_MAX_TOKENS_BF16 or out_dtype == torch.float32 or epi != 0)
             and not through_workspace and scale is None and resid is None
             and stream(x, weight, bias_f32, out, epi, act_consts)):
@@ -232,14 +233,15 @@ def plain_limit(weight) -> int:
 _ACTIVATION_EPILOGUES = {None: 0, "relu2": 1, "xielu": 4}
 
 
-def try_linear(x, weight, bias_f32, out_dtype, activation: str | None = None, act_consts=None):
-    """Run the tcgen05 kernel where it is the faster one (the small batches of decode steps and
+def try_linear(x, weight, bias_f32, out_dtype, activation: str | None = None, act_consts=None,
+               streamed: bool = True):
+    """Run the tcgen05 kernel, or the register-streaming one, where it is the faster one (the small batches of decode steps and
     short prompt portions); ``None`` hands the product to cuBLAS.  ``activation``: the
     result passes it in the kernel's epilogue (see :func:`gemm`)."""
     if x.shape[0] > plain_limit(weight):
         return None
     return gemm(x, weight, bias_f32, out_dtype, epi=_ACTIVATION_EPILOGUES[activation],
-                act_consts=act_consts)
+                act_consts=act_consts, streamed=streamed)
 
 
 # Plain products leave for cuBLAS above this many tokens.  In a CUDA graph on a B200, 1.5B shapes,

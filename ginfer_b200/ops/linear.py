@@ -38,17 +38,18 @@ class Linear:
     output head).  ``activation``: the product passes ``"relu2"`` (``relu(.)^2``) or ``"xielu"``
     (``act_consts = (a, b)``: ``a z^2 + z/2`` above zero, ``b (e^z - 1 - z) + z/2`` below), in the
     product's epilogue where the tcgen05 kernel runs it (few tokens), else in a kernel behind the
-    library's."""
+    library's.  ``streamed`` false: products of few rows stay off the register-streaming kernel
+    (``csrc/gemm_stream.cu``), which sums in another order than the tcgen05 kernel."""
 
     def __init__(self, weight: torch.Tensor, bias: torch.Tensor | None = None,
                  out_dtype: torch.dtype | None = None, activation: str | None = None,
-                 act_consts: tuple[float, float] | None = None):
+                 act_consts: tuple[float, float] | None = None, streamed: bool = True):
         _cuda(weight, bias)
         if activation not in (None, "relu2", "xielu"):
             raise ValueError(f"activation {activation!r}: 'relu2' and 'xielu' are there")
         if (activation == "xielu") != (act_consts is not None):
             raise ValueError("'xielu' takes two constants, other activations none")
-        self.activation, self.act_consts = activation, act_consts
+        self.activation, self.act_consts, self.streamed = activation, act_consts, bool(streamed)
         self.weight = weight.contiguous()
         self.bias = bias
         self.out_features, self.in_features = weight.shape
@@ -70,7 +71,8 @@ class Linear:
         if (self.dtype == torch.bfloat16 and not hasattr(x, "materialize")
                 and x.dtype == self.dtype):
             y = gemm_bf16.try_linear(x, self.weight, self._bias_f32, self.out_dtype,
-                                     activation=self.activation, act_consts=self.act_consts)
+                                     activation=self.activation, act_consts=self.act_consts,
+                                     streamed=self.streamed)
             if y is not None:
                 return y
         return activation_(self._product(x), self.activation, *(self.act_consts or ()))
@@ -83,7 +85,8 @@ class Linear:
         if (self.activation is None and self.dtype == torch.bfloat16 and self.bias is not None
                 and self.out_dtype == torch.float32 and not hasattr(x, "materialize")
                 and x.dtype == self.dtype):
-            y = gemm_bf16.try_linear(x, self.weight, self._bias_f32, self.out_dtype)
+            y = gemm_bf16.try_linear(x, self.weight, self._bias_f32, self.out_dtype,
+                                     streamed=self.streamed)
             if y is not None:
                 return y, None
             return torch.mm(x, self.weight.t(), out_dtype=torch.float32), self._bias_f32
@@ -101,7 +104,7 @@ class Linear:
             raise TypeError(f"Linear holds {self.dtype} weights but got {x.dtype} input")
         if self.dtype == torch.float32:
             return gemm_f32(x, self.weight, self.bias)
-        y = gemm_bf16.try_linear(x, self.weight, self._bias_f32, self.out_dtype)
+        y = gemm_bf16.try_linear(x, self.weight, self._bias_f32, self.out_dtype, streamed=self.streamed)
         if y is not None:
             return y
         if self.out_dtype == torch.float32:
@@ -150,10 +153,11 @@ class GatedLinear:
     sigmoid(alpha * min(g, limit)) * (clamp(u, -limit, limit) + up_shift)``; the kernels' gated
     epilogues take the three constants where a plain product would take its bias."""
 
-    def __init__(self, gate: torch.Tensor, up: torch.Tensor, clamped=None):
+    def __init__(self, gate: torch.Tensor, up: torch.Tensor, clamped=None, streamed: bool = True):
         assert gate.shape == up.shape and gate.dtype == up.dtype
         self.intermediate, k = gate.shape
-        self.proj = Linear(torch.stack([gate, up], dim=1).reshape(2 * self.intermediate, k))
+        self.proj = Linear(torch.stack([gate, up], dim=1).reshape(2 * self.intermediate, k),
+                           streamed=streamed)
         self.clamped = None if clamped is None else tuple(float(c) for c in clamped)
         self.act = None if clamped is None else torch.tensor(
             self.clamped, dtype=torch.float32, device=gate.device)
@@ -169,7 +173,8 @@ class GatedLinear:
             x = x.materialize()
         if x.dtype == torch.bfloat16:
             if x.shape[0] <= gemm_bf16.MAX_TOKENS:
-                z = gemm_bf16.gemm(x, self.proj.weight, self.act, torch.bfloat16, epi=2)
+                z = gemm_bf16.gemm(x, self.proj.weight, self.act, torch.bfloat16, epi=2,
+                                   streamed=self.proj.streamed)
                 if z is not None:
                     return z
             elif x.shape[0] >= PREFILL_GATED_MIN_TOKENS:

@@ -14,12 +14,13 @@ _tile_rows: dict = {}
 
 def tile_rows(tensor_cores) -> int:
     """Rows of a tile of the plain kernel (``False``), of the ``mma.sync`` kernel (``True``), of
-    the tcgen05 kernel (``"tcgen05"``) or of the weight-streaming kernel (``"few"``)."""
+    the tcgen05 kernel (``"tcgen05"``), of the weight-streaming kernel (``"few"``) or of the kernel with
+    plain multiply-adds for a handful of pairs (``"gemv"``)."""
     if tensor_cores not in _tile_rows:
         if tensor_cores == "tcgen05":
             _tile_rows[tensor_cores] = int(load_library("gemm_prefill").gf_gemm_grouped_tile_rows())
-        elif tensor_cores == "few":
-            _tile_rows[tensor_cores] = int(load_library("moe").gf_moe_tile_rows(2))
+        elif tensor_cores in ("few", "gemv"):
+            _tile_rows[tensor_cores] = int(load_library("moe").gf_moe_tile_rows(2 if tensor_cores == "few" else 3))
         else:
             _tile_rows[tensor_cores] = int(load_library("moe").gf_moe_tile_rows(int(tensor_cores)))
     return _tile_rows[tensor_cores]
@@ -37,18 +38,22 @@ TCGEN05_MIN_PAIRS = 1024
 # choices: 510 pairs 47 against 62.
 FEW_MAX_PAIRS = 768
 FEW_MAX_K = 4096
+# Without that kernel (``streamed`` false: its sums run in another order than those of the others), up
+# to this many pairs run on one that multiplies on the FMA pipes, more on the mma.sync kernel.
+GEMV_MAX_PAIRS = 20
 
 
-def kernel_for(x: torch.Tensor, pairs: int, reductions, widths) -> object:
+def kernel_for(x: torch.Tensor, pairs: int, reductions, widths, streamed: bool = True) -> object:
     """Which grouped-product kernel serves activations ``x`` with these reduction sizes and output
-    widths: ``"tcgen05"``, ``"few"`` (weights streamed), ``True`` (``mma.sync``) or ``False``
-    (plain)."""
+    widths: ``"tcgen05"``, ``"few"`` (weights streamed; not without ``streamed``), ``"gemv"`` (a handful
+    of pairs), ``True`` (``mma.sync``) or ``False`` (plain)."""
     if not (on_tensor_cores(x.dtype, *reductions) and x.stride(0) % 8 == 0):
         return False
     if pairs >= TCGEN05_MIN_PAIRS and all(n % 8 == 0 for n in widths):
         return "tcgen05"
-    if pairs <= FEW_MAX_PAIRS and max(reductions) <= FEW_MAX_K and all(n % 2 == 0 for n in widths):
-        return "few"
+    if (pairs <= (FEW_MAX_PAIRS if streamed else GEMV_MAX_PAIRS) and max(reductions) <= FEW_MAX_K
+            and all(n % 2 == 0 for n in widths)):
+        return "few" if streamed else "gemv"
     return True
 
 
@@ -127,6 +132,7 @@ class Plan:
         self.tcgen05 = tensor_cores == "tcgen05"
         self.few = tensor_cores == "few"
         self.tensor_cores = bool(tensor_cores)
+        self.kernel = {"few": 2, "gemv": 3}.get(tensor_cores, int(self.tensor_cores))
         rows = tile_rows(tensor_cores if isinstance(tensor_cores, str) else self.tensor_cores)
         P = T * top
         dev = idx.device
@@ -243,7 +249,7 @@ def _gemm(a, w, plan, out, first, limit, alpha, up_shift, row_w=None):
     _ok(f(_p(a), a.stride(0), _p(w), w.shape[1], w.shape[2], _p(plan.offsets),
           _p(plan.pair_of_pos), plan.top, _p(plan.tile_expert), _p(plan.tile_row0),
           _p(plan.num_tiles), plan.max_tiles, _p(out), int(first), float(limit), float(alpha),
-          float(up_shift), _p(row_w), _code(a.dtype), 2 if plan.few else int(plan.tensor_cores),
+          float(up_shift), _p(row_w), _code(a.dtype), plan.kernel,
           _stream(), plan.pairs),
         "moe_gemm")
 

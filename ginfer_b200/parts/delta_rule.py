@@ -30,13 +30,15 @@ from .base import Mixer, StateSpec, TensorSpec, register_mixer
 class ChannelDelta(Mixer):
     def __init__(self, hidden_size: int, num_heads: int, num_kv_heads: int, key_dim: int,
                  v_dim: int, conv_taps: int, out_norm_eps: float = 1e-6,
-                 decay_rank: int = -1, gate_rank: int = -1, prefix: str = "mix"):
+                 decay_rank: int = -1, gate_rank: int = -1, prefix: str = "mix",
+                 streamed: bool = True):
         if num_heads % num_kv_heads:
             raise ValueError(f"{num_heads} heads are not a multiple of {num_kv_heads} kv heads")
         self.hidden_size, self.H, self.G = int(hidden_size), int(num_heads), int(num_kv_heads)
         self.D, self.Vd, self.taps = int(key_dim), int(v_dim), int(conv_taps)
         self.eps = float(out_norm_eps)
         self.decay_rank, self.gate_rank = int(decay_rank), int(gate_rank)   # -1: the file's
+        self.streamed = bool(streamed)                                      # see ops.Linear
         self.prefix = prefix + "." if prefix else ""
         self.channels = 2 * self.G * self.D + self.H * self.Vd
         self.state_floats = self.H * self.D * self.Vd
@@ -73,14 +75,14 @@ class ChannelDelta(Mixer):
         pad = -n % 8
         if pad:
             rows.append(torch.zeros((pad, self.hidden_size), dtype=rows[0].dtype, device=device))
-        self.first = ops.Linear(torch.cat(rows, dim=0))
+        self.first = ops.Linear(torch.cat(rows, dim=0), streamed=self.streamed)
         self.a1_off = self.channels
         self.g1_off = self.a1_off + ra
         self.b_off = self.g1_off + rg
         self.ra, self.rg = ra, rg
-        self.decay = ops.Linear(t["a2"], None, out_dtype=torch.float32)
-        self.gate = ops.Linear(t["g2"])
-        self.out = ops.Linear(t["o"], None, out_dtype=torch.float32)
+        self.decay = ops.Linear(t["a2"], None, out_dtype=torch.float32, streamed=self.streamed)
+        self.gate = ops.Linear(t["g2"], streamed=self.streamed)
+        self.out = ops.Linear(t["o"], None, out_dtype=torch.float32, streamed=self.streamed)
         self.conv_w = torch.cat([t["q.conv"], t["k.conv"], t["v.conv"]], dim=0).float().contiguous()
         self.A_log = t["A_log"].float().contiguous()
         self.dt_bias = t["dt_bias"].float().contiguous()

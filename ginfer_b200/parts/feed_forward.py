@@ -61,8 +61,10 @@ class ClampedGLU(FeedForward):
 
     def __init__(self, hidden_size: int, intermediate_size: int, limit: float,
                  alpha: float = 1.702, up_shift: float = 1.0, prefix: str = "mlp",
-                 gate_name: str = "gate", up_name: str = "up", down_name: str = "down"):
+                 gate_name: str = "gate", up_name: str = "up", down_name: str = "down",
+                 streamed: bool = True):
         self.hidden_size, self.intermediate_size = int(hidden_size), int(intermediate_size)
+        self.streamed = bool(streamed)                 # see ops.Linear
         self.limit, self.alpha, self.up_shift = float(limit), float(alpha), float(up_shift)
         p = prefix + "." if prefix else ""
         self.gate_key, self.up_key, self.down_key = p + gate_name, p + up_name, p + down_name
@@ -74,8 +76,10 @@ class ClampedGLU(FeedForward):
 
     def load(self, tensors, dtype, device):
         self.gate_up = ops.GatedLinear(tensors[self.gate_key], tensors[self.up_key],
-                                       clamped=(self.limit, self.alpha, self.up_shift))
-        self.down = ops.Linear(tensors[self.down_key], None, out_dtype=torch.float32)
+                                       clamped=(self.limit, self.alpha, self.up_shift),
+                                       streamed=self.streamed)
+        self.down = ops.Linear(tensors[self.down_key], None, out_dtype=torch.float32,
+                               streamed=self.streamed)
 
     def forward(self, x, ctx):
         return self.down(self.gate_up(x))

@@ -40,7 +40,8 @@ class LatentAttention(Mixer):
     def __init__(self, hidden_size: int, num_heads: int, nope_dim: int, rope_dim: int, v_dim: int,
                  kv_rank: int, scale: float, window: int = 0, rotary_dims: int | None = None,
                  rotary_base: float = 10000.0, latent_eps: float = 1e-6, prefix: str = "mix",
-                 q_rank: int = 0, head_gate: bool = False, own_latent: bool = True):
+                 q_rank: int = 0, head_gate: bool = False, own_latent: bool = True,
+                 streamed: bool = True):
         self.hidden_size, self.H = int(hidden_size), int(num_heads)
         self.D, self.R, self.Vd, self.C = int(nope_dim), int(rope_dim), int(v_dim), int(kv_rank)
         self.scale, self.window = float(scale), int(window)
@@ -50,6 +51,7 @@ class LatentAttention(Mixer):
         self.base, self.eps = float(rotary_base), float(latent_eps)
         self.prefix = prefix + "." if prefix else ""
         self.Q, self.gated, self.own = int(q_rank), bool(head_gate), bool(own_latent)
+        self.streamed = bool(streamed)                     # see ops.Linear
         if not self.own and self.R:
             raise ValueError("a layer that reads another layer's latent vectors has no rotated "
                              "key part of its own")
@@ -90,13 +92,14 @@ class LatentAttention(Mixer):
         n = sum(r.shape[0] for r in rows)
         if -n % 8 and not self.classic:
             rows.append(torch.zeros((-n % 8, self.hidden_size), dtype=rows[0].dtype, device=device))
-        self.q_dkv = ops.Linear(torch.cat(rows, dim=0) if len(rows) > 1 else rows[0])
+        self.q_dkv = ops.Linear(torch.cat(rows, dim=0) if len(rows) > 1 else rows[0],
+                                streamed=self.streamed)
         self.latent_w = tensors[self._n("dkv.norm")].float().contiguous() if self.own else None
         self.q_w = tensors[self._n("dq.norm")].float().contiguous() if self.Q else None
-        self.uq = ops.Linear(tensors[self._n("uq")]) if self.Q else None
+        self.uq = ops.Linear(tensors[self._n("uq")], streamed=self.streamed) if self.Q else None
         self.uk = tensors[self._n("uk")].view(H, D, C)                     # q_lat = q_plain @ uk[h]
         self.uv_t = tensors[self._n("uv")].view(H, Vd, C).transpose(1, 2)  # values = o_lat @ uv[h]^T
-        self.out = ops.Linear(tensors[self._n("o")], None, out_dtype=torch.float32)
+        self.out = ops.Linear(tensors[self._n("o")], None, out_dtype=torch.float32, streamed=self.streamed)
         i = np.arange(self.rot // 2, dtype=np.float64)
         freq = np.power(np.float64(self.base), -2.0 * i / self.rot).astype(np.float32)
         self.freq = torch.from_numpy(freq).to(device)

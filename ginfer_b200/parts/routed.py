@@ -24,11 +24,12 @@ from .linear_attention import joined_rows
 class RoutedGLU(FeedForward):
     def __init__(self, hidden_size: int, intermediate_size: int, limit: float, num_experts: int,
                  top_k: int, renormalize: bool = False, alpha: float = 1.702,
-                 up_shift: float = 1.0, prefix: str = "mlp"):
+                 up_shift: float = 1.0, prefix: str = "mlp", streamed: bool = True):
         self.hidden_size, self.intermediate_size = int(hidden_size), int(intermediate_size)
         self.E, self.top = int(num_experts), int(top_k)
         if not (0 < self.top <= self.E):
             raise ValueError(f"{self.top} of {self.E} experts cannot be chosen")
+        self.streamed = bool(streamed)         # see ops.Linear and moe.kernel_for
         self.limit, self.alpha, self.up_shift = float(limit), float(alpha), float(up_shift)
         self.renormalize = bool(renormalize)
         self.prefix = prefix + "." if prefix else ""
@@ -50,7 +51,8 @@ class RoutedGLU(FeedForward):
         self.w_gate_up = torch.stack(gu).contiguous()                       # [E, 2 F, H]
         self.w_down = torch.stack([tensors[f"{self.prefix}e{e}.down"]
                                    for e in range(self.E)]).contiguous()    # [E, H, F]
-        self.router = ops.Linear(tensors[self.prefix + "router"], None, out_dtype=torch.float32)
+        self.router = ops.Linear(tensors[self.prefix + "router"], None, out_dtype=torch.float32,
+                                 streamed=self.streamed)
         self.act = torch.tensor([self.limit, self.alpha, self.up_shift], dtype=torch.float32,
                                 device=device)
 
@@ -61,7 +63,7 @@ class RoutedGLU(FeedForward):
         idx, wgt = moe.route(self.router(x), self.top, self.renormalize)
         plan = moe.Plan(idx, self.E, moe.kernel_for(
             x, T * self.top, (self.hidden_size, self.intermediate_size),
-            (self.intermediate_size, self.hidden_size)))
+            (self.intermediate_size, self.hidden_size), self.streamed))
         y = moe.grouped_glu(x, self.w_gate_up, plan, self.limit, self.alpha, self.up_shift,
                             act=self.act)
         rows = moe.grouped_down(y, self.w_down, plan)

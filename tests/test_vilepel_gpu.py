@@ -502,3 +502,56 @@ def test_latent_attention_of_a_token_does_not_depend_on_its_step(H, C, R, window
                                 table, ctx, window, 0.05, page)
     whole = run(0, T)
     assert torch.equal(whole, torch.cat([run(a, min(a + 110, T)) for a in range(0, T, 110)], dim=1))
+
+
+def test_layers_before_and_behind_routers_keep_their_kernels(monkeypatch, tmp_path):
+    """Prompts, decode steps of one and of several requests: no product of a layer runs on the kernels that
+    stream the weights through registers, and no recurrence on the kernel for single tokens (they sum in
+    another order than the kernels of longer steps)."""
+    from ginfer_b200.engine.runner import StepEntry
+    from ginfer_b200.ops import delta, gemm_bf16, moe
+    cfg = tv.config([tv.layer(tv.latent(), tv.dense()), tv.layer(tv.delta(vdim=16), tv.moe()),
+                     tv.layer(tv.latent(), tv.moe())], width=64)
+    streamed, kinds, step = [], [], delta.state_step
+    stream, kernel_for = gemm_bf16.stream, moe.kernel_for
+    monkeypatch.setattr(gemm_bf16, "stream", lambda x, w, *a, **k: streamed.append(w.shape[0]) or stream(x, w, *a, **k))
+    monkeypatch.setattr(delta, "state_step", lambda *a, **k: streamed.append("step") or step(*a, **k))
+    monkeypatch.setattr(moe, "kernel_for", lambda *a, **k: kinds.append(kernel_for(*a, **k)) or kinds[-1])
+    runner = make_runner(tv.write_folder(str(tmp_path), cfg, storage=torch.bfloat16), "bfloat16", 256)
+    for n in (1, 9, 40):
+        runner.step([StepEntry(n, list(range(n)), [n - 1])])
+    for live in ([1], [1, 9, 40]):
+        runner.step([StepEntry(r, [7], [0]) for r in live])
+    assert set(streamed) <= {cfg["vocab"]}                   # the head, behind the last router
+    assert set(kinds) == {"gemv", True}
+
+
+@pytest.mark.parametrize("K, F, T, E, top", [(8, 2, 1, 1, 1), (256, 136, 2, 6, 3), (1416, 34, 5, 4, 4),
+                                             (4096, 72, 12, 3, 1)])
+def test_grouped_products_of_a_handful_of_pairs_on_plain_multiply_adds(K, F, T, E, top):
+    """One pair to two tiles of an expert, reductions that fill no step of a warp: against 64 bits."""
+    from ginfer_b200.ops import moe
+    g = torch.Generator(device="cuda").manual_seed(K + F)
+    x = torch.randn(T, K, generator=g, device="cuda").bfloat16()
+    gate_up = (torch.randn(E, 2 * F, K, generator=g, device="cuda") * K ** -0.5).bfloat16()
+    idx = torch.rand(T, E, generator=g, device="cuda").argsort(1)[:, :top].int()
+    if T == 12:
+        idx[:9, 0] = 2                                       # nine pairs of one expert: two tiles
+    assert moe.kernel_for(x, T * top, (K, 8), (8, K), streamed=False) == "gemv"
+    plan = moe.Plan(idx, E, "gemv")
+    tok, exp = torch.arange(T, device="cuda").repeat_interleave(top), idx.reshape(-1).long()
+    place = plan.pos_of_pair.long()
+    h = torch.einsum("pk,pfk->pf", x[tok].double(), gate_up[exp].double())
+    size = torch.einsum("pk,pfk->pf", x[tok].double().abs(), gate_up[exp].double().abs()) * K * 2.0 ** -24
+    gt, u = h[:, 0::2], h[:, 1::2]
+    og, ou = (a.abs() * 2.0 ** -8 + e for a, e in ((gt, size[:, 0::2]), (u, size[:, 1::2])))
+    s = gt * torch.sigmoid(gt)                               # its slope is at most 1.1
+    off = 1.1 * og * (u.abs() + ou) + s.abs() * ou
+    y = moe.grouped_glu(x, gate_up, plan, 1e9, 1.0, 0.0)
+    assert ((y[place].double() - s * u).abs() <= off + 2.0 ** -8 * ((s * u).abs() + off) + 1e-6).all()
+    if F % 8 == 0:
+        down = (torch.randn(E, K, F, generator=g, device="cuda") * F ** -0.5).bfloat16()
+        yp = y[place].double()
+        want = torch.einsum("pf,pkf->pk", yp, down[exp].double())
+        size = torch.einsum("pf,pkf->pk", yp.abs(), down[exp].double().abs())
+        assert ((moe.grouped_down(y, down, plan)[place].double() - want).abs() <= (F + 8) * 2.0 ** -24 * size).all()
