@@ -585,7 +585,7 @@ __global__ void latent_merge_kernel(const float* __restrict__ part_o,
   for (int z = 0; z < kMaxSplits; ++z) M = fmaxf(M, m[z]);
 #pragma unroll
   for (int z = 0; z < kMaxSplits; ++z)
-    if (l[z] > 0.f) {                              // (an empty share's is 0)
+    if (l[z] != 0.f) {                             // (an empty share's is 0; a NaN stays one)
       const float w = expf(m[z] - M);
       L += l[z] * w;
 #pragma unroll

@@ -690,6 +690,12 @@ def test_shares_of_a_tokens_keys_are_put_together(C, lens):
         p = torch.softmax(q[:, b].double() @ c.t() * C ** -0.5, dim=-1)
         # probabilities and result are rounded to bf16: 2^-8 each, of at most sum p |c|
         assert ((out[:, b] - p @ c).abs() <= 2 * 2.0 ** -8 * (p @ c.abs()) + 1e-6).all()
+    # a key that is no number makes its request's outputs none, whichever share it falls into
+    for at in (0, lens[0] // 2, lens[0] - 1):
+        bad = pages.clone()
+        bad[int(table[0, at // page]), at % page, 0, 3] = float("nan")
+        got = latent.attention(q, None, bad, None, table, ctx, 0, C ** -0.5, page).double()
+        assert got[:, 0].isnan().all() and torch.equal(got[:, 1:], out[:, 1:])
 
 
 @pytest.mark.parametrize("H,G,D,Vd,B", [(2, 1, 12, 20, 3), (4, 2, 64, 64, 1), (16, 16, 128, 128, 5), (3, 3, 100, 36, 2),
