@@ -1,4 +1,4 @@
-// One token of every request through the recurrences over per-request state S [H, D, Vd] (decode steps):
+// One token (or none) of every request through the recurrences over per-request state S [H, D, Vd] (decode steps):
 //
 //   linear   S <- g S + (c k) v^T,                      o = S^T q + skip_h v
 //   delta    S <- g S, u = beta (v - S^T k), S <- S + k u^T, o = S^T q      (= S'^T q + u (k . q), S' = g S)
@@ -38,6 +38,7 @@ state_step_kernel(const StepArgs a) {
   pdl_trigger();
   pdl_wait();
   const size_t r = a.cu_seqlens[b];
+  if (a.cu_seqlens[b + 1] == (int)r) return;         // a request without a token: no row, no change
   const int kvh = h / (a.H / a.G);
   float* S = a.state + (size_t)a.slot_ids[b] * a.state_stride + (size_t)h * D * Vd + col;
   float s[NR][4];
@@ -172,7 +173,7 @@ GF_DEFINE_PDL_SWITCH
 
 // Rows of q and k: G heads of D; v and o: H of Vd; g: H (gD 1) or H of D (gD D); c: H; beta [B, H] by token
 // (null: the linear form, which may have c and skip).  Every request of the step has one token, at row
-// cu_seqlens[b].  Returns -6 for what it does not take (keys over 256, values, rows, slots or addresses that
+// cu_seqlens[b], or none (cu_seqlens[b + 1] == cu_seqlens[b]).  Returns -6 for what it does not take (keys over 256, values, rows, slots or addresses that
 // are no multiples of four floats).
 GF_EXPORT int gf_state_step(const float* q, int ld_q, const float* k, int ld_k, const float* v, int ld_v,
                             const float* g, int ld_g, int gD, const float* c, int ld_c, const float* skip,

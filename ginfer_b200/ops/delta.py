@@ -86,7 +86,7 @@ def prepare_heads(proj: torch.Tensor, a_off: int, b_off: int, conv_w: torch.Tens
 
 def state_step(q, k, v, g, state, ctx, H: int, G: int, D: int, Vd: int, o, c=None, skip=None,
                beta=None) -> bool:
-    """One token of every request (``csrc/state_step.cu``): rows of ``q``, ``k`` (``G D``), ``v``, ``o``
+    """One token, or none, of every request (``csrc/state_step.cu``): rows of ``q``, ``k`` (``G D``), ``v``, ``o``
     (``H Vd``), ``g`` (``H`` or ``H D``) and ``c`` (``H``), all fp32 with a row stride; with ``beta [T, H]``
     the delta rule, else ``S <- g S + c k v^T``.  ``False`` where the kernel does not take the case."""
     f = _fn("state_step", "gf_state_step",

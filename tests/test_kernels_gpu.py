@@ -744,6 +744,34 @@ def test_one_token_of_every_request_through_its_state(H, G, D, Vd, B, channels, 
     assert torch.equal(state[rest], state0[rest])
 
 
+@pytest.mark.parametrize("rule", ["delta", "linear"])
+@pytest.mark.parametrize("lens", [[1, 0, 1], [0, 1], [1, 1, 0, 0]])
+def test_requests_without_a_token_keep_their_state(rule, lens):
+    """Steps of single tokens in which some requests bring none, the last one among them: as if those were
+    not in the step."""
+    from types import SimpleNamespace
+    from ginfer_b200.ops import decay, delta
+    H, D, Vd, B, T = 2, 16, 8, len(lens), sum(lens)
+    g0 = torch.Generator(device=DEV).manual_seed(B)
+    q, k, v, state0 = (torch.randn(*s, generator=g0, device=DEV)
+                       for s in ((T, H, D), (T, H, D), (T, H, Vd), (B + 1, H * D * Vd)))
+    g, beta = torch.rand(T, H, generator=g0, device=DEV), torch.rand(T, H, generator=g0, device=DEV)
+    got = []
+    for who in (range(B), [b for b in range(B) if lens[b]]):
+        ctx = SimpleNamespace(num_seqs=len(who), slot_ids=torch.tensor(who, dtype=torch.int32, device=DEV),
+                              max_q_len=1, q_lens_host=[lens[b] for b in who],
+                              cu_seqlens_q=torch.tensor([0] + [lens[b] for b in who], device=DEV).cumsum(0).int())
+        state = state0.clone()
+        if rule == "delta":
+            o = delta.recurrence(q, k, v, g, beta, state, ctx)
+        else:
+            o = decay.recurrence(q.view(T, -1), k.view(T, -1), v.view(T, -1), g, state, ctx, H, H, D, Vd)
+        got.append((o, state))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    for b in range(B + 1):
+        assert torch.equal(got[0][1][b], state0[b]) == (b == B or not lens[b])
+
+
 @pytest.mark.parametrize("T,top,N", [(1, 1, 4), (3, 4, 2048), (5, 6, 516), (2, 9, 37), (40, 2, 130)])
 @pytest.mark.parametrize("weighted", [False, True])
 def test_pairs_rows_are_added_up_in_the_order_chosen(T, top, N, weighted):
