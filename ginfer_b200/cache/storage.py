@@ -78,7 +78,8 @@ class CacheStorage:
         self.num_slots = num_slots
         self.state = {cid: torch.zeros((num_slots + 1, *s.shape), dtype=s.dtype, device=device)
                       for cid, s in cache_specs.items() if isinstance(s, StateSpec)}
-        self._spans = None           # the states' addresses and slot sizes on the device
+        # the states' addresses and slot sizes, and the same on the device
+        self._span_rows, self._spans = None, None
 
     def group_of(self, cache_id: int) -> int:
         return self._where[cache_id][0]
@@ -97,18 +98,25 @@ class CacheStorage:
         return cache_id in self._where
 
     def reset_slots(self, slots: list[int]) -> None:
-        """The slots' state becomes zero, all of it by one kernel."""
+        """The slots' state becomes zero: on a device all of it by one kernel."""
         if not self.state or not slots:
             return
         if any(not 0 <= s <= self.num_slots for s in slots):
             raise IndexError(f"slots {slots} of {self.num_slots}")
-        if self._spans is None:
-            self._spans = torch.tensor([[t.data_ptr(), t.stride(0) * t.element_size()]
-                                        for t in self.state.values()], dtype=torch.int64,
-                                       device=next(iter(self.state.values())).device)
+        rows = []
+        for t in self.state.values():
+            if t.is_cuda and t.is_contiguous():
+                if t.numel():
+                    rows.append([t.data_ptr(), t.stride(0) * t.element_size()])
+            else:
+                for s in slots:
+                    t[s].zero_()
+        if not rows:
+            return
+        if rows != self._span_rows:      # (a state's tensor may have been replaced)
+            self._span_rows = rows
+            self._spans = torch.tensor(rows, dtype=torch.int64, device=next(
+                t.device for t in self.state.values() if t.is_cuda))
         from ..ops import zero_slots
         with torch.cuda.device(self._spans.device):      # (a step is prepared outside any guard)
             zero_slots(self._spans, slots)
-
-    def reset_slot(self, slot: int) -> None:
-        self.reset_slots([slot])

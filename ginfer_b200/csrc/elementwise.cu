@@ -10,7 +10,6 @@ namespace gf {
 // one kernel does.
 struct SlotList {
   static constexpr int kMax = 64;
-  int count;
   int slot[kMax];
 };
 __global__ void zero_slots_kernel(const longlong2* __restrict__ spans, const SlotList list) {
@@ -21,8 +20,10 @@ __global__ void zero_slots_kernel(const longlong2* __restrict__ spans, const Slo
   const long long at = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
   if (((uintptr_t)base | s.y) % 16 == 0)
     for (long long i = at; i < s.y / 16; i += step) reinterpret_cast<uint4*>(base)[i] = make_uint4(0, 0, 0, 0);
-  else
+  else if (((uintptr_t)base | s.y) % 4 == 0)
     for (long long i = at; i < s.y / 4; i += step) reinterpret_cast<uint32_t*>(base)[i] = 0;
+  else
+    for (long long i = at; i < s.y; i += step) base[i] = 0;
 }
 
 // ----------------------------------------------------------------------------- embedding
@@ -438,14 +439,14 @@ GF_EXPORT int gf_rope_kv_write(void* qkv, int row_stride, const float* table, in
 }
 
 // spans[i] = {address of a state's first slot, bytes a slot}, i < n; the slots named by `slots` (host) of
-// each become zero.  Slot sizes are multiples of four bytes.
+// each become zero.
 GF_EXPORT int gf_zero_slots(const long long* spans, int n, const int* slots, int count, void* stream) {
   for (int at = 0; at < count; at += SlotList::kMax) {
     SlotList list;
-    list.count = count - at < SlotList::kMax ? count - at : SlotList::kMax;
-    for (int i = 0; i < list.count; ++i) list.slot[i] = slots[at + i];
+    const int here = count - at < SlotList::kMax ? count - at : SlotList::kMax;
+    for (int i = 0; i < here; ++i) list.slot[i] = slots[at + i];
     if (n <= 0) return 0;
-    const int rc = launch_kernel(zero_slots_kernel, dim3(16, n, list.count), dim3(256), 0,
+    const int rc = launch_kernel(zero_slots_kernel, dim3(16, n, here), dim3(256), 0,
                                  (cudaStream_t)stream, (const longlong2*)spans, list);
     if (rc) return rc;
   }

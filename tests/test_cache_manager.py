@@ -237,3 +237,18 @@ def test_native_manager_does_what_the_python_manager_does(seed):
                 (rb.slot, rb.num_tokens, rb.reserved, rb.first_page, rb.next_page)
         for ta, tb in zip(a.tables, b.tables):
             assert (ta == tb).all()
+
+
+def test_a_storage_on_the_host_clears_slots():
+    import torch
+    from ginfer_b200.cache.storage import CacheStorage
+    from ginfer_b200.parts.base import StateSpec
+    st = CacheStorage({0: StateSpec((5, 3)), 1: StateSpec((3,), torch.bfloat16), 2: StateSpec((0,))}, [], [], 16, 4,
+                      torch.float32, "cpu")
+    for t in st.state.values():
+        t.fill_(1)
+    st.reset_slots([1, 4])
+    for t in st.state.values():
+        assert t[[1, 4]].eq(0).all() and t[[0, 2, 3]].eq(1).all()
+    with pytest.raises(IndexError):
+        st.reset_slots([5])

@@ -617,10 +617,12 @@ def test_delta_rule_with_channel_decays(H, G, D, Vd, lens):
 
 @pytest.mark.parametrize("slots", [[2], [0, 4, 1], list(range(69, -1, -1))])
 def test_zero_slots_clears_the_named_slots_of_every_state(slots):
-    """States of several types and slot sizes (whole 16 bytes and not), more slots than a launch names."""
+    """States of several types and slot sizes (whole 16 bytes, whole words, and neither), more slots than a
+    launch names."""
     n = max(max(slots) + 2, 6)
     states = [torch.ones((n, 7), dtype=torch.int32, device=DEV), torch.ones((n, 1), dtype=torch.int32, device=DEV),
-              torch.ones((n, 12345), device=DEV), torch.ones((n, 64), device=DEV)]
+              torch.ones((n, 12345), device=DEV), torch.ones((n, 64), device=DEV),
+              torch.ones((n, 3), dtype=torch.bfloat16, device=DEV), torch.ones((n, 5), dtype=torch.int8, device=DEV)]
     from ginfer_b200 import ops
     spans = torch.tensor([[t.data_ptr(), t.stride(0) * t.element_size()] for t in states], device=DEV)
     ops.zero_slots(spans, slots)
@@ -628,6 +630,20 @@ def test_zero_slots_clears_the_named_slots_of_every_state(slots):
         want = torch.ones(n, dtype=torch.bool, device=DEV)
         want[slots] = False
         assert torch.equal((t == 1).all(dim=1), want) and torch.equal((t == 0).all(dim=1), ~want)
+
+
+def test_a_storage_clears_the_tensors_it_holds_now():
+    """States of other types than the engine's own, and one that has been replaced since the last time."""
+    from ginfer_b200.cache.storage import CacheStorage
+    from ginfer_b200.parts.base import StateSpec
+    st = CacheStorage({0: StateSpec((5, 3)), 1: StateSpec((3,), torch.bfloat16)}, [], [], 16, 4, torch.float32, DEV)
+    for again in range(2):
+        for t in st.state.values():
+            t.fill_(1)
+        st.reset_slots([1, 4])
+        for t in st.state.values():
+            assert t[[1, 4]].eq(0).all() and t[[0, 2, 3]].eq(1).all()
+        st.state[0] = torch.empty_like(st.state[0])
 
 
 @pytest.mark.parametrize("H,G,D,Vd,lens", [(2, 1, 12, 20, [64, 1, 7]), (4, 2, 64, 64, [80, 8, 9]),
