@@ -81,11 +81,11 @@ template <int MT, int VEC, int STAGES>
 __global__ void __launch_bounds__(32)
 gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W,
                      const float* __restrict__ bias, float* __restrict__ C, int M, int N, int K,
-                     int lda, int ldc, int seg) {
+                     int lda, int ldc, int seg, int ranks) {
   extern __shared__ __align__(16) uint8_t raw[];
   auto& sm = *reinterpret_cast<RowsShared<MT, STAGES>*>(raw);
   const int lane = threadIdx.x, half = lane >> 4, row = lane & 15;
-  const int rank = blockIdx.x, ranks = gridDim.x, n0 = blockIdx.y * 32;
+  const int rank = blockIdx.x % ranks, n0 = blockIdx.x / ranks * 32;     // (x: the grid's long side)
   const int kbase = 2 * rank * seg;                       // seg: a multiple of KS
   const int steps = max(0, min(seg, K - kbase) + KU - 1) / KU;
   pdl_trigger();
@@ -180,11 +180,11 @@ template <int BM, int VEC>
 __global__ void __launch_bounds__(BM * 2, BM == 128 ? 1 : BM == 64 ? 2 : 3)
 gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W,
                      const float* __restrict__ bias, float* __restrict__ C, int M, int N, int K,
-                     int lda, int ldc, int seg) {
+                     int lda, int ldc, int seg, int ranks) {
   extern __shared__ __align__(16) float ring[];           // TILE_STAGES x (BM + BN) rows of BP
   constexpr int THREADS = BM * 2, TY = BM / 8;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int rank = blockIdx.x, ranks = gridDim.x, n0 = blockIdx.y * BN, m0 = blockIdx.z * BM;
+  const int rank = blockIdx.x % ranks, n0 = blockIdx.x / ranks * BN, m0 = blockIdx.y * BM;
   const int kbase = rank * seg;
   const int steps = max(0, min(seg, K - kbase) + BK - 1) / BK;
   pdl_trigger();
@@ -270,18 +270,19 @@ struct F32Args {
 };
 
 template <typename Kernel>
-int start(Kernel* kernel, OncePerDevice& once, dim3 grid, int threads, size_t smem, const F32Args& a) {
+int start(Kernel* kernel, OncePerDevice& once, int ranks, int columns, int rows, int threads, size_t smem,
+          const F32Args& a) {
   const int rc = once.run([&] {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   });
   if (rc) return rc;
-  return launch_kernel_cluster_dims(kernel, grid, dim3(threads), smem, a.stream, (int)grid.x, true, a.A, a.W,
-                                    a.bias, a.C, a.M, a.N, a.K, a.lda, a.ldc, a.seg);
+  return launch_kernel_cluster_dims(kernel, dim3(ranks * columns, rows), dim3(threads), smem, a.stream, ranks,
+                                    true, a.A, a.W, a.bias, a.C, a.M, a.N, a.K, a.lda, a.ldc, a.seg, ranks);
 }
 
 template <int MT, int VEC, int STAGES> int start_rows_staged(const F32Args& a) {
   static OncePerDevice once;
-  return start(gemm_f32_rows_kernel<MT, VEC, STAGES>, once, dim3(a.segments / 2, (a.N + 31) / 32), 32,
+  return start(gemm_f32_rows_kernel<MT, VEC, STAGES>, once, a.segments / 2, (a.N + 31) / 32, 1, 32,
                sizeof(RowsShared<MT, STAGES>), a);
 }
 
@@ -292,7 +293,7 @@ template <int MT, int VEC> int start_rows(const F32Args& a) {
 
 template <int BM, int VEC> int start_tile(const F32Args& a) {
   static OncePerDevice once;
-  return start(gemm_f32_tile_kernel<BM, VEC>, once, dim3(a.segments, (a.N + BN - 1) / BN, (a.M + BM - 1) / BM),
+  return start(gemm_f32_tile_kernel<BM, VEC>, once, a.segments, (a.N + BN - 1) / BN, (a.M + BM - 1) / BM,
                BM * 2, tile_shared<BM>(), a);
 }
 

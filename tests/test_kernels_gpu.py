@@ -151,6 +151,19 @@ def test_gemm_f32_at_the_edges_of_its_kernels(M, N, K, lda):
         assert torch.equal(gemm_f32(x[m:m + 1], w, b), got[m:m + 1])
 
 
+@pytest.mark.parametrize("M", [2, 20])
+def test_gemm_f32_of_more_than_two_million_columns(M):
+    """More tiles of columns than a grid's shorter sides hold."""
+    from ginfer_b200.ops.linear import gemm_f32
+    N, K = (65536 * 32 if M == 2 else 65536 * 128) + 5, 4
+    g = torch.Generator(device=DEV).manual_seed(M)
+    x, w = torch.randn(M, K, device=DEV, generator=g), torch.randn(N, K, device=DEV, generator=g)
+    got = gemm_f32(x, w)
+    for a in (0, N - 1000):
+        want, size = (f(x.double()) @ f(w[a:a + 1000].double()).t() for f in (lambda t: t, torch.abs))
+        assert ((got[:, a:a + 1000].double() - want).abs() <= 8 * 2.0 ** -24 * size).all()
+
+
 def _paged_case(B_lens, q_lens, nh, nkv, hd, P, window, dtype, seed=0, spike=True):
     """Random paged cache and queries for requests with kv lengths ``B_lens`` whose last
     ``q_lens`` tokens are this step's queries.  Returns the kernel inputs and the plain result."""
