@@ -558,20 +558,21 @@ delta_chunk_coef_kernel(const float* __restrict__ qn, const float* __restrict__ 
 // prompts of 1,500 and 1,700 tokens, 16 heads of 128 x 128: 20 us, and 360 for the recurrence behind it.
 // (The delta rule itself with a decay a channel goes token by token in steps of every length: a router
 // behind it makes close calls, so its sums keep one order.)  ld_q, ld_k, ld_g: floats between two tokens.
+// The launch takes `heads` heads from number `head0` on, so that what it leaves is bounded: [T, heads, D].
 __global__ void __launch_bounds__(128)
 linear_chunk_coef_kernel(const float* __restrict__ qn, int ld_q, const float* __restrict__ kn,
                          int ld_k, const float* __restrict__ g, int ld_g,
-                         const int* __restrict__ cu_seqlens, DeltaDims dm,
+                         const int* __restrict__ cu_seqlens, DeltaDims dm, int head0, int heads,
                          float* __restrict__ coef, float* __restrict__ total,
                          float* __restrict__ qg, float* __restrict__ ke) {
   const int lane = threadIdx.x & 31;
-  const int c = blockIdx.x * 4 + (threadIdx.x >> 5), b = blockIdx.y, h = blockIdx.z;
+  const int c = blockIdx.x * 4 + (threadIdx.x >> 5), b = blockIdx.y, hl = blockIdx.z, h = head0 + hl;
   pdl_wait();
   const int t0 = cu_seqlens[b], ta = t0 + c * CT, n = min(CT, cu_seqlens[b + 1] - ta);
   if (n <= 0) return;
-  const int D = dm.D, H = dm.H, kvh = h / (H / dm.G);
-  const size_t HD = (size_t)H * D;
-  const size_t chunk = (size_t)chunk_number(t0, b, c) * H + h;
+  const int D = dm.D, kvh = h / (dm.H / dm.G);
+  const size_t HD = (size_t)heads * D;
+  const size_t chunk = (size_t)chunk_number(t0, b, c) * heads + hl;
   float val[64];                                             // pairs as above
 #pragma unroll
   for (int m = 0; m < 64; ++m) val[m] = 0.f;
@@ -600,7 +601,7 @@ linear_chunk_coef_kernel(const float* __restrict__ qn, int ld_q, const float* __
           kr[x] *= gd[i][x];
           val[8 * j + i] = fmaf(kr[x], q[i][x], val[8 * j + i]);
         }
-      if (j < n) Quad<float>::store(ke + (size_t)(ta + j) * HD + (size_t)h * D + d, kr);
+      if (j < n) Quad<float>::store(ke + (size_t)(ta + j) * HD + (size_t)hl * D + d, kr);
     }
     float G[4] = {1.f, 1.f, 1.f, 1.f};
 #pragma unroll
@@ -608,7 +609,7 @@ linear_chunk_coef_kernel(const float* __restrict__ qn, int ld_q, const float* __
       float e[4];
 #pragma unroll
       for (int x = 0; x < 4; ++x) G[x] *= gd[i][x], e[x] = G[x] * q[i][x];
-      if (i < n) Quad<float>::store(qg + (size_t)(ta + i) * HD + (size_t)h * D + d, e);
+      if (i < n) Quad<float>::store(qg + (size_t)(ta + i) * HD + (size_t)hl * D + d, e);
     }
     Quad<float>::store(total + chunk * D + d, G);
   }
@@ -639,8 +640,9 @@ linear_chunk_coef_kernel(const float* __restrict__ qn, int ld_q, const float* __
 // the rows 4 (p + LANES i) .. + 3, i < DPER / 4, so that the lanes' reads of a token's k and q are one run of
 // shared memory.  Stages as in the kernel above, one barrier a chunk.
 // HEADS: the delta rule with a decay a head; ke and total are not read.  PLAIN: linear attention with a
-// decay a key channel (u = v; kn is not read; eight lanes a column); qn and ke are [T, H, D] as
-// linear_chunk_coef_kernel leaves them, total the chunks' G_7.
+// decay a key channel (u = v; kn is not read; eight lanes a column); qn and ke are [T, heads, D] as
+// linear_chunk_coef_kernel leaves them, total the chunks' G_7.  The launch takes `heads` heads from number
+// `head0` on (HEADS: all).
 enum { HEADS = 0, PLAIN = 1 };
 template <int DPER, int LANES, int CP, int MODE>
 __global__ void __launch_bounds__(16 * LANES)
@@ -648,7 +650,8 @@ delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restr
                               const float* __restrict__ ke, const float* __restrict__ total,
                               const float* __restrict__ v, int ld_v, const float* __restrict__ coef,
                               float* __restrict__ state, const int* __restrict__ cu_seqlens,
-                              const int* __restrict__ slot_ids, DeltaDims dm, float* __restrict__ o) {
+                              const int* __restrict__ slot_ids, DeltaDims dm, int head0, int heads,
+                              float* __restrict__ o) {
   constexpr int Dp = LANES * DPER, COLS = 16 * CP, NQ = DPER / 4;
   static_assert(MODE != PLAIN || LANES == CT, "a lane a token of a chunk");
   // two sets of [CT][Dp]: k | q, or q | ke
@@ -656,7 +659,7 @@ delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restr
   constexpr int kVc = kG + (MODE == HEADS ? 0 : Dp), kC = kVc + CT * COLS, kStage = kC + kCoefs;
   constexpr int DOTS = MODE == PLAIN ? CT : 2 * CT;            // with S: the chunk's q, and k in front of them
   extern __shared__ __align__(16) float stage[];               // [kStages][kStage]
-  const int b = blockIdx.x / dm.H, h = blockIdx.x - b * dm.H;
+  const int b = blockIdx.x / heads, hl = blockIdx.x - b * heads, h = head0 + hl;
   const int p = threadIdx.x % LANES, lc = threadIdx.x / LANES;
   const int col0 = blockIdx.y * COLS;                          // a lane's columns: col0 + lc + 16 c
   pdl_trigger();
@@ -664,7 +667,7 @@ delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restr
   for (int i = threadIdx.x; i < kStages * kStage; i += blockDim.x) stage[i] = 0.f;
   __syncthreads();
   pdl_wait();
-  const int kvh = MODE == HEADS ? h / (dm.H / dm.G) : h;
+  const int kvh = MODE == HEADS ? h / (dm.H / dm.G) : hl;
   float* Sg = state + (size_t)slot_ids[b] * dm.state_stride + ((size_t)h * D) * Vd;
   float S[CP][NQ][4];
 #pragma unroll
@@ -677,11 +680,11 @@ delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restr
         S[y][i][x] = row < D ? Sg[(size_t)row * Vd + (col < Vd ? col : 0)] : 0.f;
       }
   const int t0 = cu_seqlens[b], t1 = cu_seqlens[b + 1];
-  const size_t KD = (size_t)(MODE == HEADS ? dm.G : dm.H) * D, HV = (size_t)dm.H * Vd;
+  const size_t KD = (size_t)(MODE == HEADS ? dm.G : heads) * D, HV = (size_t)dm.H * Vd;
   const int vq = min(COLS, Vd - col0) >> 2, dq = D >> 2;
   const int nchunks = (t1 - t0 + CT - 1) / CT;
   const int chunk0 = chunk_number(t0, b, 0);
-  const float* coef0 = coef + ((size_t)chunk0 * dm.H + h) * kCoefs;
+  const float* coef0 = coef + ((size_t)chunk0 * heads + hl) * kCoefs;
   auto copy16 = [](float* dst, const float* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
   };
@@ -697,13 +700,13 @@ delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restr
     }
     if (MODE != HEADS)
       for (int e = threadIdx.x; e < dq; e += blockDim.x)
-        copy16(st + kG + 4 * e, total + ((size_t)(chunk0 + c) * dm.H + h) * D + 4 * e);
+        copy16(st + kG + 4 * e, total + ((size_t)(chunk0 + c) * heads + hl) * D + 4 * e);
     for (int e = threadIdx.x; e < n * vq; e += blockDim.x) {
       const int t = e / vq, d = 4 * (e - t * vq);
       copy16(st + kVc + t * COLS + d, v + (size_t)(ta + t) * ld_v + (size_t)h * Vd + col0 + d);
     }
     for (int e = threadIdx.x; e < kCoefs / 4; e += blockDim.x)
-      copy16(st + kC + 4 * e, coef0 + (size_t)c * dm.H * kCoefs + 4 * e);
+      copy16(st + kC + 4 * e, coef0 + (size_t)c * heads * kCoefs + 4 * e);
   };
   for (int c = 0; c < kStages - 1; ++c) {
     if (c < nchunks) ask(c);
@@ -836,6 +839,7 @@ struct ChunkArgs {
   const float* coef;
   float* state;
   const int *cu_seqlens, *slot_ids;
+  int head0, heads;
   float* o;
 };
 
@@ -850,15 +854,16 @@ static int launch_chunk_columns(int B, const DeltaDims& dm, const ChunkArgs& a, 
       }))
     return rc;
   return launch_kernel(delta_chunk_recurrence_kernel<DPER, LANES, CP, MODE>,
-                       dim3(B * dm.H, (dm.Vd + 16 * CP - 1) / (16 * CP)), dim3(16 * LANES), smem, st, a.q,
-                       a.k, a.ke, a.total, a.v, a.ld_v, a.coef, a.state, a.cu_seqlens, a.slot_ids, dm, a.o);
+                       dim3(B * a.heads, (dm.Vd + 16 * CP - 1) / (16 * CP)), dim3(16 * LANES), smem, st, a.q,
+                       a.k, a.ke, a.total, a.v, a.ld_v, a.coef, a.state, a.cu_seqlens, a.slot_ids, dm, a.head0,
+                       a.heads, a.o);
 }
 
 template <int DPER, int LANES, int MODE>
 static int launch_chunks(int B, const DeltaDims& dm, const ChunkArgs& a, cudaStream_t st) {
   // two blocks an SM of 16 columns: then one of 32 each does the same work with half the reads (512
   // blocks of 16 columns 434 us, 256 of 32 391)
-  if (LANES * DPER <= 128 && (long long)B * dm.H * ((dm.Vd + 15) / 16) >= 2 * 148 && dm.Vd > 16)
+  if (LANES * DPER <= 128 && (long long)B * a.heads * ((dm.Vd + 15) / 16) >= 2 * 148 && dm.Vd > 16)
     return launch_chunk_columns<DPER, LANES, LANES * DPER <= 128 ? 2 : 1, MODE>(B, dm, a, st);
   return launch_chunk_columns<DPER, LANES, 1, MODE>(B, dm, a, st);
 }
@@ -974,11 +979,11 @@ GF_EXPORT int gf_delta_prepare_heads(const float* proj, int ld, int a_off, int b
                        0, st, proj, ld, state, cu_seqlens, slot_ids, dm);
 }
 
-// fp32 words of scratch with which a step goes eight tokens at a time: gf_delta_recurrence (one_decay 1),
-// gf_decay_channels_chunked (0).
-GF_EXPORT long long gf_delta_chunk_words(int T, int B, int H, int D, int one_decay) {
-  const long long chunks = (long long)(T / CT + B + 1) * H;
-  return one_decay ? chunks * kCoefs : chunks * (kCoefs + D) + 2ll * T * H * D;
+// fp32 words of scratch with which a step of `heads` heads goes eight tokens at a time: gf_delta_recurrence
+// (one_decay 1), gf_decay_channels_chunked (0).
+GF_EXPORT long long gf_delta_chunk_words(int T, int B, int heads, int D, int one_decay) {
+  const long long chunks = (long long)(T / CT + B + 1) * heads;
+  return one_decay ? chunks * kCoefs : chunks * (kCoefs + D) + 2ll * T * heads * D;
 }
 
 // one_decay: g is [T, H] (a decay a head), else [T, H, D].  scratch (gf_delta_chunk_words; null: token by
@@ -998,7 +1003,7 @@ GF_EXPORT int gf_delta_recurrence(const float* qn, const float* kn, const float*
     if (int rc = launch_kernel(delta_chunk_coef_kernel, dim3((chunks + 3) / 4, B, G), dim3(128), 0, st,
                                qn, kn, g, beta, cu_seqlens, dm, scratch))
       return rc;
-    const ChunkArgs a{qn, kn, nullptr, nullptr, v, H * Vd, scratch, state, cu_seqlens, slot_ids, o};
+    const ChunkArgs a{qn, kn, nullptr, nullptr, v, H * Vd, scratch, state, cu_seqlens, slot_ids, 0, H, o};
 #define GF_GO(DPER, LANES)                                                                         \
   if (D <= DPER * LANES) return launch_chunks<DPER, LANES, HEADS>(B, dm, a, st);
     GF_GO(4, 8)
@@ -1042,28 +1047,28 @@ GF_EXPORT int gf_delta_recurrence(const float* qn, const float* kn, const float*
 }
 
 // A plain linear attention with a decay a key channel, S <- diag(g) S + k v^T, o = S^T q, eight tokens at a
-// time.  Rows of q, k (G heads of D), v (H of Vd) and g (H of D) are ld_* floats apart; scratch:
-// gf_delta_chunk_words with one_decay 0; o [T, H, Vd].  Returns -6 for what it does not take (key sizes over
+// time.  Rows of q, k (G heads of D), v (H of Vd) and g (H of D) are ld_* floats apart; `heads` of the H
+// from number `head0` on; scratch: gf_delta_chunk_words with one_decay 0; o [T, H, Vd].  Returns -6 for what it does not take (key sizes over
 // 128, sizes or rows that are no multiples of four).
 GF_EXPORT int gf_decay_channels_chunked(const float* q, int ld_q, const float* k, int ld_k, const float* v,
                                         int ld_v, const float* g, int ld_g, float* state, int state_stride,
                                         const int* cu_seqlens, const int* slot_ids, int T, int B, int H,
                                         int G, int D, int Vd, float* o, float* scratch, int max_q_len,
-                                        void* stream) {
+                                        int head0, int heads, void* stream) {
   if (B <= 0) return 0;
   if (H % G || D > 128 || D % 4 || Vd % 4 || ld_q % 4 || ld_k % 4 || ld_v % 4 || ld_g % 4 || B > 65535 ||
-      H > 65535 ||
+      H > 65535 || head0 < 0 || heads <= 0 || head0 + heads > H ||
       (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)g | (uintptr_t)scratch) & 15))
     return -6;
   const DeltaDims dm = dims_of(H, G, D, Vd, 1, state_stride, 0);
   auto st = (cudaStream_t)stream;
-  const size_t chunks = (size_t)(T / CT + B + 1) * H, HTD = (size_t)T * H * D;
+  const size_t chunks = (size_t)(T / CT + B + 1) * heads, HTD = (size_t)T * heads * D;
   float *total = scratch + chunks * kCoefs, *qg = total + chunks * D, *ke = qg + HTD;
-  if (int rc = launch_kernel(linear_chunk_coef_kernel, dim3(((max_q_len + CT - 1) / CT + 3) / 4, B, H),
-                             dim3(128), 0, st, q, ld_q, k, ld_k, g, ld_g, cu_seqlens, dm, scratch, total, qg,
-                             ke))
+  if (int rc = launch_kernel(linear_chunk_coef_kernel, dim3(((max_q_len + CT - 1) / CT + 3) / 4, B, heads),
+                             dim3(128), 0, st, q, ld_q, k, ld_k, g, ld_g, cu_seqlens, dm, head0, heads,
+                             scratch, total, qg, ke))
     return rc;
-  const ChunkArgs a{qg, nullptr, ke, total, v, ld_v, scratch, state, cu_seqlens, slot_ids, o};
+  const ChunkArgs a{qg, nullptr, ke, total, v, ld_v, scratch, state, cu_seqlens, slot_ids, head0, heads, o};
   if (D <= 32) return launch_chunks<4, 8, PLAIN>(B, dm, a, st);
   if (D <= 64) return launch_chunks<8, 8, PLAIN>(B, dm, a, st);
   return launch_chunks<16, 8, PLAIN>(B, dm, a, st);

@@ -86,6 +86,9 @@ WIDE_MIN_TOKENS = 64
 # B200, two prompts of 1,500 and 1,700 tokens, 16 heads of 128 x 128: 360 us and 20 before it, against 997
 # token by token).
 CHUNK_MIN_TOKENS = 64
+# The second leaves scaled keys and queries of every token in scratch: at most this many words (256 MB; a
+# step of 8,192 tokens with 32 heads of 128), or one head's; more heads go a group after the other.
+CHANNELS_MAX_WORDS = 1 << 26
 
 
 def _chunked(q, k, v, g, state, ctx, first: int, H, G, D, Vd, k_scale, skip, normaliser, o, o_n) -> bool:
@@ -113,17 +116,19 @@ def _channels_chunked(q, k, v, g, state, ctx, H, G, D, Vd, o) -> bool:
     """The step eight tokens at a time with a decay a key channel; ``False`` if not served."""
     if D > 128 or D % 4 or Vd % 4:
         return False
-    T = v.shape[0]
-    scratch = torch.empty(delta.chunk_words(T, ctx.num_seqs, H, D, 0), dtype=torch.float32, device=v.device)
+    T, B = v.shape[0], ctx.num_seqs
+    group = max(1, min(H, CHANNELS_MAX_WORDS // delta.chunk_words(T, B, 1, D, 0)))
+    scratch = torch.empty(delta.chunk_words(T, B, group, D, 0), dtype=torch.float32, device=v.device)
     f = _fn("delta_rule", "gf_decay_channels_chunked",
-            [c_void_p, c_int] * 5 + [c_void_p, c_void_p] + [c_int] * 6 + [c_void_p, c_void_p, c_int, c_void_p],
-            kernels=2)
-    rc = f(_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(g), g.stride(0), _p(state),
-           state.stride(0), _p(ctx.cu_seqlens_q), _p(ctx.slot_ids), T, ctx.num_seqs, H, G, D, Vd, _p(o),
-           _p(scratch), int(ctx.max_q_len), _stream())
-    if rc == -6:
-        return False
-    _ok(rc, "decay_channels_chunked")
+            [c_void_p, c_int] * 5 + [c_void_p, c_void_p] + [c_int] * 6 + [c_void_p, c_void_p] + [c_int] * 3 +
+            [c_void_p], kernels=2)
+    for head in range(0, H, group):
+        rc = f(_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(g), g.stride(0), _p(state),
+               state.stride(0), _p(ctx.cu_seqlens_q), _p(ctx.slot_ids), T, B, H, G, D, Vd, _p(o),
+               _p(scratch), int(ctx.max_q_len), head, min(group, H - head), _stream())
+        if rc == -6:                     # (of sizes and addresses: the same for every group)
+            return False
+        _ok(rc, "decay_channels_chunked")
     return True
 
 

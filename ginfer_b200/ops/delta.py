@@ -102,14 +102,14 @@ def state_step(q, k, v, g, state, ctx, H: int, G: int, D: int, Vd: int, o, c=Non
     return True
 
 
-def chunk_words(T: int, B: int, H: int, D: int, one_decay: int) -> int:
-    """fp32 words of scratch with which a step goes eight tokens at a time."""
+def chunk_words(T: int, B: int, heads: int, D: int, one_decay: int) -> int:
+    """fp32 words of scratch with which ``heads`` heads of a step go eight tokens at a time."""
     from ctypes import c_longlong
 
     from .build import load_library
     f = load_library("delta_rule").gf_delta_chunk_words
     f.argtypes, f.restype = [c_int] * 5, c_longlong
-    return int(f(T, B, H, D, one_decay))
+    return int(f(T, B, heads, D, one_decay))
 
 
 def recurrence(qn, kn, v, g, beta, state: torch.Tensor, ctx) -> torch.Tensor:

@@ -662,11 +662,11 @@ def test_a_storage_clears_the_tensors_it_holds_now():
 @pytest.mark.parametrize("H,G,D,Vd,lens", [(2, 1, 12, 20, [64, 1, 7]), (4, 2, 64, 64, [80, 8, 9]),
                                            (2, 2, 128, 128, [66, 17]), (3, 3, 100, 36, [24, 65, 1]),
                                            (16, 16, 128, 48, [64, 3, 9, 70, 8, 1, 65, 64]), (1, 1, 32, 4, [71])])
-def test_linear_attention_with_channel_decays_eight_tokens_at_a_time(H, G, D, Vd, lens):
+def test_linear_attention_with_channel_decays_eight_tokens_at_a_time(monkeypatch, H, G, D, Vd, lens):
     """Rows of a wider projection, chunks whole and cut, one and two columns a lane, decays from none to all
     gone: outputs and states against the recurrence token by token in 64 bits."""
     from types import SimpleNamespace
-    from ginfer_b200.ops import decay
+    from ginfer_b200.ops import decay, delta
     g0 = torch.Generator().manual_seed(D + Vd)
     B, T = len(lens), sum(lens)
     q, k = torch.randn(T, G, D, generator=g0) / D ** 0.5, torch.randn(T, G, D, generator=g0) / D ** 0.5
@@ -693,6 +693,12 @@ def test_linear_attention_with_channel_decays_eight_tokens_at_a_time(H, G, D, Vd
         assert torch.equal(state[slots[b], H * D * Vd:], state0[slots[b], H * D * Vd:])
     # values of a few units (a state holds some 200 terms of at most one), fp32 sums of at most 128 of them
     assert err <= 2e-5, err
+    # scratch for fewer heads than there are: a group of them after the other, the same bits
+    for heads in {1, H // 2 + 1}:
+        monkeypatch.setattr(decay, "CHANNELS_MAX_WORDS", delta.chunk_words(T, B, heads, D, 0))
+        again = state0.clone().cuda()
+        o2 = decay.recurrence(qd, kd, vd, g.reshape(T, -1).cuda(), again, ctx, H, G, D, Vd)
+        assert torch.equal(o2.cpu().double().reshape(T, H, Vd), o) and torch.equal(again.cpu(), state)
     rest = [s for s in range(B + 2) if s not in slots.tolist()]
     assert torch.equal(state[rest], state0[rest])
 
