@@ -685,25 +685,30 @@ delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restr
   const int nchunks = (t1 - t0 + CT - 1) / CT;
   const int chunk0 = chunk_number(t0, b, 0);
   const float* coef0 = coef + ((size_t)chunk0 * heads + hl) * kCoefs;
-  auto copy16 = [](float* dst, const float* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+  auto copy16 = [](float* dst, const float* src, bool in = true) {         // zeros where !in
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src),
+                 "r"(in ? 16 : 0)
+                 : "memory");
   };
   auto ask = [&](int c) {
     float* st = stage + (size_t)(c % kStages) * kStage;
     const int ta = t0 + c * CT, n = min(CT, t1 - ta);
-    for (int e = threadIdx.x; e < n * dq; e += blockDim.x) {
+    // (tokens behind the portion's end are zeros, not an older chunk's)
+    for (int e = threadIdx.x; e < CT * dq; e += blockDim.x) {
       const int t = e / dq, d = 4 * (e - t * dq);
-      const size_t at = (size_t)(ta + t) * KD + (size_t)kvh * D + d;
-      if (MODE != PLAIN) copy16(st + t * Dp + d, kn + at);
-      copy16(st + kQ + t * Dp + d, qn + at);
-      if (MODE != HEADS) copy16(st + kE + t * Dp + d, ke + at);
+      const bool in = t < n;
+      const size_t at = (size_t)(ta + (in ? t : 0)) * KD + (size_t)kvh * D + d;
+      if (MODE != PLAIN) copy16(st + t * Dp + d, kn + at, in);
+      copy16(st + kQ + t * Dp + d, qn + at, in);
+      if (MODE != HEADS) copy16(st + kE + t * Dp + d, ke + at, in);
     }
     if (MODE != HEADS)
       for (int e = threadIdx.x; e < dq; e += blockDim.x)
         copy16(st + kG + 4 * e, total + ((size_t)(chunk0 + c) * heads + hl) * D + 4 * e);
-    for (int e = threadIdx.x; e < n * vq; e += blockDim.x) {
+    for (int e = threadIdx.x; e < CT * vq; e += blockDim.x) {
       const int t = e / vq, d = 4 * (e - t * vq);
-      copy16(st + kVc + t * COLS + d, v + (size_t)(ta + t) * ld_v + (size_t)h * Vd + col0 + d);
+      const bool in = t < n;
+      copy16(st + kVc + t * COLS + d, v + (size_t)(ta + (in ? t : 0)) * ld_v + (size_t)h * Vd + col0 + d, in);
     }
     for (int e = threadIdx.x; e < kCoefs / 4; e += blockDim.x)
       copy16(st + kC + 4 * e, coef0 + (size_t)c * heads * kCoefs + 4 * e);
@@ -758,11 +763,10 @@ delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restr
     const float Gp = MODE == HEADS ? cf[kCoefG + tok] : 1.f;
     float u[CP][CT];
     if constexpr (MODE == PLAIN) {
-      const int n = t1 - t0 - c * CT;                           // (what lies behind the end is an older chunk's)
 #pragma unroll
       for (int y = 0; y < CP; ++y)
 #pragma unroll
-        for (int i = 0; i < CT; ++i) u[y][i] = i < n ? st[kVc + i * COLS + lc + 16 * y] : 0.f;
+        for (int i = 0; i < CT; ++i) u[y][i] = st[kVc + i * COLS + lc + 16 * y];
     } else {
 #pragma unroll
     for (int y = 0; y < CP; ++y) {
@@ -787,8 +791,10 @@ delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restr
       for (int y = 0; y < CP; ++y) {
         const float(&w)[CT] = u[y];
         float out = Gp * x[y][LANES == CT && MODE != PLAIN ? CT : 0];
-        out = fmaf(m0.x, w[0], fmaf(m0.y, w[1], fmaf(m0.z, w[2], fmaf(m0.w, w[3], out))));
-        out = fmaf(m1.x, w[4], fmaf(m1.y, w[5], fmaf(m1.z, w[6], fmaf(m1.w, w[7], out))));
+        // (M is 0 behind a token, but 0 times what is no number would reach back)
+        auto seen = [&](int j) { return j <= tok ? w[j] : 0.f; };
+        out = fmaf(m0.x, w[0], fmaf(m0.y, seen(1), fmaf(m0.z, seen(2), fmaf(m0.w, seen(3), out))));
+        out = fmaf(m1.x, seen(4), fmaf(m1.y, seen(5), fmaf(m1.z, seen(6), fmaf(m1.w, seen(7), out))));
         const int col = col0 + lc + 16 * y;
         if (col < Vd && row < t1 && p >= LANES - CT) o[(size_t)row * HV + (size_t)h * Vd + col] = out;
       }

@@ -703,6 +703,40 @@ def test_linear_attention_with_channel_decays_eight_tokens_at_a_time(monkeypatch
     assert torch.equal(state[rest], state0[rest])
 
 
+@pytest.mark.parametrize("rule", ["linear", "delta"])
+def test_what_is_no_number_stays_with_its_token_and_later_ones(rule):
+    """Portions eight tokens at a time: a value that is infinite or no number leaves the outputs of earlier
+    tokens, of other columns and of other requests as they were, and is not forgotten by later ones."""
+    from types import SimpleNamespace
+    from ginfer_b200.ops import decay, delta
+    H, D, Vd, lens = 2, 32, 20, [70, 66]
+    T, g0 = sum(lens), torch.Generator(device=DEV).manual_seed(5)
+    q, k = (torch.randn(T, H, D, generator=g0, device=DEV) * D ** -0.5 for _ in range(2))
+    v, beta = torch.randn(T, H, Vd, generator=g0, device=DEV), torch.rand(T, H, generator=g0, device=DEV)
+    g = torch.rand(T, H * D if rule == "linear" else H, generator=g0, device=DEV) * 0.5 + 0.5
+    ctx = SimpleNamespace(num_seqs=2, slot_ids=torch.tensor([1, 0], dtype=torch.int32, device=DEV), max_q_len=70,
+                          cu_seqlens_q=torch.tensor([0, 70, 136], dtype=torch.int32, device=DEV), q_lens_host=lens)
+
+    def run(v):
+        state = torch.zeros(2, H * D * Vd, device=DEV)
+        if rule == "delta":
+            return delta.recurrence(q, k, v, g, beta, state, ctx), state.view(2, H, D, Vd)
+        o = decay.recurrence(q.view(T, -1), k.view(T, -1), v.view(T, -1), g, state, ctx, H, H, D, Vd)
+        return o.view(T, H, Vd), state.view(2, H, D, Vd)
+    want, kept = run(v)
+    for at in (3, 37, 64, 69):
+        for bad in (float("nan"), float("inf")):
+            w = v.clone()
+            w[at, 1, 6] = bad
+            o, state = run(w)
+            hit = torch.zeros(T, H, Vd, dtype=torch.bool, device=DEV)
+            hit[at:70, 1, 6] = True
+            assert torch.equal(o[~hit], want[~hit]) and not o[hit].isfinite().any()
+            away = torch.ones_like(state, dtype=torch.bool)
+            away[1, 1, :, 6] = False
+            assert torch.equal(state[away], kept[away]) and not state[~away].isfinite().any()
+
+
 @pytest.mark.parametrize("C", [16, 48, 80, 512])
 @pytest.mark.parametrize("lens", [[600], [700, 3, 64], [1000, 520, 1, 65]])
 def test_shares_of_a_tokens_keys_are_put_together(C, lens):
