@@ -24,10 +24,11 @@ namespace gf {
 constexpr int kMaxHeadDim = 256;
 constexpr int kWarps = 8;
 
-// VEC channels as one access: 4, or 1 for sizes and addresses that are no multiples of four elements.
+// VEC channels as one access: 4, or 1 for sizes and addresses that are no multiples of four elements; from L2
+// (the kernel ahead has just rotated q and written this step's keys and values).
 template <typename T, int VEC> __device__ __forceinline__ void load_channels(const T* p, float (&v)[VEC]) {
-  if constexpr (VEC == 4) Quad<T>::load(p, v);
-  else v[0] = to_f32(*p);
+  if constexpr (VEC == 4) Quad<T>::fresh(p, v);
+  else v[0] = fresh(p);
 }
 
 // QN, VN: steps of eight lanes over a key's channels, of a warp over a value's.

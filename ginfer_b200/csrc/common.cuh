@@ -60,9 +60,14 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(flo
   return __float2bfloat16_rn(v);
 }
 
-// Four channels of one type as one access (the address a multiple of four elements).
+// Four channels of one type as one access (the address a multiple of four elements).  fresh: past L1,
+// for what a kernel shortly before this one wrote (see below).
 template <typename T> struct Quad;
 template <> struct Quad<float> {
+  static __device__ __forceinline__ void fresh(const float* p, float (&v)[4]) {
+    const float4 a = __ldcg(reinterpret_cast<const float4*>(p));
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+  }
   static __device__ __forceinline__ void load(const float* p, float (&v)[4]) {
     const float4 a = *reinterpret_cast<const float4*>(p);
     v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
@@ -72,11 +77,16 @@ template <> struct Quad<float> {
   }
 };
 template <> struct Quad<__nv_bfloat16> {
-  static __device__ __forceinline__ void load(const __nv_bfloat16* p, float (&v)[4]) {
-    const uint2 raw = *reinterpret_cast<const uint2*>(p);
+  static __device__ __forceinline__ void unpack(const uint2& raw, float (&v)[4]) {
     const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
     const float2 a = __bfloat1622float2(h[0]), b = __bfloat1622float2(h[1]);
     v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+  }
+  static __device__ __forceinline__ void fresh(const __nv_bfloat16* p, float (&v)[4]) {
+    unpack(__ldcg(reinterpret_cast<const uint2*>(p)), v);
+  }
+  static __device__ __forceinline__ void load(const __nv_bfloat16* p, float (&v)[4]) {
+    unpack(*reinterpret_cast<const uint2*>(p), v);
   }
   static __device__ __forceinline__ void store(__nv_bfloat16* p, const float (&v)[4]) {
     uint2 raw;
@@ -162,10 +172,17 @@ __device__ __forceinline__ void pdl_trigger() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// An index that a kernel shortly before this one wrote, read from L2.  A kernel that was launched while
-// that one still ran may share its SM with kernels that read the same memory when it held something
-// else (a recycled buffer), and what they left in L1 must not be taken for an index.
+// What a kernel shortly before this one wrote, read from L2.  A kernel that was launched while that one
+// still ran may share its SM with kernels that read the same memory when it held something else (a
+// recycled buffer), and what they left in L1 must not be taken for it; nor may it be loaded as data that
+// is constant for the kernel's whole life, which a load through a `const __restrict__` pointer allows.
+// An index is always read so; values are in kernels that start early, where they come by plain loads
+// (cp.async and TMA copies go past L1).
 __device__ __forceinline__ int fresh_index(const int* p) { return __ldcg(p); }
+__device__ __forceinline__ float fresh(const float* p) { return __ldcg(p); }
+__device__ __forceinline__ float fresh(const __nv_bfloat16* p) {
+  return __uint_as_float((uint32_t)__ldcg(reinterpret_cast<const unsigned short*>(p)) << 16);
+}
 
 inline int& pdl_flag() {
   static int enabled = 1;

@@ -584,9 +584,9 @@ linear_chunk_coef_kernel(const float* __restrict__ qn, int ld_q, const float* __
       for (int x = 0; x < 4; ++x) k[i][x] = q[i][x] = 0.f, gd[i][x] = 1.f;
       if (i < n) {
         const size_t r = ta + i;
-        Quad<float>::load(kn + r * ld_k + (size_t)kvh * D + d, k[i]);
-        Quad<float>::load(qn + r * ld_q + (size_t)kvh * D + d, q[i]);
-        Quad<float>::load(g + r * ld_g + (size_t)h * D + d, gd[i]);
+        Quad<float>::fresh(kn + r * ld_k + (size_t)kvh * D + d, k[i]);
+        Quad<float>::fresh(qn + r * ld_q + (size_t)kvh * D + d, q[i]);
+        Quad<float>::fresh(g + r * ld_g + (size_t)h * D + d, gd[i]);
       }
     }
 #pragma unroll

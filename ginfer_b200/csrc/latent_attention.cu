@@ -575,9 +575,9 @@ __global__ void latent_merge_kernel(const float* __restrict__ part_o,
   for (int z = 0; z < kMaxSplits; ++z) {
     m[z] = -INFINITY, l[z] = 0.f;
     if (z < nsplit) {
-      const float2 ml = *reinterpret_cast<const float2*>(part_ml + 2 * (z * pairs + pair));
+      const float2 ml = __ldcg(reinterpret_cast<const float2*>(part_ml + 2 * (z * pairs + pair)));
       m[z] = ml.x, l[z] = ml.y;
-      Quad<float>::load(part_o + (z * pairs + pair) * C + c, v[z]);
+      Quad<float>::fresh(part_o + (z * pairs + pair) * C + c, v[z]);
     }
   }
   float M = -INFINITY, L = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};

@@ -632,7 +632,7 @@ moe_stream_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfloa
       const size_t s = (size_t)(row0 + r);
       const float c0 = acc[j][i], c1 = acc[j][2 + i];        // weight rows n, n + 1
       if (MODE == 2) {
-        const float rw = row_w ? row_w[fresh_index(pair_of_pos + s)] : 1.f;
+        const float rw = row_w ? fresh(row_w + fresh_index(pair_of_pos + s)) : 1.f;
         const float v0 = fmaxf(to_f32(from_f32<__nv_bfloat16>(c0 * rw)), 0.f);
         const float v1 = fmaxf(to_f32(from_f32<__nv_bfloat16>(c1 * rw)), 0.f);
         *reinterpret_cast<__nv_bfloat162*>((__nv_bfloat16*)out_ + s * N + n) =
@@ -791,13 +791,13 @@ moe_combine_kernel(const float* __restrict__ y, const int* __restrict__ pos_of_p
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       p[i] = k0 + i < top ? fresh_index(pos_of_pair + t * top + k0 + i) : -1;
-      w[i] = wgt && k0 + i < top ? wgt[t * top + k0 + i] : 1.f;
+      w[i] = wgt && k0 + i < top ? fresh(wgt + t * top + k0 + i) : 1.f;
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i)
       if (p[i] >= 0) {
-        if constexpr (VEC == 4) Quad<float>::load(y + (size_t)p[i] * N + n, v[i]);
-        else v[i][0] = y[(size_t)p[i] * N + n];
+        if constexpr (VEC == 4) Quad<float>::fresh(y + (size_t)p[i] * N + n, v[i]);
+        else v[i][0] = fresh(y + (size_t)p[i] * N + n);
       }
 #pragma unroll
     for (int i = 0; i < 4; ++i)                      // in the order chosen

@@ -49,11 +49,11 @@ state_step_kernel(const StepArgs a) {
     if (live && d < D) Quad<float>::load(S + (size_t)d * Vd, s[i]);
   }
   float v[4] = {0.f, 0.f, 0.f, 0.f};
-  if (live) Quad<float>::load(a.v + r * a.ld_v + (size_t)h * Vd + col, v);
+  if (live) Quad<float>::fresh(a.v + r * a.ld_v + (size_t)h * Vd + col, v);
   for (int d = threadIdx.x; d < D; d += kStepThreads) {
-    qs[d] = a.q[r * a.ld_q + (size_t)kvh * D + d];
-    ks[d] = a.k[r * a.ld_k + (size_t)kvh * D + d];
-    gs[d] = a.g[r * a.ld_g + (a.gD == 1 ? h : h * D + d)];
+    qs[d] = fresh(a.q + r * a.ld_q + (size_t)kvh * D + d);
+    ks[d] = fresh(a.k + r * a.ld_k + (size_t)kvh * D + d);
+    gs[d] = fresh(a.g + r * a.ld_g + (a.gD == 1 ? h : h * D + d));
   }
   __syncthreads();
   float dq[4] = {0.f, 0.f, 0.f, 0.f};
@@ -78,7 +78,7 @@ state_step_kernel(const StepArgs a) {
     for (int d = lane; d < D; d += 32) kq = fmaf(ks[d], qs[d], kq);
     kq = warp_sum(kq);
     __syncthreads();
-    const float beta = a.beta[r * a.H + h];
+    const float beta = fresh(a.beta + r * a.H + h);
     float u[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int j = 0; j < RG; ++j) {
@@ -112,7 +112,7 @@ state_step_kernel(const StepArgs a) {
       Quad<float>::store(a.o + r * a.ld_o + (size_t)h * Vd + col, out);
     }
   } else {
-    const float c = a.c ? a.c[r * a.ld_c + h] : 1.f;
+    const float c = a.c ? fresh(a.c + r * a.ld_c + h) : 1.f;
     float cv[4];
 #pragma unroll
     for (int x = 0; x < 4; ++x) cv[x] = c * v[x];

@@ -77,8 +77,8 @@ __global__ void outnorm_add_vec_kernel(const float* __restrict__ x, const Y* __r
   for (int u = 0; u < OPT; ++u) {
     const int q = threadIdx.x + u * blockDim.x;
     if (q < nq) {
-      Quad<Y>::load(y + base + 4 * q, yv[u]);
-      Quad<float>::load(x + base + 4 * q, xv[u]);    // (behind the sum it was waited for: 2.8 us a decode step's, 1.9 so)
+      Quad<Y>::fresh(y + base + 4 * q, yv[u]);
+      Quad<float>::fresh(x + base + 4 * q, xv[u]);    // (behind the sum it was waited for: 2.8 us a decode step's, 1.9 so)
 #pragma unroll
       for (int i = 0; i < 4; ++i) ss += yv[u][i] * yv[u][i];
     }
