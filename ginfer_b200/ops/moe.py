@@ -32,27 +32,34 @@ def tile_rows(tensor_cores) -> int:
 # experts' weight bytes there.
 TCGEN05_MIN_PAIRS = 1024
 # Up to this many pairs (decode steps) the products run on the kernel that streams an expert's weights
-# once for up to 16 pairs; it keeps the pairs' rows in shared memory, which bounds the reduction size.
+# once for every 16 pairs; it keeps the pairs' rows in shared memory, which bounds the reduction size.
 # On a B200, both products of 32 experts of 2048 x 2112 with 4 choices a token: 512 pairs 144 us
 # against 182 on the mma.sync kernel, 1,020 pairs 214 against 209; 16 experts of 1024 x 1056 with 2
-# choices: 510 pairs 47 against 62.
+# choices: 510 pairs 47 against 62.  Up to this many pairs an expert as well, three readings of its weights
+# where the 64-row tiles make one (streamed / tiles, weights from HBM): 4 experts of 2048 x 1408, 48 pairs
+# an expert 60 / 84, 96 90 / 93, 128 113 / 93; 8 such, 48 107 / 108, 64 118 / 113, 96 153 / 127; 16 of
+# 1024 x 704, 32 51 / 56, 48 67 / 65.
 FEW_MAX_PAIRS = 768
+FEW_MAX_PAIRS_AN_EXPERT = 48
 FEW_MAX_K = 4096
 # Without that kernel (``streamed`` false: its sums run in another order than those of the others), up
 # to this many pairs run on one that multiplies on the FMA pipes, more on the mma.sync kernel.
 GEMV_MAX_PAIRS = 20
 
 
-def kernel_for(x: torch.Tensor, pairs: int, reductions, widths, streamed: bool = True) -> object:
+def kernel_for(x: torch.Tensor, pairs: int, reductions, widths, streamed: bool = True,
+               experts: int | None = None) -> object:
     """Which grouped-product kernel serves activations ``x`` with these reduction sizes and output
-    widths: ``"tcgen05"``, ``"few"`` (weights streamed; not without ``streamed``), ``"gemv"`` (a handful
+    widths, of ``experts`` that the pairs are spread over: ``"tcgen05"``, ``"few"`` (weights streamed; not without ``streamed``), ``"gemv"`` (a handful
     of pairs), ``True`` (``mma.sync``) or ``False`` (plain)."""
     if not (on_tensor_cores(x.dtype, *reductions) and x.stride(0) % 8 == 0):
         return False
     if pairs >= TCGEN05_MIN_PAIRS and all(n % 8 == 0 for n in widths):
         return "tcgen05"
-    if (pairs <= (FEW_MAX_PAIRS if streamed else GEMV_MAX_PAIRS) and max(reductions) <= FEW_MAX_K
-            and all(n % 2 == 0 for n in widths)):
+    most = GEMV_MAX_PAIRS
+    if streamed:
+        most = FEW_MAX_PAIRS if experts is None else min(FEW_MAX_PAIRS, FEW_MAX_PAIRS_AN_EXPERT * experts)
+    if pairs <= most and max(reductions) <= FEW_MAX_K and all(n % 2 == 0 for n in widths):
         return "few" if streamed else "gemv"
     return True
 

@@ -63,7 +63,7 @@ class RoutedGLU(FeedForward):
         idx, wgt = moe.route(self.router(x), self.top, self.renormalize)
         plan = moe.Plan(idx, self.E, moe.kernel_for(
             x, T * self.top, (self.hidden_size, self.intermediate_size),
-            (self.intermediate_size, self.hidden_size), self.streamed))
+            (self.intermediate_size, self.hidden_size), self.streamed, self.E))
         y = moe.grouped_glu(x, self.w_gate_up, plan, self.limit, self.alpha, self.up_shift,
                             act=self.act)
         rows = moe.grouped_down(y, self.w_down, plan)
@@ -119,7 +119,7 @@ class RoutedExperts(FeedForward):
         idx, wgt = moe.route(self.router(x), self.top, self.renormalize, self.score)
         plan = moe.Plan(idx, self.E, moe.kernel_for(
             x, T * self.top, (self.hidden_size, self.intermediate_size),
-            (self.intermediate_size, self.hidden_size)))
+            (self.intermediate_size, self.hidden_size), experts=self.E))
         on_input = self.weight_on == "input"
         y = moe.grouped_relu2(x, self.w_up, plan, wgt if on_input else None)
         rows, w = moe.grouped_down(y, self.w_down, plan), None if on_input else wgt
@@ -210,7 +210,7 @@ class GroupRoutedGLU(RoutedGLU):
         top = self.top + self.always
         plan = moe.Plan(idx, self.E + self.always, moe.kernel_for(
             x, T * top, (self.hidden_size, self.intermediate_size),
-            (self.intermediate_size, self.hidden_size)))
+            (self.intermediate_size, self.hidden_size), experts=self.E + self.always))
         y = moe.grouped_glu(x, self.w_gate_up, plan, self.limit, self.alpha, self.up_shift,
                             act=self.act)
         rows = moe.grouped_down(y, self.w_down, plan)
