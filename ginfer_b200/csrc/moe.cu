@@ -514,7 +514,11 @@ moe_gemm_mma_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfl
 // the pairs' rows, at most 16 of one expert, are staged in shared memory and are the 8-column operand.
 // No weight is staged, so a warp keeps 8 loads of 16 bytes a lane under way whatever the other warps do.
 // A warp owns 16 weight rows; `parts` warps (1, 2, 4 or 8 of the block's eight) split its reduction
-// where the rows alone give too few warps.  Lane group g has weight rows 2 g and 2 g + 1: a gate and
+// where the rows alone give too few warps.  `parts` is the order of a pair's sums, so it follows from the
+// matrices and from a step's range (up to 20 pairs, up to 16 an expert, more), not from its pairs'
+// number: within a range a pair's result does not depend on the batch.  Against `parts` from the number
+// itself (both products, weights from HBM, us): 32 experts of 2048 x 2112, 8 pairs 69.6 -> 63.6, 20 pairs 107
+// -> 109; 8 of 2048 x 1408, 24 pairs 45 -> 49, 64 pairs 61.5 -> 57.4; elsewhere within 3 %, or faster.  Lane group g has weight rows 2 g and 2 g + 1: a gate and
 // its up value meet in one lane.
 // Measured on a B200 (both products of a layer, 32 experts of 2048 x 2112, 4 choices; floor = the
 // reached experts' bytes at 6.54 TB/s), against a kernel that kept eight rows in shared memory and
@@ -522,7 +526,9 @@ moe_gemm_mma_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfl
 // us (29.5; floor 10.6), 20 pairs 53.5 (97.5; 39.6), 64 pairs 91.6 (120; 60.8), 256 pairs 113.5 (172; 82),
 // 512 pairs 144.5 (182; 84.6), 1,020 pairs 214 (209: the line lies at 768).
 constexpr int kStRows = 16, kStWarps = 8, kStUnroll = 2;
-constexpr int kStMaxShared = 160 * 1024;                     // K up to 5,088
+constexpr int kStMaxShared = 160 * 1024;                     // K up to 5,056
+// The tiles of rows that `parts` reckons with: for a handful of pairs, at most otherwise.
+constexpr int kStHandful = 20, kStHandfulTiles = 12, kStTiles = 32;
 
 __host__ __device__ inline size_t stream_pitch(int K) {      // of a staged row, bytes: 64 mod 128
   return ((size_t)K * 2 + 127) / 128 * 128 + 64;
@@ -870,7 +876,7 @@ GF_EXPORT int gf_moe_gemm(const void* a, int lda, const void* w, int N, int K, c
                           const int* tile_row0, const int* num_tiles, int max_tiles, void* out,
                           int first, float limit, float alpha, float up_shift,
                           const float* row_w, int dtype, int tensor_cores, void* stream,
-                          int pairs) {
+                          int pairs, int experts) {
   if (max_tiles <= 0) return 0;
   auto st = (cudaStream_t)stream;
   if (tensor_cores == 2) {                     // the weight-streaming kernel
@@ -878,8 +884,10 @@ GF_EXPORT int gf_moe_gemm(const void* a, int lda, const void* w, int N, int K, c
     if (dtype != GF_BF16 || K % 8 || lda % 8 || N % 2 || (uintptr_t)a % 16 || (uintptr_t)w % 16 ||
         (uintptr_t)out % 8 || smem > kStMaxShared)
       return -3;
-    // at most min(pairs, max_tiles) tiles hold rows; about 16 warps an SM should be busy
-    const int busy = pairs > 0 && pairs < max_tiles ? pairs : max_tiles;
+    // about 16 warps an SM should be busy
+    const int each = pairs <= kStRows * experts ? 2 : 4;       // tiles an expert
+    const int most = pairs <= kStHandful ? kStHandfulTiles : kStTiles;
+    const int busy = most < each * experts ? most : each * experts;
     int parts = 1;
     while (parts < kStWarps && (long long)busy * (N / 16 + 1) * parts < 16 * 148 && K >= parts * 256) parts *= 2;
     const int span = 16 * (kStWarps / parts);

@@ -252,12 +252,12 @@ def _gemm(a, w, plan, out, first, limit, alpha, up_shift, row_w=None):
     f = _fn("moe", "gf_moe_gemm",
             [c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p,
              c_void_p, c_void_p, c_int, c_void_p, c_int, c_float, c_float, c_float, c_void_p,
-             c_int, c_int, c_void_p, c_int])
+             c_int, c_int, c_void_p, c_int, c_int])
     _ok(f(_p(a), a.stride(0), _p(w), w.shape[1], w.shape[2], _p(plan.offsets),
           _p(plan.pair_of_pos), plan.top, _p(plan.tile_expert), _p(plan.tile_row0),
           _p(plan.num_tiles), plan.max_tiles, _p(out), int(first), float(limit), float(alpha),
           float(up_shift), _p(row_w), _code(a.dtype), plan.kernel,
-          _stream(), plan.pairs),
+          _stream(), plan.pairs, plan.num_experts),
         "moe_gemm")
 
 

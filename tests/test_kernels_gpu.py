@@ -562,6 +562,28 @@ def test_grouped_products_that_stream_the_weights(K, F, T, E, top):
         assert ((got - want).abs() <= (F + 8) * 2.0 ** -24 * size).all()
 
 
+@pytest.mark.parametrize("K,F,E,top", [(2048, 1408, 32, 4), (1024, 704, 16, 2), (256, 96, 8, 1)])
+@pytest.mark.parametrize("counts", [(1, 2, 3, 5), (24, 25, 40, 100)])
+def test_a_pairs_result_does_not_depend_on_the_batch(K, F, E, top, counts):
+    """Up to 20 pairs, and up to 16 an expert: the first tokens' rows of a step are those of a shorter step, bit
+    for bit."""
+    from ginfer_b200.ops import moe
+    g = torch.Generator(device=DEV).manual_seed(K)
+    T = max(counts)
+    x = torch.randn(T, K, generator=g, device=DEV).bfloat16()
+    up = (torch.randn(E, 2 * F, K, generator=g, device=DEV) * K ** -0.5).bfloat16()
+    down = (torch.randn(E, K, F, generator=g, device=DEV) * F ** -0.5).bfloat16()
+    idx = torch.rand(T, E, generator=g, device=DEV).argsort(1)[:, :top].int()
+    got = []
+    for n in counts:
+        assert (n * top <= 20) == (counts[0] == 1) and moe.kernel_for(x, n * top, (K, F), (F, K)) == "few"
+        plan = moe.Plan(idx[:n].contiguous(), E, "few")
+        y = moe.grouped_glu(x[:n], up, plan, 1e9, 1.0, 0.0)
+        got.append((y[plan.pos_of_pair.long()], moe.grouped_down(y, down, plan)[plan.pos_of_pair.long()]))
+    for n, (y, rows) in zip(counts, got):
+        assert torch.equal(y, got[-1][0][:n * top]) and torch.equal(rows, got[-1][1][:n * top])
+
+
 @pytest.mark.parametrize("H,G,D,Vd,lens", [(2, 1, 12, 20, [16, 1, 7]), (4, 2, 64, 64, [40, 8, 9, 3]),
                                            (2, 2, 128, 128, [33, 17]), (3, 3, 100, 36, [24, 25, 31, 1]),
                                            (2, 1, 256, 48, [65]), (1, 1, 128, 4, [1, 1, 23]),
