@@ -685,30 +685,30 @@ delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restr
   const int nchunks = (t1 - t0 + CT - 1) / CT;
   const int chunk0 = chunk_number(t0, b, 0);
   const float* coef0 = coef + ((size_t)chunk0 * heads + hl) * kCoefs;
-  auto copy16 = [](float* dst, const float* src, bool in = true) {         // zeros where !in
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src),
-                 "r"(in ? 16 : 0)
-                 : "memory");
+  auto copy16 = [](float* dst, const float* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
   };
   auto ask = [&](int c) {
     float* st = stage + (size_t)(c % kStages) * kStage;
     const int ta = t0 + c * CT, n = min(CT, t1 - ta);
-    // (tokens behind the portion's end are zeros, not an older chunk's)
-    for (int e = threadIdx.x; e < CT * dq; e += blockDim.x) {
+    for (int e = threadIdx.x; e < n * dq; e += blockDim.x) {
       const int t = e / dq, d = 4 * (e - t * dq);
-      const bool in = t < n;
-      const size_t at = (size_t)(ta + (in ? t : 0)) * KD + (size_t)kvh * D + d;
-      if (MODE != PLAIN) copy16(st + t * Dp + d, kn + at, in);
-      copy16(st + kQ + t * Dp + d, qn + at, in);
-      if (MODE != HEADS) copy16(st + kE + t * Dp + d, ke + at, in);
+      const size_t at = (size_t)(ta + t) * KD + (size_t)kvh * D + d;
+      if (MODE != PLAIN) copy16(st + t * Dp + d, kn + at);
+      copy16(st + kQ + t * Dp + d, qn + at);
+      if (MODE != HEADS) copy16(st + kE + t * Dp + d, ke + at);
     }
     if (MODE != HEADS)
       for (int e = threadIdx.x; e < dq; e += blockDim.x)
         copy16(st + kG + 4 * e, total + ((size_t)(chunk0 + c) * heads + hl) * D + 4 * e);
-    for (int e = threadIdx.x; e < CT * vq; e += blockDim.x) {
+    for (int e = threadIdx.x; e < n * vq; e += blockDim.x) {
       const int t = e / vq, d = 4 * (e - t * vq);
-      const bool in = t < n;
-      copy16(st + kVc + t * COLS + d, v + (size_t)(ta + (in ? t : 0)) * ld_v + (size_t)h * Vd + col0 + d, in);
+      copy16(st + kVc + t * COLS + d, v + (size_t)(ta + t) * ld_v + (size_t)h * Vd + col0 + d);
+    }
+    if (n < CT) {                    // behind the portion's end: zeros, not an older chunk's tokens
+      for (int e = threadIdx.x; e < (CT - n) * Dp; e += blockDim.x)
+        st[n * Dp + e] = st[CT * Dp + n * Dp + e] = 0.f;
+      for (int e = threadIdx.x; e < (CT - n) * COLS; e += blockDim.x) st[kVc + n * COLS + e] = 0.f;
     }
     for (int e = threadIdx.x; e < kCoefs / 4; e += blockDim.x)
       copy16(st + kC + 4 * e, coef0 + (size_t)c * heads * kCoefs + 4 * e);
@@ -787,16 +787,28 @@ delta_chunk_recurrence_kernel(const float* __restrict__ qn, const float* __restr
       const float4* Mp = reinterpret_cast<const float4*>(cf + kCoefM + tok * CT);
       const float4 m0 = Mp[0], m1 = Mp[1];
       const int row = t0 + c * CT + tok;
+      const float m[CT] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+      float out[CP], all = 0.f;
 #pragma unroll
       for (int y = 0; y < CP; ++y) {
-        const float(&w)[CT] = u[y];
-        float out = Gp * x[y][LANES == CT && MODE != PLAIN ? CT : 0];
-        // (M is 0 behind a token, but 0 times what is no number would reach back)
-        auto seen = [&](int j) { return j <= tok ? w[j] : 0.f; };
-        out = fmaf(m0.x, w[0], fmaf(m0.y, seen(1), fmaf(m0.z, seen(2), fmaf(m0.w, seen(3), out))));
-        out = fmaf(m1.x, seen(4), fmaf(m1.y, seen(5), fmaf(m1.z, seen(6), fmaf(m1.w, seen(7), out))));
+        out[y] = Gp * x[y][LANES == CT && MODE != PLAIN ? CT : 0];
+#pragma unroll
+        for (int j = 0; j < CT; ++j) out[y] = fmaf(m[j ^ 3], u[y][j ^ 3], out[y]);
+        all += out[y];
+      }
+      if (isnan(all)) {          // M is 0 for later tokens, but 0 times what is no number would reach back
+#pragma unroll
+        for (int y = 0; y < CP; ++y) {
+          out[y] = Gp * x[y][LANES == CT && MODE != PLAIN ? CT : 0];
+#pragma unroll
+          for (int j = 0; j < CT; ++j)
+            if ((j ^ 3) <= tok) out[y] = fmaf(m[j ^ 3], u[y][j ^ 3], out[y]);
+        }
+      }
+#pragma unroll
+      for (int y = 0; y < CP; ++y) {
         const int col = col0 + lc + 16 * y;
-        if (col < Vd && row < t1 && p >= LANES - CT) o[(size_t)row * HV + (size_t)h * Vd + col] = out;
+        if (col < Vd && row < t1 && p >= LANES - CT) o[(size_t)row * HV + (size_t)h * Vd + col] = out[y];
       }
     }
     const float Gc = MODE == HEADS ? cf[kCoefG + CT - 1] : 1.f;
