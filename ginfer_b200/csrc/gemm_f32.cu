@@ -6,9 +6,10 @@
 // The order of every sum is fixed by N and K alone, so a row's result does not depend on what else is
 // in the batch, nor on which of the two kernels below computes it: K is cut into 2, 4 or 8 segments, a
 // segment is two chains of FMAs in ascending k (even and odd k) and their sum, and the segments are
-// added in pairs, pairs of pairs, and so on.  The two chains are the halves of fma.rn.f32x2: one FMA an instruction
-// leaves the pipes of an sm_100 SM at half their rate (37 TFLOP/s at 148 SMs), and pairs of
-// neighbouring k are what a 16-byte load of either operand holds.
+// added in pairs, pairs of pairs, and so on.  The two chains are the halves of fma.rn.f32x2: pairs of
+// neighbouring k are what a 16-byte load of either operand holds, and half as many instructions issue.
+// (It is not the pipes' rate that asks for pairs: tiles of 64 rows with one FMA an instruction measured the
+// same 37 TFLOP/s, half of what the pipes of 148 SMs can do.)
 //
 //   rows_kernel   up to 16 rows of A, as a decode step has them: bound by reading W once.  A block is
 //                 one warp: 32 rows of W and two segments of K, which half a warp each takes; the

@@ -9,7 +9,8 @@
 // has four columns of D / (256 / lanes a row) rows: 16 loads of 16 bytes under way, whole rows at a time.
 // Then one sum over the block (both of the delta rule's, S'^T k and S'^T q, at once).  fp32 throughout.
 // Measured on a B200, 16 heads of 128 x 128: 32 requests 14.0 us (67 MB: 10.3 at 6.54 TB/s), 29.4 with a lane a
-// column; 8 requests 7.1 and 9.7; the delta rule with channel decays, 4 requests 5.2 and 14.8.
+// column; 8 requests 7.1 and 9.7.  (Layers with the delta rule and channel decays stay with the kernel that
+// walks over tokens, ops/delta.py: recurrence.)
 #include "common.cuh"
 
 namespace gf {

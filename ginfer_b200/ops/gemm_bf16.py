@@ -1,5 +1,6 @@
-"""bf16 matrix products on the 5th-generation tensor cores (``csrc/gemm_bf16.cu``: tcgen05.mma with
-the accumulator in tensor memory, operands staged by TMA)."""
+"""bf16 matrix products of few tokens: on the 5th-generation tensor cores (``csrc/gemm_bf16.cu``: tcgen05.mma
+with the accumulator in tensor memory, operands staged by TMA), and for up to 8 tokens and small weights
+by streaming the weights through mma.sync's registers (``csrc/gemm_stream.cu``, :func:`stream`)."""
 from __future__ import annotations
 
 from ctypes import c_float, c_int, c_void_p
@@ -184,7 +185,7 @@ def gemm(x, weight, bias_f32=None, out_dtype=torch.bfloat16, epi: int = 0, split
 # much again is streamed) the products run on the kernel that has its weights in registers before the
 # kernel ahead is done (csrc/gemm_stream.cu).  Decode steps on a B200 with products of up to 9.7 MB / of
 # up to 14.5 MB / of up to 27 MB on it, none: pimidra m, 2 requests 0.589 / 0.569 / 0.581, 0.610 ms;
-# lasizen m, 4 requests 0.513 / 0.499 / 0.501, 0.509; vilepel m, 4 requests 0.872 / 0.874 / 0.892, 0.960.
+# lasizen m, 4 requests 0.513 / 0.499 / 0.501, 0.509.  (A layer may ask to be left out: ``streamed``.)
 # Plain products with bf16 results come up to four rows only: beside Qwen2's large products they cost its
 # decode step of 8 requests 2 % at the 1.5B shape (47.5 -> 48.4 ms for the whole batch of 512-token prompts)
 # and give 4 requests 1 %; lasizen s, one request: 9.7 ms without them, 9.1 with; bapivik s, 4 requests:

@@ -3,8 +3,9 @@ reference reads the same memory as a column-major ``[in, out]`` view:
 ``ginfer/core/layer/linear.cc:13-16``).
 
 float32: the hand-written FMA kernel of ``csrc/gemm_f32.cu`` (no reduced-precision mode).
-bfloat16: the tcgen05 kernels of ``csrc/gemm_bf16.cu`` (few tokens) and ``csrc/gemm_prefill.cu``
-(the gated product of many tokens) where they are the faster ones, else cuBLAS through ``torch``
+bfloat16: ``csrc/gemm_stream.cu`` (mma.sync, up to 8 tokens and small weights) and the tcgen05 kernels of
+``csrc/gemm_bf16.cu`` (few tokens) and ``csrc/gemm_prefill.cu`` (the gated product of many tokens)
+where they are the faster ones, else cuBLAS through ``torch``
 (fp32 accumulation), which is what the reference uses for every product.
 """
 from __future__ import annotations
@@ -37,7 +38,7 @@ class Linear:
     """``y = x W^T + b``.  ``out_dtype`` float32 asks for fp32 results from bf16 operands (the
     output head).  ``activation``: the product passes ``"relu2"`` (``relu(.)^2``) or ``"xielu"``
     (``act_consts = (a, b)``: ``a z^2 + z/2`` above zero, ``b (e^z - 1 - z) + z/2`` below), in the
-    product's epilogue where the tcgen05 kernel runs it (few tokens), else in a kernel behind the
+    product's epilogue where one of this package's kernels runs it (few tokens), else in a kernel behind the
     library's.  ``streamed`` false: products of few rows stay off the register-streaming kernel
     (``csrc/gemm_stream.cu``), which sums in another order than the tcgen05 kernel."""
 
