@@ -230,6 +230,19 @@ inline int launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t
   return launch_kernel_cluster_dims(kernel, grid, block, smem, stream, 1, false, args...);
 }
 
+// Behind everything ahead in the stream, not beside it: for a grid whose blocks run long and unequally, which
+// the device spreads evenly over the SMs only where they are empty.
+template <typename... KArgs, typename... Args>
+inline int launch_kernel_behind(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                cudaStream_t stream, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  return (int)cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+
 }  // namespace gf
 
 // Every library exports this switch for programmatic dependent launch (on by default).

@@ -16,6 +16,7 @@
 //                            independent: four lanes or a warp share a column (a share of the rows
 //                            each, in registers).  The tokens' operands come through two stages of
 //                            shared memory, a chunk ahead (cp.async).
+//   delta_tree_kernel        the same with eight or sixteen lanes for two columns (see there).
 //   delta_chunk_coef_kernel, linear_chunk_coef_kernel, delta_chunk_recurrence_kernel   the recurrence of
 //                            long portions, eight tokens at a time: the delta rule with one decay a head,
 //                            plain linear attention with a decay a key channel (see there).
@@ -272,6 +273,62 @@ __device__ __forceinline__ void copy_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// What a block of the recurrence stages of a token: q, k, decay and v rows and beta of its head (and columns),
+// GD, GD, HD, HV and H floats from one token to the next.  vec: 16-byte copies.
+struct DeltaStage {
+  const float *q, *k, *v, *g, *beta;
+  size_t GD, HD, HV;
+  int H, D, ncols;
+  bool vec;
+};
+// Tokens ta .. ta + n - 1 into a stage: k | q | g rows of Dp floats (g only with a decay a channel), v columns,
+// beta, the head's decay.  Of a row, quad x (four neighbours) lies at quad x / QL + x % QL * (Dp / 4 / QL): where
+// a lane has QL quads in a row, its lanes' reads of one of them are then neighbours and meet every bank once.
+template <int Dp, bool ONE_DECAY, int QL>
+__device__ __forceinline__ void ask_tokens(const DeltaStage& src, float* st, int ta, int n, int tid,
+                                           int threads) {
+  constexpr int kV = (ONE_DECAY ? 2 : 3) * Dp, kB = kV + kMaxColumnsPerBlock, kTok = kB + 4;
+  const int D = src.D;
+  auto quad = [](int x) { return 4 * (QL == 1 ? x : x / QL + x % QL * (Dp / 4 / QL)); };
+  auto place = [&](int d) { return QL == 1 ? d : quad(d >> 2) + (d & 3); };
+  if (src.vec) {                                   // (a thread keeps the same piece of every token)
+    const int dq = D >> 2, nd = (ONE_DECAY ? 2 : 3) * dq, pieces = nd + (src.ncols >> 2);
+    for (int e = tid; e < pieces; e += threads) {
+      const float* from;
+      int dst, step;                               // source floats from one token to the next
+      if (e < dq) from = src.k + (size_t)ta * src.GD + 4 * e, dst = quad(e), step = (int)src.GD;
+      else if (e < 2 * dq)
+        from = src.q + (size_t)ta * src.GD + 4 * (e - dq), dst = Dp + quad(e - dq), step = (int)src.GD;
+      else if (!ONE_DECAY && e < nd)
+        from = src.g + (size_t)ta * src.HD + 4 * (e - 2 * dq), dst = 2 * Dp + quad(e - 2 * dq),
+        step = (int)src.HD;
+      else from = src.v + (size_t)ta * src.HV + 4 * (e - nd), dst = kV + 4 * (e - nd), step = (int)src.HV;
+      for (int tt = 0; tt < n; ++tt)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(st + (size_t)tt * kTok + dst)),
+                     "l"(from + (size_t)tt * step)
+                     : "memory");
+    }
+    if (tid < n) {
+      copy_async_4(st + (size_t)tid * kTok + kB, src.beta + (size_t)(ta + tid) * src.H);
+      if (ONE_DECAY) copy_async_4(st + (size_t)tid * kTok + kB + 1, src.g + (size_t)(ta + tid) * src.H);
+    }
+    return;
+  }
+  const int rd = (ONE_DECAY ? 2 : 3) * D;
+  const int per = rd + src.ncols + (ONE_DECAY ? 2 : 1);
+  for (int i = tid; i < n * per; i += threads) {
+    const int tt = i / per, e = i - tt * per;
+    const size_t t = (size_t)(ta + tt);
+    float* dst = st + (size_t)tt * kTok;
+    if (e < D) copy_async_4(dst + place(e), src.k + t * src.GD + e);
+    else if (e < 2 * D) copy_async_4(dst + Dp + place(e - D), src.q + t * src.GD + (e - D));
+    else if (!ONE_DECAY && e < rd) copy_async_4(dst + 2 * Dp + place(e - 2 * D), src.g + t * src.HD + (e - 2 * D));
+    else if (e < rd + src.ncols) copy_async_4(dst + kV + (e - rd), src.v + t * src.HV + (e - rd));
+    else if (e == rd + src.ncols) copy_async_4(dst + kB, src.beta + t * src.H);
+    else copy_async_4(dst + kB + 1, src.g + t * src.H);
+  }
+}
+
 // A block = (request, head, 128 / LP columns of S); LP lanes share a column, DPER rows each.  The
 // tokens' k, q, g rows (padded to Dp = LP * DPER floats, the padding zero), the block's v columns and
 // beta come through three stages of shared memory, CHUNK tokens each, asked for two chunks ahead
@@ -312,54 +369,13 @@ delta_recurrence_kernel(const float* __restrict__ qn, const float* __restrict__ 
   const int t0 = cu_seqlens[b], t1 = cu_seqlens[b + 1];
   const size_t GD = (size_t)dm.G * D, HD = (size_t)dm.H * D, HV = (size_t)dm.H * Vd;
   const int ncols = min(cols, Vd - col0);
-  // 16-byte copies where rows allow it (a thread keeps the same piece of every token), else 4-byte
-  const bool vec = (D & 3) == 0 && (Vd & 3) == 0 && (ncols & 3) == 0;
-  const int dq = D >> 2, nd = (ONE_DECAY ? 2 : 3) * dq, pieces = nd + (ncols >> 2);
+  const DeltaStage src{qn + (size_t)kvh * D, kn + (size_t)kvh * D, v + (size_t)h * Vd + col0,
+                       ONE_DECAY ? g + h : g + (size_t)h * D, beta + h, GD, HD, HV, dm.H, D, ncols,
+                       (D & 3) == 0 && (Vd & 3) == 0 && (ncols & 3) == 0};
   auto ask = [&](int chunk) {                      // the chunk's tokens into stage chunk % kStages
-    float* st = stage + (size_t)(chunk % kStages) * CHUNK * kTok;
-    const int ta = t0 + chunk * CHUNK, n = min(CHUNK, t1 - ta);
-    if (vec) {
-      for (int e = threadIdx.x; e < pieces; e += blockDim.x) {
-        const float* src;
-        int dst, step;                             // source floats from one token to the next
-        if (e < dq) src = kn + (size_t)ta * GD + (size_t)kvh * D + 4 * e, dst = 4 * e, step = (int)GD;
-        else if (e < 2 * dq)
-          src = qn + (size_t)ta * GD + (size_t)kvh * D + 4 * (e - dq), dst = Dp + 4 * (e - dq), step = (int)GD;
-        else if (!ONE_DECAY && e < nd)
-          src = g + (size_t)ta * HD + (size_t)h * D + 4 * (e - 2 * dq), dst = 2 * Dp + 4 * (e - 2 * dq),
-          step = (int)HD;
-        else
-          src = v + (size_t)ta * HV + (size_t)h * Vd + col0 + 4 * (e - nd),
-          dst = kV + 4 * (e - nd), step = (int)HV;
-        for (int tt = 0; tt < n; ++tt)
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                           smem_u32(st + (size_t)tt * kTok + dst)),
-                       "l"(src + (size_t)tt * step)
-                       : "memory");
-      }
-      if (threadIdx.x < n) {
-        copy_async_4(st + (size_t)threadIdx.x * kTok + kB,
-                     beta + (size_t)(ta + threadIdx.x) * dm.H + h);
-        if (ONE_DECAY)
-          copy_async_4(st + (size_t)threadIdx.x * kTok + kB + 1,
-                       g + (size_t)(ta + threadIdx.x) * dm.H + h);
-      }
-    } else {
-      const int rd = (ONE_DECAY ? 2 : 3) * D;
-      const int per = rd + ncols + (ONE_DECAY ? 2 : 1);
-      for (int i = threadIdx.x; i < n * per; i += blockDim.x) {
-        const int tt = i / per, e = i - tt * per;
-        const size_t t = (size_t)(ta + tt);
-        float* dst = st + (size_t)tt * kTok;
-        if (e < D) copy_async_4(dst + e, kn + t * GD + (size_t)kvh * D + e);
-        else if (e < 2 * D) copy_async_4(dst + Dp + (e - D), qn + t * GD + (size_t)kvh * D + (e - D));
-        else if (!ONE_DECAY && e < rd) copy_async_4(dst + 2 * Dp + (e - 2 * D), g + t * HD + (size_t)h * D + (e - 2 * D));
-        else if (e < rd + ncols)
-          copy_async_4(dst + kV + (e - rd), v + t * HV + (size_t)h * Vd + col0 + (e - rd));
-        else if (e == rd + ncols) copy_async_4(dst + kB, beta + t * dm.H + h);
-        else copy_async_4(dst + kB + 1, g + t * dm.H + h);
-      }
-    }
+    const int ta = t0 + chunk * CHUNK;
+    ask_tokens<Dp, ONE_DECAY, 1>(src, stage + (size_t)(chunk % kStages) * CHUNK * kTok, ta,
+                                 min(CHUNK, t1 - ta), threadIdx.x, THREADS);
     copy_async_commit();
   };
   const int nchunks = (t1 - t0 + CHUNK - 1) / CHUNK;
@@ -438,6 +454,225 @@ delta_recurrence_kernel(const float* __restrict__ qn, const float* __restrict__ 
     for (int i = 0; i < DPER; ++i)
       if (row0 + i < D) Sg[(size_t)(row0 + i) * Vd] = S[i];
   }
+}
+
+// ---- few long portions ----------------------------------------------------------------------------
+// Where requests x heads x columns do not fill the device (one long prompt, a small decode batch) the time
+// is the longest portion's chain from token to token, and behind that what shared memory gives an SM a
+// cycle: with a warp a column a token took three 16-byte reads a lane and ten shuffles for every column.
+// Here LP lanes share two neighbouring columns, DPER rows each: a read of k, q and g serves both, and most of
+// a sum's tree lies in registers.  While a token's sum goes through the lanes, the warp reads the next
+// token's operands and multiplies the state that the token before left by that token's q.
+// The sums over the rows are one binary tree over LP * DPER products in the rows' order (a lane's rows, then
+// lanes 1, 2, 4, 8 apart), as they were with 4 rows a lane: the same bits for every LP and DPER.
+// A block is up to four groups of 128 threads that share nothing but the SM, each with a request of its own,
+// long and short ones together: blocks of one request each are placed two and more to an SM while others are
+// empty (1,201 tokens beside three single ones: 423 us; alone 298).
+// On a B200, prompts of 150, 300, 600 and 1,201 tokens, 16 heads of 128 x 128: 420 us a layer (a warp a column:
+// 740); one of 1,201 tokens 288 (446).
+constexpr int kTreeThreads = 128, kTreeChunk = 8, kTreeGroups = 4;
+
+template <int N> __device__ __forceinline__ float tree_sum(const float* p) {
+  if constexpr (N == 1) return p[0];
+  else return tree_sum<N / 2>(p) + tree_sum<N / 2>(p + N / 2);
+}
+
+template <int DPER, int LP, bool ONE_DECAY>
+__global__ void __launch_bounds__(kTreeThreads * kTreeGroups, 1)
+delta_tree_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
+                  const float* __restrict__ v, const float* __restrict__ g,
+                  const float* __restrict__ beta, float* __restrict__ state,
+                  const int* __restrict__ cu_seqlens, const int* __restrict__ slot_ids,
+                  DeltaDims dm, int B, int by_length, int whole, float* __restrict__ o) {
+  constexpr int Dp = LP * DPER, CHUNK = kTreeChunk, COLS = 2;
+  constexpr int kV = (ONE_DECAY ? 2 : 3) * Dp;                 // where a token's v columns start
+  constexpr int kB = kV + kMaxColumnsPerBlock;                 // beta (and the head's decay)
+  constexpr int kTok = kB + 4;                                 // floats a token in a stage
+  constexpr int cols = kTreeThreads / LP * COLS;
+  static_assert(cols <= kMaxColumnsPerBlock && DPER % 4 == 0 && CHUNK * COLS >= LP);
+  extern __shared__ __align__(16) float stages[];              // a group: [kStages][CHUNK][kTok]
+  __shared__ int request[kTreeGroups];
+  const int tid = threadIdx.x % kTreeThreads, group = threadIdx.x / kTreeThreads;
+  float* stage = stages + (size_t)group * kStages * CHUNK * kTok;
+  auto group_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(kTreeThreads) : "memory"); };
+  const int part = tid % LP, lc = tid / LP * COLS;
+  const int of = blockIdx.x / dm.H, h = blockIdx.x - of * dm.H, nz = gridDim.x / dm.H;
+  const int col0 = blockIdx.y * cols, col = col0 + lc;
+  pdl_trigger();
+  const int D = dm.D, Vd = dm.Vd;
+  if (D != Dp) {                                               // the rows that are not there are zero
+    for (int i = tid; i < kStages * CHUNK * kTok; i += kTreeThreads) stage[i] = 0.f;
+    group_sync();
+  }
+  pdl_wait();
+  // the group's request: the b-th longest portion's; groups of odd number take theirs from the other end
+  int b = group * nz + (group & 1 ? nz - 1 - of : of);
+  if (b >= B) return;
+  if (by_length) {
+    for (int i = tid; i < B; i += kTreeThreads) {
+      const int mine = cu_seqlens[i + 1] - cu_seqlens[i];
+      int before = 0;
+      for (int j = 0; j < B; ++j) {
+        const int its = cu_seqlens[j + 1] - cu_seqlens[j];
+        before += its > mine || (its == mine && j < i);
+      }
+      if (before == b) request[group] = i;
+    }
+    group_sync();
+    b = request[group];
+  }
+  const int row0 = part * DPER;
+  const int kvh = h / (dm.H / dm.G);
+  const int t0 = cu_seqlens[b], t1 = cu_seqlens[b + 1];
+  const size_t GD = (size_t)dm.G * D, HD = (size_t)dm.H * D, HV = (size_t)dm.H * Vd;
+  const int ncols = min(cols, Vd - col0);
+  const DeltaStage src{qn + (size_t)kvh * D, kn + (size_t)kvh * D, v + (size_t)h * Vd + col0,
+                       ONE_DECAY ? g + h : g + (size_t)h * D, beta + h, GD, HD, HV, dm.H, D, ncols,
+                       (D & 3) == 0 && (Vd & 3) == 0 && (ncols & 3) == 0};
+  auto ask = [&](int chunk) {                      // the chunk's tokens into stage chunk % kStages
+    const int ta = t0 + chunk * CHUNK;
+    ask_tokens<Dp, ONE_DECAY, DPER / 4>(src, stage + (size_t)(chunk % kStages) * CHUNK * kTok, ta,
+                                        min(CHUNK, t1 - ta), tid, kTreeThreads);
+    copy_async_commit();
+  };
+  const int nchunks = (t1 - t0 + CHUNK - 1) / CHUNK;
+  for (int c = 0; c < kStages - 1; ++c) {
+    if (c < nchunks) ask(c);
+    else copy_async_commit();
+  }
+  // the state, while the first chunks come: both columns at once where rows are whole and aligned
+  float* Sg = state + (size_t)slot_ids[b] * dm.state_stride + (size_t)h * D * Vd + col;
+  float S[DPER][COLS];
+#pragma unroll
+  for (int i = 0; i < DPER; ++i) {
+    S[i][0] = S[i][1] = 0.f;
+    if (row0 + i < D) {
+      const float* at = Sg + (size_t)(row0 + i) * Vd;
+      if (whole) {
+        if (col < Vd) {
+          const float2 two = *reinterpret_cast<const float2*>(at);
+          S[i][0] = two.x, S[i][1] = two.y;
+        }
+      } else {
+#pragma unroll
+        for (int c = 0; c < COLS; ++c)
+          if (col + c < Vd) S[i][c] = at[c];
+      }
+    }
+  }
+  for (int ch = 0; ch < nchunks; ++ch) {
+    if (ch + kStages - 1 < nchunks) ask(ch + kStages - 1);     // (the stage that chunk ch - 1 left)
+    else copy_async_commit();
+    copy_async_wait<kStages - 1>();
+    group_sync();
+    const float* tok = stage + (size_t)(ch % kStages) * CHUNK * kTok;
+    const int ta = t0 + ch * CHUNK, n = min(CHUNK, t1 - ta);
+    float outp[CHUNK * COLS];                                  // summed over the lanes behind the chunk
+    float k[DPER], gd[DPER], q[DPER], vb[COLS + 1], before[DPER][COLS];
+    auto quads = [&](const float* from, float (&to)[DPER]) {
+#pragma unroll
+      for (int i = 0; i < DPER; i += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(from + (i / 4 * LP + part) * 4);
+        to[i] = x.x, to[i + 1] = x.y, to[i + 2] = x.z, to[i + 3] = x.w;
+      }
+    };
+    auto operands = [&](const float* t) {                      // all but q
+      quads(t, k);
+      if (!ONE_DECAY) quads(t + 2 * Dp, gd);
+      else gd[0] = t[kB + 1];
+      const float2 vv = *reinterpret_cast<const float2*>(t + kV + lc);
+      vb[0] = vv.x, vb[1] = vv.y, vb[2] = t[kB];
+    };
+    auto read_out = [&](int tt) {
+#pragma unroll
+      for (int c = 0; c < COLS; ++c) {
+        float p[DPER];
+#pragma unroll
+        for (int i = 0; i < DPER; ++i) p[i] = fmaf(before[i][c], q[i], 0.f);
+        outp[tt * COLS + c] = tree_sum<DPER>(p);
+      }
+    };
+    auto token = [&](int tt, bool more) {
+      float dot[COLS], kc[DPER];
+#pragma unroll
+      for (int i = 0; i < DPER; ++i) kc[i] = k[i];
+#pragma unroll
+      for (int c = 0; c < COLS; ++c) {
+        float p[DPER];
+#pragma unroll
+        for (int i = 0; i < DPER; ++i) {
+          S[i][c] *= gd[ONE_DECAY ? 0 : i];
+          p[i] = fmaf(S[i][c], kc[i], 0.f);
+        }
+        dot[c] = tree_sum<DPER>(p);
+      }
+      const float vc[COLS] = {vb[0], vb[1]}, bc = vb[2];
+#pragma unroll
+      for (int c = 0; c < COLS; ++c) dot[c] += __shfl_xor_sync(0xffffffffu, dot[c], 1);
+      if (more) operands(tok + kTok);
+#pragma unroll
+      for (int c = 0; c < COLS; ++c) dot[c] += __shfl_xor_sync(0xffffffffu, dot[c], 2);
+      if (tt > 0) read_out(tt - 1);
+#pragma unroll
+      for (int sh = 4; sh < LP; sh <<= 1) {
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) dot[c] += __shfl_xor_sync(0xffffffffu, dot[c], sh);
+        if (sh == 4) quads(tok + Dp, q);
+      }
+#pragma unroll
+      for (int c = 0; c < COLS; ++c) {
+        const float u = bc * (vc[c] - dot[c]);
+#pragma unroll
+        for (int i = 0; i < DPER; ++i) before[i][c] = S[i][c] = fmaf(kc[i], u, S[i][c]);
+      }
+      tok += kTok;
+    };
+    operands(tok);
+    if (n == CHUNK) {                                          // (no branch between tokens)
+#pragma unroll
+      for (int tt = 0; tt < CHUNK; ++tt) token(tt, tt + 1 < CHUNK);
+      read_out(CHUNK - 1);
+    } else {
+#pragma unroll
+      for (int tt = 0; tt < CHUNK; ++tt) {
+        outp[tt * COLS] = outp[tt * COLS + 1] = 0.f;
+        if (tt < n) token(tt, tt + 1 < n);
+        if (tt == n - 1) read_out(tt);
+      }
+    }
+    // add up across the lanes; every halving of the list leaves a lane the half that its bit names
+    int first = 0;
+    constexpr int kAll = CHUNK * COLS;
+#pragma unroll
+    for (int sh = 1; sh < LP; sh <<= 1) {
+      const int half = kAll / (2 * sh);
+      const bool up = part & sh;
+#pragma unroll
+      for (int m = 0; m < half; ++m) {
+        const float got = __shfl_xor_sync(0xffffffffu, up ? outp[m] : outp[m + half], sh);
+        outp[m] = (up ? outp[m + half] : outp[m]) + got;
+      }
+      if (up) first += half;
+    }
+#pragma unroll
+    for (int m = 0; m < kAll / LP; ++m) {
+      const int tt = (first + m) / COLS, c = (first + m) % COLS;
+      if (tt < n && col + c < Vd) o[(size_t)(ta + tt) * HV + (size_t)h * Vd + col + c] = outp[m];
+    }
+    group_sync();                                  // the stage is free for the chunk after next
+  }
+#pragma unroll
+  for (int i = 0; i < DPER; ++i)
+    if (row0 + i < D) {
+      float* at = Sg + (size_t)(row0 + i) * Vd;
+      if (whole) {
+        if (col < Vd) *reinterpret_cast<float2*>(at) = make_float2(S[i][0], S[i][1]);
+      } else {
+#pragma unroll
+        for (int c = 0; c < COLS; ++c)
+          if (col + c < Vd) at[c] = S[i][c];
+      }
+    }
 }
 
 // ---- eight tokens at a time ---------------------------------------------------------------------
@@ -1031,10 +1266,46 @@ GF_EXPORT int gf_delta_recurrence(const float* qn, const float* kn, const float*
     GF_GO(16, 16)
 #undef GF_GO
   }
-  // few (request, head, column) triples: a warp (sixteen lanes for key sizes up to 64) a column
-  // instead of four lanes (see the kernel)
+  // few (request, head, column) triples: more lanes a column than four (see the kernels)
   const bool wide = (long long)B * H * ((Vd + 31) / 32) < 2 * 148;
-  const int lp = !wide ? 4 : (D <= 64 ? 16 : 32);
+  if (wide && D <= 128) {
+    const int whole = Vd % 2 == 0 && state_stride % 2 == 0 && ((uintptr_t)state & 7) == 0;
+#define GF_TREE(DPER, LP, ONE)                                                                     \
+  {                                                                                                \
+    constexpr int cols = kTreeThreads / LP * 2;                                                    \
+    constexpr size_t smem = (size_t)kStages * kTreeChunk *                                         \
+                            ((ONE ? 2 : 3) * LP * DPER + kMaxColumnsPerBlock + 4) * sizeof(float); \
+    const int ny = (Vd + cols - 1) / cols;                                                         \
+    if (max_q_len == 1)                                                                            \
+      return launch_kernel(delta_tree_kernel<DPER, LP, ONE>, dim3(B * H, ny), dim3(kTreeThreads),  \
+                           smem, st, qn, kn, v, g, beta, state, cu_seqlens, slot_ids, dm, B, 0,    \
+                           whole, o);                                                              \
+    /* the fewest requests a block with which every block has an SM of its own */                  \
+    int groups = 1;                                                                                \
+    while (groups < kTreeGroups && (long long)H * ny * ((B + groups - 1) / groups) > 148) groups *= 2; \
+    const int nz = (B + groups - 1) / groups;                                                      \
+    const size_t alone = 120 * 1024, all = smem * groups;                                          \
+    static OncePerDevice attrs;                                                                    \
+    if (int rc = attrs.run([&] {                                                                   \
+          return cudaFuncSetAttribute(delta_tree_kernel<DPER, LP, ONE>,                            \
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);    \
+        }))                                                                                        \
+      return rc;                                                                                   \
+    return launch_kernel_behind(delta_tree_kernel<DPER, LP, ONE>, dim3(nz * H, ny),                \
+                                dim3(kTreeThreads * groups),                                       \
+                                (long long)H * ny * nz <= 148 && all < alone ? alone : all, st,    \
+                                qn, kn, v, g, beta, state, cu_seqlens, slot_ids, dm, B, B > 1,     \
+                                whole, o);                                                         \
+  }
+    if (D <= 64) {
+      if (one_decay) GF_TREE(8, 8, true)
+      GF_TREE(8, 8, false)
+    }
+    if (one_decay) GF_TREE(8, 16, true)
+    GF_TREE(8, 16, false)
+#undef GF_TREE
+  }
+  const int lp = wide ? 32 : 4;
   const int threads = lp == 32 ? 256 : kRecurrenceThreads;
   const int cols = threads / lp;
   const dim3 grid(B * H, (Vd + cols - 1) / cols);
@@ -1057,8 +1328,6 @@ GF_EXPORT int gf_delta_recurrence(const float* qn, const float* kn, const float*
   GF_GO(16, 4, 8, kRecurrenceThreads)
   GF_GO(32, 4, 8, kRecurrenceThreads)
   GF_GO(64, 4, 4, kRecurrenceThreads)
-  GF_GO(4, 16, 8, kRecurrenceThreads)
-  GF_GO(4, 32, 8, 256)
   GF_GO(8, 32, 4, 256)
 #undef GF_GO
 #undef GF_AS

@@ -123,11 +123,11 @@ def recurrence(qn, kn, v, g, beta, state: torch.Tensor, ctx) -> torch.Tensor:
     f = _fn("delta_rule", "gf_delta_recurrence",
             [c_void_p] * 8 + [c_int] * 6 + [c_void_p, c_int, c_void_p, c_int, c_void_p])
     one = int(g.dim() == 2)
-    scratch, longest = None, int(ctx.max_q_len) if one else 0
-    if longest == 1 and state_step(qn.view(T, G * D), kn.view(T, G * D), v.view(T, H * Vd), g.view(T, -1),
-                                   state, ctx, H, G, D, Vd, o.view(T, H * Vd), beta=beta):
+    scratch, longest = None, int(ctx.max_q_len if one else getattr(ctx, "max_q_len", 0))
+    if one and longest == 1 and state_step(qn.view(T, G * D), kn.view(T, G * D), v.view(T, H * Vd),
+                                           g.view(T, -1), state, ctx, H, G, D, Vd, o.view(T, H * Vd), beta=beta):
         return o
-    if longest >= CHUNKED_MIN_TOKENS:
+    if one and longest >= CHUNKED_MIN_TOKENS:
         scratch = torch.empty(chunk_words(T, ctx.num_seqs, H, D, one), dtype=torch.float32,
                               device=qn.device)
     rc = f(_p(qn), _p(kn), _p(v), _p(g), _p(beta), _p(state), _p(ctx.cu_seqlens_q),

@@ -584,6 +584,40 @@ def test_a_pairs_result_does_not_depend_on_the_batch(K, F, E, top, counts):
         assert torch.equal(y, got[-1][0][:n * top]) and torch.equal(rows, got[-1][1][:n * top])
 
 
+@pytest.mark.parametrize("H,G,D,Vd,lens,one", [
+    (16, 16, 128, 128, [70, 9, 33, 5], 0), (16, 8, 100, 126, [8, 16, 1, 7], 0), (4, 4, 64, 64, [24, 3], 0),
+    (2, 1, 40, 31, [17, 8, 9], 0), (3, 3, 128, 32, [1, 1, 1], 0), (2, 2, 96, 48, [9, 15, 8], 1),
+    (1, 1, 128, 20, [3, 1, 8, 2, 9, 7, 16, 5] * 20, 0)])
+def test_delta_rule_of_several_portions_is_that_of_each(H, G, D, Vd, lens, one):
+    """Requests of a step share blocks, the longest first: outputs and states are, bit for bit, those of each
+    request in a step of its own (the sums over the rows are one tree, wherever the request is), at lengths
+    around the chunks of eight tokens, key sizes with rows that are not there and odd numbers of columns."""
+    from types import SimpleNamespace
+    from ginfer_b200.ops import delta
+    g0 = torch.Generator().manual_seed(D + Vd)
+    B, T = len(lens), sum(lens)
+    q, k = (torch.nn.functional.normalize(torch.randn(T, G, D, generator=g0), dim=-1).cuda() for _ in "qk")
+    v, beta = torch.randn(T, H, Vd, generator=g0).cuda(), torch.rand(T, H, generator=g0).cuda()
+    g = torch.rand(*((T, H) if one else (T, H, D)), generator=g0).cuda()
+    state0 = torch.randn(B + 1, H * D * Vd + 1, generator=g0).cuda()
+    slots = torch.randperm(B + 1, generator=g0)[:B]
+
+    def run(requests):
+        state = state0.clone()
+        rows = torch.cat([torch.arange(sum(lens[:b]), sum(lens[:b + 1])) for b in requests]).cuda()
+        own = [lens[b] for b in requests]
+        ctx = SimpleNamespace(num_seqs=len(own), slot_ids=slots[requests].int().cuda(), max_q_len=max(own),
+                              cu_seqlens_q=torch.tensor([0] + own).cumsum(0).int().cuda())
+        return delta.recurrence(*(t[rows] for t in (q, k, v, g, beta)), state, ctx), state
+    o, state = run(list(range(B)))
+    for b in range(B):
+        o1, state1 = run([b])
+        assert torch.equal(o[sum(lens[:b]):sum(lens[:b + 1])], o1)
+        assert torch.equal(state[slots[b]], state1[slots[b]])
+    assert torch.equal(state[[i for i in range(B + 1) if i not in slots.tolist()]],
+                       state0[[i for i in range(B + 1) if i not in slots.tolist()]])
+
+
 @pytest.mark.parametrize("H,G,D,Vd,lens", [(2, 1, 12, 20, [16, 1, 7]), (4, 2, 64, 64, [40, 8, 9, 3]),
                                            (2, 2, 128, 128, [33, 17]), (3, 3, 100, 36, [24, 25, 31, 1]),
                                            (2, 1, 256, 48, [65]), (1, 1, 128, 4, [1, 1, 23]),
