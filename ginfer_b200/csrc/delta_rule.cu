@@ -284,13 +284,16 @@ struct DeltaStage {
 // Tokens ta .. ta + n - 1 into a stage: k | q | g rows of Dp floats (g only with a decay a channel), v columns,
 // beta, the head's decay.  Of a row, quad x (four neighbours) lies at quad x / QL + x % QL * (Dp / 4 / QL): where
 // a lane has QL quads in a row, its lanes' reads of one of them are then neighbours and meet every bank once.
-template <int Dp, bool ONE_DECAY, int QL>
+// RUN > 0: runs of RUN quads lie a quad apart (four lanes share a run, four runs a sum).
+template <int Dp, bool ONE_DECAY, int QL, int RUN = 0>
 __device__ __forceinline__ void ask_tokens(const DeltaStage& src, float* st, int ta, int n, int tid,
                                            int threads) {
   constexpr int kV = (ONE_DECAY ? 2 : 3) * Dp, kB = kV + kMaxColumnsPerBlock, kTok = kB + 4;
   const int D = src.D;
-  auto quad = [](int x) { return 4 * (QL == 1 ? x : x / QL + x % QL * (Dp / 4 / QL)); };
-  auto place = [&](int d) { return QL == 1 ? d : quad(d >> 2) + (d & 3); };
+  auto quad = [](int x) {
+    return 4 * (RUN > 0 ? x + x / (RUN > 0 ? RUN : 1) : QL == 1 ? x : x / QL + x % QL * (Dp / 4 / QL));
+  };
+  auto place = [&](int d) { return quad(d >> 2) + (d & 3); };
   if (src.vec) {                                   // (a thread keeps the same piece of every token)
     const int dq = D >> 2, nd = (ONE_DECAY ? 2 : 3) * dq, pieces = nd + (src.ncols >> 2);
     for (int e = tid; e < pieces; e += threads) {
@@ -456,20 +459,23 @@ delta_recurrence_kernel(const float* __restrict__ qn, const float* __restrict__ 
   }
 }
 
-// ---- few long portions ----------------------------------------------------------------------------
+// ---- portions of many tokens ----------------------------------------------------------------------------
 // Where requests x heads x columns do not fill the device (one long prompt, a small decode batch) the time
 // is the longest portion's chain from token to token, and behind that what shared memory gives an SM a
 // cycle: with a warp a column a token took three 16-byte reads a lane and ten shuffles for every column.
 // Here LP lanes share two neighbouring columns, DPER rows each: a read of k, q and g serves both, and most of
 // a sum's tree lies in registers.  While a token's sum goes through the lanes, the warp reads the next
 // token's operands and multiplies the state that the token before left by that token's q.
-// The sums over the rows are one binary tree over LP * DPER products in the rows' order (a lane's rows, then
-// lanes 1, 2, 4, 8 apart), as they were with 4 rows a lane: the same bits for every LP and DPER.
+// The orders of the sums over the rows are older than this kernel, and a router behind the layer makes close
+// calls, so they stay.  Where the triples are few: one binary tree over LP * DPER products in the rows' order
+// (a lane's rows, then lanes 1, 2, 4, 8 apart).  Where they are many (CHAIN): four runs of D / 4 rows; of a
+// run four chains of multiply-adds, over every fourth row, a lane each; chains, then runs, added in pairs.
 // A block is up to four groups of 128 threads that share nothing but the SM, each with a request of its own,
 // long and short ones together: blocks of one request each are placed two and more to an SM while others are
 // empty (1,201 tokens beside three single ones: 423 us; alone 298).
 // On a B200, prompts of 150, 300, 600 and 1,201 tokens, 16 heads of 128 x 128: 420 us a layer (a warp a column:
-// 740); one of 1,201 tokens 288 (446).
+// 740); one of 1,201 tokens 288 (446); eight of 200
+// 202 (four lanes a column: 680), seven of 1 to 900 375 (1,620).
 constexpr int kTreeThreads = 128, kTreeChunk = 8, kTreeGroups = 4;
 
 template <int N> __device__ __forceinline__ float tree_sum(const float* p) {
@@ -477,19 +483,19 @@ template <int N> __device__ __forceinline__ float tree_sum(const float* p) {
   else return tree_sum<N / 2>(p) + tree_sum<N / 2>(p + N / 2);
 }
 
-template <int DPER, int LP, bool ONE_DECAY>
+template <int DPER, int LP, bool ONE_DECAY, bool CHAIN>
 __global__ void __launch_bounds__(kTreeThreads * kTreeGroups, 1)
 delta_tree_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
                   const float* __restrict__ v, const float* __restrict__ g,
                   const float* __restrict__ beta, float* __restrict__ state,
                   const int* __restrict__ cu_seqlens, const int* __restrict__ slot_ids,
                   DeltaDims dm, int B, int by_length, int whole, float* __restrict__ o) {
-  constexpr int Dp = LP * DPER, CHUNK = kTreeChunk, COLS = 2;
+  constexpr int D4 = LP * DPER, Dp = D4 + (CHAIN ? 16 : 0), CHUNK = kTreeChunk, COLS = 2;
   constexpr int kV = (ONE_DECAY ? 2 : 3) * Dp;                 // where a token's v columns start
   constexpr int kB = kV + kMaxColumnsPerBlock;                 // beta (and the head's decay)
   constexpr int kTok = kB + 4;                                 // floats a token in a stage
   constexpr int cols = kTreeThreads / LP * COLS;
-  static_assert(cols <= kMaxColumnsPerBlock && DPER % 4 == 0 && CHUNK * COLS >= LP);
+  static_assert(cols <= kMaxColumnsPerBlock && DPER % 4 == 0 && CHUNK * COLS >= LP && (!CHAIN || LP == 16));
   extern __shared__ __align__(16) float stages[];              // a group: [kStages][CHUNK][kTok]
   __shared__ int request[kTreeGroups];
   const int tid = threadIdx.x % kTreeThreads, group = threadIdx.x / kTreeThreads;
@@ -500,7 +506,7 @@ delta_tree_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
   const int col0 = blockIdx.y * cols, col = col0 + lc;
   pdl_trigger();
   const int D = dm.D, Vd = dm.Vd;
-  if (D != Dp) {                                               // the rows that are not there are zero
+  if (D != D4) {                                               // the rows that are not there are zero
     for (int i = tid; i < kStages * CHUNK * kTok; i += kTreeThreads) stage[i] = 0.f;
     group_sync();
   }
@@ -521,7 +527,8 @@ delta_tree_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
     group_sync();
     b = request[group];
   }
-  const int row0 = part * DPER;
+  // the lane's i-th row
+  auto row = [&](int i) { return CHAIN ? part / 4 * (4 * DPER) + 4 * i + part % 4 : part * DPER + i; };
   const int kvh = h / (dm.H / dm.G);
   const int t0 = cu_seqlens[b], t1 = cu_seqlens[b + 1];
   const size_t GD = (size_t)dm.G * D, HD = (size_t)dm.H * D, HV = (size_t)dm.H * Vd;
@@ -531,7 +538,7 @@ delta_tree_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
                        (D & 3) == 0 && (Vd & 3) == 0 && (ncols & 3) == 0};
   auto ask = [&](int chunk) {                      // the chunk's tokens into stage chunk % kStages
     const int ta = t0 + chunk * CHUNK;
-    ask_tokens<Dp, ONE_DECAY, DPER / 4>(src, stage + (size_t)(chunk % kStages) * CHUNK * kTok, ta,
+    ask_tokens<Dp, ONE_DECAY, DPER / 4, CHAIN ? DPER : 0>(src, stage + (size_t)(chunk % kStages) * CHUNK * kTok, ta,
                                         min(CHUNK, t1 - ta), tid, kTreeThreads);
     copy_async_commit();
   };
@@ -546,8 +553,8 @@ delta_tree_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
 #pragma unroll
   for (int i = 0; i < DPER; ++i) {
     S[i][0] = S[i][1] = 0.f;
-    if (row0 + i < D) {
-      const float* at = Sg + (size_t)(row0 + i) * Vd;
+    if (row(i) < D) {
+      const float* at = Sg + (size_t)row(i) * Vd;
       if (whole) {
         if (col < Vd) {
           const float2 two = *reinterpret_cast<const float2*>(at);
@@ -570,6 +577,11 @@ delta_tree_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
     float outp[CHUNK * COLS];                                  // summed over the lanes behind the chunk
     float k[DPER], gd[DPER], q[DPER], vb[COLS + 1], before[DPER][COLS];
     auto quads = [&](const float* from, float (&to)[DPER]) {
+      if constexpr (CHAIN) {
+#pragma unroll
+        for (int i = 0; i < DPER; ++i) to[i] = from[part / 4 * (4 * DPER + 4) + part % 4 + 4 * i];
+        return;
+      }
 #pragma unroll
       for (int i = 0; i < DPER; i += 4) {
         const float4 x = *reinterpret_cast<const float4*>(from + (i / 4 * LP + part) * 4);
@@ -588,8 +600,8 @@ delta_tree_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
       for (int c = 0; c < COLS; ++c) {
         float p[DPER];
 #pragma unroll
-        for (int i = 0; i < DPER; ++i) p[i] = fmaf(before[i][c], q[i], 0.f);
-        outp[tt * COLS + c] = tree_sum<DPER>(p);
+        for (int i = 0; i < DPER; ++i) p[i] = fmaf(before[i][c], q[i], CHAIN && i ? p[i - (i > 0)] : 0.f);
+        outp[tt * COLS + c] = CHAIN ? p[DPER - 1] : tree_sum<DPER>(p);
       }
     };
     auto token = [&](int tt, bool more) {
@@ -602,9 +614,9 @@ delta_tree_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
 #pragma unroll
         for (int i = 0; i < DPER; ++i) {
           S[i][c] *= gd[ONE_DECAY ? 0 : i];
-          p[i] = fmaf(S[i][c], kc[i], 0.f);
+          p[i] = fmaf(S[i][c], kc[i], CHAIN && i ? p[i - (i > 0)] : 0.f);
         }
-        dot[c] = tree_sum<DPER>(p);
+        dot[c] = CHAIN ? p[DPER - 1] : tree_sum<DPER>(p);
       }
       const float vc[COLS] = {vb[0], vb[1]}, bc = vb[2];
 #pragma unroll
@@ -663,8 +675,8 @@ delta_tree_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
   }
 #pragma unroll
   for (int i = 0; i < DPER; ++i)
-    if (row0 + i < D) {
-      float* at = Sg + (size_t)(row0 + i) * Vd;
+    if (row(i) < D) {
+      float* at = Sg + (size_t)row(i) * Vd;
       if (whole) {
         if (col < Vd) *reinterpret_cast<float2*>(at) = make_float2(S[i][0], S[i][1]);
       } else {
@@ -1268,16 +1280,19 @@ GF_EXPORT int gf_delta_recurrence(const float* qn, const float* kn, const float*
   }
   // few (request, head, column) triples: more lanes a column than four (see the kernels)
   const bool wide = (long long)B * H * ((Vd + 31) / 32) < 2 * 148;
-  if (wide && D <= 128) {
+  // (many requests of a token each are their states' bytes, which four lanes a column read in longer runs:
+  // 16 requests of 16 heads of 128 x 128 19 us against 29)
+  if (D <= 128 && (wide || (D > 32 && max_q_len != 1))) {
     const int whole = Vd % 2 == 0 && state_stride % 2 == 0 && ((uintptr_t)state & 7) == 0;
-#define GF_TREE(DPER, LP, ONE)                                                                     \
+#define GF_TREE(DPER, LP, ONE, CHAIN)                                                                    \
   {                                                                                                \
     constexpr int cols = kTreeThreads / LP * 2;                                                    \
     constexpr size_t smem = (size_t)kStages * kTreeChunk *                                         \
-                            ((ONE ? 2 : 3) * LP * DPER + kMaxColumnsPerBlock + 4) * sizeof(float); \
+                            ((ONE ? 2 : 3) * (LP * DPER + (CHAIN ? 16 : 0)) + kMaxColumnsPerBlock + 4) * \
+                            sizeof(float);                                                         \
     const int ny = (Vd + cols - 1) / cols;                                                         \
     if (max_q_len == 1)                                                                            \
-      return launch_kernel(delta_tree_kernel<DPER, LP, ONE>, dim3(B * H, ny), dim3(kTreeThreads),  \
+      return launch_kernel(delta_tree_kernel<DPER, LP, ONE, CHAIN>, dim3(B * H, ny), dim3(kTreeThreads),  \
                            smem, st, qn, kn, v, g, beta, state, cu_seqlens, slot_ids, dm, B, 0,    \
                            whole, o);                                                              \
     /* the fewest requests a block with which every block has an SM of its own */                  \
@@ -1287,22 +1302,26 @@ GF_EXPORT int gf_delta_recurrence(const float* qn, const float* kn, const float*
     const size_t alone = 120 * 1024, all = smem * groups;                                          \
     static OncePerDevice attrs;                                                                    \
     if (int rc = attrs.run([&] {                                                                   \
-          return cudaFuncSetAttribute(delta_tree_kernel<DPER, LP, ONE>,                            \
+          return cudaFuncSetAttribute(delta_tree_kernel<DPER, LP, ONE, CHAIN>,                            \
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);    \
         }))                                                                                        \
       return rc;                                                                                   \
-    return launch_kernel_behind(delta_tree_kernel<DPER, LP, ONE>, dim3(nz * H, ny),                \
+    return launch_kernel_behind(delta_tree_kernel<DPER, LP, ONE, CHAIN>, dim3(nz * H, ny),                \
                                 dim3(kTreeThreads * groups),                                       \
                                 (long long)H * ny * nz <= 148 && all < alone ? alone : all, st,    \
                                 qn, kn, v, g, beta, state, cu_seqlens, slot_ids, dm, B, B > 1,     \
                                 whole, o);                                                         \
   }
     if (D <= 64) {
-      if (one_decay) GF_TREE(8, 8, true)
-      GF_TREE(8, 8, false)
+      if (one_decay && wide) GF_TREE(8, 8, true, false)
+      if (one_decay) GF_TREE(4, 16, true, true)
+      if (wide) GF_TREE(8, 8, false, false)
+      GF_TREE(4, 16, false, true)
     }
-    if (one_decay) GF_TREE(8, 16, true)
-    GF_TREE(8, 16, false)
+    if (one_decay && wide) GF_TREE(8, 16, true, false)
+    if (one_decay) GF_TREE(8, 16, true, true)
+    if (wide) GF_TREE(8, 16, false, false)
+    GF_TREE(8, 16, false, true)
 #undef GF_TREE
   }
   const int lp = wide ? 32 : 4;

@@ -618,6 +618,49 @@ def test_delta_rule_of_several_portions_is_that_of_each(H, G, D, Vd, lens, one):
                        state0[[i for i in range(B + 1) if i not in slots.tolist()]])
 
 
+@pytest.mark.parametrize("H,G,D,Vd,lens,one", [
+    (16, 16, 128, 128, [7, 30, 8, 1, 16, 9], 0), (8, 4, 64, 62, [9, 2, 17, 8] * 5, 0), (8, 8, 36, 64, [3, 25] * 10, 0),
+    (16, 16, 100, 128, [12, 1, 15, 8, 7], 1), (10, 10, 64, 31, [8, 4] * 15, 1)])
+def test_delta_rule_of_many_portions(H, G, D, Vd, lens, one):
+    """Where the requests' columns fill the device, portions of many tokens and single tokens run on different
+    kernels with one order of the sums: a token a step gives the same bits, and the recurrence in 64 bits is
+    within the rounding of D terms a sum over the tokens so far (decays below one)."""
+    from types import SimpleNamespace
+    from ginfer_b200.ops import delta
+    g0 = torch.Generator().manual_seed(D + Vd)
+    B, T = len(lens), sum(lens)
+    assert B * H * -(-Vd // 32) >= 2 * 148
+    q, k = (torch.nn.functional.normalize(torch.randn(T, G, D, generator=g0), dim=-1) for _ in "qk")
+    v, beta = torch.randn(T, H, Vd, generator=g0), torch.rand(T, H, generator=g0)
+    g = torch.rand(*((T, H) if one else (T, H, D)), generator=g0)
+    state0 = torch.randn(B, H * D * Vd, generator=g0)
+    cu = torch.tensor([0] + lens).cumsum(0)
+
+    def run(rows, own, state, longest):
+        ctx = SimpleNamespace(num_seqs=B, slot_ids=torch.arange(B).int().cuda(), max_q_len=longest,
+                              cu_seqlens_q=torch.tensor([0] + own).cumsum(0).int().cuda())
+        return delta.recurrence(*(t[rows].cuda() for t in (q, k, v, g, beta)), state, ctx).cpu()
+    state = state0.clone().cuda()
+    o = run(torch.arange(T), lens, state, max(lens))
+    if not one:                                    # (single tokens with a decay a head: a kernel of their own)
+        n = min(lens)
+        alone = state0.clone().cuda()
+        for t in range(n):
+            rows = cu[:-1] + t
+            assert torch.equal(run(rows, [1] * B, alone, 1), o[rows])
+    kv = torch.arange(H) // (H // G)
+    for b in range(B):
+        S = state0[b].double().view(H, D, Vd).clone()
+        for t in range(int(cu[b]), int(cu[b + 1])):
+            S = (g[t].double()[:, None, None] if one else g[t].double()[:, :, None]) * S
+            u = beta[t].double()[:, None] * (v[t].double() - torch.einsum("hdv,hd->hv", S, k[t].double()[kv]))
+            S = S + k[t].double()[kv][:, :, None] * u[:, None, :]
+            want = torch.einsum("hdv,hd->hv", S, q[t].double()[kv])
+            assert (o[t].double() - want).abs().max() <= 2.0 ** -24 * D * 8 * S.abs().max()
+        got = state[b].cpu().double().view(H, D, Vd)
+        assert (got - S).abs().max() <= 2.0 ** -24 * D * 8 * S.abs().max()
+
+
 @pytest.mark.parametrize("H,G,D,Vd,lens", [(2, 1, 12, 20, [16, 1, 7]), (4, 2, 64, 64, [40, 8, 9, 3]),
                                            (2, 2, 128, 128, [33, 17]), (3, 3, 100, 36, [24, 25, 31, 1]),
                                            (2, 1, 256, 48, [65]), (1, 1, 128, 4, [1, 1, 23]),
