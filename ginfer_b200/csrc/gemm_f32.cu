@@ -18,14 +18,19 @@
 //                 the same or not) is used twice.  cp.async in a ring of its own, three stages deep
 //                 where every SM has five such warps, six where it has fewer.
 //   tile_kernel   more rows: bound by the FMA pipes and the shared-memory reads alike (8 x 8 outputs a
-//                 thread: 64 cycles of either for a warp's step of four k).  Block tiles of 32, 64 or
-//                 128 rows by 128 columns, a segment of K, a four-stage ring.
+//                 thread: 64 cycles of either for a warp's step of four k), and with two warps a scheduler,
+//                 as many as the accumulators allow, by what either waits for the other.  So the next four
+//                 k of A and the next column of W are read ahead, stages are 32 k long (half the barriers),
+//                 and a short last tile multiplies the rows that are there only.  Block tiles of 32 or 64
+//                 rows by 128 columns, a segment of K (of 128 rows, one block an SM: 128 rows of 17,920 x
+//                 1,536 take 231 us, in two tiles 180).
 // Measured on a B200 (floor: W's bytes at 6.54 TB/s, or FMAs at 74 TFLOP/s), 3 rows: 17,920 x
-// 1,536 in 30 us (floor 17), 1,536 x 8,960 in 23 (8.4), 151,936 x 1,536 in 155 (143); 164 rows: 17,920 x
-// 1,536 in 285 us (122), 1,536 x 8,960 in 200 (61).  One kernel of 64 x 64 tiles for all rows, which
-// these two replace, took about 580 us a product at 3 rows (28-layer decode step 69.2 -> 2.65 ms with
-// the attention's part) and at 164 alike (that step 73.0 -> 18.7 ms).
+// 1,536 in 30 us (floor 17), 1,536 x 8,960 in 23 (8.4), 151,936 x 1,536 in 155 (143); 164 rows, against
+// stages of 16 k read as they are multiplied in tiles of 64 whole rows: 17,920 x 1,536 in 233 us (290; floor
+// 122), 1,536 x 8,960 in 157 (202; 61), 2,048 x 1,536 in 41 (53); 1,000 rows of the last 174 (240).
 #include <cooperative_groups.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -170,10 +175,15 @@ gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W,
 }
 
 // ---------------------------------------------------------------------------------- more rows
-constexpr int BN = 128, BK = 16, BP = BK + 4, TILE_STAGES = 4, OP = BN + 16;
+constexpr int BN = 128, OP = BN + 16;
+// k of a stage and stages: long stages where a block has enough warps to fill them with 16-byte copies
+template <int BM, int VEC> struct TileRing {
+  static constexpr int BK = BM >= 64 && VEC == 4 ? 32 : 16, BP = BK + 4, STAGES = BK == 32 ? 3 : 4;
+};
 
-template <int BM> constexpr size_t tile_shared() {
-  const size_t ring = (size_t)TILE_STAGES * (BM + BN) * BP, out = (size_t)BM * OP;
+template <int BM, int VEC> constexpr size_t tile_shared() {
+  using R = TileRing<BM, VEC>;
+  const size_t ring = (size_t)R::STAGES * (BM + BN) * R::BP, out = (size_t)BM * OP;
   return (ring > out ? ring : out) * sizeof(float);
 }
 
@@ -184,6 +194,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W,
                      int lda, int ldc, int seg, int ranks) {
   extern __shared__ __align__(16) float ring[];           // TILE_STAGES x (BM + BN) rows of BP
   constexpr int THREADS = BM * 2, TY = BM / 8;
+  constexpr int BK = TileRing<BM, VEC>::BK, BP = TileRing<BM, VEC>::BP, TILE_STAGES = TileRing<BM, VEC>::STAGES;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int rank = blockIdx.x % ranks, n0 = blockIdx.x / ranks * BN, m0 = blockIdx.y * BM;
   const int kbase = rank * seg;
@@ -219,28 +230,46 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W,
     for (int j = 0; j < 8; ++j) acc[i][j] = 0;
 #pragma unroll
   for (int s = 0; s < TILE_STAGES - 1; ++s) fetch(s);
-  for (int step = 0; step < steps; ++step) {
-    copy_wait<TILE_STAGES - 2>();
-    __syncthreads();                                      // this step is there, the last one is read
-    fetch(step + TILE_STAGES - 1);
-    const float* as = ring + (size_t)(step % TILE_STAGES) * (BM + BN) * BP;
-    const float* ws = as + BM * BP;
+  // NI: rows a thread has at most (the last tile of rows may be short).  The next four k of A, and the next
+  // column of W, are read while the ones at hand are multiplied.
+  auto products = [&](auto rows_of) {
+    constexpr int NI = decltype(rows_of)::value;
+    for (int step = 0; step < steps; ++step) {
+      copy_wait<TILE_STAGES - 2>();
+      __syncthreads();                                    // this step is there, the last one is read
+      fetch(step + TILE_STAGES - 1);
+      const float* as = ring + (size_t)(step % TILE_STAGES) * (BM + BN) * BP + ty * BP;
+      const float* ws = ring + (size_t)(step % TILE_STAGES) * (BM + BN) * BP + (BM + tx) * BP;
+      ulonglong2 a[2][NI], w[2];
 #pragma unroll
-    for (int kk = 0; kk < BK; kk += 4) {
-      ulonglong2 a[8];
+      for (int i = 0; i < NI; ++i) a[0][i] = *reinterpret_cast<const ulonglong2*>(as + TY * i * BP);
+      w[0] = *reinterpret_cast<const ulonglong2*>(ws);
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        a[i] = *reinterpret_cast<const ulonglong2*>(as + (ty + TY * i) * BP + kk);
+      for (int kk = 0; kk < BK; kk += 4) {
+        const int now = kk / 4 & 1;
+        if (kk + 4 < BK) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(ws + (tx + 16 * j) * BP + kk);
+          for (int i = 0; i < NI; ++i)
+            a[now ^ 1][i] = *reinterpret_cast<const ulonglong2*>(as + TY * i * BP + kk + 4);
+        }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) fma2(acc[i][j], a[i].x, w.x);
+        for (int j = 0; j < 8; ++j) {
+          if (j < 7) w[(j & 1) ^ 1] = *reinterpret_cast<const ulonglong2*>(ws + 16 * (j + 1) * BP + kk);
+          else if (kk + 4 < BK) w[(j & 1) ^ 1] = *reinterpret_cast<const ulonglong2*>(ws + kk + 4);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) fma2(acc[i][j], a[i].y, w.y);
+          for (int i = 0; i < NI; ++i) fma2(acc[i][j], a[now][i].x, w[j & 1].x);
+#pragma unroll
+          for (int i = 0; i < NI; ++i) fma2(acc[i][j], a[now][i].y, w[j & 1].y);
+        }
       }
     }
-  }
+  };
+  const int most = min(8, (M - m0 + TY - 1) / TY);
+  if (most > 6) products(std::integral_constant<int, 8>{});
+  else if (most == 6) products(std::integral_constant<int, 6>{});
+  else if (most == 5) products(std::integral_constant<int, 5>{});
+  else if (most > 2) products(std::integral_constant<int, 4>{});
+  else products(std::integral_constant<int, 2>{});
   copy_wait<0>();
   __syncthreads();                                        // the ring becomes the segment's sums
 #pragma unroll
@@ -295,7 +324,7 @@ template <int MT, int VEC> int start_rows(const F32Args& a) {
 template <int BM, int VEC> int start_tile(const F32Args& a) {
   static OncePerDevice once;
   return start(gemm_f32_tile_kernel<BM, VEC>, once, a.segments, (a.N + BN - 1) / BN, (a.M + BM - 1) / BM,
-               BM * 2, tile_shared<BM>(), a);
+               BM * 2, tile_shared<BM, VEC>(), a);
 }
 
 template <int VEC> int start_by_rows(const F32Args& a) {
@@ -304,11 +333,7 @@ template <int VEC> int start_by_rows(const F32Args& a) {
   if (a.M <= 4) return start_rows<4, VEC>(a);
   if (a.M <= 8) return start_rows<8, VEC>(a);
   if (a.M <= 16) return start_rows<16, VEC>(a);
-  // the largest tile that computes at most an eighth more rows (with those that are not there) than
-  // the next smaller one
-  const int p32 = (a.M + 31) / 32 * 32, p64 = (a.M + 63) / 64 * 64, p128 = (a.M + 127) / 128 * 128;
-  if (p128 * 8 <= p64 * 9) return start_tile<128, VEC>(a);
-  return p64 * 8 <= p32 * 9 ? start_tile<64, VEC>(a) : start_tile<32, VEC>(a);
+  return a.M <= 32 ? start_tile<32, VEC>(a) : start_tile<64, VEC>(a);
 }
 
 }  // namespace gf

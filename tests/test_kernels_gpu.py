@@ -151,6 +151,20 @@ def test_gemm_f32_at_the_edges_of_its_kernels(M, N, K, lda):
         assert torch.equal(gemm_f32(x[m:m + 1], w, b), got[m:m + 1])
 
 
+@pytest.mark.parametrize("M", [18, 25, 40, 41, 48, 49, 57, 72, 81, 97, 105, 113, 121, 164])
+@pytest.mark.parametrize("N,K", [(130, 100), (1536, 264), (257, 77)])
+def test_gemm_f32_multiplies_the_rows_that_are_there(M, N, K):
+    """Last tiles with every number of rows a thread, chunks of K that end inside a stage: each row's sums as
+    if it were alone."""
+    from ginfer_b200.ops.linear import gemm_f32
+    g = torch.Generator(device=DEV).manual_seed(M * 31 + N)
+    x, w = torch.randn(M, K, device=DEV, generator=g), torch.randn(N, K, device=DEV, generator=g)
+    got = gemm_f32(x, w)
+    assert torch.equal(torch.cat([gemm_f32(x[m:m + 1], w) for m in range(M)]), got)
+    bound = (K / 4 + 26) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())
+    assert ((got.double() - x.double() @ w.double().t()).abs() <= bound).all()
+
+
 @pytest.mark.parametrize("M", [2, 20])
 def test_gemm_f32_of_more_than_two_million_columns(M):
     """More tiles of columns than a grid's shorter sides hold."""
