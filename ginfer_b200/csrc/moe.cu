@@ -25,6 +25,8 @@
 //                       not depend on the batch.
 //   moe_combine_kernel  out[t] = sum over the token's choices, in the order chosen, of weight *
 //                       the pair's row.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace gf {
@@ -655,14 +657,20 @@ moe_stream_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfloa
 
 // ---- the same for a handful of pairs on the FMA pipes ----------------------------------------------
 // For layers that stay off moe_stream_kernel (their routers' close calls ask for sums in one order).  The
-// work is the experts' weight bytes, and a tile of 64 rows that walks its whole reduction alone keeps too
-// few of them under way (4 pairs, 35 MB: 45 us; here 29.5, streamed 26.5; 20 pairs 97.5 and 53.5).  A
-// tile is up to 8 rows of one expert, kept in shared memory; a block takes 16, 32 or 64 weight rows of
-// that expert (the fewer pairs, the fewer rows, so that enough blocks keep loads under way), a warp two
-// neighbouring rows at a time (a gate and its up value in the gated form), streamed once with 16-byte
-// loads, each lane a strided share of the reduction, a warp sum at the end.  The order of the sums
-// depends on K alone, so a pair's result does not depend on the batch.
-constexpr int kFewRows = 8, kFewWarps = 8, kFewChunkMax = 64;
+// work is the experts' weight bytes.  A tile is up to 8 rows of one expert, kept in shared memory; the (tile,
+// two neighbouring weight rows) items of the step, one list, are cut into one equal run a block, two blocks
+// an SM, and of a block's run every warp takes every eighth item (a gate and its up value in the gated form).
+// A warp reads its items' weights once, with 16-byte loads, in batches of 1,024 k of both rows, each lane a
+// strided share of the reduction; while one batch is multiplied the next one, of the same item or of the next,
+// is under way, so that the stream does not stop at an item's end.  A warp sum ends an item.  The order of the
+// sums depends on K alone, so a pair's result does not depend on the batch.
+// The loops over a tile's rows are most of the instructions, so their number is the compiler's; tiles of
+// three rows and more hold each batch's code once (kernels alternate, and code that is not there is waited for).
+// On a B200, weights from HBM, both products, us (floor in brackets), against a grid of (tile, 16 to 64 weight
+// rows) blocks whose warps waited for each batch and branched for each row: 32 experts of 2048 x 1408, 4 choices, 1
+// token 21.6 / 31.8 (10.7), 2 tokens 33.6 / 50.2 (18.8), 4 tokens 60 / 75 (34.9), 5 tokens 66 / 94 (40.2); 16 of 1024 x 704,
+// 2 choices, 4 tokens 16.2 / 19.0, 8 tokens 27.3 / 26.7, 10 tokens 33.6 / 31.1.
+constexpr int kFewRows = 8, kFewWarps = 8, kFewBlocks = 2, kFewSteps = 4;
 constexpr int kFewMaxShared = 64 * 1024;                     // K up to 4,096
 
 __device__ __forceinline__ void bf16x8_to_f32(const uint4& raw, float (&v)[8]) {
@@ -674,59 +682,72 @@ __device__ __forceinline__ void bf16x8_to_f32(const uint4& raw, float (&v)[8]) {
   }
 }
 
+// Weights are read once: past L1, and without a claim on it.
+__device__ __forceinline__ uint4 load_once(const __nv_bfloat16* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p));
+  return v;
+}
+
 template <int MODE>
-__global__ void __launch_bounds__(kFewWarps * 32)
+__global__ void __launch_bounds__(kFewWarps * 32, kFewBlocks)
 moe_gemv_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfloat16* __restrict__ w,
                 int N, int K, const int* __restrict__ offsets, const int* __restrict__ pair_of_pos,
                 int top, const int* __restrict__ tile_expert, const int* __restrict__ tile_row0,
                 const int* __restrict__ num_tiles, void* __restrict__ out_, float limit,
-                float alpha, float up_shift, int chunk) {
+                float alpha, float up_shift) {
   extern __shared__ __align__(16) __nv_bfloat16 xrows[];           // [kFewRows][K]
-  pdl_trigger();
   pdl_wait();
-  if ((int)blockIdx.x >= fresh_index(num_tiles)) return;
-  const int e = fresh_index(tile_expert + blockIdx.x), row0 = fresh_index(tile_row0 + blockIdx.x);
-  const int rows = min(kFewRows, fresh_index(offsets + e + 1) - row0);
-  const int k8 = K >> 3;
-  for (int i = threadIdx.x; i < rows * k8; i += blockDim.x) {
-    const int r = i / k8, c = (i - r * k8) * 8;
-    const int src = MODE != 0 ? fresh_index(pair_of_pos + row0 + r) / top : row0 + r;
-    *reinterpret_cast<uint4*>(xrows + (size_t)r * K + c) =
-        __ldcg(reinterpret_cast<const uint4*>(a + (size_t)src * lda + c));
-  }
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const __nv_bfloat16* we = w + (size_t)e * N * K;
-  for (int i = warp; i < chunk / 2; i += kFewWarps) {
-    const int n = blockIdx.y * chunk + 2 * i;
-    if (n >= N) break;                                             // N is even
-    const __nv_bfloat16 *w0 = we + (size_t)n * K, *w1 = w0 + K;
-    float acc0[kFewRows], acc1[kFewRows];
+  pdl_trigger();
+  const int items = N >> 1;                                        // of a tile; N is even
+  const long long all = (long long)fresh_index(num_tiles) * items;
+  const int i0 = (int)(all * blockIdx.x / gridDim.x), i1 = (int)(all * (blockIdx.x + 1) / gridDim.x);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, k8 = K >> 3;
+  for (int at = i0; at < i1;) {
+    const int tile = at / items, p0 = at - tile * items, p1 = min(items, p0 + (i1 - at));
+    const int e = fresh_index(tile_expert + tile), row0 = fresh_index(tile_row0 + tile);
+    const int rows = min(kFewRows, fresh_index(offsets + e + 1) - row0);
+    const __nv_bfloat16* we = w + (size_t)e * N * K + lane * 8;
+    int ask_item = p0 + warp, ask_k = 0;
+    auto load = [&](uint4 (&wa)[kFewSteps], uint4 (&wb)[kFewSteps]) {
+      if (ask_item >= p1) return;
+      const __nv_bfloat16* src = we + (size_t)(2 * ask_item) * K + ask_k;
 #pragma unroll
-    for (int r = 0; r < kFewRows; ++r) acc0[r] = acc1[r] = 0.f;
-    // four steps of the reduction at a time: their eight loads go out together, before any
-    // arithmetic (left to the compiler, the loads of a step waited behind the branches of the
-    // step before: 1.2 TB/s)
-    for (int c0 = lane * 8; c0 < K; c0 += 4 * 256) {
-      uint4 wa[4], wb[4];
+      for (int u = 0; u < kFewSteps; ++u)
+        if (ask_k + lane * 8 + u * 256 < K) wa[u] = load_once(src + u * 256), wb[u] = load_once(src + u * 256 + K);
+      ask_k += kFewSteps * 256;
+      if (ask_k >= K) ask_k = 0, ask_item += kFewWarps;
+    };
+    uint4 wa[kFewSteps], wb[kFewSteps], va[kFewSteps], vb[kFewSteps];
+    load(wa, wb);
+    load(va, vb);
+    for (int i = threadIdx.x; i < rows * k8; i += kFewWarps * 32) {
+      const int r = i / k8, c = (i - r * k8) * 8;
+      const int src = MODE != 0 ? fresh_index(pair_of_pos + row0 + r) / top : row0 + r;
+      *reinterpret_cast<uint4*>(xrows + (size_t)r * K + c) =
+          __ldcg(reinterpret_cast<const uint4*>(a + (size_t)src * lda + c));
+    }
+    __syncthreads();
+    // ROWS: of the tile, known to the compiler (its loops over them are most of the instructions)
+    auto run = [&](auto rows_of) {
+      constexpr int ROWS = decltype(rows_of)::value;
+      int item = p0 + warp, k = 0;
+      float acc0[ROWS], acc1[ROWS];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int c = c0 + u * 256;
-        if (c < K) {
-          wa[u] = __ldg(reinterpret_cast<const uint4*>(w0 + c));
-          wb[u] = __ldg(reinterpret_cast<const uint4*>(w1 + c));
-        }
-      }
+      for (int r = 0; r < ROWS; ++r) acc0[r] = acc1[r] = 0.f;
+      auto multiply = [&](const uint4 (&pa)[kFewSteps], const uint4 (&pb)[kFewSteps]) {
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int c = c0 + u * 256;
-        if (c >= K) break;
-        float f0[8], f1[8];
-        bf16x8_to_f32(wa[u], f0);
-        bf16x8_to_f32(wb[u], f1);
+        for (int u = 0; u < kFewSteps; ++u) {
+          const int c = k + lane * 8 + u * 256;
+          if (c >= K) break;
+          float f0[8], f1[8];
+          bf16x8_to_f32(pa[u], f0);
+          bf16x8_to_f32(pb[u], f1);
 #pragma unroll
-        for (int r = 0; r < kFewRows; ++r) {
-          if (r < rows) {
+          for (int r = 0; r < ROWS; ++r) {
+            if (ROWS > 4 && r >= rows) break;
             float x[8];
             bf16x8_to_f32(*reinterpret_cast<const uint4*>(xrows + (size_t)r * K + c), x);
 #pragma unroll
@@ -736,24 +757,60 @@ moe_gemv_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfloat1
             }
           }
         }
-      }
-    }
+      };
+      auto finish = [&]() {                                        // behind a batch: the item's end, if it is
+        k += kFewSteps * 256;
+        if (k < K) return;
+        const int n = 2 * item;
 #pragma unroll
-    for (int r = 0; r < kFewRows; ++r) {
-      if (r >= rows) break;                                        // uniform over the warp
-      const float c0 = warp_sum(acc0[r]), c1 = warp_sum(acc1[r]);
-      if (lane != 0) continue;
-      const size_t s = (size_t)(row0 + r);
-      if (MODE == 1) {
-        const float gt = to_f32(from_f32<__nv_bfloat16>(c0)), up = to_f32(from_f32<__nv_bfloat16>(c1));
-        ((__nv_bfloat16*)out_)[s * (N / 2) + n / 2] =
-            from_f32<__nv_bfloat16>(clamped_glu(gt, up, limit, alpha, up_shift));
-      } else {
-        float* out = (float*)out_ + s * N + n;
-        out[0] = c0;
-        out[1] = c1;
+        for (int o = 16; o > 0; o >>= 1)                           // (warp_sum, all rows side by side)
+#pragma unroll
+          for (int r = 0; r < ROWS; ++r) {
+            acc0[r] += __shfl_xor_sync(0xffffffffu, acc0[r], o);
+            acc1[r] += __shfl_xor_sync(0xffffffffu, acc1[r], o);
+          }
+        if (lane == 0) {
+#pragma unroll
+          for (int r = 0; r < ROWS; ++r) {
+            if (r >= rows) break;
+            const size_t s = (size_t)(row0 + r);
+            if (MODE == 1) {
+              const float gt = to_f32(from_f32<__nv_bfloat16>(acc0[r])), up = to_f32(from_f32<__nv_bfloat16>(acc1[r]));
+              ((__nv_bfloat16*)out_)[s * (N / 2) + n / 2] =
+                  from_f32<__nv_bfloat16>(clamped_glu(gt, up, limit, alpha, up_shift));
+            } else {
+              *reinterpret_cast<float2*>((float*)out_ + s * N + n) = make_float2(acc0[r], acc1[r]);
+            }
+          }
+        }
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) acc0[r] = acc1[r] = 0.f;
+        k = 0, item += kFewWarps;
+      };
+      while (item < p1) {
+        multiply(wa, wb);
+        if (ROWS > 2) {                                            // (once in the code: there is much of it)
+#pragma unroll
+          for (int u = 0; u < kFewSteps; ++u) wa[u] = va[u], wb[u] = vb[u];
+          load(va, vb);
+          finish();
+          continue;
+        }
+        load(wa, wb);
+        finish();
+        if (item >= p1) break;
+        multiply(va, vb);
+        load(va, vb);
+        finish();
       }
-    }
+    };
+    if (rows == 1) run(std::integral_constant<int, 1>{});
+    else if (rows == 2) run(std::integral_constant<int, 2>{});
+    else if (rows == 3) run(std::integral_constant<int, 3>{});
+    else if (rows == 4) run(std::integral_constant<int, 4>{});
+    else run(std::integral_constant<int, 8>{});
+    at += p1 - p0;
+    if (at < i1) __syncthreads();                                  // the rows are free for the next tile's
   }
 }
 
@@ -821,6 +878,17 @@ using namespace gf;
 using bf = __nv_bfloat16;
 
 GF_DEFINE_PDL_SWITCH
+
+// Streaming multiprocessors of the current device, asked of it once.
+static int sm_count(int* sms) {
+  static OncePerDevice once;
+  static int count[OncePerDevice::kMaxDevices];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= OncePerDevice::kMaxDevices) return -9;
+  const int rc = once.run([&] { return cudaDeviceGetAttribute(&count[dev], cudaDevAttrMultiProcessorCount, dev); });
+  *sms = count[dev];
+  return rc;
+}
 
 // Rows of a tile: of the plain kernel (tensor_cores == 0), of the tensor-core kernel (1), of the
 // weight-streaming kernel (2) or of the one with FMAs for a handful of pairs (3).
@@ -914,11 +982,9 @@ GF_EXPORT int gf_moe_gemm(const void* a, int lda, const void* w, int N, int K, c
     if (dtype != GF_BF16 || K % 8 || lda % 8 || N % 2 || (uintptr_t)a % 16 || (uintptr_t)w % 16 ||
         smem > kFewMaxShared || first == 2)
       return -3;
-    // at most min(pairs, max_tiles) tiles hold rows; about four blocks an SM should be busy
-    int chunk = kFewChunkMax;
-    const int busy = pairs > 0 && pairs < max_tiles ? pairs : max_tiles;
-    while (chunk > 2 * kFewWarps && (long long)busy * ((N + chunk - 1) / chunk) < 4 * 148) chunk /= 2;
-    const dim3 fgrid(max_tiles, (N + chunk - 1) / chunk), fblock(kFewWarps * 32);
+    int sms = 0;
+    if (int rc = sm_count(&sms)) return rc;
+    const dim3 fgrid(sms * kFewBlocks), fblock(kFewWarps * 32);
 #define GF_FEW(MODE)                                                                              \
   {                                                                                               \
     static OncePerDevice attrs;                                                                   \
@@ -929,7 +995,7 @@ GF_EXPORT int gf_moe_gemm(const void* a, int lda, const void* w, int N, int K, c
       return rc;                                                                                  \
     return launch_kernel(moe_gemv_kernel<MODE>, fgrid, fblock, smem, st, (const bf*)a, lda,       \
                          (const bf*)w, N, K, offsets, pair_of_pos, top, tile_expert, tile_row0,   \
-                         num_tiles, out, limit, alpha, up_shift, chunk);                          \
+                         num_tiles, out, limit, alpha, up_shift);                                 \
   }
     if (first) GF_FEW(1)
     GF_FEW(0)

@@ -576,6 +576,34 @@ def test_grouped_products_that_stream_the_weights(K, F, T, E, top):
         assert ((got - want).abs() <= (F + 8) * 2.0 ** -24 * size).all()
 
 
+@pytest.mark.parametrize("K,N", [(8, 2), (264, 38), (1024, 16), (1032, 34), (2056, 20), (4096, 10)])
+@pytest.mark.parametrize("counts", [(1, 2, 3, 4, 0, 5), (8, 9, 0, 1, 1, 1), (0, 0, 20, 0, 0, 0), (0, 0, 0, 0, 0, 1)])
+def test_products_of_a_handful_of_pairs(K, N, counts):
+    """Tiles of every number of rows, reductions around a batch of 1,024 and a warp's 256, fewer items than
+    warps: against 64 bits, and each pair as if it were alone."""
+    from ginfer_b200.ops import moe
+    g = torch.Generator(device=DEV).manual_seed(K + N)
+    E, P = len(counts), sum(counts)
+    idx = torch.tensor([e for e, n in enumerate(counts) for _ in range(n)])
+    idx = idx[torch.randperm(P, generator=torch.Generator().manual_seed(K))].int().cuda().view(P, 1)
+    x = torch.randn(P, K, generator=g, device=DEV).bfloat16()
+    up = (torch.randn(E, N, K, generator=g, device=DEV) * K ** -0.5).bfloat16()
+    plan = moe.Plan(idx, E, "gemv")
+    rows = moe.grouped_down(x[plan.pair_of_pos.long()].contiguous(), up, plan)[plan.pos_of_pair.long()]
+    glu = moe.grouped_glu(x, up, plan, 1e9, 1.0, 0.0)[plan.pos_of_pair.long()]
+    want = torch.einsum("pk,pnk->pn", x.double(), up[idx[:, 0].long()].double())
+    size = torch.einsum("pk,pnk->pn", x.double().abs(), up[idx[:, 0].long()].double().abs())
+    # a lane's chain of K / 32 products (rounded up to its 8 k) and five additions across the lanes
+    assert ((rows.double() - want).abs() <= (K / 32 + 16) * 2.0 ** -24 * size).all()
+    gate, lift = rows[:, 0::2].bfloat16().double(), rows[:, 1::2].bfloat16().double()
+    ref = gate / (1 + torch.exp(-gate)) * lift
+    assert ((glu.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-30).all()
+    for p in {0, P // 2, P - 1}:
+        one = moe.Plan(idx[p:p + 1].contiguous(), E, "gemv")
+        assert torch.equal(moe.grouped_down(x[p:p + 1], up, one)[0], rows[p])
+        assert torch.equal(moe.grouped_glu(x[p:p + 1], up, one, 1e9, 1.0, 0.0)[0], glu[p])
+
+
 @pytest.mark.parametrize("K,F,E,top", [(2048, 1408, 32, 4), (1024, 704, 16, 2), (256, 96, 8, 1)])
 @pytest.mark.parametrize("counts", [(1, 2, 3, 5), (24, 25, 40, 100)])
 def test_a_pairs_result_does_not_depend_on_the_batch(K, F, E, top, counts):
