@@ -434,6 +434,20 @@ def test_attention_bf16_decode_with_several_clusters_a_request(case, splits, par
     torch.testing.assert_close(out.float(), one.float(), atol=1e-2, rtol=2e-2)
 
 
+@pytest.mark.parametrize("window", [0, 70, -128])
+@pytest.mark.parametrize("splits,parts", [(8, 1), (2, 1), (8, 2), (1, 3)])
+def test_attention_bf16_decode_of_few_keys(splits, parts, window):
+    """Requests whose keys one CTA holds (it writes the result itself) beside requests with one key more, with
+    as many as all splits take, with a window and with chunks."""
+    from ginfer_b200.ops import attention_bf16, gemm_bf16
+    lens, nh, nkv, hd, P = [1, 63, 64, 65, 127, 128, 129, 130, 200, 256, 257, 1030], 6, 2, 64, 16
+    dev, want, scale = _paged_case(lens, [1] * len(lens), nh, nkv, hd, P, window, torch.bfloat16)
+    out = attention_bf16.decode(_qkv(dev, nh, nkv, hd), dev["pages"], dev["table"], dev["cu"], dev["positions"],
+                                len(lens), nh, nkv, hd, scale, window, P, splits, parts=parts)
+    gemm_bf16.check_errors()
+    torch.testing.assert_close(out.double().cpu(), want, atol=1e-2, rtol=2e-2)
+
+
 @pytest.mark.parametrize("case", DEC_CASES)
 @pytest.mark.parametrize("splits", [1, 4, 8, -3])
 @pytest.mark.parametrize("rot_frac", [1.0, 0.5])
