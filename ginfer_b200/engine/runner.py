@@ -33,10 +33,14 @@ def _align4(n: int) -> int:
 
 GRAPH_WIDTH_STEP = 64        # block-table widths of graph-replayed steps, in pages
 # Steps with prompt portions are replayed from a graph when the same shape (portion lengths, table
-# width, wanted rows) comes a second time: whole-budget portions of long prompts do.  Only steps
-# of at most this many requests and at least this many tokens, and this many graphs at most.
+# width, wanted rows) comes again: whole-budget portions of long prompts do, and prompts of a few
+# tokens.  Only steps of at most this many requests, and this many graphs at most of steps up to
+# PORTION_GRAPH_SHORT tokens and as many of longer ones.  A short step's host work is most of its time (28
+# layers, a prompt of 17 tokens on a B200: 4.4 ms of launches for 1.4 ms of kernels), but a capture
+# costs two eager steps' launches, and lengths seldom repeat as portions do: it is captured when it
+# comes a fourth time, a long one the second time.
 PORTION_GRAPH_MAX_SEQS = 4
-PORTION_GRAPH_MIN_TOKENS = 256
+PORTION_GRAPH_SHORT = 255
 PORTION_GRAPH_LIMIT = 16
 
 
@@ -195,13 +199,14 @@ class ModelRunner:
         logit_rows = np.asarray(rows, dtype=np.int64)
         width = int(-(-int(kv_lens.max()) // P))
         decode_only = int(q_lens.max()) == 1
-        graphable = decode_only or (B <= PORTION_GRAPH_MAX_SEQS and T >= PORTION_GRAPH_MIN_TOKENS)
+        graphable = decode_only or (B <= PORTION_GRAPH_MAX_SEQS and T > PORTION_GRAPH_SHORT)
         if graphable and not self.enforce_eager:
             # such steps are replayed from CUDA graphs, one per (shape, table width): widths come
             # in steps of GRAPH_WIDTH_STEP pages so that few graphs are needed.  Steps with
             # portions take the next power of two of such steps (the portions of one long prompt
             # then share a handful of graphs; nothing in such a step is chosen by the width, while
-            # a decode step splits its keys by it).
+            # a decode step splits its keys by it, and so may a short step with portions, which
+            # keeps its own width).
             steps = -(-width // GRAPH_WIDTH_STEP)
             if not decode_only:
                 steps = 1 << (steps - 1).bit_length()
@@ -375,9 +380,10 @@ class ModelRunner:
             if any(len(e.want) != 1 for e in entries):
                 return None
             return (self.graph_batch(facts["B"]), facts["width"])
-        if facts["B"] > PORTION_GRAPH_MAX_SEQS or facts["T"] < PORTION_GRAPH_MIN_TOKENS:
+        if facts["B"] > PORTION_GRAPH_MAX_SEQS:
             return None
-        key = ("portions", tuple(int(n) for n in facts["q_lens"]), facts["width"],
+        short = facts["T"] <= PORTION_GRAPH_SHORT
+        key = ("short" if short else "portions", tuple(int(n) for n in facts["q_lens"]), facts["width"],
                tuple(tuple(int(w) for w in e.want) for e in entries))
         if key in self._graphs:
             return key
@@ -385,8 +391,8 @@ class ModelRunner:
         if len(self._portion_seen) > 4096:
             self._portion_seen.clear()
         self._portion_seen[key] = seen
-        graphs = sum(1 for k in self._graphs if isinstance(k[0], str))
-        return key if seen >= 2 and graphs < PORTION_GRAPH_LIMIT else None
+        graphs = sum(1 for k in self._graphs if k[0] == key[0])
+        return key if seen >= (4 if short else 2) and graphs < PORTION_GRAPH_LIMIT else None
 
     def _capture(self, key, arrays, facts) -> _StepGraph:
         from .. import ops

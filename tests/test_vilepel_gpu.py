@@ -555,3 +555,30 @@ def test_grouped_products_of_a_handful_of_pairs_on_plain_multiply_adds(K, F, T, 
         want = torch.einsum("pf,pkf->pk", yp, down[exp].double())
         size = torch.einsum("pf,pkf->pk", yp.abs(), down[exp].double().abs())
         assert ((moe.grouped_down(y, down, plan)[place].double() - want).abs() <= (F + 8) * 2.0 ** -24 * size).all()
+
+
+@pytest.mark.parametrize("name, dtype", [("MIXED", "bfloat16"), ("OTHER", "float32")])
+def test_short_prompts_of_one_length_replay_a_graph(tmp_path_factory, name, dtype):
+    """Prompts of a few tokens, two a step, whose lengths come again: from the fourth step of a shape on it is
+    captured and replayed, with other tokens, pages and slots than it was captured with.  The rows are those of
+    an eager runner bit for bit, other lengths stay eager, and a request that goes on decoding keeps its state."""
+    from ginfer_b200.engine import StepEntry
+    cfg = getattr(tv, name)
+    d = folder(tmp_path_factory, name, cfg, dtype)
+    rng = random.Random(3)
+    runners = [make_runner(d, dtype, 512, eager=e, max_live=6) for e in (True, False)]
+    kept = [rng.randrange(cfg["vocab"]) for _ in range(40)]
+    for turn in range(8):
+        a, b = ([rng.randrange(cfg["vocab"]) for _ in range(n)] for n in (21, 9 if turn != 4 else 10))
+        tokens = kept[:30] if turn == 0 else kept[29 + turn:30 + turn]
+        steps = [[StepEntry("kept", tokens, [len(tokens) - 1])],
+                 [StepEntry(f"a{turn}", a, [0, 20]), StepEntry(f"b{turn}", b, [8])]]
+        for entries in steps:
+            eager, graph = (r.step(entries).clone() for r in runners)
+            assert torch.equal(eager, graph), (turn, len(entries))
+        for r in runners:
+            if turn % 2:                           # (the slots and pages differ from turn to turn)
+                r.end(f"a{turn}"), r.end(f"b{turn}"), r.end(f"a{turn - 1}")
+                r.end(f"b{turn - 1}")
+    short = [k for k in runners[1]._graphs if k[0] == "short"]
+    assert [k[1] for k in short] == [(21, 9)] and not runners[0]._graphs
