@@ -69,10 +69,11 @@ def token_tile(M: int) -> int:
     return 16 if M <= 16 else 32 if M <= 32 else 64 if M <= 64 else 128 if M <= 128 else 256
 
 
-def split_k_for(M: int, N: int, K: int, sms: int | None = None) -> int:
+def split_k_for(M: int, N: int, K: int, sms: int | None = None, settled: bool = False) -> int:
     """Split the K range of products whose tiles alone would leave most SMs idle: 2, 4, 8 or 12
     splits, which form a thread-block cluster and add up through distributed shared memory.
-    ``sms``: the device's SM count (asked of the current device if ``None``)."""
+    ``sms``: the device's SM count (asked of the current device if ``None``).  ``settled``: only the splits
+    of up to about a CTA an SM (a layer whose sums keep the order that they have)."""
     sms = sms or num_sms()
     tiles = -(-N // 128) * -(-M // token_tile(M))
     nkb = -(-K // 64)
@@ -83,6 +84,18 @@ def split_k_for(M: int, N: int, K: int, sms: int | None = None) -> int:
         split = 12      # a long reduction on few tiles (the down product): 144 CTAs instead of 96
     if split == 1 and M <= 64 and sms // 2 < tiles <= sms and nkb >= 16:
         split = 2       # about one tile an SM (gate/up): pairs of CTAs have more under way
+    elif M <= 64 and not settled:
+        # up to two CTAs an SM where a CTA's K range stays long: its K steps, not its bytes, bound it.  In a
+        # CUDA graph on a B200, 8 tokens, weights from HBM (us, splits as above / these): 8192 x 2048 9.7 / 8.4,
+        # 8448 x 2048 9.9 / 8.6, 3584 x 18944 28.7 / 25.5, 2048 x 8448 9.9 / 9.3.  Not gained: 11264 x 2048 in
+        # four 12.0 / 14.9 (more than two an SM), 4608 x 3584 in eight 9.7 / 12.4 (clusters of eight that find no
+        # place), 2048 x 8448 in twelve at 32 tokens 11.2 / 11.5.
+        if split == 2 and tiles * 4 <= 2 * sms and nkb // 4 >= 8:
+            split = 4
+        elif split == 4 and tiles * 8 * 5 <= 8 * sms and nkb // 8 >= 24:
+            split = 8
+        elif split == 8 and M <= 16 and tiles * 12 * 10 <= 13 * sms and nkb // 12 >= 7:
+            split = 12
     return split
 
 
@@ -146,7 +159,7 @@ def gemm(x, weight, bias_f32=None, out_dtype=torch.bfloat16, epi: int = 0, split
             and not through_workspace and scale is None and resid is None
             and stream(x, weight, bias_f32, out, epi, act_consts)):
         return out
-    sk = split_k_for(M, N, K) if split_k is None else int(split_k)
+    sk = split_k_for(M, N, K, settled=not streamed) if split_k is None else int(split_k)
     ws = None
     if sk > 1 and through_workspace:
         bn = token_tile(M)

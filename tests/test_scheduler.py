@@ -534,3 +534,13 @@ def test_the_bench_scenarios_fit_the_engines_they_ask_for():
             # pages for every request at its full length, so that nobody is preempted
             pages = sum(-(-(len(p) + q.max_tokens) // bench.PAGE) for p, q in zip(prompts, params))
             assert pages <= kwargs["num_kvcache_blocks"], (name, shape, pages)
+
+
+@pytest.mark.parametrize("M,N,K,splits,settled", [
+    (8, 8192, 2048, 4, 2), (33, 8448, 2048, 4, 2), (8, 3584, 18944, 8, 4), (16, 2048, 8448, 12, 8),
+    (17, 2048, 8448, 8, 8), (8, 11264, 2048, 2, 2), (8, 4608, 3584, 4, 4), (65, 8192, 2048, 2, 2),
+    (8, 9472, 2048, 4, 2), (8, 9600, 2048, 2, 2), (8, 8192, 1984, 2, 2)])
+def test_splits_of_up_to_two_blocks_an_sm(M, N, K, splits, settled):
+    from ginfer_b200.ops import gemm_bf16
+    assert gemm_bf16.split_k_for(M, N, K, sms=148) == splits
+    assert gemm_bf16.split_k_for(M, N, K, sms=148, settled=True) == settled
