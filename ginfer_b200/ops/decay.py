@@ -3,7 +3,7 @@ convolution and step sizes of a state-space mixer, the decays of gated linear at
 recurrence both share, and the gated norm of its output."""
 from __future__ import annotations
 
-from ctypes import c_float, c_int, c_void_p
+from ctypes import c_float, c_int, c_longlong, c_void_p
 
 import torch
 
@@ -98,10 +98,14 @@ def _chunked(q, k, v, g, state, ctx, first: int, H, G, D, Vd, k_scale, skip, nor
     if not _chunk_tokens:
         _chunk_tokens.append(int(load_library("decay_chunk").gf_decay_chunk_tokens()))
     chunks = sum(-(-n // _chunk_tokens[0]) for n in ctx.q_lens_host[first:])
-    scratch = torch.empty(chunks * H * (D * Vd + D + 1), dtype=torch.float32, device=v.device)
+    if len(_chunk_tokens) == 1:
+        words = load_library("decay_chunk").gf_decay_chunk_words
+        words.argtypes, words.restype = [c_int] * 5, c_longlong
+        _chunk_tokens.append(words)
+    scratch = torch.empty(int(_chunk_tokens[1](chunks, H, G, D, Vd)), dtype=torch.float32, device=v.device)
     f = _fn("decay_chunk", "gf_decay_chunked",
             [c_void_p, c_int] * 5 + [c_void_p, c_void_p, c_int, c_void_p, c_void_p] + [c_int] * 6 +
-            [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p], kernels=3)
+            [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p], kernels=4 if H > G else 3)
     rc = f(_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(g), g.stride(0), _p(k_scale),
            k_scale.stride(0) if k_scale is not None else 0, _p(skip), _p(state), state.stride(0),
            _p(ctx.cu_seqlens_q[first:]), _p(ctx.slot_ids[first:]), ctx.num_seqs - first, chunks, H, G, D,
@@ -132,7 +136,7 @@ def _channels_chunked(q, k, v, g, state, ctx, H, G, D, Vd, o) -> bool:
     return True
 
 
-_chunk_tokens: list = []
+_chunk_tokens: list = []               # tokens a chunk; the function that gives a step's words of scratch
 
 
 def recurrence(q, k, v, g, state: torch.Tensor, ctx, H: int, G: int, D: int, Vd: int,

@@ -1015,3 +1015,30 @@ def test_pairs_rows_are_added_up_in_the_order_chosen(T, top, N, weighted):
         row = torch.where(p[:, None] >= 0, y[p.clamp(min=0)], 0.0) * (wgt[:, k:k + 1] if weighted else 1.0)
         want, size = want + row.double(), size + row.abs()
     assert ((got.double() - want).abs() <= top * 2.0 ** -23 * size).all()
+
+
+@pytest.mark.parametrize("H,G,D,Vd,lens", [(8, 1, 128, 64, [64, 65, 200]), (6, 2, 36, 132, [130, 64]), (4, 2, 4, 4, [66]),
+                                           (64, 1, 64, 64, [127])])
+@pytest.mark.parametrize("norm", [False, True])
+def test_heads_that_share_queries_and_keys_share_their_scores(H, G, D, Vd, lens, norm):
+    """A chunk at a time with fewer key heads than heads: outputs, states and normalisers are, bit for bit,
+    those of the same queries and keys written out for every head."""
+    from types import SimpleNamespace
+    from ginfer_b200.ops import decay
+    g0 = torch.Generator(device=DEV).manual_seed(D + Vd)
+    B, T = len(lens), sum(lens)
+    q, k, v = (torch.randn(T, n, device=DEV, generator=g0) / D ** 0.5 for n in (G * D, G * D, H * Vd))
+    g, c = torch.rand(T, H, device=DEV, generator=g0) ** 0.1, torch.rand(T, H, device=DEV, generator=g0)
+    skip = torch.randn(H, device=DEV, generator=g0)
+    state0 = torch.randn(B, (H * D * Vd + H * D + 3) // 4 * 4, device=DEV, generator=g0)
+    ctx = SimpleNamespace(num_seqs=B, slot_ids=torch.arange(B).int().cuda(), max_q_len=max(lens), q_lens_host=lens,
+                          cu_seqlens_q=torch.tensor([0] + lens).cumsum(0).int().cuda())
+    got = []
+    for heads in (G, H):
+        state = state0.clone()
+        qh, kh = (t.view(T, G, D).repeat_interleave(heads // G, 1).reshape(T, heads * D) for t in (q, k))
+        o = decay.recurrence(qh, kh, v, g, state, ctx, H, heads, D, Vd, k_scale=c, skip=skip,
+                             normaliser=H * D * Vd if norm else None)
+        got.append((o if norm else (o,)) + (state,))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
