@@ -338,6 +338,14 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+constexpr int kRowTokens = 4;       // tokens that share a block of latent_attention_rows_kernel
+// Whether token t is one of four that share a block.
+__device__ __forceinline__ bool in_rows(int t, int num_tokens, const int* seq_of_token, const int* positions,
+                                        int window) {
+  const int base = t / kRowTokens * kRowTokens, end = base + kRowTokens - 1;
+  return end < num_tokens && seq_of_token[base] == seq_of_token[end] && (window <= 0 || positions[end] < window);
+}
+
 template <int NT>
 __global__ void __launch_bounds__(kMmaWarps * 32)
 latent_attention_mma_kernel(const float* __restrict__ q_lat, const float* __restrict__ q_rot,
@@ -347,7 +355,7 @@ latent_attention_mma_kernel(const float* __restrict__ q_lat, const float* __rest
                             const int* __restrict__ positions, bf16* __restrict__ out,
                             int num_tokens, int H, int C, int R, int page_size, int window,
                             float scale, int nsplit, float* __restrict__ part_o,
-                            float* __restrict__ part_ml) {
+                            float* __restrict__ part_ml, int left_out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int Dk = C + R, ld = Dk + 8;
   constexpr int pld = kMmaTile + 8;
@@ -360,6 +368,7 @@ latent_attention_mma_kernel(const float* __restrict__ q_lat, const float* __rest
   const int t = blockIdx.x, h0 = blockIdx.y * 16;
   pdl_trigger();
   pdl_wait();
+  if (left_out && in_rows(t, num_tokens, seq_of_token, positions, window)) return;
   const int b = seq_of_token[t];
   const int p = positions[t];
   const int lo = window > 0 ? max(0, p - window + 1) : 0;
@@ -557,6 +566,255 @@ latent_attention_mma_kernel(const float* __restrict__ q_lat, const float* __rest
   }
 }
 
+// ---- four tokens a block (prompt portions) ---------------------------------------------------------
+// A block a token reads the token's keys for that token alone, and between its four barriers a tile most warps
+// wait.  Neighbouring tokens of a request whose window reaches back to its first key see the same tiles, so a block
+// takes four of them: 64 rows (16 heads each) share every tile.  A warp belongs to one token and a quarter: 16
+// of the tile's keys for the scores and the softmax, a quarter of the latent channels for the output; the
+// barriers inside a tile are the four warps' of a token.  Half tiles of 32 keys go through three places, so that
+// half of the next tile is under way while a tile is multiplied.
+// Every sum is the kernel's above in its order (tiles of 64 keys from the first one, two halves of the key
+// channels with two accumulators each, eight keys' sums a thread, channels over the tile's keys); keys behind
+// a token count as zeros for it, as they do there: the same bits.  Groups of four that reach over a request's
+// end, or tokens whose window starts behind key 0 (their tiles start where no other token's do), are left to that
+// kernel, which leaves out the others: both are launched.
+// 2,251 tokens of four prompts (16 heads, 512 + 64 channels, a window of 1,024) on a B200: 417 us a layer (a block a
+// token 624; both with the table's copy), 2,000 tokens of one 665 (801).
+// A block's tile takes longer than a block a token's, so a step needs enough blocks: 182, 17 tiles the longest,
+// 225 us against 213; 250 blocks 124 against 142.
+constexpr int kRowMinBlocks = 192;
+constexpr int kRowHalf = 32, kRowSlots = 3, kRowPld = kMmaTile + 8;
+
+__device__ __forceinline__ void ldsm_x4_trans(uint32_t (&r)[4], const void* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(smem_u32(p)));
+}
+__host__ __device__ inline size_t rows_shared(int Dk) {
+  return (size_t)(16 * kRowTokens + kRowSlots * kRowHalf) * (Dk + 8) * 2 + (size_t)16 * kRowTokens * kRowPld * 2 +
+         8 * 16 * kRowTokens * 4;
+}
+
+// NT: tiles of 8 latent channels a warp has (a quarter of them).
+template <int NT>
+__global__ void __launch_bounds__(512, 1)
+latent_attention_rows_kernel(const float* __restrict__ q_lat, const float* __restrict__ q_rot,
+                             const bf16* __restrict__ c_pages, const bf16* __restrict__ r_pages,
+                             const int* __restrict__ block_table, int table_stride,
+                             const int* __restrict__ seq_of_token, const int* __restrict__ positions,
+                             bf16* __restrict__ out, int num_tokens, int H, int C, int R, int page_size,
+                             int window, float scale) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int Dk = C + R, ld = Dk + 8;
+  bf16* Qs = reinterpret_cast<bf16*>(smem_raw);              // [64][ld], row 16 token + head
+  bf16* Ks = Qs + 16 * kRowTokens * ld;                      // [kRowSlots][32][ld]
+  bf16* Ps = Ks + kRowSlots * kRowHalf * ld;                 // [64][kRowPld]
+  float* red = reinterpret_cast<float*>(Ps + 16 * kRowTokens * kRowPld);   // [8][64]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+  const int tok = warp & 3, qr = warp >> 2, h0 = blockIdx.y * 16;
+  // the last tokens of a prompt see the most keys: they go first
+  const int base = ((int)gridDim.x - 1 - (int)blockIdx.x) * kRowTokens;
+  pdl_trigger();
+  pdl_wait();
+  if (!in_rows(base, num_tokens, seq_of_token, positions, window)) return;
+  const int b = seq_of_token[base], t = base + tok;
+  const int p_last = positions[base + kRowTokens - 1], p = positions[t];
+  const int* tbl = block_table + (size_t)b * table_stride;
+  const int nchunk = Dk >> 3, kj = threadIdx.x >> 4;         // sixteen threads a key
+  // (a key's page is looked up a tile ahead of its copy, so that no copy waits for the table)
+  auto page_of = [&](int half) {
+    const int c = half * kRowHalf + kj;
+    return c <= p_last ? tbl[c / page_size] : -1;
+  };
+  auto ask = [&](int half, int page) {                       // keys 32 half .. + 31
+    bf16* dst = Ks + ((size_t)(half % kRowSlots) * kRowHalf + kj) * ld;
+    const bool ok = page >= 0;
+    const size_t slot = ok ? (size_t)page * page_size + (half * kRowHalf + kj) % page_size : 0;
+    for (int i = threadIdx.x & 15; i < nchunk; i += 16) {
+      const int d = i << 3;
+      cp_async_16(dst + d, d < C ? c_pages + slot * C + d : r_pages + slot * R + (d - C), ok);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  ask(0, page_of(0));
+  ask(1, page_of(1));
+  int page_a = page_of(2), page_b = page_of(3);
+  const int dq = Dk >> 2;
+  for (int i = threadIdx.x; i < 16 * kRowTokens * dq; i += 512) {
+    const int row = i / dq, d = (i - row * dq) * 4, tt = base + (row >> 4), h = h0 + (row & 15);
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    if (h < H)
+      Quad<float>::fresh(d < C ? q_lat + ((size_t)h * num_tokens + tt) * C + d
+                               : q_rot + ((size_t)tt * H + h) * R + (d - C), v);
+    Quad<bf16>::store(Qs + row * ld + d, v);
+  }
+  auto token_sync = [&] { asm volatile("bar.sync %0, 128;" ::"r"(tok + 1) : "memory"); };
+  float o[NT][4];
+#pragma unroll
+  for (int j = 0; j < NT; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
+  float m[2] = {-INFINITY, -INFINITY}, lsum[2][2] = {{0.f, 0.f}, {0.f, 0.f}};   // [eight keys][row]
+  const int ctiles = C >> 3, ntw = (((ctiles + 3) >> 2) + 1) & ~1, ct0 = qr * ntw;   // (ctiles is even)
+  const bf16* qa = Qs + (tok * 16 + (lane & 15)) * ld + ((lane >> 4) << 3);
+  const int k_mid = ((Dk >> 4) >> 1) << 4;
+  const int all_tiles = p_last / kMmaTile + 1, my_tiles = p / kMmaTile + 1;
+  for (int it = 0; it < all_tiles; ++it) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                         // this tile is there, the third place is free
+    if (it + 1 < all_tiles) ask(2 * it + 2, page_a);
+    page_a = page_of(2 * it + 4);
+    const bf16* K[2] = {Ks + (size_t)(2 * it % kRowSlots) * kRowHalf * ld,
+                        Ks + (size_t)((2 * it + 1) % kRowSlots) * kRowHalf * ld};
+    const bool mine = it < my_tiles;
+    float corr[2] = {1.f, 1.f};
+    if (mine) {
+      // ---- scores of 16 keys: 16 qr .. + 15 of the tile
+      float s[2][4];
+      const bf16* kb = K[qr >> 1] + (size_t)((qr & 1) * 16 + ((lane >> 4) << 3) + (lane & 7)) * ld + (((lane >> 3) & 1) << 3);
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        float s0[2][4] = {}, s1[2][4] = {};
+        const int k_hi = half ? Dk : k_mid;
+        int kk = half ? k_mid : 0;
+#pragma unroll 2
+        for (; kk + 32 <= k_hi; kk += 32) {
+          uint32_t a0[4], a1[4], x0[4], x1[4];
+          ldsm_x4(a0, qa + kk);
+          ldsm_x4(x0, kb + kk);
+          ldsm_x4(a1, qa + kk + 16);
+          ldsm_x4(x1, kb + kk + 16);
+          const uint32_t b00[2] = {x0[0], x0[1]}, b01[2] = {x0[2], x0[3]};
+          const uint32_t b10[2] = {x1[0], x1[1]}, b11[2] = {x1[2], x1[3]};
+          mma_bf16(s0[0], a0, b00);
+          mma_bf16(s0[1], a0, b01);
+          mma_bf16(s1[0], a1, b10);
+          mma_bf16(s1[1], a1, b11);
+        }
+        if (kk < k_hi) {
+          uint32_t a0[4], x0[4];
+          ldsm_x4(a0, qa + kk);
+          ldsm_x4(x0, kb + kk);
+          const uint32_t b00[2] = {x0[0], x0[1]}, b01[2] = {x0[2], x0[3]};
+          mma_bf16(s0[0], a0, b00);
+          mma_bf16(s0[1], a0, b01);
+        }
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float both = s0[n][e] + s1[n][e];
+            s[n][e] = half ? s[n][e] + both : both;
+          }
+      }
+      float mx[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        const int key0 = it * kMmaTile + 16 * qr + 8 * n + 2 * t4;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          s[n][e] = key0 + (e & 1) <= p ? s[n][e] * scale : -INFINITY;
+          mx[e >> 1] = fmaxf(mx[e >> 1], s[n][e]);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
+        mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
+        if (t4 == 0) red[qr * 64 + tok * 16 + g + 8 * r] = mx[r];
+      }
+      token_sync();
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const float* at = red + tok * 16 + g + 8 * r;
+        const float mn = fmaxf(m[r], fmaxf(fmaxf(at[0], at[64]), fmaxf(at[128], at[192])));
+        corr[r] = expf(m[r] - mn);
+        m[r] = mn;
+      }
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        lsum[n][0] *= corr[0];
+        lsum[n][1] *= corr[1];
+        const float p0 = expf(s[n][0] - m[0]), p1 = expf(s[n][1] - m[0]);
+        const float p2 = expf(s[n][2] - m[1]), p3 = expf(s[n][3] - m[1]);
+        lsum[n][0] += p0 + p1;
+        lsum[n][1] += p2 + p3;
+        bf16* pw = Ps + (size_t)(tok * 16) * kRowPld + 16 * qr + 8 * n + 2 * t4;
+        *reinterpret_cast<uint32_t*>(pw + g * kRowPld) = pack_bf16(p0, p1);
+        *reinterpret_cast<uint32_t*>(pw + (g + 8) * kRowPld) = pack_bf16(p2, p3);
+      }
+#pragma unroll
+      for (int j = 0; j < NT; ++j) {
+        o[j][0] *= corr[0], o[j][1] *= corr[0];
+        o[j][2] *= corr[1], o[j][3] *= corr[1];
+      }
+      token_sync();
+    }
+    // ---- this warp's quarter of the latent channels, half a tile of keys at a time
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      if (mine) {
+#pragma unroll
+        for (int ks = 0; ks < kRowHalf; ks += 16) {
+          uint32_t a[4];
+          ldsm_x4(a, Ps + (size_t)(tok * 16 + (lane & 15)) * kRowPld + half * kRowHalf + ks + ((lane >> 4) << 3));
+          const bf16* vrow = K[half] + (size_t)(ks + (lane & 15)) * ld + ((lane >> 4) << 3);
+          // keys 2 t4, 2 t4 + 1 (and + 8, + 9) behind the token are zeros to it, whatever they hold
+          const int key = it * kMmaTile + half * kRowHalf + ks + 2 * t4;
+          uint32_t keep[2];
+#pragma unroll
+          for (int x = 0; x < 2; ++x)
+            keep[x] = (key + 8 * x <= p ? 0xffffu : 0u) | (key + 8 * x + 1 <= p ? 0xffff0000u : 0u);
+#pragma unroll
+          for (int j = 0; j < NT; j += 2) {
+            const int ct = ct0 + j;
+            if (j < ntw && ct < ctiles) {
+              uint32_t v[4];
+              ldsm_x4_trans(v, vrow + ct * 8);
+              const uint32_t v0[2] = {v[0] & keep[0], v[1] & keep[1]}, v1[2] = {v[2] & keep[0], v[3] & keep[1]};
+              mma_bf16(o[j], a, v0);
+              mma_bf16(o[j + 1], a, v1);
+            }
+          }
+        }
+      }
+      if (half == 0) {
+        __syncthreads();                                     // the tile's first place is free
+        if (it + 1 < all_tiles) ask(2 * it + 3, page_b);
+        page_b = page_of(2 * it + 5);
+      }
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      lsum[n][r] += __shfl_xor_sync(0xffffffffu, lsum[n][r], 1);
+      lsum[n][r] += __shfl_xor_sync(0xffffffffu, lsum[n][r], 2);
+    }
+  token_sync();                                              // the maxima have been read
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+      if (t4 == 0) red[(2 * qr + n) * 64 + tok * 16 + g + 8 * r] = lsum[n][r];
+  token_sync();
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int h = h0 + g + 8 * r;
+    if (h >= H) continue;
+    float l = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) l += red[w * 64 + tok * 16 + g + 8 * r];
+    const float inv = 1.f / l;
+    bf16* dst = out + ((size_t)h * num_tokens + t) * C;
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+      const int ct = ct0 + j;
+      if (j < ntw && ct < ctiles)
+        *reinterpret_cast<uint32_t*>(dst + ct * 8 + 2 * t4) = pack_bf16(o[j][2 * r] * inv, o[j][2 * r + 1] * inv);
+    }
+  }
+}
+
 // out[h, t, :] = sum_z o_z exp(m_z - M) / sum_z l_z exp(m_z - M): a block a (token, head), a thread four
 // channels.  Bound by latency: the shares' sums are asked for before their weights are known (what an
 // empty share left there is not used), all at once.  32 tokens, 16 heads of 512 channels in 4 shares on a
@@ -664,7 +922,7 @@ GF_EXPORT int gf_latent_attention(const float* q_lat, const float* q_rot, const 
                                   const int* seq_of_token, const int* positions, void* out, int T,
                                   int H, int C, int R, int page_size, int window, float scale,
                                   int dtype, int nsplit, float* part_o, float* part_ml,
-                                  void* stream) {
+                                  int max_q_len, void* stream) {
   if (T <= 0) return 0;
   if (C > kLatMaxC || C <= 0 || R < 0) return -3;
   const int Dk = C + R;
@@ -689,13 +947,38 @@ GF_EXPORT int gf_latent_attention(const float* q_lat, const float* q_rot, const 
       if (nsplit < 1 || nsplit > 16 || (nsplit > 1 && (!part_o || !part_ml))) nsplit = 1;
       const dim3 grid(T, (H + 15) / 16, nsplit), block(kMmaWarps * 32);
       auto st = (cudaStream_t)stream;
+      // steps with portions: their groups of four tokens first, then what is left
+      const int rows = nsplit == 1 && max_q_len >= 4 * kRowTokens &&
+                       (long long)(T / kRowTokens) * ((H + 15) / 16) >= kRowMinBlocks && C <= 512 &&
+                       rows_shared(Dk) <= 220 * 1024 && (uintptr_t)q_lat % 16 == 0 && (uintptr_t)q_rot % 16 == 0;
+      if (rows) {
+        static OncePerDevice once_rows;
+        if (int rc = once_rows.run([] {
+              for (auto k : {latent_attention_rows_kernel<4>, latent_attention_rows_kernel<8>,
+                             latent_attention_rows_kernel<16>}) {
+                const cudaError_t e =
+                    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+                if (e != cudaSuccess) return e;
+              }
+              return cudaSuccess;
+            }))
+          return rc;
+        const auto kernel = C <= 128   ? latent_attention_rows_kernel<4>
+                            : C <= 256 ? latent_attention_rows_kernel<8>
+                                       : latent_attention_rows_kernel<16>;
+        if (int rc = launch_kernel(kernel, dim3((T + kRowTokens - 1) / kRowTokens, (H + 15) / 16), dim3(512),
+                                   rows_shared(Dk), st, q_lat, q_rot, (const bf*)c_pages, (const bf*)r_pages,
+                                   block_table, table_stride, seq_of_token, positions, (bf*)out, T, H, C, R,
+                                   page_size, window, scale))
+          return rc;
+      }
       int rc2 = -3;
 #define GF_GO(NT)                                                                              \
   if (rc2 == -3 && C <= 128 * NT)                                                              \
     rc2 = launch_kernel(latent_attention_mma_kernel<NT>, grid, block, bytes, st, q_lat, q_rot,  \
                         (const bf*)c_pages, (const bf*)r_pages, block_table, table_stride,      \
                         seq_of_token, positions, (bf*)out, T, H, C, R, page_size, window, scale, \
-                        nsplit, part_o, part_ml)
+                        nsplit, part_o, part_ml, rows)
       GF_GO(1);
       GF_GO(2);
       GF_GO(4);

@@ -116,14 +116,17 @@ def attention(q_lat: torch.Tensor, q_rot: torch.Tensor, c_pages: torch.Tensor,
         if nsplit > 1:
             part_o = torch.empty((nsplit, T, H, C), dtype=torch.float32, device=q_lat.device)
             part_ml = torch.empty((nsplit, T, H, 2), dtype=torch.float32, device=q_lat.device)
+    # portions whose tokens see their request from its first key on share tiles of keys (same bits); where most
+    # windows start behind it, the kernel for them would only be launched
+    longest = int(getattr(ctx, "max_q_len", 0) or 0) if window <= 0 or max_keys <= 2 * window else 0
     f = _fn("latent_attention", "gf_latent_attention",
             [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
              c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p,
-             c_void_p, c_void_p], kernels=2 if nsplit > 1 else 1)
+             c_void_p, c_int, c_void_p], kernels=2 if nsplit > 1 else 1)
     rc = f(_p(q_lat), _p(q_rot), _p(c_pages), _p(r_pages), _p(block_table),
            block_table.stride(0), _p(ctx.seq_of_token), _p(ctx.positions), _p(out), T, H, C, R,
            int(page_size), int(window), float(scale), _code(c_pages.dtype), nsplit, _p(part_o),
-           _p(part_ml), _stream())
+           _p(part_ml), longest, _stream())
     if rc == -3:
         raise ValueError(f"latent attention takes latent vectors of up to 1024 channels whose key "
                          f"tile fits shared memory; got kv_rank={C}, rot_dim={R}")

@@ -1042,3 +1042,37 @@ def test_heads_that_share_queries_and_keys_share_their_scores(H, G, D, Vd, lens,
         got.append((o if norm else (o,)) + (state,))
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("H,C,R,window,portions,broken", [
+    (16, 64, 16, 0, [(0, 801)], ()), (16, 272, 16, 900, [(0, 401), (700, 402), (3, 2)], ()),
+    (20, 48, 0, 512, [(0, 129), (0, 300), (400, 99)], ()), (3, 512, 32, 1024, [(0, 770)], (66, 300)),
+    (16, 16, 16, 0, [(0, 63), (0, 65), (64, 641)], (62, 64))])
+def test_latent_attention_of_neighbouring_tokens(H, C, R, window, portions, broken):
+    """Tokens in fours that share tiles of keys: the bits of a block a token, with remainders of four, requests
+    that meet inside a four, windows that start behind key 0, odd numbers of 32 channels, and keys that are no
+    number, which no token in front of them sees."""
+    from types import SimpleNamespace
+    from ginfer_b200.ops import latent
+    page, g = 16, torch.Generator(device=DEV).manual_seed(C + R)
+    lens, T = [a + n for a, n in portions], sum(n for _, n in portions)
+    pages = [-(-n // page) for n in lens]
+    table = torch.zeros(len(lens), max(pages), dtype=torch.int32)
+    order = torch.randperm(sum(pages), generator=torch.Generator().manual_seed(C)).int()
+    for i, n in enumerate(pages):
+        table[i, :n] = order[sum(pages[:i]):sum(pages[:i + 1])]
+    c = torch.randn(sum(pages), page, 1, C, device=DEV, generator=g).bfloat16()
+    r = torch.randn(sum(pages), page, 1, R, device=DEV, generator=g).bfloat16() if R else None
+    for p in broken:
+        c.view(-1, C)[int(table[0, p // page]) * page + p % page, ::3] = float("nan")
+    q = torch.randn(H, T, C, device=DEV, generator=g) * 3 * C ** -0.5
+    qr = torch.randn(T, H, R, device=DEV, generator=g) if R else None
+    seq = torch.cat([torch.full((n,), i) for i, (_, n) in enumerate(portions)]).int().cuda()
+    pos = torch.cat([torch.arange(a, a + n) for a, n in portions]).int().cuda()
+    out = []
+    for longest in (max(n for _, n in portions), 0):       # 0: a block a token
+        ctx = SimpleNamespace(seq_of_token=seq, positions=pos, max_kv_len=max(lens), max_q_len=longest)
+        out.append(latent.attention(q, qr, c, r, table.cuda(), ctx, window, (C + R) ** -0.5, page))
+    assert torch.equal(*(torch.nan_to_num(o.float(), nan=1e9) for o in out))
+    if broken:
+        assert torch.isnan(out[0]).any() and not torch.isnan(out[0][:, :min(broken)]).any()
