@@ -655,6 +655,193 @@ moe_stream_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfloa
     }
 }
 
+// ---- the same for more pairs of large experts ------------------------------------------------------
+// The grid above is (tile, weight rows) blocks, about one and a half rounds of them: while the last round runs
+// half of the places are empty.  Here one block an SM takes an equal run of the step's (tile of pairs, 16 weight
+// rows) items, one list.  Its sixteen warps share an item's reduction: step f of a matrix (16-row groups in
+// order, steps of 64 k inside) belongs to warp f mod 16, whatever block has it, so that a pair's sums follow from
+// the matrix alone.  A warp's steps come through a ring of its own in shared memory, each lane with its own
+// 16-byte copies (nobody else reads them: no barrier), which runs on across items and tiles; after every two
+// items the warps' sums meet, two warps add them up in order and store.
+// For steps of one to two and a half pairs an expert.  Whole batches on a B200 (ms, the grid above / here), 32 experts
+// of 2048 x 2112, 4 choices: 9 requests 35.7 / 30.8, 16 requests 42.5 / 34.2, 32 requests 29.18 / 29.16, 64 requests
+// 24.4 / 24.9; 29 of 2048 x 1408, 5 choices: 8 requests 28.5 / 27.9, 30 requests 26.5 / 27.3.  Both products alone,
+// weights from HBM: 64 pairs of the first 91.9 / 87.1 us (floor 69.7), 24 pairs 52.9 / 59.8; of 8 experts of 2048 x
+// 1408, 48 pairs, 37.2 / 40.8: with few tiles of pairs the start of a run (the tile's rows, the first steps) is too
+// much of it, with many their rows are.
+constexpr int kRgWarps = 16, kRgRing = 3, kRgItems = 2;
+constexpr int kRgSlot = 2048;                                // a step: 16 rows x 64 k
+constexpr int kRgHead = 128;                                 // the rows' weights
+constexpr int kRgSums = kRgItems * kRgWarps * 2 * 32 * 16;
+constexpr int kRgMaxShared = 227 * 1024;
+// From this many bytes of weights an expert and experts: 16 of 1024 x 704, 8 pairs, take 12.5 us above and 16.4 here.
+constexpr size_t kRgMinBytes = 4 << 20;
+constexpr int kRgMinExperts = 24;
+__host__ __device__ inline size_t ring_shared(int K) {
+  return kRgHead + (size_t)kRgWarps * kRgRing * kRgSlot + kRgSums + kStRows * stream_pitch(K);
+}
+__device__ __forceinline__ void ring_copy(uint32_t dst, const void* src, bool there) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(there ? 16 : 0) : "memory");
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kRgWarps * 32, 1)
+moe_ring_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfloat16* __restrict__ w,
+                int N, int K, const int* __restrict__ offsets, const int* __restrict__ pair_of_pos,
+                int top, const int* __restrict__ tile_expert, const int* __restrict__ tile_row0,
+                const int* __restrict__ num_tiles, void* __restrict__ out_, float limit,
+                float alpha, float up_shift, const float* __restrict__ row_w) {
+  extern __shared__ __align__(128) uint8_t shared[];         // head | rings | sums | [kStRows] rows of stream_pitch(K)
+  float* weight_of = reinterpret_cast<float*>(shared);       // [kStRows]
+  float4* sums = reinterpret_cast<float4*>(shared + kRgHead + kRgWarps * kRgRing * kRgSlot);
+  uint8_t* staged = shared + kRgHead + kRgWarps * kRgRing * kRgSlot + kRgSums;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int units = (K + 63) / 64, groups = (N + 15) / 16;
+  pdl_wait();
+  pdl_trigger();
+  const long long items = (long long)fresh_index(num_tiles) * groups;
+  const long long i0 = items * blockIdx.x / gridDim.x, i1 = items * (blockIdx.x + 1) / gridDim.x;
+  if (i0 >= i1) return;
+  const int first_tile = (int)(i0 / groups), first_group = (int)(i0 % groups);
+  const int last_tile = (int)((i1 - 1) / groups), last_group = (int)((i1 - 1) % groups);
+
+  // the warp's next step to ask for: step pu of group pg of tile pt; from group `pend` on the block has no more
+  // of this tile
+  int pt = first_tile, pg, pu, pend;
+  const __nv_bfloat16* pw;
+  auto enter = [&](int tile, int group) {                    // the warp's first step at or behind `group`
+    const int ahead = (warp - group * units) & (kRgWarps - 1);
+    pg = group + ahead / units, pu = ahead % units;
+    pend = tile == last_tile ? last_group + 1 : groups;
+    pw = w + (size_t)fresh_index(tile_expert + tile) * N * K + 8 * t;
+  };
+  enter(pt, first_group);
+  const uint32_t ring = smem_u32(shared) + kRgHead + warp * kRgRing * kRgSlot + lane * 16;
+  auto ask = [&](int slot) {
+    while (pg >= pend && pt < last_tile) {
+      ++pt;
+      enter(pt, 0);
+    }
+    if (pg < pend) {
+      const int n = pg * 16 + 2 * g;                         // N is even: both rows are there, or none
+      const __nv_bfloat16* src = pw + (size_t)n * K + pu * 64;
+      const uint32_t dst = ring + slot * kRgSlot;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const bool there = n < N && pu * 64 + h * 32 + 8 * t < K;
+        ring_copy(dst + h * 1024, there ? src + h * 32 : w, there);
+        ring_copy(dst + h * 1024 + 512, there ? src + h * 32 + K : w, there);
+      }
+      pu += kRgWarps;
+      while (pu >= units) pu -= units, ++pg;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int i = 0; i < kRgRing; ++i) ask(i);
+
+  int slot = 0;
+  const size_t pitch = stream_pitch(K);
+  const uint8_t* x0 = staged + g * pitch + 16 * t;
+  const uint8_t* mine = shared + kRgHead + warp * kRgRing * kRgSlot + lane * 16;
+  for (int tile = first_tile; tile <= last_tile; ++tile) {
+    const int e = fresh_index(tile_expert + tile), row0 = fresh_index(tile_row0 + tile);
+    const int rows = min(kStRows, fresh_index(offsets + e + 1) - row0);
+    const bool second = rows > 8;
+    if (MODE == 2 && (int)threadIdx.x < rows)
+      weight_of[threadIdx.x] = row_w ? fresh(row_w + fresh_index(pair_of_pos + row0 + threadIdx.x)) : 1.f;
+    {                                                        // the rows, zeros up to whole steps
+      const int k8 = units * 8, staged_rows = second ? 16 : 8;
+      for (int i = threadIdx.x; i < staged_rows * k8; i += kRgWarps * 32) {
+        const int r = i / k8, c = (i - r * k8) * 8;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (r < rows && c < K) {
+          const int src = MODE != 0 ? fresh_index(pair_of_pos + row0 + r) / top : row0 + r;
+          v = __ldcg(reinterpret_cast<const uint4*>(a + (size_t)src * lda + c));
+        }
+        *reinterpret_cast<uint4*>(staged + r * pitch + (size_t)c * 2) = v;
+      }
+    }
+    __syncthreads();
+    const int g0 = tile == first_tile ? first_group : 0, g1 = tile == last_tile ? last_group + 1 : groups;
+    for (int from = g0; from < g1; from += kRgItems) {
+      const int many = min(kRgItems, g1 - from);
+      for (int b = 0; b < many; ++b) {
+        float acc[2][2][4] = {};                             // [run][8 j ..]: pairs 8 j + 2 t, + 1 of rows 2 g | 2 g + 1
+        for (int u = (warp - (from + b) * units) & (kRgWarps - 1); u < units; u += kRgWarps) {
+          asm volatile("cp.async.wait_group %0;" ::"n"(kRgRing - 1) : "memory");
+          const uint8_t *x = x0 + (size_t)u * 128, *at = mine + slot * kRgSlot;
+          uint4 wa[2], wb[2];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            wa[h] = *reinterpret_cast<const uint4*>(at + h * 1024);
+            wb[h] = *reinterpret_cast<const uint4*>(at + h * 1024 + 512);
+          }
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const uint32_t lo[4] = {wa[h].x, wb[h].x, wa[h].y, wb[h].y};
+            const uint32_t hi[4] = {wa[h].z, wb[h].z, wa[h].w, wb[h].w};
+            const uint4 v = *reinterpret_cast<const uint4*>(x + h * 64);
+            const uint32_t b0[2] = {v.x, v.y}, b1[2] = {v.z, v.w};
+            mma_bf16(acc[h][0], lo, b0);
+            mma_bf16(acc[h][0], hi, b1);
+            if (second) {
+              const uint4 y = *reinterpret_cast<const uint4*>(x + 8 * pitch + h * 64);
+              const uint32_t d0[2] = {y.x, y.y}, d1[2] = {y.z, y.w};
+              mma_bf16(acc[h][1], lo, d0);
+              mma_bf16(acc[h][1], hi, d1);
+            }
+          }
+          ask(slot);                                         // its old contents are in registers
+          slot = slot + 1 == kRgRing ? 0 : slot + 1;
+        }
+        float4* to = sums + (b * kRgWarps + warp) * 64 + lane;
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+          if (j == 0 || second)
+            to[j * 32] = make_float4(acc[0][j][0] + acc[1][j][0], acc[0][j][1] + acc[1][j][1],
+                                     acc[0][j][2] + acc[1][j][2], acc[0][j][3] + acc[1][j][3]);
+      }
+      __syncthreads();
+      const int n = (from + warp) * 16 + 2 * g;
+      if (warp < many && n < N) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          if (j == 1 && !second) break;
+          const float4* of = sums + warp * kRgWarps * 64 + j * 32 + lane;
+          float4 s = of[0];
+#pragma unroll
+          for (int p = 1; p < kRgWarps; ++p) {
+            const float4 v = of[p * 64];
+            s.x += v.x, s.y += v.y, s.z += v.z, s.w += v.w;
+          }
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const int r = 8 * j + 2 * t + i;
+            if (r >= rows) continue;
+            const size_t at = (size_t)(row0 + r);
+            const float c0 = i ? s.y : s.x, c1 = i ? s.w : s.z;    // weight rows n, n + 1
+            if (MODE == 2) {
+              const float rw = weight_of[r];
+              const float v0 = fmaxf(to_f32(from_f32<__nv_bfloat16>(c0 * rw)), 0.f);
+              const float v1 = fmaxf(to_f32(from_f32<__nv_bfloat16>(c1 * rw)), 0.f);
+              *reinterpret_cast<__nv_bfloat162*>((__nv_bfloat16*)out_ + at * N + n) =
+                  __floats2bfloat162_rn(v0 * v0, v1 * v1);
+            } else if (MODE == 1) {
+              const float gt = to_f32(from_f32<__nv_bfloat16>(c0)), up = to_f32(from_f32<__nv_bfloat16>(c1));
+              ((__nv_bfloat16*)out_)[at * (N / 2) + n / 2] =
+                  from_f32<__nv_bfloat16>(clamped_glu(gt, up, limit, alpha, up_shift));
+            } else {
+              *reinterpret_cast<float2*>((float*)out_ + at * N + n) = make_float2(c0, c1);
+            }
+          }
+        }
+      }
+      __syncthreads();                                       // the sums (and the rows) may be written again
+    }
+  }
+}
+
 // ---- the same for a handful of pairs on the FMA pipes ----------------------------------------------
 // For layers that stay off moe_stream_kernel (their routers' close calls ask for sums in one order).  The
 // work is the experts' weight bytes.  A tile is up to 8 rows of one expert, kept in shared memory; the (tile,
@@ -952,6 +1139,27 @@ GF_EXPORT int gf_moe_gemm(const void* a, int lda, const void* w, int N, int K, c
     if (dtype != GF_BF16 || K % 8 || lda % 8 || N % 2 || (uintptr_t)a % 16 || (uintptr_t)w % 16 ||
         (uintptr_t)out % 8 || smem > kStMaxShared)
       return -3;
+    if (experts >= kRgMinExperts && pairs >= experts && 2 * pairs <= 5 * experts &&
+        (size_t)N * K * sizeof(bf) >= kRgMinBytes && ring_shared(K) <= kRgMaxShared) {
+      int sms = 0;
+      if (int rc = sm_count(&sms)) return rc;
+#define GF_RING(MODE)                                                                             \
+  {                                                                                               \
+    static OncePerDevice attrs;                                                                   \
+    if (int rc = attrs.run([&] {                                                                  \
+          return cudaFuncSetAttribute(moe_ring_kernel<MODE>,                                      \
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, kRgMaxShared); \
+        }))                                                                                       \
+      return rc;                                                                                  \
+    return launch_kernel(moe_ring_kernel<MODE>, dim3(sms), dim3(kRgWarps * 32), ring_shared(K), st, \
+                         (const bf*)a, lda, (const bf*)w, N, K, offsets, pair_of_pos, top,        \
+                         tile_expert, tile_row0, num_tiles, out, limit, alpha, up_shift, row_w);  \
+  }
+      if (first == 2) GF_RING(2)
+      if (first) GF_RING(1)
+      GF_RING(0)
+#undef GF_RING
+    }
     // about 16 warps an SM should be busy
     const int each = pairs <= kStRows * experts ? 2 : 4;       // tiles an expert
     const int most = pairs <= kStHandful ? kStHandfulTiles : kStTiles;

@@ -618,6 +618,46 @@ def test_products_of_a_handful_of_pairs(K, N, counts):
         assert torch.equal(moe.grouped_glu(x[p:p + 1], up, one, 1e9, 1.0, 0.0)[0], glu[p])
 
 
+@pytest.mark.parametrize("E,K,N,counts", [
+    (24, 2048, 1026, [1] * 24), (32, 1096, 2050, [0] * 20 + [17, 1, 2, 8, 9, 16, 0, 0, 0, 0, 0, 27]),
+    (40, 2120, 1056, [2, 0] * 20), (30, 520, 4034, [3] * 10 + [1] * 20)])
+def test_routed_products_of_one_or_two_pairs_an_expert(E, K, N, counts):
+    """Equal runs of items over all SMs: runs that begin and end inside a tile or hold several, tiles of up to
+    16 pairs and experts of more, reductions and rows that are no multiples of a step: against 64 bits, and the
+    same bits for the same pairs in another step of that range."""
+    from ginfer_b200.ops import moe
+    g = torch.Generator(device=DEV).manual_seed(K + N)
+    P = sum(counts)
+    assert E <= P <= 2.5 * E and 2 * N * K >= 4 << 20
+    idx = torch.tensor([e for e, n in enumerate(counts) for _ in range(n)])
+    idx = idx[torch.randperm(P, generator=torch.Generator().manual_seed(K))].int().cuda().view(P, 1)
+    x = torch.randn(P, K, generator=g, device=DEV).bfloat16()
+    w = (torch.randn(E, N, K, generator=g, device=DEV) * K ** -0.5).bfloat16()
+    wgt = torch.rand(P, 1, generator=g, device=DEV) + 0.5
+
+    def run(idx, x, wgt):
+        plan = moe.Plan(idx, E, "few")
+        back = plan.pos_of_pair.long()
+        return (moe.grouped_down(x[plan.pair_of_pos.long()].contiguous(), w, plan)[back],
+                moe.grouped_glu(x, w, plan, 1e9, 1.0, 0.0)[back], moe.grouped_relu2(x, w, plan, wgt)[back])
+    rows, glu, relu2 = run(idx, x, wgt)
+    for at in range(0, P, 16):
+        e = idx[at:at + 16, 0].long()
+        want = torch.einsum("pk,pnk->pn", x[at:at + 16].double(), w[e].double())
+        size = torch.einsum("pk,pnk->pn", x[at:at + 16].double().abs(), w[e].double().abs())
+        # sums of 16 warps with two accumulators each: chains of K / 32 products at most, of fp32 in the tensor
+        # cores (four a step), then 17 additions
+        assert ((rows[at:at + 16].double() - want).abs() <= (K / 32 + 40) * 2.0 ** -23 * size).all()
+    gate, lift = rows[:, 0::2].bfloat16().double(), rows[:, 1::2].bfloat16().double()
+    ref = gate / (1 + torch.exp(-gate)) * lift
+    assert ((glu.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-30).all()
+    ref = (rows * wgt).bfloat16().double().clamp(min=0) ** 2
+    assert ((relu2.double() - ref).abs() <= 2.0 ** -8 * ref).all()
+    some = torch.arange(P - 1, -1, -1, device=DEV)[:max(E, P - 3)]
+    for a, b in zip((rows, glu, relu2), run(idx[some].contiguous(), x[some].contiguous(), wgt[some].contiguous())):
+        assert torch.equal(a[some], b)
+
+
 @pytest.mark.parametrize("K,F,E,top", [(2048, 1408, 32, 4), (1024, 704, 16, 2), (256, 96, 8, 1)])
 @pytest.mark.parametrize("counts", [(1, 2, 3, 5), (24, 25, 40, 100)])
 def test_a_pairs_result_does_not_depend_on_the_batch(K, F, E, top, counts):
