@@ -91,18 +91,22 @@ CHUNK_MIN_TOKENS = 64
 CHANNELS_MAX_WORDS = 1 << 26
 
 
+def _chunk_scratch(q_lens, H: int, G: int, D: int, Vd: int) -> tuple[int, int]:
+    """Chunks of portions of ``q_lens`` tokens, and the fp32 words of scratch that they take."""
+    lib = load_library("decay_chunk")
+    words = lib.gf_decay_chunk_words
+    words.argtypes, words.restype = [c_int] * 5, c_longlong
+    size = int(lib.gf_decay_chunk_tokens())
+    chunks = sum(-(-n // size) for n in q_lens)
+    return chunks, int(words(chunks, H, G, D, Vd))
+
+
 def _chunked(q, k, v, g, state, ctx, first: int, H, G, D, Vd, k_scale, skip, normaliser, o, o_n) -> bool:
     """The requests from number ``first`` on, a chunk of tokens at a time; ``False`` if not served."""
     if D > 128 or D % 4 or Vd % 4:
         return False
-    if not _chunk_tokens:
-        _chunk_tokens.append(int(load_library("decay_chunk").gf_decay_chunk_tokens()))
-    chunks = sum(-(-n // _chunk_tokens[0]) for n in ctx.q_lens_host[first:])
-    if len(_chunk_tokens) == 1:
-        words = load_library("decay_chunk").gf_decay_chunk_words
-        words.argtypes, words.restype = [c_int] * 5, c_longlong
-        _chunk_tokens.append(words)
-    scratch = torch.empty(int(_chunk_tokens[1](chunks, H, G, D, Vd)), dtype=torch.float32, device=v.device)
+    chunks, words = _chunk_scratch(ctx.q_lens_host[first:], H, G, D, Vd)
+    scratch = torch.empty(words, dtype=torch.float32, device=v.device)
     f = _fn("decay_chunk", "gf_decay_chunked",
             [c_void_p, c_int] * 5 + [c_void_p, c_void_p, c_int, c_void_p, c_void_p] + [c_int] * 6 +
             [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p], kernels=4 if H > G else 3)
@@ -134,9 +138,6 @@ def _channels_chunked(q, k, v, g, state, ctx, H, G, D, Vd, o) -> bool:
             return False
         _ok(rc, "decay_channels_chunked")
     return True
-
-
-_chunk_tokens: list = []               # tokens a chunk; the function that gives a step's words of scratch
 
 
 def recurrence(q, k, v, g, state: torch.Tensor, ctx, H: int, G: int, D: int, Vd: int,
