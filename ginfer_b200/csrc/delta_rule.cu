@@ -476,7 +476,9 @@ delta_recurrence_kernel(const float* __restrict__ qn, const float* __restrict__ 
 // On a B200, prompts of 150, 300, 600 and 1,201 tokens, 16 heads of 128 x 128: 420 us a layer (a warp a column:
 // 740); one of 1,201 tokens 288 (446); eight of 200
 // 202 (four lanes a column: 680), seven of 1 to 900 375 (1,620).
-constexpr int kTreeThreads = 128, kTreeChunk = 8, kTreeGroups = 4;
+// Up to kTreeSorted requests are sorted by length, in every block (B^2 / 128 comparisons a thread: 512 requests of 5 tokens
+// 7.9 ms so, 0.8 as they come); more of them fill the device in any order.
+constexpr int kTreeThreads = 128, kTreeChunk = 8, kTreeGroups = 4, kTreeSorted = 64;
 
 template <int N> __device__ __forceinline__ float tree_sum(const float* p) {
   if constexpr (N == 1) return p[0];
@@ -1252,13 +1254,24 @@ GF_EXPORT long long gf_delta_chunk_words(int T, int B, int heads, int D, int one
   return one_decay ? chunks * kCoefs : chunks * (kCoefs + D) + 2ll * T * heads * D;
 }
 
+// Many (request, head, column) triples: whether T tokens of B requests take the kernel of portions of many tokens
+// instead of four lanes a column, which give the same bits.  A request costs that kernel more before its first
+// token (one block of up to four requests an SM), a token less.  Its time over that of four lanes on a B200, 8 to
+// 512 requests of equal portions: 16 heads of 128 x 128, 2 tokens 1.3 to 1.75, 4 tokens 0.95 to 1.2, 6 tokens 0.84 to 0.95, 8 tokens
+// 0.62 to 0.75, 16 tokens 0.5; with a decay a head 6 tokens 1.1, 8 tokens 0.79 to 0.95; 64 x 64, 16 tokens 1.0 to 1.26,
+// 32 tokens 0.8 to 1.0, 64 tokens 0.7 to 0.9.
+inline bool tree_pays(long long T, int B, int D, bool one_decay) {
+  return D > 32 && T >= (long long)(D <= 64 ? 32 : one_decay ? 8 : 5) * B;
+}
+
 // one_decay: g is [T, H] (a decay a head), else [T, H, D].  scratch (gf_delta_chunk_words; null: token by
-// token) and max_q_len, the longest portion, are for steps with one decay a head.
+// token) is for steps with one decay a head; max_q_len: the longest portion (0: not known); singles: how many
+// requests in front have one token.
 GF_EXPORT int gf_delta_recurrence(const float* qn, const float* kn, const float* v, const float* g,
                                   const float* beta, float* state, const int* cu_seqlens,
                                   const int* slot_ids, int B, int H, int G, int D, int Vd,
                                   int state_stride, float* o, int one_decay, float* scratch,
-                                  int max_q_len, void* stream) {
+                                  int max_q_len, int T, int singles, void* stream) {
   if (B <= 0) return 0;
   if (H % G) return -3;
   const DeltaDims dm = dims_of(H, G, D, Vd, 1, state_stride, 0);
@@ -1278,57 +1291,14 @@ GF_EXPORT int gf_delta_recurrence(const float* qn, const float* kn, const float*
     GF_GO(16, 16)
 #undef GF_GO
   }
-  // few (request, head, column) triples: more lanes a column than four (see the kernels)
-  const bool wide = (long long)B * H * ((Vd + 31) / 32) < 2 * 148;
-  // (many requests of a token each are their states' bytes, which four lanes a column read in longer runs:
-  // 16 requests of 16 heads of 128 x 128 19 us against 29)
-  if (D <= 128 && (wide || (D > 32 && max_q_len != 1))) {
-    const int whole = Vd % 2 == 0 && state_stride % 2 == 0 && ((uintptr_t)state & 7) == 0;
-#define GF_TREE(DPER, LP, ONE, CHAIN)                                                                    \
-  {                                                                                                \
-    constexpr int cols = kTreeThreads / LP * 2;                                                    \
-    constexpr size_t smem = (size_t)kStages * kTreeChunk *                                         \
-                            ((ONE ? 2 : 3) * (LP * DPER + (CHAIN ? 16 : 0)) + kMaxColumnsPerBlock + 4) * \
-                            sizeof(float);                                                         \
-    const int ny = (Vd + cols - 1) / cols;                                                         \
-    if (max_q_len == 1)                                                                            \
-      return launch_kernel(delta_tree_kernel<DPER, LP, ONE, CHAIN>, dim3(B * H, ny), dim3(kTreeThreads),  \
-                           smem, st, qn, kn, v, g, beta, state, cu_seqlens, slot_ids, dm, B, 0,    \
-                           whole, o);                                                              \
-    /* the fewest requests a block with which every block has an SM of its own */                  \
-    int groups = 1;                                                                                \
-    while (groups < kTreeGroups && (long long)H * ny * ((B + groups - 1) / groups) > 148) groups *= 2; \
-    const int nz = (B + groups - 1) / groups;                                                      \
-    const size_t alone = 120 * 1024, all = smem * groups;                                          \
-    static OncePerDevice attrs;                                                                    \
-    if (int rc = attrs.run([&] {                                                                   \
-          return cudaFuncSetAttribute(delta_tree_kernel<DPER, LP, ONE, CHAIN>,                            \
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);    \
-        }))                                                                                        \
-      return rc;                                                                                   \
-    return launch_kernel_behind(delta_tree_kernel<DPER, LP, ONE, CHAIN>, dim3(nz * H, ny),                \
-                                dim3(kTreeThreads * groups),                                       \
-                                (long long)H * ny * nz <= 148 && all < alone ? alone : all, st,    \
-                                qn, kn, v, g, beta, state, cu_seqlens, slot_ids, dm, B, B > 1,     \
-                                whole, o);                                                         \
-  }
-    if (D <= 64) {
-      if (one_decay && wide) GF_TREE(8, 8, true, false)
-      if (one_decay) GF_TREE(4, 16, true, true)
-      if (wide) GF_TREE(8, 8, false, false)
-      GF_TREE(4, 16, false, true)
-    }
-    if (one_decay && wide) GF_TREE(8, 16, true, false)
-    if (one_decay) GF_TREE(8, 16, true, true)
-    if (wide) GF_TREE(8, 16, false, false)
-    GF_TREE(8, 16, false, true)
-#undef GF_TREE
-  }
-  const int lp = wide ? 32 : 4;
-  const int threads = lp == 32 ? 256 : kRecurrenceThreads;
-  const int cols = threads / lp;
-  const dim3 grid(B * H, (Vd + cols - 1) / cols);
-  const dim3 block(threads);
+  // few (request, head, column) triples: more lanes a column than four (see the kernels).  Which it is decides
+  // the order of the sums, for all requests of the step
+  const long long units = (long long)B * H * ((Vd + 31) / 32);
+  const bool wide = units < 2 * 148;
+  auto lanes = [&](int lp, int n) -> int {         // the first n requests, lp lanes a column
+    const int threads = lp == 32 ? 256 : kRecurrenceThreads;
+    const int cols = threads / lp;
+    const dim3 grid(n * H, (Vd + cols - 1) / cols), block(threads);
 #define GF_AS(DPER, LP, CHUNK, THREADS, ONE)                                                       \
   {                                                                                                \
     const size_t smem =                                                                            \
@@ -1342,15 +1312,81 @@ GF_EXPORT int gf_delta_recurrence(const float* qn, const float* kn, const float*
     if (one_decay) GF_AS(DPER, LP, CHUNK, THREADS, true)                                           \
     GF_AS(DPER, LP, CHUNK, THREADS, false)                                                         \
   }
-  GF_GO(4, 4, 8, kRecurrenceThreads)
-  GF_GO(8, 4, 8, kRecurrenceThreads)
-  GF_GO(16, 4, 8, kRecurrenceThreads)
-  GF_GO(32, 4, 8, kRecurrenceThreads)
-  GF_GO(64, 4, 4, kRecurrenceThreads)
-  GF_GO(8, 32, 4, 256)
+    GF_GO(4, 4, 8, kRecurrenceThreads)
+    GF_GO(8, 4, 8, kRecurrenceThreads)
+    GF_GO(16, 4, 8, kRecurrenceThreads)
+    GF_GO(32, 4, 8, kRecurrenceThreads)
+    GF_GO(64, 4, 4, kRecurrenceThreads)
+    GF_GO(4, 16, 8, kRecurrenceThreads)
+    GF_GO(8, 32, 4, 256)
 #undef GF_GO
 #undef GF_AS
-  return -3;
+    return -3;
+  };
+  auto tree = [&](int first) -> int {              // the requests from number `first` on
+    const int n = B - first;
+    const int *cu = cu_seqlens + first, *slots = slot_ids + first;
+    const int whole = Vd % 2 == 0 && state_stride % 2 == 0 && ((uintptr_t)state & 7) == 0;
+#define GF_TREE(DPER, LP, ONE, CHAIN)                                                              \
+  {                                                                                                \
+    constexpr int cols = kTreeThreads / LP * 2;                                                    \
+    constexpr size_t smem = (size_t)kStages * kTreeChunk *                                         \
+                            ((ONE ? 2 : 3) * (LP * DPER + (CHAIN ? 16 : 0)) + kMaxColumnsPerBlock + 4) * \
+                            sizeof(float);                                                         \
+    const int ny = (Vd + cols - 1) / cols;                                                         \
+    if (max_q_len == 1 || n == 1)                                                                  \
+      return launch_kernel(delta_tree_kernel<DPER, LP, ONE, CHAIN>, dim3(n * H, ny),               \
+                           dim3(kTreeThreads), smem, st, qn, kn, v, g, beta, state, cu, slots, dm, \
+                           n, 0, whole, o);                                                        \
+    /* the fewest requests a block with which every block has an SM of its own */                  \
+    int groups = 1;                                                                                \
+    while (groups < kTreeGroups && (long long)H * ny * ((n + groups - 1) / groups) > 148) groups *= 2; \
+    const int nz = (n + groups - 1) / groups;                                                      \
+    const size_t alone = 120 * 1024, all = smem * groups;                                          \
+    static OncePerDevice attrs;                                                                    \
+    if (int rc = attrs.run([&] {                                                                   \
+          return cudaFuncSetAttribute(delta_tree_kernel<DPER, LP, ONE, CHAIN>,                     \
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);    \
+        }))                                                                                        \
+      return rc;                                                                                   \
+    return launch_kernel_behind(delta_tree_kernel<DPER, LP, ONE, CHAIN>, dim3(nz * H, ny),         \
+                                dim3(kTreeThreads * groups),                                       \
+                                (long long)H * ny * nz <= 148 && all < alone ? alone : all, st,    \
+                                qn, kn, v, g, beta, state, cu, slots, dm, n, n <= kTreeSorted,     \
+                                whole, o);                                                         \
+  }
+    if (D <= 64) {
+      if (one_decay && wide) GF_TREE(8, 8, true, false)
+      if (one_decay) GF_TREE(4, 16, true, true)
+      if (wide) GF_TREE(8, 8, false, false)
+      GF_TREE(4, 16, false, true)
+    }
+    if (one_decay && wide) GF_TREE(8, 16, true, false)
+    if (one_decay) GF_TREE(8, 16, true, true)
+    if (wide) GF_TREE(8, 16, false, false)
+    GF_TREE(8, 16, false, true)
+#undef GF_TREE
+  };
+  if (wide) {
+    // Key sizes up to 64: sixteen lanes a column (four rows each: the tree kernel's sums) start sooner, and with few
+    // columns nothing waits for shared memory.  On a B200, us, tree kernel / sixteen lanes, 64 x 64: one request of 8
+    // heads 1.16 at 1 token, 1.23 at 17, 1.04 at 100; 64 units 1.13 (17 tokens 1.15, 100 0.95); 128 units 0.86 at 1 token, 1.04
+    // at 2, 1.06 at 15, 0.91 at 17, 0.69 at 100; 256 units 0.55 to 0.87.
+    if (D <= 64 && !(units >= 192 || (units >= 128 && (max_q_len == 1 || T >= 16ll * B)))) return lanes(16, B);
+    return D <= 128 ? tree(0) : lanes(32, B);
+  }
+  // (many requests of a token each are their states' bytes, which four lanes a column read in longer runs:
+  // 16 requests of 16 heads of 128 x 128 19 us against 29)
+  if (D > 128 || max_q_len == 1) return lanes(4, B);
+  if (tree_pays(T, B, D, one_decay)) return tree(0);
+  // a few portions behind many decoding requests: each on the kernel that it would have alone (16 heads of 128 x
+  // 128, 127 single tokens and a portion of 64: 157 us, all on four lanes 204, all on the tree kernel 330; 255 and a
+  // portion of 300: 386, 751 and 1,340)
+  if (singles > 0 && singles < B && tree_pays((long long)T - singles, B - singles, D, one_decay)) {
+    if (int rc = lanes(4, singles)) return rc;
+    return tree(singles);
+  }
+  return lanes(4, B);
 }
 
 // A plain linear attention with a decay a key channel, S <- diag(g) S + k v^T, o = S^T q, eight tokens at a

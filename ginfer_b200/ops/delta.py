@@ -121,7 +121,7 @@ def recurrence(qn, kn, v, g, beta, state: torch.Tensor, ctx) -> torch.Tensor:
     H, Vd = v.shape[1], v.shape[2]
     o = torch.empty((T, H, Vd), dtype=torch.float32, device=qn.device)
     f = _fn("delta_rule", "gf_delta_recurrence",
-            [c_void_p] * 8 + [c_int] * 6 + [c_void_p, c_int, c_void_p, c_int, c_void_p])
+            [c_void_p] * 8 + [c_int] * 6 + [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p])
     one = int(g.dim() == 2)
     scratch, longest = None, int(ctx.max_q_len if one else getattr(ctx, "max_q_len", 0))
     if one and longest == 1 and state_step(qn.view(T, G * D), kn.view(T, G * D), v.view(T, H * Vd),
@@ -130,9 +130,14 @@ def recurrence(qn, kn, v, g, beta, state: torch.Tensor, ctx) -> torch.Tensor:
     if one and longest >= CHUNKED_MIN_TOKENS:
         scratch = torch.empty(chunk_words(T, ctx.num_seqs, H, D, one), dtype=torch.float32,
                               device=qn.device)
+    # single tokens in front of portions, as the scheduler orders a mixed step
+    singles, q_lens = 0, getattr(ctx, "q_lens_host", ())
+    if longest > 1 and len(q_lens) == ctx.num_seqs:
+        while singles < len(q_lens) and q_lens[singles] == 1:
+            singles += 1
     rc = f(_p(qn), _p(kn), _p(v), _p(g), _p(beta), _p(state), _p(ctx.cu_seqlens_q),
            _p(ctx.slot_ids), ctx.num_seqs, H, G, D, Vd, state.stride(0), _p(o), one,
-           _p(scratch), longest, _stream())
+           _p(scratch), longest, T, singles, _stream())
     if rc == -3:
         raise ValueError(f"the delta-rule recurrence takes key sizes up to {MAX_KEY_SIZE}, got {D}")
     _ok(rc, "delta_recurrence")

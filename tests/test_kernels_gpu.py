@@ -1,8 +1,6 @@
 """Each kernel alone against a plain PyTorch reference of the same operation, at sizes other than
 the tiny models': widths and vocabularies that are no power of two, head sizes in steps of 16,
 odd head counts and groups, page sizes, windows, and inputs made so that a fault shows."""
-import math
-
 import pytest
 import torch
 
@@ -755,6 +753,68 @@ def test_delta_rule_of_many_portions(H, G, D, Vd, lens, one):
             assert (o[t].double() - want).abs().max() <= 2.0 ** -24 * D * 8 * S.abs().max()
         got = state[b].cpu().double().view(H, D, Vd)
         assert (got - S).abs().max() <= 2.0 ** -24 * D * 8 * S.abs().max()
+
+
+def _delta_step(H, G, D, Vd, lens, one=0):
+    from types import SimpleNamespace
+    from ginfer_b200.ops import delta
+    g0 = torch.Generator(device=DEV).manual_seed(D + Vd + sum(lens))
+    B, T = len(lens), sum(lens)
+    q, k = (torch.nn.functional.normalize(torch.randn(T, G, D, device=DEV, generator=g0), dim=-1) for _ in "qk")
+    v, beta = torch.randn(T, H, Vd, device=DEV, generator=g0), torch.rand(T, H, device=DEV, generator=g0)
+    g = torch.rand(*((T, H) if one else (T, H, D)), device=DEV, generator=g0)
+    state0 = torch.randn(B, H * D * Vd, device=DEV, generator=g0)
+
+    def step(rows=slice(None), own=lens, host=False):
+        ctx = SimpleNamespace(num_seqs=len(own), slot_ids=torch.arange(len(own)).int().to(DEV), max_q_len=max(own),
+                              cu_seqlens_q=torch.tensor([0] + list(own)).cumsum(0).int().to(DEV))
+        if host:
+            ctx.q_lens_host = list(own)
+        given = [t[rows] for t in (q, k, v, g, beta)]
+        return lambda state: delta.recurrence(*given, state, ctx)
+    return step, state0
+
+
+@pytest.mark.parametrize("H,G,D,Vd,lens", [
+    (16, 16, 128, 128, [1] * 20 + [70, 9]), (16, 8, 100, 128, [1] * 20 + [17]), (8, 4, 64, 62, [1] * 40 + [90, 33]),
+    (8, 8, 64, 64, [1] * 3 + [40, 5]), (16, 16, 64, 64, [1, 1, 30]), (16, 16, 128, 128, [1] * 30 + [3, 2]),
+    (16, 16, 64, 64, [40, 33] * 10), (16, 16, 128, 64, [5, 4] * 20), (32, 32, 64, 64, [20, 17, 16])])
+def test_delta_rule_of_single_tokens_in_front_of_portions(H, G, D, Vd, lens):
+    """Whatever kernels share a step: known lengths or not, outputs and states are the same bits, and where there are
+    many requests those of steps of one token each."""
+    step, state0 = _delta_step(H, G, D, Vd, lens)
+    states = [state0.clone() for _ in range(3)]
+    o = step()(states[0])
+    assert torch.equal(o, step(host=True)(states[1])) and torch.equal(*states[:2])
+    if min(lens) > 1 and len(lens) * H * -(-Vd // 32) >= 2 * 148:
+        at = torch.tensor([0] + lens).cumsum(0)[:-1].to(DEV)
+        for t in range(min(lens)):
+            assert torch.equal(step(at + t, [1] * len(lens))(states[2]), o[at + t])
+
+
+@pytest.mark.parametrize("H,D,Vd,B,n,one", [(16, 128, 128, 512, 5, 0), (8, 64, 64, 512, 5, 0), (16, 64, 64, 256, 3, 1)])
+def test_delta_rule_of_many_short_portions_costs_no_more_than_its_tokens_one_by_one(H, D, Vd, B, n, one):
+    """Hundreds of requests with a handful of tokens each, as one step and as steps of one token: the step reads and
+    writes the states once, so it may not take longer (with a third for what the steps do otherwise)."""
+    step, state = _delta_step(H, H, D, Vd, [n] * B, one)
+    at = torch.arange(B, device=DEV) * n
+    whole, parts = step(), [step(at + t, [1] * B) for t in range(n)]
+
+    def timed(steps):
+        times = []
+        for _ in range(7):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            torch.cuda._sleep(4000000)               # (the launches of all turns are there when the first begins)
+            a.record()
+            for _ in range(4):
+                for f in steps:
+                    f(state)
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        return sorted(times)[3]
+    assert timed([whole]) <= 1.34 * timed(parts)
 
 
 @pytest.mark.parametrize("H,G,D,Vd,lens", [(2, 1, 12, 20, [16, 1, 7]), (4, 2, 64, 64, [40, 8, 9, 3]),
