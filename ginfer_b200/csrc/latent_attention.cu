@@ -581,8 +581,11 @@ latent_attention_mma_kernel(const float* __restrict__ q_lat, const float* __rest
 // 2,251 tokens of four prompts (16 heads, 512 + 64 channels, a window of 1,024) on a B200: 417 us a layer (a block a
 // token 624; both with the table's copy), 2,000 tokens of one 665 (801).
 // A block's tile takes longer than a block a token's, so a step needs enough blocks: 182, 17 tiles the longest,
-// 225 us against 213; 250 blocks 124 against 142.
-constexpr int kRowMinBlocks = 192;
+// 225 us against 213; 250 blocks 124 against 142.  Where only the first tokens of a portion share, the other kernel runs
+// behind this one, and what it has left fills fewer rounds: a portion behind 400 keys (156 blocks here) 607 us against
+// 669, behind 650 (93) 593 against 629, 700 (81) 593 against 580, 900 (31) 592 against 524; 8 heads of 256 + 32, a window of
+// 512, 800 tokens behind 100 keys (103) 120.5 against 128.3.
+constexpr int kRowMinBlocks = 192, kRowMinSharing = 90;
 constexpr int kRowHalf = 32, kRowSlots = 3, kRowPld = kMmaTile + 8;
 
 __device__ __forceinline__ void ldsm_x4_trans(uint32_t (&r)[4], const void* p) {
@@ -917,12 +920,13 @@ GF_EXPORT int gf_latent_gather(const void* c_pages, const int* table, int table_
                        W, page, row_bytes, num_pages, vec, (unsigned char*)out, own);
 }
 
+// sharing: how many of the T tokens see their request from its first key on.
 GF_EXPORT int gf_latent_attention(const float* q_lat, const float* q_rot, const void* c_pages,
                                   const void* r_pages, const int* block_table, int table_stride,
                                   const int* seq_of_token, const int* positions, void* out, int T,
                                   int H, int C, int R, int page_size, int window, float scale,
                                   int dtype, int nsplit, float* part_o, float* part_ml,
-                                  int max_q_len, void* stream) {
+                                  int max_q_len, int sharing, void* stream) {
   if (T <= 0) return 0;
   if (C > kLatMaxC || C <= 0 || R < 0) return -3;
   const int Dk = C + R;
@@ -949,7 +953,8 @@ GF_EXPORT int gf_latent_attention(const float* q_lat, const float* q_rot, const 
       auto st = (cudaStream_t)stream;
       // steps with portions: their groups of four tokens first, then what is left
       const int rows = nsplit == 1 && max_q_len >= 4 * kRowTokens &&
-                       (long long)(T / kRowTokens) * ((H + 15) / 16) >= kRowMinBlocks && C <= 512 &&
+                       (long long)(T / kRowTokens) * ((H + 15) / 16) >= kRowMinBlocks &&
+                       (long long)(sharing / kRowTokens) * ((H + 15) / 16) >= kRowMinSharing && C <= 512 &&
                        rows_shared(Dk) <= 220 * 1024 && (uintptr_t)q_lat % 16 == 0 && (uintptr_t)q_rot % 16 == 0;
       if (rows) {
         static OncePerDevice once_rows;

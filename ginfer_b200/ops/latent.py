@@ -95,6 +95,19 @@ def key_splits(num_tokens: int, num_heads: int, max_keys: int, sms: int = 148) -
     return max(1, min(tiles // MIN_TILES_A_SPLIT, sms // blocks, MAX_SPLITS))
 
 
+def sharing_tokens(ctx, T: int, window: int, max_keys: int) -> int:
+    """How many of a step's ``T`` tokens see their request from its first key on: neighbours among them can share
+    tiles of keys.  (Where the requests' places are not known: all or none.)"""
+    if window <= 0 or max_keys <= window:
+        return T
+    if max_keys > 2 * window:                            # most windows start behind the first key
+        return 0
+    starts, lens = getattr(ctx, "q_starts_host", ()), getattr(ctx, "q_lens_host", ())
+    if not lens or len(starts) != len(lens):
+        return T
+    return sum(max(0, min(n, window - a)) for a, n in zip(starts, lens))
+
+
 def attention(q_lat: torch.Tensor, q_rot: torch.Tensor, c_pages: torch.Tensor,
               r_pages: torch.Tensor, block_table: torch.Tensor, ctx, window: int, scale: float,
               page_size: int) -> torch.Tensor:
@@ -116,17 +129,15 @@ def attention(q_lat: torch.Tensor, q_rot: torch.Tensor, c_pages: torch.Tensor,
         if nsplit > 1:
             part_o = torch.empty((nsplit, T, H, C), dtype=torch.float32, device=q_lat.device)
             part_ml = torch.empty((nsplit, T, H, 2), dtype=torch.float32, device=q_lat.device)
-    # portions whose tokens see their request from its first key on share tiles of keys (same bits); where most
-    # windows start behind it, the kernel for them would only be launched
-    longest = int(getattr(ctx, "max_q_len", 0) or 0) if window <= 0 or max_keys <= 2 * window else 0
+    shared = sharing_tokens(ctx, T, window, max_keys)
     f = _fn("latent_attention", "gf_latent_attention",
             [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
              c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p,
-             c_void_p, c_int, c_void_p], kernels=2 if nsplit > 1 else 1)
+             c_void_p, c_int, c_int, c_void_p], kernels=2 if nsplit > 1 else 1)
     rc = f(_p(q_lat), _p(q_rot), _p(c_pages), _p(r_pages), _p(block_table),
            block_table.stride(0), _p(ctx.seq_of_token), _p(ctx.positions), _p(out), T, H, C, R,
            int(page_size), int(window), float(scale), _code(c_pages.dtype), nsplit, _p(part_o),
-           _p(part_ml), longest, _stream())
+           _p(part_ml), int(getattr(ctx, "max_q_len", 0) or 0), shared, _stream())
     if rc == -3:
         raise ValueError(f"latent attention takes latent vectors of up to 1024 channels whose key "
                          f"tile fits shared memory; got kv_rank={C}, rot_dim={R}")
