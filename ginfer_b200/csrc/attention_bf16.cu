@@ -446,9 +446,12 @@ constexpr uint32_t HALF_BYTES = KT * 128;                // [64 keys][64 channel
 constexpr uint32_t TILE_BYTES = HALVES * HALF_BYTES;     // K (or V) of a stage
 constexpr uint32_t STAGE_BYTES = 2 * TILE_BYTES;
 constexpr int kMaxTableCopyTma = 2048;
-// The fewest keys a split takes: a cluster's merge costs about what two tiles do (12 query heads on a B200, 40
-// keys: 5.9 us in a cluster of 8, 4.9 in one CTA; 100 keys 6.2 and 5.4; 16 requests of 100 keys 7.7 and 6.2).
-constexpr int LEAST_KEYS = 2 * KT;
+// Requests of up to this many keys go to one CTA: a cluster's merge costs about what two tiles do.  12 query heads
+// on a B200, in a cluster of 8 / in one CTA: 40 keys 5.9 / 4.9 us, 128 keys 6.15 / 5.4, 16 requests of 100 keys 7.7 / 6.2,
+// 64 requests (clusters of 2) 8.2 / 6.7; 4 requests of 8 heads of 256 channels, 128 keys 6.9 / 6.7.  More keys keep
+// splits of one tile: two tiles a split are slower at 200 to 256, 384 and 512 keys (6.16 / 6.42, 6.67 / 6.93 with 8
+// requests) and level or 4 % faster between.
+constexpr int ONE_CTA_KEYS = 2 * KT;
 
 __device__ __forceinline__ uint32_t movmatrix_t(uint32_t v) {
   uint32_t d;
@@ -519,12 +522,13 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap kmap,
   const int lo = first_visible_key(p, window);
   const int lo_al = lo / KT * KT;                               // tiles start on tile boundaries
   const int nkeys = p - lo_al + 1;
+  if (nkeys <= ONE_CTA_KEYS) {                                  // the other splits have nothing to do
+    if (split > 0) return;
+    splits = 1;
+  }
   const int pieces = splits * parts;
   int per = (nkeys + pieces - 1) / pieces;
-  per = max((per + KT - 1) / KT * KT, LEAST_KEYS);
-  // keys that one CTA holds: it writes the result itself, the other splits have nothing to do
-  const bool one = splits == 1 || nkeys <= per;
-  if (one && split > 0) return;
+  per = (per + KT - 1) / KT * KT;
   const int begin = lo_al + (part * splits + split) * per;
   const int end = min(p + 1, begin + per);
   const int first = max(begin, lo);                             // first visible key of this split
@@ -784,21 +788,21 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap kmap,
 #pragma unroll
     for (int w = 0; w < 4; ++w) acc += cw[w * 8 + r] * so[(w * 8 + r) * SOP + d];
     float mm = -INFINITY, lsum = 0.f;
-    if (d == 0 || one) {
+    if (d == 0 || splits == 1) {
 #pragma unroll
       for (int w = 0; w < 4; ++w) {
         mm = fmaxf(mm, sm[w * 8 + r]);
         lsum += cw[w * 8 + r] * sl[w * 8 + r];
       }
     }
-    if (one && parts > 1) {
+    if (splits == 1 && parts > 1) {
       const size_t at = ((size_t)b * nh + h0 + r) * parts + part;
       po[at * HD + d] = acc;
       if (d == 0) {
         pml[at * 2] = mm;
         pml[at * 2 + 1] = lsum;
       }
-    } else if (one) {
+    } else if (splits == 1) {
       out[((size_t)row * nh + h0 + r) * HD + d] =
           __float2bfloat16_rn(lsum > 0.f ? acc / (lsum + sink_share(sink.at(h0 + r), mm)) : 0.f);
     } else {
@@ -809,7 +813,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap kmap,
       }
     }
   }
-  if (!one) {
+  if (splits > 1) {
     float* part_o = parts > 1 ? po + (((size_t)b * nh + h0) * parts + part) * HD : nullptr;
     float* part_ml = parts > 1 ? pml + (((size_t)b * nh + h0) * parts + part) * 2 : nullptr;
     cluster_sync_all();          // also orders the weights above before they are overwritten

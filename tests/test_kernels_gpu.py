@@ -1,6 +1,8 @@
 """Each kernel alone against a plain PyTorch reference of the same operation, at sizes other than
 the tiny models': widths and vocabularies that are no power of two, head sizes in steps of 16,
 odd head counts and groups, page sizes, windows, and inputs made so that a fault shows."""
+import math
+
 import pytest
 import torch
 
@@ -444,6 +446,34 @@ def test_attention_bf16_decode_of_few_keys(splits, parts, window):
                                 len(lens), nh, nkv, hd, scale, window, P, splits, parts=parts)
     gemm_bf16.check_errors()
     torch.testing.assert_close(out.double().cpu(), want, atol=1e-2, rtol=2e-2)
+
+
+@pytest.mark.parametrize("keys,splits", [(129, 8), (192, 4), (200, 4), (256, 8), (300, 8), (512, 8)])
+def test_attention_bf16_decode_gives_a_split_one_tile_while_there_are_splits(keys, splits):
+    """Above the keys that one CTA takes and up to a tile a split, the probabilities are rounded against the largest
+    score of their warp's sixteen keys, of which it has no more: the same values computed in 64 bits from such
+    groups.  (With a second tile a split a warp's probabilities follow its running maximum: about a quarter of the
+    bf16 results are then others.)"""
+    from ginfer_b200.ops import attention_bf16, gemm_bf16
+    nh, nkv, hd, P, B = 12, 2, 128, 16, 4
+    g = torch.Generator(device=DEV).manual_seed(keys)
+    n = -(-keys // P)
+    pages = torch.randn(2, B * n, P, nkv, hd, device=DEV, generator=g).bfloat16()
+    table = torch.arange(B * n, device=DEV, dtype=torch.int32).view(B, n)
+    qkv = torch.randn(B, (nh + 2 * nkv) * hd, device=DEV, generator=g).bfloat16()
+    out = attention_bf16.decode(qkv, pages, table, torch.arange(B + 1, device=DEV, dtype=torch.int32),
+                                torch.full((B,), keys - 1, device=DEV, dtype=torch.int32), B, nh, nkv, hd,
+                                hd ** -0.5, 0, P, splits).view(B, nh, hd)
+    gemm_bf16.check_errors()
+    k, v = (t.view(B, n * P, nkv, hd)[:, :keys].double().repeat_interleave(nh // nkv, 2) for t in pages)
+    s = torch.einsum("bhd,bkhd->bhk", qkv[:, :nh * hd].view(B, nh, hd).double(), k) * (hd ** -0.5 / math.log(2))
+    s = torch.nn.functional.pad(s, (0, -keys % 16), value=-math.inf).unflatten(2, (-1, 16))
+    m = s.amax(3, keepdim=True)
+    p, weight = torch.exp2(s - m), torch.exp2(m - m.amax(2, keepdim=True))
+    v = torch.nn.functional.pad(v, (0, 0, 0, 0, 0, -keys % 16)).unflatten(1, (-1, 16))
+    want = torch.einsum("bhgk,bgkhd->bhd", p.float().bfloat16().double() * weight, v) / (p * weight).sum((2, 3))[..., None]
+    # a result that another rounding of fp32 sums moves over the middle between two bf16 values: one in some hundred
+    assert (out == want.float().bfloat16()).float().mean() > 0.95
 
 
 @pytest.mark.parametrize("case", DEC_CASES)
