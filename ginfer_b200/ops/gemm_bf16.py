@@ -85,16 +85,21 @@ def split_k_for(M: int, N: int, K: int, sms: int | None = None, settled: bool = 
     if split == 1 and M <= 64 and sms // 2 < tiles <= sms and nkb >= 16:
         split = 2       # about one tile an SM (gate/up): pairs of CTAs have more under way
     elif M <= 64 and not settled:
-        # up to two CTAs an SM where a CTA's K range stays long: its K steps, not its bytes, bound it.  In a
-        # CUDA graph on a B200, 8 tokens, weights from HBM (us, splits as above / these): 8192 x 2048 9.7 / 8.4,
-        # 8448 x 2048 9.9 / 8.6, 3584 x 18944 28.7 / 25.5, 2048 x 8448 9.9 / 9.3.  Not gained: 11264 x 2048 in
-        # four 12.0 / 14.9 (more than two an SM), 4608 x 3584 in eight 9.7 / 12.4 (clusters of eight that find no
-        # place), 2048 x 8448 in twelve at 32 tokens 11.2 / 11.5.
-        if split == 2 and tiles * 4 <= 2 * sms and nkb // 4 >= 8:
+        # More CTAs than SMs where a CTA's K range stays long: its K steps, not its bytes, bound it.  The lines are
+        # those of the places: clusters of 4, 8 and 12 CTAs, two CTAs an SM, fit 71, 33 and 21 times on 148 SMs
+        # (a cluster lies inside one of the device's groups of SMs), and one more waits for a whole round.  In a
+        # CUDA graph on a B200, weights from HBM, us, splits as above / these.  Two / four, 2048 columns: 64 tiles 10.0 /
+        # 8.6 at 8 tokens, 11.6 / 10.9 at 64, 71 tiles 10.3 / 9.1 and 11.6 / 11.6, 72 tiles 10.3 / 13.0 and 11.8 / 17.6;
+        # 1024 columns at 64 tokens 8.0 / 8.3.  Four / eight: 18944 columns, 28 tiles 28.9 / 25.6 at 8 tokens, 32.6 /
+        # 30.6 at 64, 32 tiles 31.1 / 28.1 and 34.0 / 33.0, 33 tiles 31.9 / 29.0 and 34.1 / 34.3, 34 tiles 32.5 / 38.3;
+        # 12288 columns, 32 tiles 22.9 / 20.4 and 25.0 / 24.6; 8192 columns at 64 tokens 18.0 / 18.5.  Eight / twelve:
+        # 5376 columns, 16 tiles 7.8 / 7.2 at 8 tokens, 8.2 / 7.9 at 16, 9.0 / 9.4 at 32, 19 tiles 8.4 / 8.0 and 8.8 /
+        # 8.7, 21 tiles at 16 9.1 / 9.4, 22 tiles 8.9 / 12.0; 4608 columns, 19 tiles at 16 7.8 / 8.0.
+        if split == 2 and tiles * 148 <= 71 * sms and nkb // 4 >= 8:
             split = 4
-        elif split == 4 and tiles * 8 * 5 <= 8 * sms and nkb // 8 >= 24:
+        elif split == 4 and tiles * 148 <= 32 * sms and nkb // 8 >= 24:
             split = 8
-        elif split == 8 and M <= 16 and tiles * 12 * 10 <= 13 * sms and nkb // 12 >= 7:
+        elif split == 8 and M <= 16 and tiles * 148 <= 19 * sms and nkb // 12 >= 7:
             split = 12
     return split
 
