@@ -188,7 +188,7 @@ template <int BM, int VEC> constexpr size_t tile_shared() {
 }
 
 template <int BM, int VEC>
-__global__ void __launch_bounds__(BM * 2, BM == 128 ? 1 : BM == 64 ? 2 : 3)
+__global__ void __launch_bounds__(BM * 2, BM == 64 ? 2 : 3)
 gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W,
                      const float* __restrict__ bias, float* __restrict__ C, int M, int N, int K,
                      int lda, int ldc, int seg, int ranks) {
@@ -265,7 +265,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W,
     }
   };
   const int most = min(8, (M - m0 + TY - 1) / TY);
-  if (most > 6) products(std::integral_constant<int, 8>{});
+  if (BM > 32 && most > 6) products(std::integral_constant<int, 8>{});     // (24 rows at most in tiles of 32)
   else if (most == 6) products(std::integral_constant<int, 6>{});
   else if (most == 5) products(std::integral_constant<int, 5>{});
   else if (most > 2) products(std::integral_constant<int, 4>{});
@@ -333,7 +333,10 @@ template <int VEC> int start_by_rows(const F32Args& a) {
   if (a.M <= 4) return start_rows<4, VEC>(a);
   if (a.M <= 8) return start_rows<8, VEC>(a);
   if (a.M <= 16) return start_rows<16, VEC>(a);
-  return a.M <= 32 ? start_tile<32, VEC>(a) : start_tile<64, VEC>(a);
+  // 25 rows and more leave half of the rows of a tile of 64 out and still gain: its stages are longer and its blocks have
+  // four warps.  28 rows, tiles of 32 / 64 (20 rows): 8192 x 2048 54.7 / 37.4 us (40.0 / 37.1), 1536 x 8960 72.9 / 53.9 (51.4 /
+  // 53.8), 2048 x 1536 18.2 / 16.4 (14.6 / 16.4), 37888 x 3584 244 / 220 (173 / 216), 17920 x 1536 58.0 / 59.3 (43.3 / 59.1).
+  return a.M <= 24 ? start_tile<32, VEC>(a) : start_tile<64, VEC>(a);
 }
 
 }  // namespace gf

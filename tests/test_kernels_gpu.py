@@ -165,6 +165,12 @@ def test_gemm_f32_multiplies_the_rows_that_are_there(M, N, K):
     assert ((got.double() - x.double() @ w.double().t()).abs() <= bound).all()
 
 
+@pytest.mark.parametrize("M", [17, 24, 26, 32, 33])
+@pytest.mark.parametrize("N,K", [(130, 100), (1536, 264), (257, 77)])
+def test_gemm_f32_around_the_rows_where_its_tiles_change(M, N, K):
+    test_gemm_f32_multiplies_the_rows_that_are_there(M, N, K)
+
+
 @pytest.mark.parametrize("M", [2, 20])
 def test_gemm_f32_of_more_than_two_million_columns(M):
     """More tiles of columns than a grid's shorter sides hold."""
