@@ -966,7 +966,9 @@ moe_gemv_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfloat1
               ((__nv_bfloat16*)out_)[s * (N / 2) + n / 2] =
                   from_f32<__nv_bfloat16>(clamped_glu(gt, up, limit, alpha, up_shift));
             } else {
-              *reinterpret_cast<float2*>((float*)out_ + s * N + n) = make_float2(acc0[r], acc1[r]);
+              float* to = (float*)out_ + s * N + n;                // (aligned to four bytes is enough)
+              to[0] = acc0[r];
+              to[1] = acc1[r];
             }
           }
         }

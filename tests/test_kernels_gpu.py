@@ -652,6 +652,20 @@ def test_products_of_a_handful_of_pairs(K, N, counts):
         assert torch.equal(moe.grouped_glu(x[p:p + 1], up, one, 1e9, 1.0, 0.0)[0], glu[p])
 
 
+def test_products_of_a_handful_of_pairs_take_any_fp32_result():
+    """A result that starts at an odd multiple of four bytes: its values, and nothing beside it."""
+    from ginfer_b200.ops import moe
+    g = torch.Generator(device=DEV).manual_seed(2)
+    x = torch.randn(5, 264, generator=g, device=DEV).bfloat16()
+    w = torch.randn(3, 38, 264, generator=g, device=DEV).bfloat16()
+    plan = moe.Plan(torch.tensor([[0], [2], [0], [1], [2]], dtype=torch.int32, device=DEV), 3, "gemv")
+    place = torch.full((5 * 38 + 2,), 7.0, device=DEV)
+    assert place.data_ptr() % 8 == 0
+    moe._gemm(x, w, plan, place[1:-1].view(5, 38), 0, 0.0, 0.0, 0.0)
+    assert torch.equal(place[1:-1].view(5, 38), moe.grouped_down(x, w, plan))
+    assert place[0] == 7 and place[-1] == 7
+
+
 @pytest.mark.parametrize("E,K,N,counts", [
     (24, 2048, 1026, [1] * 24), (32, 1096, 2050, [0] * 20 + [17, 1, 2, 8, 9, 16, 0, 0, 0, 0, 0, 27]),
     (40, 2120, 1056, [2, 0] * 20), (30, 520, 4034, [3] * 10 + [1] * 20)])
