@@ -13,6 +13,7 @@
 //                       the sorted order, each pair's place, and the list of row tiles (expert,
 //                       first row) that the grouped products walk over.
 //   moe_stream_kernel   the grouped products of decode steps: an expert's weights streamed once (see there).
+//   moe_ring_kernel     those of one to two and a half pairs an expert, where that grid takes more than a round.
 //   moe_gemv_kernel     those of a handful of pairs for layers that stay off it (see there).
 //   moe_gemm_mma_kernel those of more pairs, in tiles of 64 rows (see there).
 //   moe_gemm_kernel     (32-bit path, and sizes the other refuses) grouped product over the sorted pairs, a block a (row tile, column tile):
@@ -25,6 +26,7 @@
 //                       not depend on the batch.
 //   moe_combine_kernel  out[t] = sum over the token's choices, in the order chosen, of weight *
 //                       the pair's row.
+#include <cmath>
 #include <type_traits>
 
 #include "common.cuh"
@@ -518,7 +520,8 @@ moe_gemm_mma_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfl
 // A warp owns 16 weight rows; `parts` warps (1, 2, 4 or 8 of the block's eight) split its reduction
 // where the rows alone give too few warps.  `parts` is the order of a pair's sums, so it follows from the
 // matrices and from a step's range (up to 20 pairs, up to 16 an expert, more), not from its pairs'
-// number: within a range a pair's result does not depend on the batch.  Against `parts` from the number
+// number: within a range a pair's result does not depend on the batch.  (Steps that ring_serves() takes, from a number
+// of pairs on that follows from the matrices up to two and a half an expert, are a range of their own.)  Against `parts` from the number
 // itself (both products, weights from HBM, us): 32 experts of 2048 x 2112, 8 pairs 69.6 -> 63.6, 20 pairs 107
 // -> 109; 8 of 2048 x 1408, 24 pairs 45 -> 49, 64 pairs 61.5 -> 57.4; elsewhere within 3 %, or faster.  Lane group g has weight rows 2 g and 2 g + 1: a gate and
 // its up value meet in one lane.
@@ -663,22 +666,38 @@ moe_stream_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfloa
 // the matrix alone.  A warp's steps come through a ring of its own in shared memory, each lane with its own
 // 16-byte copies (nobody else reads them: no barrier), which runs on across items and tiles; after every two
 // items the warps' sums meet, two warps add them up in order and store.
-// For steps of one to two and a half pairs an expert.  Whole batches on a B200 (ms, the grid above / here), 32 experts
-// of 2048 x 2112, 4 choices: 9 requests 35.7 / 30.8, 16 requests 42.5 / 34.2, 32 requests 29.18 / 29.16, 64 requests
-// 24.4 / 24.9; 29 of 2048 x 1408, 5 choices: 8 requests 28.5 / 27.9, 30 requests 26.5 / 27.3.  Both products alone,
-// weights from HBM: 64 pairs of the first 91.9 / 87.1 us (floor 69.7), 24 pairs 52.9 / 59.8; of 8 experts of 2048 x
-// 1408, 48 pairs, 37.2 / 40.8: with few tiles of pairs the start of a run (the tile's rows, the first steps) is too
-// much of it, with many their rows are.
+// Whole batches on a B200 (ms, the grid above / here), 32 experts of 2048 x 2112, 4 choices: 9 requests 35.7 / 30.8,
+// 16 requests 42.5 / 34.2, 32 requests 29.18 / 29.16, 64 requests 24.4 / 24.9; 29 of 2048 x 1408, 5 choices: 8
+// requests 28.5 / 27.9, 30 requests 26.5 / 27.3.  See ring_serves() for the line.
 constexpr int kRgWarps = 16, kRgRing = 3, kRgItems = 2;
 constexpr int kRgSlot = 2048;                                // a step: 16 rows x 64 k
 constexpr int kRgHead = 128;                                 // the rows' weights
 constexpr int kRgSums = kRgItems * kRgWarps * 2 * 32 * 16;
 constexpr int kRgMaxShared = 227 * 1024;
-// From this many bytes of weights an expert and experts: 16 of 1024 x 704, 8 pairs, take 12.5 us above and 16.4 here.
+constexpr int kRgMinExperts = 16, kRgMinK = 1280;
 constexpr size_t kRgMinBytes = 4 << 20;
-constexpr int kRgMinExperts = 24;
 __host__ __device__ inline size_t ring_shared(int K) {
   return kRgHead + (size_t)kRgWarps * kRgRing * kRgSlot + kRgSums + kStRows * stream_pitch(K);
+}
+// Steps of one to two and a half pairs an expert, where the grid above would come to more than one round of blocks:
+// a grid that fits at once has nothing to gain, and the second round costs what a full one does.  The
+// grid's blocks follow from the experts that P pairs reach of E, about E (1 - (1 - 1 / E)^P); at 0.95 rounds nearly as
+// many steps have an expert more as have one less, and the second round costs more than the ring.  In us a product on a
+// B200, weights from HBM, grid / ring, by rounds: 2112 x 2048, 24 experts, 24 pairs (0.88) 27.8 / 29.9, 28 pairs (0.96,
+// one expert more than that reached) 41.6 / 34.4, 36 pairs (1.08) 41.8 / 34.0, 32 experts, 64 pairs (1.60) 48.1 / 45.9, 80 (1.70)
+// 50.2 / 49.2; 64 experts, 96 pairs (2.9) 76.7 / 72.6; 2816 x 2048, 32 experts, 48 pairs (1.86) 50.4 / 51.6; 1280 x 2048, 32
+// experts, 40 pairs (0.78) 25.7 / 29.0, 80 pairs (1.00) 43.1 / 35.5; 1536 x 2048 28.3 / 30.3 (0.93), 44.9 / 38.2 (1.2); 2048 x
+// 1408, 32 experts, 32 pairs (1.1) 29.6 / 25.6, 80 (1.6) 34.4 / 35.4; 2048 x 3072 (a block an SM), 24 experts, 28 pairs 89 /
+// 45.  A shorter reduction leaves warps without a step in an item: 4096 x 512, 24 experts, 28 pairs (1.8) 15.3 / 18.7, 3072 x 1024
+// (1.4) 25.7 / 28.3.  Fewer experts: 16 of 2816 x 2048, 24 pairs 41.9 / 34.7; 8, 16 pairs (1.05) 18.9 / 20.9, 20 pairs 26.2 /
+// 23.5.  Small matrices: 1536 x 1024, 24 experts, 60 pairs 18.6 / 22.7.
+inline bool ring_serves(int pairs, int experts, int N, int K, int span, size_t grid_shared, int sms) {
+  if (experts < kRgMinExperts || pairs <= kStHandful || pairs < experts || 2 * pairs > 5 * experts || K < kRgMinK ||
+      (size_t)N * K * sizeof(__nv_bfloat16) < kRgMinBytes || ring_shared(K) > kRgMaxShared)
+    return false;
+  const double reached = experts * (1.0 - pow(1.0 - 1.0 / experts, pairs));
+  const int places = sms * (2 * (grid_shared + 9 * 1024) < 204 * 1024 ? 2 : 1);   // (2,816 columns are the last with two)
+  return reached * ((N + span - 1) / span) >= 0.95 * places;
 }
 __device__ __forceinline__ void ring_copy(uint32_t dst, const void* src, bool there) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(there ? 16 : 0) : "memory");
@@ -1141,10 +1160,16 @@ GF_EXPORT int gf_moe_gemm(const void* a, int lda, const void* w, int N, int K, c
     if (dtype != GF_BF16 || K % 8 || lda % 8 || N % 2 || (uintptr_t)a % 16 || (uintptr_t)w % 16 ||
         (uintptr_t)out % 8 || smem > kStMaxShared)
       return -3;
-    if (experts >= kRgMinExperts && pairs >= experts && 2 * pairs <= 5 * experts &&
-        (size_t)N * K * sizeof(bf) >= kRgMinBytes && ring_shared(K) <= kRgMaxShared) {
-      int sms = 0;
-      if (int rc = sm_count(&sms)) return rc;
+    // about 16 warps an SM should be busy
+    const int each = pairs <= kStRows * experts ? 2 : 4;       // tiles an expert
+    const int most = pairs <= kStHandful ? kStHandfulTiles : kStTiles;
+    const int busy = most < each * experts ? most : each * experts;
+    int parts = 1;
+    while (parts < kStWarps && (long long)busy * (N / 16 + 1) * parts < 16 * 148 && K >= parts * 256) parts *= 2;
+    const int span = 16 * (kStWarps / parts);
+    int sms = 0;
+    if (int rc = sm_count(&sms)) return rc;
+    if (ring_serves(pairs, experts, N, K, span, smem, sms)) {
 #define GF_RING(MODE)                                                                             \
   {                                                                                               \
     static OncePerDevice attrs;                                                                   \
@@ -1162,13 +1187,6 @@ GF_EXPORT int gf_moe_gemm(const void* a, int lda, const void* w, int N, int K, c
       GF_RING(0)
 #undef GF_RING
     }
-    // about 16 warps an SM should be busy
-    const int each = pairs <= kStRows * experts ? 2 : 4;       // tiles an expert
-    const int most = pairs <= kStHandful ? kStHandfulTiles : kStTiles;
-    const int busy = most < each * experts ? most : each * experts;
-    int parts = 1;
-    while (parts < kStWarps && (long long)busy * (N / 16 + 1) * parts < 16 * 148 && K >= parts * 256) parts *= 2;
-    const int span = 16 * (kStWarps / parts);
     const dim3 sgrid(max_tiles, (N + span - 1) / span), sblock(kStWarps * 32);
 #define GF_ST(MODE)                                                                               \
   {                                                                                               \

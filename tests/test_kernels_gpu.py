@@ -706,6 +706,15 @@ def test_routed_products_of_one_or_two_pairs_an_expert(E, K, N, counts):
         assert torch.equal(a[some], b)
 
 
+@pytest.mark.parametrize("E,K,N,counts", [
+    (24, 1288, 2050, [3] * 12 + [2] * 12), (32, 2056, 2114, [0] * 20 + [17, 1, 2, 8, 9, 16, 0, 0, 0, 0, 0, 27]),
+    (16, 1288, 4098, [1] * 16), (64, 1280, 1642, [1, 2] * 32)])
+def test_routed_products_whose_grid_takes_more_than_a_round(E, K, N, counts):
+    """The same where blocks of (tile, weight rows) would come to more than fit at once: that is where equal runs
+    of items serve."""
+    test_routed_products_of_one_or_two_pairs_an_expert(E, K, N, counts)
+
+
 @pytest.mark.parametrize("K,F,E,top", [(2048, 1408, 32, 4), (1024, 704, 16, 2), (256, 96, 8, 1)])
 @pytest.mark.parametrize("counts", [(1, 2, 3, 5), (24, 25, 40, 100)])
 def test_a_pairs_result_does_not_depend_on_the_batch(K, F, E, top, counts):
