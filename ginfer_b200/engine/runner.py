@@ -33,15 +33,20 @@ def _align4(n: int) -> int:
 
 GRAPH_WIDTH_STEP = 64        # block-table widths of graph-replayed steps, in pages
 # Steps with prompt portions are replayed from a graph when the same shape (portion lengths, table
-# width, wanted rows) comes again: whole-budget portions of long prompts do, and prompts of a few
+# width, wanted rows) comes again: whole-budget portions of long prompts do, and whole prompts of a few
 # tokens.  Only steps of at most this many requests, and this many graphs at most of steps up to
 # PORTION_GRAPH_SHORT tokens and as many of longer ones.  A short step's host work is most of its time (28
 # layers, a prompt of 17 tokens on a B200: 4.4 ms of launches for 1.4 ms of kernels), but a capture
 # costs two eager steps' launches, and lengths seldom repeat as portions do: it is captured when it
-# comes a fourth time, a long one the second time.
+# comes a fourth time, a long one the second time.  Short steps are whole prompts only (a decoding request
+# beside them makes a shape that passes with its next page, and one whose kernels an eager step may choose by the
+# exact number of keys), with few wanted rows (their logits stay with the graph: 5 MB for
+# 152k words), and the graph that was replayed longest ago gives its place to a new shape.
 PORTION_GRAPH_MAX_SEQS = 4
 PORTION_GRAPH_SHORT = 255
+PORTION_GRAPH_SHORT_ROWS = 8
 PORTION_GRAPH_LIMIT = 16
+PORTION_GRAPH_SHAPES = 1024      # shapes of short steps whose comings are counted
 
 
 @dataclass
@@ -80,7 +85,8 @@ class ModelRunner:
         self._host = None            # pinned staging for the step's integers
         self._host_cap = 0
         self._graphs: dict = {}
-        self._portion_seen: dict = {}     # shapes of steps with prompt portions -> times seen
+        self._portion_seen: dict = {}     # shapes of steps with long prompt portions -> times seen
+        self._short_seen: dict = {}       # of short steps, the one seen last at the end
         self._graph_pool = None
         self._copied = torch.cuda.Event()     # the last copy out of the staging buffer
         self._copy_pending = False
@@ -205,8 +211,7 @@ class ModelRunner:
             # in steps of GRAPH_WIDTH_STEP pages so that few graphs are needed.  Steps with
             # portions take the next power of two of such steps (the portions of one long prompt
             # then share a handful of graphs; nothing in such a step is chosen by the width, while
-            # a decode step splits its keys by it, and so may a short step with portions, which
-            # keeps its own width).
+            # a decode step splits its keys by it).  Short steps keep their own width.
             steps = -(-width // GRAPH_WIDTH_STEP)
             if not decode_only:
                 steps = 1 << (steps - 1).bit_length()
@@ -383,16 +388,35 @@ class ModelRunner:
         if facts["B"] > PORTION_GRAPH_MAX_SEQS:
             return None
         short = facts["T"] <= PORTION_GRAPH_SHORT
+        if short and (facts["q_starts"].any()
+                      or sum(len(e.want) for e in entries) > PORTION_GRAPH_SHORT_ROWS):
+            return None
         key = ("short" if short else "portions", tuple(int(n) for n in facts["q_lens"]), facts["width"],
                tuple(tuple(int(w) for w in e.want) for e in entries))
         if key in self._graphs:
+            if short:                             # the one replayed last stands last
+                self._graphs[key] = self._graphs.pop(key)
             return key
+        if short:
+            seen = self._short_seen[key] = self._short_seen.pop(key, 0) + 1
+            if len(self._short_seen) > PORTION_GRAPH_SHAPES:
+                del self._short_seen[next(iter(self._short_seen))]
+            return key if seen >= 4 else None
         seen = self._portion_seen.get(key, 0) + 1
         if len(self._portion_seen) > 4096:
             self._portion_seen.clear()
         self._portion_seen[key] = seen
-        graphs = sum(1 for k in self._graphs if k[0] == key[0])
-        return key if seen >= (4 if short else 2) and graphs < PORTION_GRAPH_LIMIT else None
+        graphs = sum(1 for k in self._graphs if k[0] == "portions")
+        return key if seen >= 2 and graphs < PORTION_GRAPH_LIMIT else None
+
+    def _make_room(self, key) -> None:
+        """Before the short step ``key`` is captured: the short graph replayed longest ago is given up where
+        there are as many as there may be.  (Its shape has to come four times again.)"""
+        self._short_seen.pop(key, None)
+        short = [k for k in self._graphs if k[0] == "short"]
+        if len(short) >= PORTION_GRAPH_LIMIT:
+            torch.cuda.synchronize(self.device)   # (a replay of it may be under way)
+            del self._graphs[short[0]]
 
     def _capture(self, key, arrays, facts) -> _StepGraph:
         from .. import ops
@@ -400,8 +424,10 @@ class ModelRunner:
         ints = torch.empty(total, dtype=torch.int32, device=self.device)
         dev = self.upload(arrays, into=ints)
         ctx = self.make_context(dev, facts)
-        # what the kernels may assume about lengths is the bucket's bound, not this step's
-        ctx.max_kv_len = min(facts["width"] * self.page_size, self.max_seq_len)
+        # what the kernels may assume about lengths is the bucket's bound, not this step's (a short step's
+        # lengths are its shape's)
+        if key[0] != "short":
+            ctx.max_kv_len = min(facts["width"] * self.page_size, self.max_seq_len)
         ctx.capturing = True
         bind = self.binder(dev)
         # once eagerly: libraries, handles, attributes.  Pages take the same values again when the
@@ -450,6 +476,8 @@ class ModelRunner:
                     padded, pfacts = self._pad_decode(arrays, facts, key[0])
                 g = self._graphs.get(key)
                 if g is None:
+                    if key[0] == "short":
+                        self._make_room(key)
                     g = self._graphs[key] = self._capture(key, padded, pfacts)
                 dev = self.upload(padded, into=g.ints)
                 self._feed_back(dev, feedback)

@@ -195,3 +195,36 @@ def test_decoding_few_requests_with_thousands_of_keys_agrees_with_plain(tmp_path
                          max_num_batched_tokens=8192, enforce_eager=False)
     rows = replay.run_in_process(runner, steps)
     replay.compare(rows, replay.plain_logits(d, reqs, "bfloat16"), "bfloat16", reqs)
+
+
+def test_short_steps_beside_a_request_of_thousands_of_keys_keep_their_bits(tmp_path):
+    """A request that decodes at 4,080 to 4,100 keys, a prompt of 17 tokens beside it in every step: the number
+    of clusters that share the long request's keys changes at 4,096, and a runner that replays graphs gives the
+    rows of an eager one bit for bit, also for prompts alone, whose shape is captured."""
+    from ginfer_b200.engine import ModelRunner, StepEntry
+    from ginfer_b200.engine.loading import load_model
+    from ginfer_b200.ops import attention_bf16
+    cfg = {"architectures": ["Qwen2ForCausalLM"], "model_type": "qwen2", "num_hidden_layers": 2,
+           "vocab_size": 300, "rope_theta": 1e6, "rms_norm_eps": 1e-6, "hidden_size": 128,
+           "num_attention_heads": 2, "num_key_value_heads": 1, "head_dim": 64,
+           "intermediate_size": 256, "max_position_embeddings": 8192,
+           "tie_word_embeddings": False, "use_sliding_window": False, "torch_dtype": "bfloat16"}
+    d = make_folder(tmp_path, "mixed_context", seed=4, storage="bfloat16", config=cfg)
+    assert attention_bf16.decode_partition(1, 2, 1, 4090) != attention_bf16.decode_partition(1, 2, 1, 4096)
+    far, near = prompt(4100, 300, seed=11), prompt(17 * 20, 300, seed=12)
+    rows = []
+    for eager in (True, False):
+        model, _ = load_model(d, "bfloat16")
+        runner = ModelRunner(model, page_size=16, max_num_seqs=3, max_seq_len=4800, num_pages=320,
+                             max_num_batched_tokens=8192, enforce_eager=eager)
+        mine = [runner.step([StepEntry("far", far[:4080], [4079])]).cpu()]
+        for k in range(20):
+            short = near[17 * k:17 * k + 17]
+            mine.append(runner.step([StepEntry("far", [far[4080 + k]], [0]),
+                                     StepEntry(f"a{k}", short, [16])]).cpu())
+            mine.append(runner.step([StepEntry(f"b{k}", short, [16])]).cpu())
+            runner.end(f"a{k}"), runner.end(f"b{k}")
+        rows.append(mine)
+    assert [k[1] for k in runner._graphs if k[0] == "short"] == [(17,)]
+    for i, (a, b) in enumerate(zip(*rows)):
+        assert torch.equal(a, b), i
