@@ -15,9 +15,10 @@
 //                             times v, and the part of the state the chunk starts from.
 // The products are bound by shared-memory reads (a thread's 4 x 4 multiply-adds take two 16-byte reads), and were
 // as long again by the slabs' loads, which nothing hid: a slab is now asked for while the one before is multiplied.
-// On a B200, all three kernels, two prompts of 1,500 and 1,700 tokens, 64 heads of 128 x 64 with one q and k: 426 us
-// a layer (581 with every head's own scores and nothing under way); 16 heads of 128 x 128, 32 prompts of 115
-// tokens 362 (404), one of 2,048 135 (144).
+// What the kernels ahead wrote is read past L1 (see fresh() in common.cuh): q and k a sector of eight channels a pair of
+// lanes, a chunk's gains once a warp.  On a B200, all kernels, two prompts of 1,500 and 1,700 tokens, 64 heads of 128
+// x 64 with one q and k: 390 us a layer (572 with every head's own scores and nothing under way; 419 with scores once, slabs ahead
+// and plain reads); 16 heads of 128 x 128, 32 prompts of 115 tokens 296 (397; 356), one of 2,048 129 (137; 127).
 //
 // Ratios of decays are products of the factors between two tokens, never quotients, so a decay of zero or
 // one loses nothing.  All products are fp32 multiply-adds: the state and what enters it are 32-bit.
@@ -29,6 +30,9 @@ constexpr int kC = 64;             // tokens a chunk
 constexpr int kSlab = 32;          // rows of S, channels of K a stage
 constexpr int kThreads = 256;      // 16 x 16, a thread 4 rows x 4 NV columns
 constexpr int kMaxSeqs = 1024;
+
+// What the kernels shortly ahead wrote, four at once (see fresh() in common.cuh).
+__device__ __forceinline__ float4 fresh4(const float* p) { return __ldcg(reinterpret_cast<const float4*>(p)); }
 
 struct ChunkDims {
   int H, G, D, Vd, B;
@@ -117,14 +121,14 @@ decay_chunk_state_kernel(const float* __restrict__ k, const float* __restrict__ 
   if (threadIdx.x < kC) {
     const bool in = threadIdx.x < at.len;
     const size_t r = (size_t)(at.row0 + threadIdx.x);
-    gs[threadIdx.x] = in ? g[r * dm.ld_g + h] : 1.f;
-    rs[threadIdx.x] = in ? (c ? c[r * dm.ld_c + h] : 1.f) : 0.f;
+    gs[threadIdx.x] = in ? fresh(g + r * dm.ld_g + h) : 1.f;
+    rs[threadIdx.x] = in ? (c ? fresh(c + r * dm.ld_c + h) : 1.f) : 0.f;
   }
   for (int i = threadIdx.x; i < kC * BV / 4; i += kThreads) {
     const int j = i / (BV / 4), col = (i - j * (BV / 4)) * 4;
     float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
     if (j < at.len && v0 + col < dm.Vd)
-      x = *reinterpret_cast<const float4*>(v + (size_t)(at.row0 + j) * dm.ld_v + (size_t)h * dm.Vd + v0 + col);
+      x = fresh4(v + (size_t)(at.row0 + j) * dm.ld_v + (size_t)h * dm.Vd + v0 + col);
     *reinterpret_cast<float4*>(vs + j * BV + col) = x;
   }
   __syncthreads();
@@ -142,7 +146,7 @@ decay_chunk_state_kernel(const float* __restrict__ k, const float* __restrict__ 
     const int j = i >> 4, d = (i & 15) * 4;
     float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
     if (j < at.len && d0 + d < dm.D) {
-      x = *reinterpret_cast<const float4*>(k + (size_t)(at.row0 + j) * dm.ld_k + (size_t)gk * dm.D + d0 + d);
+      x = fresh4(k + (size_t)(at.row0 + j) * dm.ld_k + (size_t)gk * dm.D + d0 + d);
       const float r = rs[j];
       x.x *= r, x.y *= r, x.z *= r, x.w *= r;
     }
@@ -182,7 +186,8 @@ decay_chunk_scan_kernel(float* __restrict__ parts, float* __restrict__ nparts,
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   pdl_trigger();
   pdl_wait();
-  if (e >= quads + nq) return;
+  const bool in = e < quads + nq;          // (a warp's lanes ask for gains together)
+  const int lane = threadIdx.x & 31;
   int first = 0;
   for (int i = 0; i < b; ++i) first += (cu_seqlens[i + 1] - cu_seqlens[i] + kC - 1) / kC;
   const int count = (cu_seqlens[b + 1] - cu_seqlens[b] + kC - 1) / kC;
@@ -192,26 +197,32 @@ decay_chunk_scan_kernel(float* __restrict__ parts, float* __restrict__ nparts,
   float4* p = reinterpret_cast<float4*>(isn ? nparts : parts) + ((size_t)first * dm.H + h) * size + el;
   float* slot = state + (size_t)slot_ids[b] * dm.state_stride +
                 (isn ? (size_t)dm.norm_off + (size_t)h * dm.D : (size_t)h * dm.D * dm.Vd) + 4 * el;
-  float s[4] = {slot[0], slot[1], slot[2], slot[3]};                // (a slot need not be 16-byte aligned)
+  float s[4] = {};
+  if (in)                                                           // (a slot need not be 16-byte aligned)
+    s[0] = fresh(slot), s[1] = fresh(slot + 1), s[2] = fresh(slot + 2), s[3] = fresh(slot + 3);
   const float* gain = gains + (size_t)first * dm.H + h;
   const size_t step = (size_t)dm.H * size;
   constexpr int U = 8;                                              // chunks whose loads go out together
   for (int c0 = 0; c0 < count; c0 += U) {
     float4 u[U];
-    float gn[U];
+    float gl = 0.f;
+    if (lane < U && c0 + lane < count) gl = fresh(gain + (size_t)(c0 + lane) * dm.H);
 #pragma unroll
     for (int i = 0; i < U; ++i)
-      if (c0 + i < count) u[i] = p[(c0 + i) * step], gn[i] = gain[(size_t)(c0 + i) * dm.H];
+      if (in && c0 + i < count) u[i] = __ldcg(p + (c0 + i) * step);
 #pragma unroll
-    for (int i = 0; i < U; ++i)
-      if (c0 + i < count) {
+    for (int i = 0; i < U; ++i) {
+      const float gn = __shfl_sync(0xffffffffu, gl, i);
+      if (in && c0 + i < count) {
         p[(c0 + i) * step] = make_float4(s[0], s[1], s[2], s[3]);
-        s[0] = fmaf(gn[i], s[0], u[i].x);
-        s[1] = fmaf(gn[i], s[1], u[i].y);
-        s[2] = fmaf(gn[i], s[2], u[i].z);
-        s[3] = fmaf(gn[i], s[3], u[i].w);
+        s[0] = fmaf(gn, s[0], u[i].x);
+        s[1] = fmaf(gn, s[1], u[i].y);
+        s[2] = fmaf(gn, s[2], u[i].z);
+        s[3] = fmaf(gn, s[3], u[i].w);
       }
+    }
   }
+  if (!in) return;
 #pragma unroll
   for (int i = 0; i < 4; ++i) slot[i] = s[i];
 }
@@ -223,26 +234,28 @@ __host__ __device__ constexpr int out_floats(int D, int BV) {
   return padded_keys(D) * kC + kC * (kC + 1) + kC * kC + kC * BV;
 }
 
-// Rows of q or k of a chunk, transposed: channels d0 .. of the tokens into [channel][kC].  A thread has a token
-// and every fourth quad of channels; ask() brings a slab into registers, put() into shared memory.
+// Rows of q or k of a chunk, transposed: channels d0 .. of the tokens into [channel][kC].  Two neighbouring lanes
+// have a token's eight neighbouring channels (a sector of 32 bytes: nothing is read twice past L1); ask() brings
+// a slab into registers, put() into shared memory.
 struct ChunkRows {
   const float* src;                        // of the first token and key head
-  int ld, D, len, token, quad;
+  int ld, D, len, token, chan;
   __device__ __forceinline__ ChunkRows(const float* base, int ld_, int D_, int gk, const ChunkPlace& at)
       : src(base + (size_t)at.row0 * ld_ + (size_t)gk * D_), ld(ld_), D(D_), len(at.len),
-        token(threadIdx.x & (kC - 1)), quad(threadIdx.x >> 6) {}
+        token((threadIdx.x >> 1 & 15) + (threadIdx.x >> 5 & 3) * 16),
+        chan(4 * (threadIdx.x & 1) + 8 * (threadIdx.x >> 7)) {}
   __device__ __forceinline__ void ask(float4 (&x)[kSlab / 16], int d0) const {
 #pragma unroll
     for (int i = 0; i < kSlab / 16; ++i) {
-      const int d = d0 + 16 * i + 4 * quad;
+      const int d = d0 + 16 * i + chan;
       x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (token < len && d < D) x[i] = *reinterpret_cast<const float4*>(src + (size_t)token * ld + d);
+      if (token < len && d < D) x[i] = fresh4(src + (size_t)token * ld + d);
     }
   }
   __device__ __forceinline__ void put(float* dst, const float4 (&x)[kSlab / 16]) const {
 #pragma unroll
     for (int i = 0; i < kSlab / 16; ++i) {
-      float* to = dst + (16 * i + 4 * quad) * kC + token;
+      float* to = dst + (16 * i + chan) * kC + token;
       to[0] = x[i].x, to[kC] = x[i].y, to[2 * kC] = x[i].z, to[3 * kC] = x[i].w;
     }
   }
@@ -322,8 +335,8 @@ decay_chunk_out_kernel(const float* __restrict__ q, const float* __restrict__ k,
   if (threadIdx.x < kC) {
     const bool in = threadIdx.x < at.len;
     const size_t r = (size_t)(at.row0 + threadIdx.x);
-    gs[threadIdx.x] = in ? g[r * dm.ld_g + h] : 0.f;
-    cs[threadIdx.x] = in ? (c ? c[r * dm.ld_c + h] : 1.f) : 0.f;
+    gs[threadIdx.x] = in ? fresh(g + r * dm.ld_g + h) : 0.f;
+    cs[threadIdx.x] = in ? (c ? fresh(c + r * dm.ld_c + h) : 1.f) : 0.f;
   }
   chunk_queries(qt, ChunkRows(q, dm.ld_q, D, gk, at), Dp);
   __syncthreads();
@@ -346,7 +359,7 @@ decay_chunk_out_kernel(const float* __restrict__ q, const float* __restrict__ k,
     const float* from = scores + ((size_t)chunk * dm.G + gk) * kC * kC;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const float4 x = *reinterpret_cast<const float4*>(from + (4 * ty + i) * kC + 4 * tx);
+      const float4 x = fresh4(from + (4 * ty + i) * kC + 4 * tx);
       sc[i][0] = x.x, sc[i][1] = x.y, sc[i][2] = x.z, sc[i][3] = x.w;
     }
     __syncthreads();                       // R is there
@@ -379,7 +392,7 @@ decay_chunk_out_kernel(const float* __restrict__ q, const float* __restrict__ k,
       const int i = threadIdx.x + n * kThreads, d = i / (BV / 4), col = (i - d * (BV / 4)) * 4;
       x[n] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (d0 + d < D && v0 + col < dm.Vd)
-        x[n] = *reinterpret_cast<const float4*>(S + (size_t)(d0 + d) * dm.Vd + v0 + col);
+        x[n] = fresh4(S + (size_t)(d0 + d) * dm.Vd + v0 + col);
     }
   };
   ask(0);
@@ -404,7 +417,7 @@ decay_chunk_out_kernel(const float* __restrict__ q, const float* __restrict__ k,
     const int j = i / (BV / 4), col = (i - j * (BV / 4)) * 4;
     float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
     if (j < at.len && v0 + col < dm.Vd)
-      x = *reinterpret_cast<const float4*>(v + (size_t)(at.row0 + j) * dm.ld_v + (size_t)h * dm.Vd + v0 + col);
+      x = fresh4(v + (size_t)(at.row0 + j) * dm.ld_v + (size_t)h * dm.Vd + v0 + col);
     *reinterpret_cast<float4*>(stage + j * BV + col) = x;
   }
   __syncthreads();
@@ -427,11 +440,15 @@ decay_chunk_out_kernel(const float* __restrict__ q, const float* __restrict__ k,
                       fmaf(sk, vv[2], acc[i][4 * n + 2]), fmaf(sk, vv[3], acc[i][4 * n + 3]));
     }
   }
-  if (o_norm != nullptr && blockIdx.z == 0 && threadIdx.x < at.len) {
-    const float* n0 = nstarts + ((size_t)chunk * dm.H + h) * D;
-    float s = 0.f;
-    for (int d = 0; d < D; ++d) s = fmaf(qt[d * kC + threadIdx.x], n0[d], s);
-    o_norm[(size_t)(at.row0 + threadIdx.x) * dm.ld_n + h] = fmaf(Gt[threadIdx.x], s, nsum[threadIdx.x]);
+  if (o_norm != nullptr && blockIdx.z == 0) {
+    __syncthreads();                       // the values have been read
+    if (threadIdx.x < D) stage[threadIdx.x] = fresh(nstarts + ((size_t)chunk * dm.H + h) * D + threadIdx.x);
+    __syncthreads();
+    if (threadIdx.x < at.len) {
+      float s = 0.f;
+      for (int d = 0; d < D; ++d) s = fmaf(qt[d * kC + threadIdx.x], stage[d], s);
+      o_norm[(size_t)(at.row0 + threadIdx.x) * dm.ld_n + h] = fmaf(Gt[threadIdx.x], s, nsum[threadIdx.x]);
+    }
   }
 }
 
