@@ -1266,13 +1266,15 @@ inline bool tree_pays(long long T, int B, int D, bool one_decay) {
 
 // one_decay: g is [T, H] (a decay a head), else [T, H, D].  scratch (gf_delta_chunk_words; null: token by
 // token) is for steps with one decay a head; max_q_len: the longest portion (0: not known); singles: how many
-// requests in front have one token.
+// requests in front have one token.  *launches: kernels launched.
 GF_EXPORT int gf_delta_recurrence(const float* qn, const float* kn, const float* v, const float* g,
                                   const float* beta, float* state, const int* cu_seqlens,
                                   const int* slot_ids, int B, int H, int G, int D, int Vd,
                                   int state_stride, float* o, int one_decay, float* scratch,
-                                  int max_q_len, int T, int singles, void* stream) {
+                                  int max_q_len, int T, int singles, int* launches, void* stream) {
+  *launches = 0;
   if (B <= 0) return 0;
+  *launches = 1;
   if (H % G) return -3;
   const DeltaDims dm = dims_of(H, G, D, Vd, 1, state_stride, 0);
   auto st = (cudaStream_t)stream;
@@ -1282,6 +1284,7 @@ GF_EXPORT int gf_delta_recurrence(const float* qn, const float* kn, const float*
     if (int rc = launch_kernel(delta_chunk_coef_kernel, dim3((chunks + 3) / 4, B, G), dim3(128), 0, st,
                                qn, kn, g, beta, cu_seqlens, dm, scratch))
       return rc;
+    ++*launches;
     const ChunkArgs a{qn, kn, nullptr, nullptr, v, H * Vd, scratch, state, cu_seqlens, slot_ids, 0, H, o};
 #define GF_GO(DPER, LANES)                                                                         \
   if (D <= DPER * LANES) return launch_chunks<DPER, LANES, HEADS>(B, dm, a, st);
@@ -1384,6 +1387,7 @@ GF_EXPORT int gf_delta_recurrence(const float* qn, const float* kn, const float*
   // portion of 300: 386, 751 and 1,340)
   if (singles > 0 && singles < B && tree_pays((long long)T - singles, B - singles, D, one_decay)) {
     if (int rc = lanes(4, singles)) return rc;
+    ++*launches;
     return tree(singles);
   }
   return lanes(4, B);

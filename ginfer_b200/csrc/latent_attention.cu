@@ -920,14 +920,16 @@ GF_EXPORT int gf_latent_gather(const void* c_pages, const int* table, int table_
                        W, page, row_bytes, num_pages, vec, (unsigned char*)out, own);
 }
 
-// sharing: how many of the T tokens see their request from its first key on.
+// sharing: how many of the T tokens see their request from its first key on.  *launches: kernels launched.
 GF_EXPORT int gf_latent_attention(const float* q_lat, const float* q_rot, const void* c_pages,
                                   const void* r_pages, const int* block_table, int table_stride,
                                   const int* seq_of_token, const int* positions, void* out, int T,
                                   int H, int C, int R, int page_size, int window, float scale,
                                   int dtype, int nsplit, float* part_o, float* part_ml,
-                                  int max_q_len, int sharing, void* stream) {
+                                  int max_q_len, int sharing, int* launches, void* stream) {
+  *launches = 0;
   if (T <= 0) return 0;
+  *launches = 1;
   if (C > kLatMaxC || C <= 0 || R < 0) return -3;
   const int Dk = C + R;
   if (dtype == GF_BF16 && C % 16 == 0 && R % 16 == 0 && (uintptr_t)c_pages % 16 == 0 &&
@@ -976,6 +978,7 @@ GF_EXPORT int gf_latent_attention(const float* q_lat, const float* q_rot, const 
                                    block_table, table_stride, seq_of_token, positions, (bf*)out, T, H, C, R,
                                    page_size, window, scale))
           return rc;
+        ++*launches;
       }
       int rc2 = -3;
 #define GF_GO(NT)                                                                              \
@@ -989,6 +992,7 @@ GF_EXPORT int gf_latent_attention(const float* q_lat, const float* q_rot, const 
       GF_GO(4);
 #undef GF_GO
       if (rc2 || nsplit == 1) return rc2;
+      ++*launches;
       return launch_kernel(latent_merge_kernel, dim3(T * H), dim3((C / 4 + 31) / 32 * 32), 0, st,
                            (const float*)part_o, (const float*)part_ml, (bf*)out, T, H, C, nsplit);
     }

@@ -2,11 +2,11 @@
 (``csrc/delta_rule.cu``)."""
 from __future__ import annotations
 
-from ctypes import c_float, c_int, c_void_p
+from ctypes import addressof, c_float, c_int, c_void_p
 
 import torch
 
-from . import _code, _cuda, _fn, _ok, _p, _stream
+from . import _Counter, _code, _cuda, _fn, _ok, _p, _stream
 
 
 MAX_KEY_SIZE = 256        # the recurrence kernel's largest
@@ -121,7 +121,8 @@ def recurrence(qn, kn, v, g, beta, state: torch.Tensor, ctx) -> torch.Tensor:
     H, Vd = v.shape[1], v.shape[2]
     o = torch.empty((T, H, Vd), dtype=torch.float32, device=qn.device)
     f = _fn("delta_rule", "gf_delta_recurrence",
-            [c_void_p] * 8 + [c_int] * 6 + [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p])
+            [c_void_p] * 8 + [c_int] * 6 + [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p],
+            kernels=0)
     one = int(g.dim() == 2)
     scratch, longest = None, int(ctx.max_q_len if one else getattr(ctx, "max_q_len", 0))
     if one and longest == 1 and state_step(qn.view(T, G * D), kn.view(T, G * D), v.view(T, H * Vd),
@@ -135,12 +136,14 @@ def recurrence(qn, kn, v, g, beta, state: torch.Tensor, ctx) -> torch.Tensor:
     if longest > 1 and len(q_lens) == ctx.num_seqs:
         while singles < len(q_lens) and q_lens[singles] == 1:
             singles += 1
+    launches = c_int()
     rc = f(_p(qn), _p(kn), _p(v), _p(g), _p(beta), _p(state), _p(ctx.cu_seqlens_q),
            _p(ctx.slot_ids), ctx.num_seqs, H, G, D, Vd, state.stride(0), _p(o), one,
-           _p(scratch), longest, T, singles, _stream())
+           _p(scratch), longest, T, singles, addressof(launches), _stream())
     if rc == -3:
         raise ValueError(f"the delta-rule recurrence takes key sizes up to {MAX_KEY_SIZE}, got {D}")
     _ok(rc, "delta_recurrence")
+    _Counter.launches += launches.value
     return o
 
 

@@ -2,11 +2,11 @@
 (``csrc/latent_attention.cu``)."""
 from __future__ import annotations
 
-from ctypes import c_float, c_int, c_void_p
+from ctypes import addressof, c_float, c_int, c_void_p
 
 import torch
 
-from . import _code, _cuda, _fn, _ok, _p, _stream
+from . import _Counter, _code, _cuda, _fn, _ok, _p, _stream
 
 
 def prepare(qd: torch.Tensor, H: int, D: int, R: int, C: int, rot: int, freq: torch.Tensor,
@@ -133,13 +133,15 @@ def attention(q_lat: torch.Tensor, q_rot: torch.Tensor, c_pages: torch.Tensor,
     f = _fn("latent_attention", "gf_latent_attention",
             [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
              c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p,
-             c_void_p, c_int, c_int, c_void_p], kernels=2 if nsplit > 1 else 1)
+             c_void_p, c_int, c_int, c_void_p, c_void_p], kernels=0)
+    launches = c_int()
     rc = f(_p(q_lat), _p(q_rot), _p(c_pages), _p(r_pages), _p(block_table),
            block_table.stride(0), _p(ctx.seq_of_token), _p(ctx.positions), _p(out), T, H, C, R,
            int(page_size), int(window), float(scale), _code(c_pages.dtype), nsplit, _p(part_o),
-           _p(part_ml), int(getattr(ctx, "max_q_len", 0) or 0), shared, _stream())
+           _p(part_ml), int(getattr(ctx, "max_q_len", 0) or 0), shared, addressof(launches), _stream())
     if rc == -3:
         raise ValueError(f"latent attention takes latent vectors of up to 1024 channels whose key "
                          f"tile fits shared memory; got kv_rank={C}, rot_dim={R}")
     _ok(rc, "latent_attention")
+    _Counter.launches += launches.value
     return out

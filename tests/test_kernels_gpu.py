@@ -1235,3 +1235,59 @@ def test_latent_attention_of_neighbouring_tokens(H, C, R, window, portions, brok
     assert torch.equal(*(torch.nan_to_num(o.float(), nan=1e9) for o in out))
     if broken:
         assert torch.isnan(out[0]).any() and not torch.isnan(out[0][:, :min(broken)]).any()
+
+
+def test_launches_are_counted_where_their_number_follows_from_the_step():
+    """What the counter says of a call is the number of kernels that a graph captures of it, whichever call of a kind
+    comes first: chunked recurrences with and without shared scores, latent attention plain, in shares and with
+    tokens that share tiles, the delta rule in one kernel, in two, and in chunks."""
+    from types import SimpleNamespace
+    from cuda.bindings import runtime
+    from ginfer_b200 import ops
+    from ginfer_b200.ops import decay, delta, latent
+
+    def zeros(*shape, dtype=torch.float32):
+        return torch.zeros(shape, dtype=dtype, device=DEV)
+
+    def step(lens):
+        B, T = len(lens), sum(lens)
+        return T, SimpleNamespace(
+            num_seqs=B, slot_ids=torch.arange(B).int().cuda(), max_q_len=max(lens), q_lens_host=lens,
+            q_starts_host=[0] * B, cu_seqlens_q=torch.tensor([0] + lens).cumsum(0).int().cuda(),
+            seq_of_token=torch.repeat_interleave(torch.arange(B), torch.tensor(lens)).int().cuda(),
+            positions=torch.cat([torch.arange(n) for n in lens]).int().cuda(), max_kv_len=max(lens))
+
+    def chunked(H, G):
+        T, ctx = step([70, 3])
+        q, v, g, state = zeros(T, G * 4), zeros(T, H * 8), zeros(T, H), zeros(2, H * 32)
+        return lambda: decay.recurrence(q, q, v, g, state, ctx, H, G, 4, 8)
+
+    def attention(H, lens, keys=0):
+        T, ctx = step(lens)
+        ctx.max_kv_len = keys or ctx.max_kv_len
+        q, c, table = zeros(H, T, 32), zeros(600, 16, 1, 32, dtype=torch.bfloat16), zeros(len(lens), 600, dtype=torch.int32)
+        return lambda: latent.attention(q, None, c, None, table, ctx, 0, 1.0, 16)
+
+    def rule(H, D, lens, one):
+        T, ctx = step(lens)
+        q, v, state = zeros(T, H, D), zeros(T, H, 64), zeros(len(lens), H * D * 64)
+        g, beta = zeros(T, H) if one else zeros(T, H, D), zeros(T, H)
+        return lambda: delta.recurrence(q, q, v, g, beta, state, ctx)
+    calls = [chunked(4, 4), chunked(4, 2), chunked(4, 4), attention(16, [5]), attention(16, [1, 1], 9000),
+             attention(16, [801]), attention(16, [5]), rule(16, 128, [9, 9], 0), rule(16, 128, [1] * 20 + [30], 0),
+             rule(16, 64, [40, 3], 1), rule(16, 128, [9, 9], 0)]
+    counts = []
+    for call in calls:
+        call()                                       # (libraries and attributes)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(graph):
+            before = ops.launch_count()
+            call()
+            counted = ops.launch_count() - before
+        raw = runtime.cudaGraph_t(graph.raw_cuda_graph())
+        err, _, n = runtime.cudaGraphGetNodes(raw)
+        err, nodes, n = runtime.cudaGraphGetNodes(raw, n)
+        kinds = [runtime.cudaGraphNodeGetType(node)[1] for node in nodes[:n]]
+        counts.append((counted, sum(k == runtime.cudaGraphNodeType.cudaGraphNodeTypeKernel for k in kinds)))
+    assert [a for a, _ in counts] == [b for _, b in counts] == [3, 4, 3, 1, 2, 2, 1, 1, 2, 2, 1], counts
