@@ -86,22 +86,29 @@ def split_k_for(M: int, N: int, K: int, sms: int | None = None, settled: bool = 
         split = 2       # about one tile an SM (gate/up): pairs of CTAs have more under way
     elif M <= 64 and not settled:
         # More CTAs than SMs where a CTA's K range stays long: its K steps, not its bytes, bound it.  The lines are
-        # those of the places: clusters of 4, 8 and 12 CTAs, two CTAs an SM, fit 71, 33 and 21 times on 148 SMs
-        # (a cluster lies inside one of the device's groups of SMs), and one more waits for a whole round.  In a
-        # CUDA graph on a B200, weights from HBM, us, splits as above / these.  Two / four, 2048 columns: 64 tiles 10.0 /
+        # those of the places: clusters of 4, 8 and 12 CTAs, two CTAs an SM, fit 71 (see placed_splits), 33 and 21
+        # times on 148 SMs (a cluster lies inside one of the device's groups of SMs), and one more waits for a whole
+        # round.  In a CUDA graph on a B200, weights from HBM, us, splits as above / these.  Two / four, 2048 columns: 64 tiles 10.0 /
         # 8.6 at 8 tokens, 11.6 / 10.9 at 64, 71 tiles 10.3 / 9.1 and 11.6 / 11.6, 72 tiles 10.3 / 13.0 and 11.8 / 17.6;
         # 1024 columns at 64 tokens 8.0 / 8.3.  Four / eight: 18944 columns, 28 tiles 28.9 / 25.6 at 8 tokens, 32.6 /
         # 30.6 at 64, 32 tiles 31.1 / 28.1 and 34.0 / 33.0, 33 tiles 31.9 / 29.0 and 34.1 / 34.3, 34 tiles 32.5 / 38.3;
         # 12288 columns, 32 tiles 22.9 / 20.4 and 25.0 / 24.6; 8192 columns at 64 tokens 18.0 / 18.5.  Eight / twelve:
         # 5376 columns, 16 tiles 7.8 / 7.2 at 8 tokens, 8.2 / 7.9 at 16, 9.0 / 9.4 at 32, 19 tiles 8.4 / 8.0 and 8.8 /
         # 8.7, 21 tiles at 16 9.1 / 9.4, 22 tiles 8.9 / 12.0; 4608 columns, 19 tiles at 16 7.8 / 8.0.
-        if split == 2 and tiles * 148 <= 71 * sms and nkb // 4 >= 8:
+        if split == 2 and tiles * 4 <= 2 * sms and nkb // 4 >= 8:
             split = 4
         elif split == 4 and tiles * 148 <= 32 * sms and nkb // 8 >= 24:
             split = 8
         elif split == 8 and M <= 16 and tiles * 148 <= 19 * sms and nkb // 12 >= 7:
             split = 12
     return split
+
+
+def placed_splits(split: int, M: int, N: int, sms: int | None = None) -> int:
+    """``split`` where clusters of that many CTAs all find a place at once, two for those of four that do not: two
+    CTAs an SM are 74 clusters of four on 148 SMs, of which 71 fit (measured at :func:`split_k_for`)."""
+    tiles = -(-N // 128) * -(-M // token_tile(M))
+    return 2 if split == 4 and tiles * 148 > 71 * (sms or num_sms()) else split
 
 
 def _workspace(words: int, device) -> torch.Tensor:
@@ -164,7 +171,7 @@ def gemm(x, weight, bias_f32=None, out_dtype=torch.bfloat16, epi: int = 0, split
             and not through_workspace and scale is None and resid is None
             and stream(x, weight, bias_f32, out, epi, act_consts)):
         return out
-    sk = split_k_for(M, N, K, settled=not streamed) if split_k is None else int(split_k)
+    sk = placed_splits(split_k_for(M, N, K, settled=not streamed), M, N) if split_k is None else int(split_k)
     ws = None
     if sk > 1 and through_workspace:
         bn = token_tile(M)
