@@ -1321,6 +1321,7 @@ GF_EXPORT int gf_delta_recurrence(const float* qn, const float* kn, const float*
     GF_GO(32, 4, 8, kRecurrenceThreads)
     GF_GO(64, 4, 4, kRecurrenceThreads)
     GF_GO(4, 16, 8, kRecurrenceThreads)
+    GF_GO(4, 32, 8, 256)
     GF_GO(8, 32, 4, 256)
 #undef GF_GO
 #undef GF_AS
@@ -1376,7 +1377,13 @@ GF_EXPORT int gf_delta_recurrence(const float* qn, const float* kn, const float*
     // heads 1.16 at 1 token, 1.23 at 17, 1.04 at 100; 64 units 1.13 (17 tokens 1.15, 100 0.95); 128 units 0.86 at 1 token, 1.04
     // at 2, 1.06 at 15, 0.91 at 17, 0.69 at 100; 256 units 0.55 to 0.87.
     if (D <= 64 && !(units >= 192 || (units >= 128 && (max_q_len == 1 || T >= 16ll * B)))) return lanes(16, B);
-    return D <= 128 ? tree(0) : lanes(32, B);
+    // Key sizes up to 128: while the blocks of a warp a column are few, it starts sooner, and the tree kernel's shorter
+    // token pays from some 60 tokens on.  Tree kernel / a warp a column, on a B200, one request: 16 units, 128 x 128 1.16 at 1
+    // token (3.9 us, 3.4), 1.27 at 5, 1.20 at 17, 1.04 at 60, 1.00 at 100, 0.91 at 1,201, 72 x 128 1.15, 1.10, 1.11, 0.99, 0.95,
+    // 0.87; 20 units 1.15 at 1, 1.0 at 60; 24 and 28 units 0.8 to 1.2, by the columns; 32 units 0.7 to 0.9.
+    const long long longest = max_q_len > 0 ? max_q_len : T;
+    const bool warp = D > 128 || (D > 64 && units <= 20 && longest < 64);
+    return warp ? lanes(32, B) : tree(0);
   }
   // (many requests of a token each are their states' bytes, which four lanes a column read in longer runs:
   // 16 requests of 16 heads of 128 x 128 19 us against 29)

@@ -1291,3 +1291,39 @@ def test_launches_are_counted_where_their_number_follows_from_the_step():
         kinds = [runtime.cudaGraphNodeGetType(node)[1] for node in nodes[:n]]
         counts.append((counted, sum(k == runtime.cudaGraphNodeType.cudaGraphNodeTypeKernel for k in kinds)))
     assert [a for a, _ in counts] == [b for _, b in counts] == [3, 4, 3, 1, 2, 2, 1, 1, 2, 2, 1], counts
+
+
+def _kernels(call):
+    """The names of the kernels that a call launches, as a captured graph has them."""
+    from cuda.bindings import driver
+    call()                                           # (libraries and attributes)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        call()
+    raw, names = driver.CUgraph(graph.raw_cuda_graph()), []
+    err, _, n = driver.cuGraphGetNodes(raw)
+    err, nodes, n = driver.cuGraphGetNodes(raw, n)
+    for node in nodes[:n]:
+        if driver.cuGraphNodeGetType(node)[1] != driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            continue
+        err, params = driver.cuGraphKernelNodeGetParams(node)
+        err, name = driver.cuFuncGetName(params.func) if int(params.func) else driver.cuKernelGetName(params.kern)
+        names.append(name.decode())
+    return names
+
+
+@pytest.mark.parametrize("H,D,Vd,lens,warp", [
+    (4, 128, 128, [5], True), (2, 72, 128, [1, 1, 17], True), (4, 128, 128, [63], True), (4, 128, 128, [64], False),
+    (5, 97, 128, [9], True), (6, 97, 128, [9], False), (5, 65, 128, [30], True), (8, 96, 128, [9], False)])
+def test_delta_rule_of_few_columns_and_tokens_takes_a_warp_a_column(H, D, Vd, lens, warp):
+    """While every block has an SM of its own and portions are short; the same bits as beside a long portion, where the
+    other kernel serves."""
+    step, state0 = _delta_step(H, H, D, Vd, lens)
+    one = step()
+    names = _kernels(lambda: one(state0))
+    assert any("delta_recurrence_kernel" in n for n in names) == warp != any("delta_tree_kernel" in n for n in names)
+    both, more = _delta_step(H, H, D, Vd, lens + [64])
+    less = more[:len(lens)].clone()
+    o = both()(more)
+    assert torch.equal(both(slice(0, sum(lens)), lens)(less), o[:sum(lens)]) and torch.equal(less, more[:len(lens)])
