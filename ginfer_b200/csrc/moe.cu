@@ -689,7 +689,10 @@ __host__ __device__ inline size_t ring_shared(int K) {
 // experts, 40 pairs (0.78) 25.7 / 29.0, 80 pairs (1.00) 43.1 / 35.5; 1536 x 2048 28.3 / 30.3 (0.93), 44.9 / 38.2 (1.2); 2048 x
 // 1408, 32 experts, 32 pairs (1.1) 29.6 / 25.6, 80 (1.6) 34.4 / 35.4; 2048 x 3072 (a block an SM), 24 experts, 28 pairs 89 /
 // 45.  A shorter reduction leaves warps without a step in an item: 4096 x 512, 24 experts, 28 pairs (1.8) 15.3 / 18.7, 3072 x 1024
-// (1.4) 25.7 / 28.3.  Fewer experts: 16 of 2816 x 2048, 24 pairs 41.9 / 34.7; 8, 16 pairs (1.05) 18.9 / 20.9, 20 pairs 26.2 /
+// (1.4) 25.7 / 28.3.  From 1,280 to 1,536 columns the second round has to be at least half empty, and an expert less costs
+// more than one more gains.  Ring over grid, sums over 16 to 64 experts: 4096 x 1280 0.99 at 1 to 1.5 rounds, 1.05 from there
+// to 1.9, 0.97 behind; 2048 x 1408 0.96, 1.02, 0.96 and 1.09 at 0.95 to 1; 3072 x 1408 0.94, 1.03, 0.96; 2048 x 1536 0.94, 1.01,
+// 0.95 and 1.06; 2048 x 2112 0.90, 0.96, 0.91 and 1.01; 2816 x 2048 0.90, 0.99, 0.94 and 0.82.  Fewer experts: 16 of 2816 x 2048, 24 pairs 41.9 / 34.7; 8, 16 pairs (1.05) 18.9 / 20.9, 20 pairs 26.2 /
 // 23.5.  Small matrices: 1536 x 1024, 24 experts, 60 pairs 18.6 / 22.7.
 inline bool ring_serves(int pairs, int experts, int N, int K, int span, size_t grid_shared, int sms) {
   if (experts < kRgMinExperts || pairs <= kStHandful || pairs < experts || 2 * pairs > 5 * experts || K < kRgMinK ||
@@ -697,7 +700,8 @@ inline bool ring_serves(int pairs, int experts, int N, int K, int span, size_t g
     return false;
   const double reached = experts * (1.0 - pow(1.0 - 1.0 / experts, pairs));
   const int places = sms * (2 * (grid_shared + 9 * 1024) < 204 * 1024 ? 2 : 1);   // (2,816 columns are the last with two)
-  return reached * ((N + span - 1) / span) >= 0.95 * places;
+  const double rounds = reached * ((N + span - 1) / span) / places;
+  return K < 2048 ? rounds >= 1.0 && (rounds < 1.5 || rounds >= 1.9) : rounds >= 0.95;
 }
 __device__ __forceinline__ void ring_copy(uint32_t dst, const void* src, bool there) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(there ? 16 : 0) : "memory");

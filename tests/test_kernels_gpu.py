@@ -1327,3 +1327,14 @@ def test_delta_rule_of_few_columns_and_tokens_takes_a_warp_a_column(H, D, Vd, le
     less = more[:len(lens)].clone()
     o = both()(more)
     assert torch.equal(both(slice(0, sum(lens)), lens)(less), o[:sum(lens)]) and torch.equal(less, more[:len(lens)])
+
+
+@pytest.mark.parametrize("E,N,K,pairs,ring", [
+    (24, 2048, 1408, 32, False), (24, 2048, 1408, 48, True), (24, 4096, 1280, 28, False), (24, 4096, 1280, 40, True),
+    (24, 2112, 2048, 28, True), (32, 2048, 1536, 32, True)])
+def test_routed_products_take_equal_runs_where_they_gain(E, N, K, pairs, ring):
+    from ginfer_b200.ops import moe
+    x, w = torch.zeros(pairs, K, device=DEV).bfloat16(), torch.zeros(E, N, K, device=DEV).bfloat16()
+    plan = moe.Plan(torch.arange(pairs, dtype=torch.int32, device=DEV).view(-1, 1) % E, E, "few")
+    names = _kernels(lambda: moe.grouped_down(x, w, plan))
+    assert any("moe_ring_kernel" in n for n in names) == ring != any("moe_stream_kernel" in n for n in names)
