@@ -1314,7 +1314,7 @@ def _kernels(call):
 
 
 @pytest.mark.parametrize("H,D,Vd,lens,warp", [
-    (4, 128, 128, [5], True), (2, 72, 128, [1, 1, 17], True), (4, 128, 128, [63], True), (4, 128, 128, [64], False),
+    (4, 128, 128, [5], True), (2, 72, 128, [1, 17], True), (2, 72, 128, [1, 1, 17], False), (4, 128, 128, [63], True), (4, 128, 128, [64], False),
     (5, 97, 128, [9], True), (6, 97, 128, [9], False), (5, 65, 128, [30], True), (8, 96, 128, [9], False)])
 def test_delta_rule_of_few_columns_and_tokens_takes_a_warp_a_column(H, D, Vd, lens, warp):
     """While every block has an SM of its own and portions are short; the same bits as beside a long portion, where the
